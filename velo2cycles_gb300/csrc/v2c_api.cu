@@ -253,17 +253,26 @@ int check_params(const v2c_params *p) {
   return V2C_OK;
 }
 
-// Column strip of the sweeps: the widest up to max_tx that still gives 1.5
-// waves of 7 resident CTAs on each of the 152 SMs (a strip of tx columns
-// restages one halo column).  The scatter takes strips of at most 16
-// columns, the gather 32: at C4 (126 x 32 strips of 32 columns) the
-// scatter's 4.4 waves at 6 CTAs left SMs idle in the last one, and 16
-// columns (8.8 waves, 3 % more halo work) ran 5.17 -> 5.01 ms, while the
-// gather ran 4.80 -> 4.86 ms with them.
+// Column strip of the gather: the widest up to 32 columns that still gives
+// 1.5 waves of 7 resident CTAs on each of the 152 SMs (a strip of tx columns
+// restages one halo column).
 int pick_tx(const v2c_ctx *c, int max_tx) {
   long rows = (c->yn + 31) / 32;
   int tx = max_tx;
   while (tx > 4 && rows * ((c->xn + tx - 1) / tx) < 152 * 7 * 3 / 2) tx /= 2;
+  return tx;
+}
+
+// Column strip of the scatter: the widest up to 16 columns that still gives
+// 3 waves of its 4 resident CTAs per SM.  Wide strips save the halo column
+// (C4, 13 waves: 2.98 ms at 16 columns, 3.27 at 4), narrow ones balance the
+// last wave (1001 x 401 lines: 0.385 ms at 8 columns and 2.7 waves, 0.382 at
+// 4 and 5.4) and, where one wave holds the grid, the columns a CTA takes in
+// turn are the kernel's time (51 x 21 lines: 49, 34 and 25 us at 4, 2 and 1).
+int scatter_tx(const v2c_ctx *c) {
+  const long rows = (c->yn + 31) / 32;
+  int tx = 16;
+  while (tx > 1 && rows * ((c->xn + tx - 1) / tx) < 152 * 4 * 3) tx /= 2;
   return tx;
 }
 
@@ -336,6 +345,7 @@ extern "C" int v2c_create(const v2c_params *p, long max_markers, void *cuda_stre
   AL(ctx->sb.blocksum, ctx->sb.blocksum_cap);
   AL(ctx->d_stage64, cap); AL(ctx->d_stage64b, cap);
 #undef AL
+  if (m2n_init() != cudaSuccess) { v2c_destroy(ctx); return V2C_ERR_CUDA; }
   if (newton_init(ctx->nw, cap) != cudaSuccess) { v2c_destroy(ctx); return V2C_ERR_CUDA; }
   if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) { v2c_destroy(ctx); return V2C_ERR_CUDA; }
   *out = ctx;
@@ -976,7 +986,7 @@ extern "C" int v2c_marker2nodes(v2c_ctx *ctx) {
   a.stat = ctx->d_stat;
   a.gxf = ctx->d_gxf;
   a.gyf = ctx->d_gyf;
-  a.TX = pick_tx(ctx, 16);
+  a.TX = scatter_tx(ctx);
   a.n = ctx->n;
   CK(cudaMemsetAsync(ctx->d_sticky, 0, sizeof(uint32_t) * ctx->nn, st));
   ctx->dsxx_valid = false;  // the scatter writes sxxe

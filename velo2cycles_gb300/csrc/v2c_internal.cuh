@@ -129,6 +129,55 @@ struct Acc {
   __device__ __forceinline__ float value() const { return s + c; }
 };
 
+// Two FP32 values in one 64-bit register pair (packed FP32: one instruction
+// issues both operations; the FMA pipe is busy as long as for two scalar
+// ones, so what it halves is the issue slots).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// (a w, b w), each product rounded.  Not mul.rn.f32x2: the assembler fuses a
+// packed product with the packed additions that read it, so the sums below
+// would take products that were never rounded.
+__device__ __forceinline__ f32x2 mul_w(float a, float b, float w) {
+  return pack2(__fmul_rn(a, w), __fmul_rn(b, w));
+}
+
+// Two compensated sums side by side.  The error of each addition is formed
+// by Knuth's two-sum: exact as Neumaier's is, so the sums are those of Acc
+// bit for bit, without the comparison and selection, in 7 packed
+// instructions for both instead of 16 scalar ones.
+struct Acc2 {
+  f32x2 s, c;
+  __device__ __forceinline__ void zero() { s = 0; c = 0; }
+  __device__ __forceinline__ void add(f32x2 x) {
+    const f32x2 t = add2(s, x);
+    const f32x2 bb = sub2(t, s);
+    const f32x2 e = add2(sub2(s, sub2(t, bb)), sub2(x, bb));
+    c = add2(c, e);
+    s = t;
+  }
+  __device__ __forceinline__ void split(Acc &lo, Acc &hi) const {
+    unpack2(s, lo.s, hi.s);
+    unpack2(c, lo.c, hi.c);
+  }
+};
+
 // The centre-node weight factor 1 - 2|f - 1/2| of an in-cell offset f
 // (interpolation.c:620-622), written as 2f below the middle and 2(1 - f)
 // above it: the same value, exact in FP32 (1 - f is exact for f >= 1/2),

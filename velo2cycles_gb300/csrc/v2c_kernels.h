@@ -68,9 +68,11 @@ struct M2NArgs {
   uint32_t *sticky_key;
   unsigned long long *stat;
   const float *gxf, *gyf;  // FP32 line positions (coarse band test)
-  int TX;
-  long n = 0;  // markers (chooses the sweep's occupancy)
+  int TX;      // node columns per CTA
+  long n = 0;  // markers
 };
+// the sweep's shared-memory size, set on the current device (once per context)
+cudaError_t m2n_init();
 void launch_m2n(const M2NArgs &a, cudaStream_t st);
 
 // per-marker physics (+ optional RSF Newton), marker array order

@@ -4,14 +4,13 @@
 // Tiling.  A CTA owns node rows [j0, j0+TY) and node columns [i0, i0+TX).
 // It sweeps cell columns ci = i0-1 .. i0+TX-1.  For each column it stages the
 // column's markers of cell rows j0-1 .. j0+TY-1 (one contiguous run of the
-// sorted order) in shared memory, evaluating every marker's properties once.
-// Then thread (role, jl) accumulates, for node row j = j0+jl, the
-// contributions of cells (ci, j-1) and (ci, j), which are all the cells of
-// that column that reach node (ci, j) and (ci+1, j) under the
-// interpolationmod=2 stencil (interpolation.c:539-628):
+// sorted order) in shared memory.  Then lane jl of each warp accumulates, for
+// node row j = j0+jl, its warp's sums over the contributions of cells
+// (ci, j-1) and (ci, j), which are all the cells of that column that reach
+// node (ci, j) and (ci+1, j) under the interpolationmod=2 stencil
+// (interpolation.c:539-628):
 //   * basic node (ci, j) gets the left-half quadrants of those two cells,
-//     basic node (ci+1, j) the right-half ones -> kept in a register carry
-//     and completed when column ci+1 adds its left halves;
+//     basic node (ci+1, j) the right-half ones;
 //   * vx node (ci, j) gets cell (ci, j) if u < 0.5, vx node (ci+1, j) if
 //     u > 0.5 (carry);
 //   * vy node (ci, j) gets cell (ci, j-1) if v > 0.5 and cell (ci, j) if
@@ -25,8 +24,13 @@
 // compensated sums, rounding each result once to FP32.
 // No float atomics; the result does not depend on scheduling.
 //
-// Roles (one warp each per 32 node rows): 0 basic-node stress/state group,
-// 1 basic-node thermal group, 2 centre node, 3 vx and vy nodes.
+// Eight warps share a staged column (lanes = node rows).  Warps 0, 1: the
+// basic nodes' stress/state group of even and of odd node columns; a node
+// column takes the right halves of one cell column and then the left halves
+// of the next, so a warp runs one list of markers per cell column and keeps
+// one set of sums, and no sums are carried between warps.  Warps 2, 3: the
+// same for the thermal group.  Warp 4: centre nodes, viscosities; warp 5:
+// centre nodes, stress, strain rate, pressure; warp 6: vx; warp 7: vy.
 #include <math.h>
 
 #include "v2c_ff.cuh"
@@ -38,24 +42,28 @@ namespace v2c {
 namespace {
 
 constexpr int TY = 32;
-constexpr int NTH = 4 * TY;
-constexpr int CHUNK = 384;
+constexpr int NTH = 8 * 32;
+// Markers staged at once.  A column segment (33 cells) that does not fit
+// splits into chunks, and the lanes whose cells lie in the other chunk idle:
+// at 20 markers per cell 384-marker chunks left 18.6 of 32 lanes busy.  780
+// holds 33 cells of 23 markers, in the 56 KB that four resident CTAs leave
+// each other (64 registers x 256 threads x 4 fill the register file).
+constexpr int CHUNK = 780;
 
-enum {
-  P_U = 0, P_V, P_NU, P_NUG, P_E, P_SXY, P_EXY, P_COH, P_PHI, P_RO, P_ET, P_HT,
-  P_CP, P_KT, P_TK, P_SXX, P_EXX, P_P, P_VX, P_VY, P_N
-};
+// staged fields, in pairs that one 8-byte shared-memory read brings straight
+// into the operand pair of a packed FP32 instruction; warp k stages pair k
+enum { S_UV = 0, S_NUE, S_SXYEXY, S_COHPHI, S_KTTK, S_SXXEXX, S_PRO, S_VXVY, S_N };
 
-// A chunk's markers are staged at their sorted position plus the local row
-// of their cell (one free slot after each cell): the threads of consecutive
-// node rows read consecutive cells in lockstep, and with the cells' runs
-// at a spacing of count + 1 rather than count (16 or 20 markers per cell
-// in a fresh uniform seeding) their shared-memory reads fall in different
+// The marker at position p of a chunk is staged in slot p + p / 16: the lanes
+// read consecutive cells in lockstep, and with a free slot in every 17 the
+// runs of 16 or 20 markers of a fresh uniform seeding start in different
 // banks instead of a few.
-constexpr int SKEW = TY + 1;
+constexpr int SLOTS = CHUNK + CHUNK / 16;
+__device__ __forceinline__ int slot_of(int p) { return p + (p >> 4); }
 struct Smem {
-  float p[P_N][CHUNK + SKEW];
-  uint8_t act[CHUNK + SKEW];
+  float2 p[S_N][SLOTS];
+  int32_t idx[CHUNK];  // array indices of the markers, copied a chunk ahead
+  uint8_t type[CHUNK];
 };
 
 // 4-byte asynchronous copy global -> shared (no register holds the value)
@@ -67,80 +75,82 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
-// Stage the chunk [cs, ce) of column ci's sorted markers, PER per thread,
-// all of a thread's markers at once: the sort indices, then the cells and
-// types, then every field by asynchronous copies straight into the
-// marker's slot (three rounds of memory latency per chunk rather than
-// three per marker, and no register holds a field).  Once a thread's own
-// copies have landed, the payload formed from them: strictly inside the
-// model (interpolation.c:219), the viscosity over the shear modulus, the
-// dencalcomp adiabatic term and the rock-table constants.  The per-marker
-// physics (viscosity, conductivity, density, state update) was done by the
-// marker physics kernel.
-constexpr int PER = CHUNK / NTH;
-static_assert(PER * NTH == CHUNK, "chunk = whole staging rounds");
-__device__ __forceinline__ void stage_chunk(const M2NArgs &a, Smem &sm, int cs, int ce, int ci,
-                                            int jlo, int tid) {
-  const Grid &g = a.g;
-  int idx[PER], q[PER], t[PER];
-#pragma unroll
-  for (int j = 0; j < PER; j++) {
-    const int s = cs + tid + j * NTH;
-    idx[j] = s < ce ? __ldg(a.perm + s) : -1;
+// The two marker fields this warp stages (no second one for P without
+// per-marker densities)
+struct Source {
+  const float *x, *y;
+};
+__device__ __forceinline__ Source stage_source(const M2NArgs &a, int warp) {
+  const Markers &m = a.m;
+  switch (warp) {
+    case S_UV: return {m.u_in, m.v_in};
+    case S_NUE: return {m.mnu, m.e};
+    case S_SXYEXY: return {m.sxy, m.exy};
+    case S_COHPHI: return {m.coh, m.phi};
+    case S_KTTK: return {m.mkt, m.tk};
+    case S_SXXEXX: return {m.sxx, m.exx};
+    case S_PRO: return {m.p, a.S.p.densimod ? m.mro : nullptr};
+    default: return {m.vx, m.vy};
   }
-#pragma unroll
-  for (int j = 0; j < PER; j++) {
-    q[j] = -1;
-    if (idx[j] < 0) continue;
-    // slot: the position in the chunk plus the skew of the cell's run (Smem)
-    q[j] = tid + j * NTH + a.m.cell_in[idx[j]] - ci * g.ncy - jlo;
-    t[j] = a.m.type[idx[j]];
+}
+
+// Copy this warp's pair of fields of the chunk's n markers (indices in
+// sm.idx) into their slots (asynchronous copies: all in flight at once, no register
+// holds a field), the CTA's threads the types, and wait for the copies.
+// Warp 0 then replaces u of a marker not strictly inside the model
+// (interpolation.c:219) by NaN, which fails every weight test below.
+__device__ __forceinline__ void stage_fields(const M2NArgs &a, Smem &sm, int n, int ci, bool edge,
+                                             const Source &src, int warp, int lane) {
+  float2 *dst = sm.p[warp];
+#pragma unroll 8
+  for (int p = lane; p < n; p += 32) {
+    const int i = sm.idx[p];
+    cp_async4(&dst[slot_of(p)].x, src.x + i);
+    if (src.y) cp_async4(&dst[slot_of(p)].y, src.y + i);
   }
-#pragma unroll
-  for (int j = 0; j < PER; j++) {
-    if (q[j] < 0) continue;
-    const int i = idx[j], kk = q[j];
-    cp_async4(&sm.p[P_U][kk], a.m.u_in + i);
-    cp_async4(&sm.p[P_V][kk], a.m.v_in + i);
-    cp_async4(&sm.p[P_NU][kk], a.m.mnu + i);
-    cp_async4(&sm.p[P_E][kk], a.m.e + i);
-    cp_async4(&sm.p[P_SXY][kk], a.m.sxy + i);
-    cp_async4(&sm.p[P_EXY][kk], a.m.exy + i);
-    cp_async4(&sm.p[P_COH][kk], a.m.coh + i);
-    cp_async4(&sm.p[P_PHI][kk], a.m.phi + i);
-    if (a.S.p.densimod) cp_async4(&sm.p[P_RO][kk], a.m.mro + i);
-    cp_async4(&sm.p[P_KT][kk], a.m.mkt + i);
-    cp_async4(&sm.p[P_TK][kk], a.m.tk + i);
-    cp_async4(&sm.p[P_SXX][kk], a.m.sxx + i);
-    cp_async4(&sm.p[P_EXX][kk], a.m.exx + i);
-    cp_async4(&sm.p[P_P][kk], a.m.p + i);
-    cp_async4(&sm.p[P_VX][kk], a.m.vx + i);
-    cp_async4(&sm.p[P_VY][kk], a.m.vy + i);
-  }
+#pragma unroll 4
+  for (int p = warp * 32 + lane; p < n; p += NTH) sm.type[p] = (uint8_t)a.m.type[sm.idx[p]];
   cp_async_wait_all();
-#pragma unroll
-  for (int j = 0; j < PER; j++) {
-    if (q[j] < 0) continue;
-    const int k = q[j], tt = t[j];
-    const int iy = jlo + k - (tid + j * NTH);
-    const float u = sm.p[P_U][k], v = sm.p[P_V][k];
-    bool act = true;
-    if (ci == 0 || ci == g.ncx - 1) {
-      double x = g.gx[ci] + (double)u * (g.gx[ci + 1] - g.gx[ci]);
-      act = act && x > 0 && x < g.xsize;
+  const Grid &g = a.g;
+  if (edge && warp == S_UV) {
+    const bool ex = ci == 0 || ci == g.ncx - 1;
+#pragma unroll 1
+    for (int p = lane; p < n; p += 32) {
+      const int iy = a.m.cell_in[sm.idx[p]] - ci * g.ncy;
+      const bool ey = iy == 0 || iy == g.ncy - 1;
+      if (!ex && !ey) continue;
+      float2 *uv = &sm.p[S_UV][slot_of(p)];
+      bool act = true;
+      if (ex) {
+        double x = g.gx[ci] + (double)uv->x * (g.gx[ci + 1] - g.gx[ci]);
+        act = act && x > 0 && x < g.xsize;
+      }
+      if (ey) {
+        double y = g.gy[iy] + (double)uv->y * (g.gy[iy + 1] - g.gy[iy]);
+        act = act && y > 0 && y < g.ysize;
+      }
+      if (!act) uv->x = __int_as_float(0x7fc00000);
     }
-    if (iy == 0 || iy == g.ncy - 1) {
-      double y = g.gy[iy] + (double)v * (g.gy[iy + 1] - g.gy[iy]);
-      act = act && y > 0 && y < g.ysize;
-    }
-    sm.act[k] = act;
-    const float bb = a.R(RK_BB, tt), T = sm.p[P_TK][k];
-    sm.p[P_NUG][k] = sm.p[P_NU][k] * a.R(RK_INV_GG, tt);
-    if (!a.S.p.densimod) sm.p[P_RO][k] = a.R(RK_RO, tt);
-    sm.p[P_ET][k] = __fdividef(bb, 1.f - bb * (T - 298.15f));  // dencalcomp adiabatic term
-    sm.p[P_HT][k] = a.R(RK_HT, tt);
-    sm.p[P_CP][k] = a.R(RK_CP, tt);
   }
+}
+
+// Ahead of the chunk at sorted positions [b, e): start copying its sort
+// indices (waited for before it is staged), and ask L2 for its markers'
+// fields at the array indices b .. e - 1.  The arrays were stored in sorted
+// order at the upload and markers move a fraction of a cell per step, so
+// these are nearly the right lines.
+__device__ __forceinline__ void prefetch_l2(const void *p) {
+  asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
+}
+__device__ __forceinline__ void start_chunk(const M2NArgs &a, Smem &sm, const Source &src, int b,
+                                            int e, int warp, int lane) {
+#pragma unroll 1
+  for (int s = b + warp * 32 + lane; s < e; s += NTH) cp_async4(&sm.idx[s - b], a.perm + s);
+  const int s = b + 32 * lane;
+  if (s >= e) return;
+  prefetch_l2(src.x + s);
+  if (src.y) prefetch_l2(src.y + s);
+  if (warp == 0 && (lane & 3) == 0) prefetch_l2(a.m.type + s);
 }
 
 // calc_frictionpara_nodes (calc_RSF.c:298-350), FP64; out of line, taken
@@ -187,338 +197,424 @@ __device__ __forceinline__ void node_friction(const M2NArgs &a, int ci, int j, f
   mu = (float)dmu; fa = (float)da; fb = (float)db; fL = (float)dL; fV0 = (float)dV0;
 }
 
-// role 0 / role 1 accumulation into a named register array
-#define ADD_BASIC_A(A, q, w)                                          \
-  do {                                                                \
-    A[0].add(sm.p[P_NU][q] * (w)); A[1].add(sm.p[P_NUG][q] * (w));    \
-    A[2].add(sm.p[P_E][q] * (w)); A[3].add(sm.p[P_SXY][q] * (w));     \
-    A[4].add(sm.p[P_EXY][q] * (w)); A[5].add(sm.p[P_COH][q] * (w));   \
-    A[6].add(sm.p[P_PHI][q] * (w)); A[7].add(w);                      \
-  } while (0)
-#define ADD_BASIC_B(A, q, w)                                          \
-  do {                                                                \
-    A[0].add(sm.p[P_RO][q] * (w)); A[1].add(sm.p[P_ET][q] * (w));     \
-    A[2].add(sm.p[P_HT][q] * (w)); A[3].add(sm.p[P_CP][q] * (w));     \
-    A[4].add(sm.p[P_KT][q] * (w)); A[5].add(sm.p[P_TK][q] * (w));     \
-    A[6].add(w);                                                      \
-  } while (0)
-
 // A compensated sum as a float pair.
 __device__ __forceinline__ ff acc_ff(const Acc &a) {
   ff r;
   r.hi = two_sum(a.s, a.c, r.lo);
   return r;
 }
-// num / den of two compensated sums, rounded once
-__device__ __forceinline__ float ratio(const Acc &num, const ff &den) {
-  return ff_round(ff_div_fast(acc_ff(num), den));
+__device__ __forceinline__ float acc_round(const Acc &a) { return ff_round(acc_ff(a)); }
+
+// The node averages, num / den of two compensated sums as a float pair.  Out
+// of line with the two stores built on it: the tail of one node is 17 such
+// quotients, and as inline copies their code alone outgrew the instruction
+// caches of the eight warps that run different tails (6.7 stalled cycles per
+// issue waiting for instructions, of 20).
+__device__ __forceinline__ ff quot(const Acc &num, const Acc &den) {
+  return ff_div_fast(acc_ff(num), acc_ff(den));
 }
-// the antidiffusion form cur + (n - prev) (interpolation.c:730-736, 758-763,
-// 784-806) from the float-pair node average n: cur and prev are consecutive
-// states of one field that agree in their leading digits, so cur - prev is
-// formed exactly and the sum is rounded once.
-__device__ __forceinline__ float antid_rn(const ff &n, float cur, float prev) {
-  return ff_round(ff_add(n, ff_diff(cur, prev)));
+struct NodeRef {
+  float *base;  // node fields at this node
+  long nn;
+  __device__ __forceinline__ float &operator()(int f) const { return base[f * nn]; }
+};
+// field f = num / den, rounded once
+static __device__ __noinline__ void put_ratio(NodeRef n, int f, Acc num, Acc den) {
+  n(f) = ff_round(quot(num, den));
+}
+// field fn = num / den and field fo = the antidiffusion form cur + (n - prev)
+// of the average n (interpolation.c:730-736, 758-763, 784-806), or the
+// average itself without antidiffusion: cur and prev are consecutive states of one field that agree in their leading digits, so
+// cur - prev is formed exactly and the sum is rounded once.
+static __device__ __noinline__ void put_antid(NodeRef n, int fn, int fo, bool antid, float cur,
+                                              float prev, Acc num, Acc den) {
+  const ff avg = quot(num, den);
+  const float r = ff_round(avg);
+  n(fn) = r;
+  n(fo) = antid ? ff_round(ff_add(avg, ff_diff(cur, prev))) : r;
+}
+static __device__ __noinline__ void put_zeros(NodeRef n, int first, int count) {
+#pragma unroll 1
+  for (int f = first; f < first + count; f++) n(f) = 0.f;
 }
 
 // The node tail of marker2nodes (interpolation.c:714-824) for node row j
-// of column ci, from the compensated sums of one role: 0 basic node (ci, j)
-// stress/state group (cur[0..7]: nu, nu/G, e, sxy, exy, C, phi, w), 1 its
-// thermal group (cur[0..6]: ro, et, ht, cp, kt, tk, w), 2 the centre node
-// (ci+1, j+1) of cell (ci, j) (cur[0..5]: nu, nu/G, sxx, exx, p, w) and the
-// centre fields of (ci, j) when no cell feeds it, 3 vx node (ci, j)
-// (cur[0..2]: vx*ro, ro, w) and vy node (ci, j) (vy3[0..2]).  The averages
-// are float-pair quotients of the float-pair sums, rounded once to FP32.
-__device__ __forceinline__ void node_tail(const M2NArgs &a, int role, int ci, int j,
-                                          const Acc (&cur)[8], const Acc (&vy3)[3]) {
+// of column ci, from the compensated sums of one group: basic node (ci, j)
+// stress/state group (cur[0..7]: nu, nu/G, e, sxy, exy, C, phi, w) or
+// thermal group (cur[0..6]: ro, et, ht, cp, kt, tk, w); the viscosities
+// (cur[0..2]: nu, nu/G, w) or the stresses (cur[0..3]: sxx, exx, p, w) of
+// the centre node (ci+1, j+1) of cell (ci, j), with the centre fields of
+// (ci, j) when no cell feeds it; vx or vy node (ci, j) (cur[0..2]: v*ro, ro,
+// w).  The averages are float-pair quotients of the float-pair sums, rounded
+// once to FP32.
+enum { T_STRESS = 0, T_THERMAL, T_CENTRE_NU, T_CENTRE_S, T_VX, T_VY };
+// the fields cleared together are neighbours in the node block
+static_assert(V2C_NF_MRY0 - V2C_NF_PHISUM == 14 && V2C_NF_ND - V2C_NF_NU == 1 &&
+                  V2C_NF_V0S - V2C_NF_MUS_S == 4 && V2C_NF_TK - V2C_NF_RO == 5,
+              "node field order");
+template <int GROUP>
+__device__ __forceinline__ void node_tail(const M2NArgs &a, int ci, int j, const Acc *cur) {
   const Grid &g = a.g;
   const int ncy = g.ncy;
   const long m3 = (long)ci * g.yn + j;
-  const Nodes &N = a.N;
-  const int antid = a.S.antid;
-  if (role == 0) {
-    const ff ssf = acc_ff(cur[7]);
-    const float ss = ff_round(ssf);
+  const NodeRef n{a.N.base + m3, a.N.nn};
+  const bool antid = a.S.antid;
+  if (GROUP == T_STRESS) {
+    const Acc w = cur[7];
     const bool interior = ci >= 1 && j >= 1 && ci < g.xn - 1 && j < g.yn - 1;
-    if (ss != 0.f && interior) {
-      const ff phin = ff_div_fast(acc_ff(cur[6]), ssf), sxyen = ff_div_fast(acc_ff(cur[3]), ssf);
-      const ff exyen = ff_div_fast(acc_ff(cur[4]), ssf), pen = ff_div_fast(acc_ff(cur[2]), ssf);
-      float phis, sxye, exye, pe;
-      if (antid) {
-        phis = antid_rn(phin, N.f(V2C_NF_PHIS_IT)[m3], N.f(V2C_NF_PHIE)[m3]);
-        sxye = antid_rn(sxyen, N.f(V2C_NF_SXY)[m3], N.f(V2C_NF_SXYEE)[m3]);
-        exye = antid_rn(exyen, N.f(V2C_NF_EXY)[m3], N.f(V2C_NF_EXYEE)[m3]);
-        pe = antid_rn(pen, N.f(V2C_NF_PES)[m3], N.f(V2C_NF_PEE)[m3]);
-      } else {
-        phis = ff_round(phin); sxye = ff_round(sxyen); exye = ff_round(exyen); pe = ff_round(pen);
-      }
-      if (pe < 0.f) pe = 0.f;
-      N.f(V2C_NF_PHIN)[m3] = ff_round(phin);
-      N.f(V2C_NF_SXYEN)[m3] = ff_round(sxyen);
-      N.f(V2C_NF_EXYEN)[m3] = ff_round(exyen);
-      N.f(V2C_NF_PEN)[m3] = ff_round(pen);
-      N.f(V2C_NF_PHIS)[m3] = phis;
-      N.f(V2C_NF_SXYE)[m3] = sxye;
-      N.f(V2C_NF_EXYE)[m3] = exye;
-      N.f(V2C_NF_PE)[m3] = pe;
-      N.f(V2C_NF_COHESION)[m3] = ratio(cur[5], ssf);
-      N.f(V2C_NF_NU_M2C)[m3] = ratio(cur[0], ssf);
+    if (acc_round(w) != 0.f && interior) {
+      // all read at once, before the calls
+      const float c0 = n(V2C_NF_PHIS_IT), p0 = n(V2C_NF_PHIE), c1 = n(V2C_NF_SXY);
+      const float p1 = n(V2C_NF_SXYEE), c2 = n(V2C_NF_EXY), p2 = n(V2C_NF_EXYEE);
+      const float c3 = n(V2C_NF_PES), p3 = n(V2C_NF_PEE);
+      put_antid(n, V2C_NF_PHIN, V2C_NF_PHIS, antid, c0, p0, cur[6], w);
+      put_antid(n, V2C_NF_SXYEN, V2C_NF_SXYE, antid, c1, p1, cur[3], w);
+      put_antid(n, V2C_NF_EXYEN, V2C_NF_EXYE, antid, c2, p2, cur[4], w);
+      put_antid(n, V2C_NF_PEN, V2C_NF_PE, antid, c3, p3, cur[2], w);
+      if (n(V2C_NF_PE) < 0.f) n(V2C_NF_PE) = 0.f;
+      put_ratio(n, V2C_NF_COHESION, cur[5], w);
+      put_ratio(n, V2C_NF_NU_M2C, cur[0], w);
       // nu_m2c / (sum nu/G w / sum w) = sum nu w / sum nu/G w
-      N.f(V2C_NF_GG)[m3] = ratio(cur[0], acc_ff(cur[1]));
+      put_ratio(n, V2C_NF_GG, cur[0], cur[1]);
     } else {
-      N.f(V2C_NF_PHIN)[m3] = 0; N.f(V2C_NF_SXYEN)[m3] = 0; N.f(V2C_NF_EXYEN)[m3] = 0;
-      N.f(V2C_NF_PHIS)[m3] = 0; N.f(V2C_NF_SXYE)[m3] = 0; N.f(V2C_NF_EXYE)[m3] = 0;
-      N.f(V2C_NF_COHESION)[m3] = 0; N.f(V2C_NF_GG)[m3] = 0;
+      n(V2C_NF_PHIN) = 0; n(V2C_NF_SXYEN) = 0; n(V2C_NF_EXYEN) = 0;
+      n(V2C_NF_PHIS) = 0; n(V2C_NF_SXYE) = 0; n(V2C_NF_EXYE) = 0;
+      n(V2C_NF_COHESION) = 0; n(V2C_NF_GG) = 0;
     }
-  } else if (role == 1) {
-    const ff ssf = acc_ff(cur[6]);
-    const float ss = ff_round(ssf);
+  } else if (GROUP == T_THERMAL) {
+    const Acc w = cur[6];
+    const bool any = acc_round(w) != 0.f;
     const bool interior = ci >= 1 && j >= 1 && ci < g.xn - 1 && j < g.yn - 1;
-    float mu = 0.f, fa = 0.f, fb = 0.f, fL = 0.f, fV0 = 0.f;
-    if (ss != 0.f && interior) node_friction(a, ci, j, mu, fa, fb, fL, fV0);
-    N.f(V2C_NF_MUS_S)[m3] = mu; N.f(V2C_NF_AS)[m3] = fa; N.f(V2C_NF_BS)[m3] = fb;
-    N.f(V2C_NF_LS)[m3] = fL; N.f(V2C_NF_V0S)[m3] = fV0;
-    if (ss != 0.f) {
-      N.f(V2C_NF_RO)[m3] = ratio(cur[0], ssf); N.f(V2C_NF_ET)[m3] = ratio(cur[1], ssf);
-      N.f(V2C_NF_HT)[m3] = ratio(cur[2], ssf); N.f(V2C_NF_CP)[m3] = ratio(cur[3], ssf);
-      N.f(V2C_NF_KT)[m3] = ratio(cur[4], ssf); N.f(V2C_NF_TK)[m3] = ratio(cur[5], ssf);
+    if (any && interior) {
+      float mu, fa, fb, fL, fV0;
+      node_friction(a, ci, j, mu, fa, fb, fL, fV0);
+      n(V2C_NF_MUS_S) = mu; n(V2C_NF_AS) = fa; n(V2C_NF_BS) = fb;
+      n(V2C_NF_LS) = fL; n(V2C_NF_V0S) = fV0;
     } else {
-      N.f(V2C_NF_RO)[m3] = 0; N.f(V2C_NF_ET)[m3] = 0; N.f(V2C_NF_HT)[m3] = 0;
-      N.f(V2C_NF_CP)[m3] = 0; N.f(V2C_NF_KT)[m3] = 0; N.f(V2C_NF_TK)[m3] = 0;
+      put_zeros(n, V2C_NF_MUS_S, 5);
+    }
+    if (any) {
+      put_ratio(n, V2C_NF_RO, cur[0], w);
+      put_ratio(n, V2C_NF_ET, cur[1], w);
+      put_ratio(n, V2C_NF_HT, cur[2], w);
+      put_ratio(n, V2C_NF_CP, cur[3], w);
+      put_ratio(n, V2C_NF_KT, cur[4], w);
+      put_ratio(n, V2C_NF_TK, cur[5], w);
+    } else {
+      put_zeros(n, V2C_NF_RO, 6);
     }
     // arrays the reference zeroes at the start (interpolation.c:58-153)
     // and that marker2nodes itself does not fill
-    static const int zl[] = {V2C_NF_NU, V2C_NF_ND, V2C_NF_WTPHISUM, V2C_NF_WTSXXSUM,
-                             V2C_NF_WTVXSUM, V2C_NF_WTVYSUM, V2C_NF_PHISUM, V2C_NF_SXYSUM,
-                             V2C_NF_EXYSUM, V2C_NF_ESUM, V2C_NF_SXXSUM, V2C_NF_EXXSUM,
-                             V2C_NF_VXSUM, V2C_NF_VYSUM, V2C_NF_PSUM, V2C_NF_MRX0,
-                             V2C_NF_MRY0};
-#pragma unroll
-    for (int q = 0; q < (int)(sizeof(zl) / sizeof(zl[0])); q++) N.f(zl[q])[m3] = 0;
-  } else if (role == 2) {
-    // centre node (ci+1, j+1) from cell (ci, j)
+    put_zeros(n, V2C_NF_NU, 2);
+    put_zeros(n, V2C_NF_PHISUM, 15);
+  } else if (GROUP == T_CENTRE_NU) {
     if (ci < g.ncx && j < ncy) {
-      const long mc = (long)(ci + 1) * g.yn + (j + 1);
-      const ff s1f = acc_ff(cur[5]);
-      const float s1 = ff_round(s1f);
-      if (s1 != 0.f) {
-        const ff sxxen = ff_div_fast(acc_ff(cur[2]), s1f), sppen = ff_div_fast(acc_ff(cur[4]), s1f);
-        const ff exxen = ff_div_fast(acc_ff(cur[3]), s1f);
-        float sxxe, sppe, exxe;
-        if (antid) {
-          sxxe = antid_rn(sxxen, N.f(V2C_NF_SXX)[mc], N.f(V2C_NF_SXXEE)[mc]);
-          sppe = antid_rn(sppen, N.f(V2C_NF_PR)[mc], N.f(V2C_NF_SPPEE)[mc]);
-          exxe = antid_rn(exxen, N.f(V2C_NF_EXX)[mc], N.f(V2C_NF_EXXEE)[mc]);
-        } else {
-          sxxe = ff_round(sxxen); sppe = ff_round(sppen); exxe = ff_round(exxen);
-        }
-        if (a.S.sppe_nstress) sppe = a.S.nstress_f;
-        N.f(V2C_NF_SXXEN)[mc] = ff_round(sxxen); N.f(V2C_NF_SPPEN)[mc] = ff_round(sppen);
-        N.f(V2C_NF_EXXEN)[mc] = ff_round(exxen); N.f(V2C_NF_SXXE)[mc] = sxxe;
-        N.f(V2C_NF_SPPE)[mc] = sppe; N.f(V2C_NF_EXXE)[mc] = exxe;
-        N.f(V2C_NF_ND_M2C)[mc] = ratio(cur[0], s1f);
-        N.f(V2C_NF_GD)[mc] = ratio(cur[0], acc_ff(cur[1]));
-        N.f(V2C_NF_BM)[mc] = 50e9f;
-        N.f(V2C_NF_DRO)[mc] = 0; N.f(V2C_NF_DRP)[mc] = 0;
+      const NodeRef c{n.base + g.yn + 1, n.nn};
+      if (acc_round(cur[2]) != 0.f) {
+        put_ratio(c, V2C_NF_ND_M2C, cur[0], cur[2]);
+        put_ratio(c, V2C_NF_GD, cur[0], cur[1]);
+        c(V2C_NF_BM) = 50e9f;
       } else {
-        N.f(V2C_NF_SXXEN)[mc] = 0; N.f(V2C_NF_SPPEN)[mc] = 0; N.f(V2C_NF_EXXEN)[mc] = 0;
-        N.f(V2C_NF_SXXE)[mc] = 0; N.f(V2C_NF_SPPE)[mc] = 0; N.f(V2C_NF_EXXE)[mc] = 0;
-        N.f(V2C_NF_GD)[mc] = 0; N.f(V2C_NF_BM)[mc] = 0;
-        N.f(V2C_NF_DRO)[mc] = 0; N.f(V2C_NF_DRP)[mc] = 0;
+        c(V2C_NF_GD) = 0; c(V2C_NF_BM) = 0;
       }
+      c(V2C_NF_DRO) = 0; c(V2C_NF_DRP) = 0;
     }
     // centre fields of nodes no cell feeds (first column / first row)
     if (ci == 0 || j == 0) {
-      N.f(V2C_NF_SXXEN)[m3] = 0; N.f(V2C_NF_SPPEN)[m3] = 0; N.f(V2C_NF_EXXEN)[m3] = 0;
-      N.f(V2C_NF_SXXE)[m3] = 0; N.f(V2C_NF_SPPE)[m3] = 0; N.f(V2C_NF_EXXE)[m3] = 0;
-      N.f(V2C_NF_GD)[m3] = 0; N.f(V2C_NF_BM)[m3] = 0;
-      N.f(V2C_NF_DRO)[m3] = 0; N.f(V2C_NF_DRP)[m3] = 0;
+      n(V2C_NF_GD) = 0; n(V2C_NF_BM) = 0; n(V2C_NF_DRO) = 0; n(V2C_NF_DRP) = 0;
+    }
+  } else if (GROUP == T_CENTRE_S) {
+    if (ci < g.ncx && j < ncy) {
+      const NodeRef c{n.base + g.yn + 1, n.nn};
+      const Acc w = cur[3];
+      if (acc_round(w) != 0.f) {
+        const float c0 = c(V2C_NF_SXX), p0 = c(V2C_NF_SXXEE), c1 = c(V2C_NF_PR);
+        const float p1 = c(V2C_NF_SPPEE), c2 = c(V2C_NF_EXX), p2 = c(V2C_NF_EXXEE);
+        put_antid(c, V2C_NF_SXXEN, V2C_NF_SXXE, antid, c0, p0, cur[0], w);
+        put_antid(c, V2C_NF_SPPEN, V2C_NF_SPPE, antid, c1, p1, cur[2], w);
+        put_antid(c, V2C_NF_EXXEN, V2C_NF_EXXE, antid, c2, p2, cur[1], w);
+        if (a.S.sppe_nstress) c(V2C_NF_SPPE) = a.S.nstress_f;
+      } else {
+        c(V2C_NF_SXXEN) = 0; c(V2C_NF_SPPEN) = 0; c(V2C_NF_EXXEN) = 0;
+        c(V2C_NF_SXXE) = 0; c(V2C_NF_SPPE) = 0; c(V2C_NF_EXXE) = 0;
+      }
+    }
+    if (ci == 0 || j == 0) {
+      n(V2C_NF_SXXEN) = 0; n(V2C_NF_SPPEN) = 0; n(V2C_NF_EXXEN) = 0;
+      n(V2C_NF_SXXE) = 0; n(V2C_NF_SPPE) = 0; n(V2C_NF_EXXE) = 0;
     }
   } else {
-    const ff wxf = acc_ff(cur[2]);
-    if (ff_round(wxf) != 0.f) {
-      const ff mrx0 = acc_ff(cur[1]);
-      const ff mvxn = ff_div_fast(acc_ff(cur[0]), mrx0);
-      N.f(V2C_NF_MVXN)[m3] = ff_round(mvxn);
+    constexpr bool X = GROUP == T_VX;
+    const int mv = X ? V2C_NF_MVX : V2C_NF_MVY, mr = X ? V2C_NF_MRX : V2C_NF_MRY;
+    if (acc_round(cur[2]) != 0.f) {
+      put_antid(n, X ? V2C_NF_MVXN : V2C_NF_MVYN, mv, antid, n(X ? V2C_NF_VX : V2C_NF_VY),
+                n(X ? V2C_NF_MVXE : V2C_NF_MVYE), cur[0], cur[1]);
       // the boundary correction (vxvy_boundarycorrection) leaves the vx
-      // ghost row at zero; only the 13-node stencil gives it weight
-      N.f(V2C_NF_MVX)[m3] = j == g.yn - 1 ? 0.f
-                            : antid ? antid_rn(mvxn, N.f(V2C_NF_VX)[m3], N.f(V2C_NF_MVXE)[m3])
-                                    : ff_round(mvxn);
-      N.f(V2C_NF_MRX)[m3] = ff_round(ff_div_fast(mrx0, wxf));
+      // ghost row and the vy ghost column at zero; only the 13-node stencil
+      // gives them weight
+      if (X ? j == g.yn - 1 : ci == g.xn - 1) n(mv) = 0;
+      put_ratio(n, mr, cur[1], cur[2]);
     } else {
-      N.f(V2C_NF_MVX)[m3] = 0; N.f(V2C_NF_MRX)[m3] = 0;
-    }
-    const ff wyf = acc_ff(vy3[2]);
-    if (ff_round(wyf) != 0.f) {
-      const ff mry0 = acc_ff(vy3[1]);
-      const ff mvyn = ff_div_fast(acc_ff(vy3[0]), mry0);
-      N.f(V2C_NF_MVYN)[m3] = ff_round(mvyn);
-      N.f(V2C_NF_MVY)[m3] = ci == g.xn - 1 ? 0.f  // the vy ghost column, likewise
-                            : antid ? antid_rn(mvyn, N.f(V2C_NF_VY)[m3], N.f(V2C_NF_MVYE)[m3])
-                                    : ff_round(mvyn);
-      N.f(V2C_NF_MRY)[m3] = ff_round(ff_div_fast(mry0, wyf));
-    } else {
-      N.f(V2C_NF_MVY)[m3] = 0; N.f(V2C_NF_MRY)[m3] = 0;
+      n(mv) = 0; n(mr) = 0;
     }
   }
 }
 
-// MINB resident CTAs per SM: 6 (80 registers, no spills); the skewed
-// staging area (33.8 KB) leaves room for 6 CTAs, and at 7 (72 registers)
-// the spills cost more than the extra CTA gave before the skew (C4 window:
-// 0.73 against 0.65 ms)
-template <int MINB>
-__global__ void __launch_bounds__(NTH, MINB) k_m2n(M2NArgs a) {
-  __shared__ Smem sm;
+// Two runs of one lane's markers in the staged chunk, walked as one list:
+// the warp's time goes with the longest of its 32 lists, and one list of two
+// runs is shorter than the two runs' longest in turn.
+struct Runs {
+  int p, n1, n, jump;  // first position, markers of run 1, of both, positions skipped between them
+};
+// sorted positions [b1, e1), then [b2, e2), clipped to the chunk [cs, ce)
+__device__ __forceinline__ Runs two_runs(int cs, int ce, int b1, int e1, int b2, int e2) {
+  b1 = max(b1, cs); e1 = min(e1, ce); b2 = max(b2, cs); e2 = min(e2, ce);
+  Runs r;
+  r.n1 = max(e1 - b1, 0);
+  r.n = r.n1 + max(e2 - b2, 0);
+  r.p = b1 - cs;
+  r.jump = (b2 - cs) - (r.p + r.n1);
+  return r;
+}
+#define FOR_RUNS(R)                                                          \
+  _Pragma("unroll 1") for (int i_ = 0, p = (R).p; i_ < (R).n; ++i_, ++p)     \
+    if (p += (i_ == (R).n1) ? (R).jump : 0; true)
+
+// what a warp of the sweep sums per marker
+struct Column {
+  int cs, ce;            // the staged chunk
+  int4 ql, qu;           // quarter class starts of cells (ci, j-1) and (ci, j)
+  int lo_e, up_e;        // their ends
+  float s1lo, s1up;      // 1 / cell area
+};
+
+__device__ __forceinline__ float marker_ro(const M2NArgs &a, const Smem &sm, int p, int q) {
+  return a.S.p.densimod ? sm.p[S_PRO][q].y : a.R(RK_RO, sm.type[p]);
+}
+
+// Basic nodes: one list of the halves (left: of node column ci; right: of
+// ci+1) of cells (ci, j-1), bottom quarter, and (ci, j), top quarter.  The
+// weight s (1-2u)(2v-1) etc. of the four quarters is written (+-s)(2u-1)(2v-1)
+// -- the same roundings -- and is positive exactly for a marker strictly
+// inside the quarter (exact halves belong to no basic node, u = NaN to none).
+template <bool THERMAL>
+__device__ __forceinline__ void sum_basic(const M2NArgs &a, const Smem &sm, const Column &C,
+                                          bool left, Acc2 (&acc)[4], Acc &wt) {
+  const Runs R = left ? two_runs(C.cs, C.ce, C.ql.z, C.ql.w, C.qu.x, C.qu.y)
+                      : two_runs(C.cs, C.ce, C.ql.w, C.lo_e, C.qu.y, C.qu.z);
+  const float s1 = left ? -C.s1lo : C.s1lo, s2 = left ? C.s1up : -C.s1up;
+  FOR_RUNS(R) {
+    const int q = slot_of(p);
+    const float2 uv = sm.p[S_UV][q];
+    const int t = sm.type[p];
+    const float w = (i_ < R.n1 ? s1 : s2) * fmaf(2.f, uv.x, -1.f) * fmaf(2.f, uv.y, -1.f);
+    const float2 ne = sm.p[S_NUE][q], cp = sm.p[S_COHPHI][q], se = sm.p[S_SXYEXY][q];
+    const float2 kt = sm.p[S_KTTK][q];
+    if (w > 0.f) {
+      if (!THERMAL) {
+        acc[0].add(mul_w(ne.x, __fmul_rn(ne.x, a.R(RK_INV_GG, t)), w));
+        acc[1].add(mul_w(ne.y, se.x, w));
+        acc[2].add(mul_w(se.y, cp.x, w));
+        acc[3].add(pack2(__fmul_rn(cp.y, w), w));
+      } else {
+        const float bb = a.R(RK_BB, t);
+        // dencalcomp adiabatic term
+        const float et = __fdividef(bb, 1.f - bb * (kt.y - 298.15f));
+        acc[0].add(mul_w(marker_ro(a, sm, p, q), et, w));
+        acc[1].add(mul_w(a.R(RK_HT, t), a.R(RK_CP, t), w));
+        acc[2].add(mul_w(kt.x, kt.y, w));
+        wt.add(w);
+      }
+    }
+  }
+}
+
+// C4 (80 M markers, 20 per cell): 4.96 -> 2.98 ms against four warps of
+// 384-marker chunks with scalar two-sums; a 1001 x 401-line model of 20 (16)
+// per cell 0.582 -> 0.382 (0.499 -> 0.316) ms, 301 x 101 lines 77 -> 48 us.
+// Bound by instruction issue (30 warp instructions per marker, 54 % issue
+// active at 4 CTAs) and the two waits of each chunk; staging alone takes
+// 1.3 ms at C4, 5.1 TB/s.  What each part gave there: whole columns in one
+// chunk and one list per warp (18.6 -> 29 active lanes), packed two-sums,
+// the loops kept rolled and the tail's quotients out of line (instruction
+// fetch was the largest stall: 6.7 cycles per issue), indices and L2
+// prefetches a chunk ahead (3.63 -> 3.15 ms), the tail's inputs read at once
+// (3.15 -> 2.98 ms).  Copying through registers instead of asynchronously
+// was slower (0.47 against 0.44 ms on the smaller model).
+__global__ void __launch_bounds__(NTH, 4) k_m2n(M2NArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
   const Grid &g = a.g;
-  const int tid = threadIdx.x, role = tid / TY, jl = tid % TY;
+  const int tid = threadIdx.x, warp = tid >> 5, jl = tid & 31;
   const int i0 = blockIdx.x * a.TX, j0 = blockIdx.y * TY;
   const int j = j0 + jl;
   const bool jvalid = j < g.yn;
   const int ncy = g.ncy;
   const int ci_end = min(i0 + a.TX, g.xn);
+  const int jlo = max(j0 - 1, 0), jhi = min(j0 + TY - 1, ncy - 1);
+  const Source src = stage_source(a, warp);
+  const int c_end = min(ci_end, g.ncx);
+  const int c0 = max(i0 - 1, 0);
+  if (c0 < c_end) {
+    const int b = __ldg(a.start + (long)c0 * ncy + jlo);
+    start_chunk(a, sm, src, b, min(b + CHUNK, __ldg(a.start + (long)c0 * ncy + jhi + 1)), warp, jl);
+  }
 
-  // role 0: nu, nu/G, e, sxy, exy, C, phi, w      role 1: ro, et, ht, cp, kt, tk, w
-  // role 2: nu, nu/G, sxx, exx, p, w (centre)     role 3: vx*ro, ro, w (vx) + vy*ro, ro, w (vy)
-  Acc cur[8], car[8], vy3[3];
+  // warps 0, 1: nu, nu/G | e, sxy | exy, C | phi, w
+  // warps 2, 3: ro, et | ht, cp | kt, tk and w      warp 4: nu, nu/G and w
+  // warp 5: sxx, exx | p, w     warps 6, 7: v*ro, ro and w (vx: [1] the carry)
+  Acc2 acc[4];
+  Acc wt, wt1;
 #pragma unroll
-  for (int q = 0; q < 8; q++) { cur[q].zero(); car[q].zero(); }
-#pragma unroll
-  for (int q = 0; q < 3; q++) vy3[q].zero();
+  for (int q = 0; q < 4; q++) acc[q].zero();
+  wt.zero(); wt1.zero();
 
-  for (int ci = max(i0 - 1, 0); ci < ci_end; ++ci) {
-#pragma unroll
-    for (int q = 0; q < 8; q++) { cur[q] = car[q]; car[q].zero(); }
-#pragma unroll
-    for (int q = 0; q < 3; q++) vy3[q].zero();
-    if (role == 2) {
-#pragma unroll
-      for (int q = 0; q < 8; q++) cur[q].zero();
-    }
-
+  for (int ci = c0; ci < ci_end; ++ci) {
+    // owned: this CTA finishes node column ci; next: it finishes column ci+1
+    const bool owned = ci >= i0, next = ci + 1 < ci_end;
+    const bool mine = ((ci ^ warp) & 1) == 0;  // warps 0..3: node column ci is this warp's
     if (ci < g.ncx) {
-      const int jlo = max(j0 - 1, 0), jhi = min(j0 + TY - 1, ncy - 1);
       const long cb = (long)ci * ncy;
       const int seg_b = __ldg(a.start + cb + jlo), seg_e = __ldg(a.start + cb + jhi + 1);
-      // quarter class starts of cell (ci, j-1) (lower) and (ci, j) (upper)
-      int4 ql = make_int4(0, 0, 0, 0), qu = make_int4(0, 0, 0, 0);
-      int lo_e = 0, up_e = 0;
-      float s1lo = 0.f, s1up = 0.f;
+      const int nseg_b = ci + 1 < c_end ? __ldg(a.start + cb + ncy + jlo) : 0;
+      const int nseg_e = ci + 1 < c_end ? __ldg(a.start + cb + ncy + jhi + 1) : 0;
+      const bool edge = ci == 0 || ci == g.ncx - 1 || jlo == 0 || jhi == ncy - 1;
+      Column C;
+      C.ql = make_int4(0, 0, 0, 0); C.qu = make_int4(0, 0, 0, 0);
+      C.lo_e = 0; C.up_e = 0;
+      C.s1lo = 0.f; C.s1up = 0.f;
       const float iwx = 1.f / __ldg(g.wx + ci);
       if (jvalid && j - 1 >= 0 && j - 1 <= ncy - 1) {
-        ql = __ldg(a.qstart + cb + j - 1);
-        lo_e = __ldg(a.start + cb + j);
-        s1lo = iwx / __ldg(g.wy + j - 1);
+        C.ql = __ldg(a.qstart + cb + j - 1);
+        C.lo_e = __ldg(a.start + cb + j);
+        C.s1lo = iwx / __ldg(g.wy + j - 1);
       }
       if (jvalid && j <= ncy - 1) {
-        qu = __ldg(a.qstart + cb + j);
-        up_e = __ldg(a.start + cb + j + 1);
-        s1up = iwx / __ldg(g.wy + j);
+        C.qu = __ldg(a.qstart + cb + j);
+        C.up_e = __ldg(a.start + cb + j + 1);
+        C.s1up = iwx / __ldg(g.wy + j);
       }
-      const int rlo = j - 1 - jlo, rup = j - jlo;  // skews of cells (ci, j-1), (ci, j)
+      if (seg_b == seg_e)
+        start_chunk(a, sm, src, nseg_b, min(nseg_b + CHUNK, nseg_e), warp, jl);
       for (int cs = seg_b; cs < seg_e; cs += CHUNK) {
         const int ce = min(cs + CHUNK, seg_e);
+        C.cs = cs; C.ce = ce;
+        cp_async_wait_all();
+        __syncthreads();  // the indices are there, the previous chunk is summed
+        stage_fields(a, sm, ce - cs, ci, edge, src, warp, jl);
         __syncthreads();
-        stage_chunk(a, sm, cs, ce, ci, jlo, tid);
-        __syncthreads();
-// the staged markers of sorted positions [b, e) (one quarter class run)
-#define CLASS_RUN(b, e, r) \
-  for (int s = max((b), cs), s_e = min((e), ce), q = s - cs + (r); s < s_e; ++s, ++q) \
-    if (sm.act[q])
-        if (role <= 1) {
-          // cell (ci, j-1), bottom halves (v > 1/2): class 2 left, class 3 right
-          CLASS_RUN(ql.z, ql.w, rlo) {
-            const float u = sm.p[P_U][q], v = sm.p[P_V][q];
-            if (u < 0.5f) {
-              const float w = s1lo * (1.f - 2.f * u) * (2.f * v - 1.f);
-              if (role == 0) ADD_BASIC_A(cur, q, w); else ADD_BASIC_B(cur, q, w);
-            }
+        const int nb = ce == seg_e ? nseg_b : ce;
+        start_chunk(a, sm, src, nb, min(nb + CHUNK, ce == seg_e ? nseg_e : seg_e), warp, jl);
+        if (warp < 4) {
+          if (mine ? owned : next) {
+            if (warp < 2) sum_basic<false>(a, sm, C, mine, acc, wt);
+            else sum_basic<true>(a, sm, C, mine, acc, wt);
           }
-          CLASS_RUN(ql.w, lo_e, rlo) {
-            const float u = sm.p[P_U][q], v = sm.p[P_V][q];
-            const float w = s1lo * (2.f * u - 1.f) * (2.f * v - 1.f);
-            if (role == 0) ADD_BASIC_A(car, q, w); else ADD_BASIC_B(car, q, w);
-          }
-          // cell (ci, j), top halves (v < 1/2): class 0 left, class 1 right
-          CLASS_RUN(qu.x, qu.y, rup) {
-            const float u = sm.p[P_U][q], v = sm.p[P_V][q];
-            if (u < 0.5f && v < 0.5f) {
-              const float w = s1up * (1.f - 2.f * u) * (1.f - 2.f * v);
-              if (role == 0) ADD_BASIC_A(cur, q, w); else ADD_BASIC_B(cur, q, w);
-            }
-          }
-          CLASS_RUN(qu.y, qu.z, rup) {
-            const float u = sm.p[P_U][q], v = sm.p[P_V][q];
-            if (v < 0.5f) {
-              const float w = s1up * (2.f * u - 1.f) * (1.f - 2.f * v);
-              if (role == 0) ADD_BASIC_A(car, q, w); else ADD_BASIC_B(car, q, w);
-            }
-          }
-        } else if (role == 2) {
+        } else if (warp < 6) {
           // the whole cell (ci, j) to its centre node
-          CLASS_RUN(qu.x, up_e, rup) {
-            const float u = sm.p[P_U][q], v = sm.p[P_V][q];
-            const float w = s1up * tent(u) * tent(v);
-            cur[0].add(sm.p[P_NU][q] * w); cur[1].add(sm.p[P_NUG][q] * w);
-            cur[2].add(sm.p[P_SXX][q] * w); cur[3].add(sm.p[P_EXX][q] * w);
-            cur[4].add(sm.p[P_P][q] * w); cur[5].add(w);
-          }
-        } else {
-          // vy node (ci, j) from the bottom halves of cell (ci, j-1)
-          CLASS_RUN(ql.z, lo_e, rlo) {
-            const float u = sm.p[P_U][q], v = sm.p[P_V][q];
-            const float w = s1lo * (1.f - fabsf(u - 0.5f)) * v;
-            const float ro = sm.p[P_RO][q];
-            vy3[0].add(sm.p[P_VY][q] * ro * w); vy3[1].add(ro * w); vy3[2].add(w);
-          }
-          // cell (ci, j): vx node (ci, j) from u < 1/2 (classes 0, 2), vx node
-          // (ci+1, j) from u > 1/2 (classes 1, 3), vy node (ci, j) from v < 1/2
-          // (classes 0, 1)
-          CLASS_RUN(qu.x, qu.y, rup) {
-            const float u = sm.p[P_U][q], v = sm.p[P_V][q];
-            const float ro = sm.p[P_RO][q];
-            if (u < 0.5f) {
-              const float w = s1up * (1.f - u) * (1.f - fabsf(v - 0.5f));
-              cur[0].add(sm.p[P_VX][q] * ro * w); cur[1].add(ro * w); cur[2].add(w);
-            }
-            if (v < 0.5f) {
-              const float w = s1up * (1.f - fabsf(u - 0.5f)) * (1.f - v);
-              vy3[0].add(sm.p[P_VY][q] * ro * w); vy3[1].add(ro * w); vy3[2].add(w);
+          if (owned) {
+            const Runs R = two_runs(cs, ce, C.qu.x, C.up_e, 0, 0);
+#pragma unroll 1
+            for (int i = 0, p = R.p; i < R.n; ++i, ++p) {
+              const int q = slot_of(p);
+              const float2 uv = sm.p[S_UV][q];
+              const float w = C.s1up * tent(uv.x) * tent(uv.y);
+              if (w >= 0.f) {
+                        if (warp == 4) {
+                  const float nu = sm.p[S_NUE][q].x;
+                  acc[0].add(mul_w(nu, __fmul_rn(nu, a.R(RK_INV_GG, sm.type[p])), w));
+                  wt.add(w);
+                } else {
+                  const float2 se = sm.p[S_SXXEXX][q];
+                  acc[0].add(mul_w(se.x, se.y, w));
+                  acc[1].add(pack2(__fmul_rn(sm.p[S_PRO][q].x, w), w));
+                }
+              }
             }
           }
-          CLASS_RUN(qu.y, qu.z, rup) {
-            const float u = sm.p[P_U][q], v = sm.p[P_V][q];
-            const float ro = sm.p[P_RO][q];
-            const float wx = s1up * u * (1.f - fabsf(v - 0.5f));
-            car[0].add(sm.p[P_VX][q] * ro * wx); car[1].add(ro * wx); car[2].add(wx);
-            if (v < 0.5f) {
-              const float w = s1up * (1.f - fabsf(u - 0.5f)) * (1.f - v);
-              vy3[0].add(sm.p[P_VY][q] * ro * w); vy3[1].add(ro * w); vy3[2].add(w);
+        } else if (warp == 6) {
+          // vx node (ci, j) from u < 1/2 of cell (ci, j) (classes 0, 2), then
+          // vx node (ci+1, j) from u > 1/2 (classes 1, 3)
+          if (owned) {
+            const Runs R = two_runs(cs, ce, C.qu.x, C.qu.y, C.qu.z, C.qu.w);
+            FOR_RUNS(R) {
+              const int q = slot_of(p);
+              const float2 uv = sm.p[S_UV][q];
+              if (uv.x < 0.5f) {
+                const float w = C.s1up * (1.f - uv.x) * (1.f - fabsf(uv.y - 0.5f));
+                const float ro = marker_ro(a, sm, p, q);
+                acc[0].add(mul_w(__fmul_rn(sm.p[S_VXVY][q].x, ro), ro, w));
+                wt.add(w);
+              }
             }
           }
-          CLASS_RUN(qu.z, qu.w, rup) {
-            const float u = sm.p[P_U][q], v = sm.p[P_V][q];
-            if (u < 0.5f) {
-              const float ro = sm.p[P_RO][q];
-              const float w = s1up * (1.f - u) * (1.f - fabsf(v - 0.5f));
-              cur[0].add(sm.p[P_VX][q] * ro * w); cur[1].add(ro * w); cur[2].add(w);
+          if (next) {
+            const Runs R = two_runs(cs, ce, C.qu.y, C.qu.z, C.qu.w, C.up_e);
+            FOR_RUNS(R) {
+              const int q = slot_of(p);
+              const float2 uv = sm.p[S_UV][q];
+              const float w = C.s1up * uv.x * (1.f - fabsf(uv.y - 0.5f));
+              if (w >= 0.f) {
+                const float ro = marker_ro(a, sm, p, q);
+                acc[1].add(mul_w(__fmul_rn(sm.p[S_VXVY][q].x, ro), ro, w));
+                wt1.add(w);
+              }
             }
           }
-          CLASS_RUN(qu.w, up_e, rup) {
-            const float u = sm.p[P_U][q], v = sm.p[P_V][q];
-            const float ro = sm.p[P_RO][q];
-            const float w = s1up * u * (1.f - fabsf(v - 0.5f));
-            car[0].add(sm.p[P_VX][q] * ro * w); car[1].add(ro * w); car[2].add(w);
+        } else if (owned) {
+          // vy node (ci, j) from the bottom halves of cell (ci, j-1) (classes
+          // 2, 3) and the top halves of cell (ci, j) (classes 0, 1)
+          const Runs R = two_runs(cs, ce, C.ql.z, C.lo_e, C.qu.x, C.qu.z);
+          FOR_RUNS(R) {
+            const int q = slot_of(p);
+            const float2 uv = sm.p[S_UV][q];
+            const bool lo = i_ < R.n1;
+            if (lo || uv.y < 0.5f) {
+              const float w = (lo ? C.s1lo : C.s1up) * (1.f - fabsf(uv.x - 0.5f)) *
+                              (lo ? uv.y : 1.f - uv.y);
+              if (w >= 0.f) {
+                const float ro = marker_ro(a, sm, p, q);
+                acc[0].add(mul_w(__fmul_rn(sm.p[S_VXVY][q].y, ro), ro, w));
+                wt.add(w);
+              }
+            }
           }
         }
-#undef CLASS_RUN
       }
     }
 
     // ------------------------------------------------------ node tail
-    if (ci < i0 || !jvalid) continue;
-    node_tail(a, role, ci, j, cur, vy3);
+    if (warp < 4 && !mine) continue;
+    if (owned && jvalid) {
+      Acc c[8];
+#pragma unroll
+      for (int q = 0; q < 4; q++) acc[q].split(c[2 * q], c[2 * q + 1]);
+      if (warp < 2) {
+        node_tail<T_STRESS>(a, ci, j, c);
+      } else if (warp < 4) {
+        c[6] = wt;
+        node_tail<T_THERMAL>(a, ci, j, c);
+      } else if (warp == 4) {
+        c[2] = wt;
+        node_tail<T_CENTRE_NU>(a, ci, j, c);
+      } else if (warp == 5) {
+        node_tail<T_CENTRE_S>(a, ci, j, c);
+      } else {
+        c[2] = wt;
+        if (warp == 6) node_tail<T_VX>(a, ci, j, c);
+        else node_tail<T_VY>(a, ci, j, c);
+      }
+    }
+    if (warp == 6) {
+      acc[0] = acc[1];
+      wt = wt1;
+    } else {
+      acc[0].zero();
+      wt.zero();
+    }
+#pragma unroll
+    for (int q = 1; q < 4; q++) acc[q].zero();
+    wt1.zero();
   }
 }
 
@@ -652,10 +748,17 @@ __global__ void __launch_bounds__(128) k_m2n_mode1(M2NArgs a) {
       }
     }
   }
-  if (ROLE != 2) {
-    node_tail(a, ROLE, ix, iy, cur, vy3);
-  } else if (ix >= 1 && iy >= 1) {
-    node_tail(a, 2, ix - 1, iy - 1, cur, vy3);  // writes centre node (ix, iy)
+  if (ROLE == 0) {
+    node_tail<T_STRESS>(a, ix, iy, cur);
+  } else if (ROLE == 1) {
+    node_tail<T_THERMAL>(a, ix, iy, cur);
+  } else if (ROLE == 3) {
+    node_tail<T_VX>(a, ix, iy, cur);
+    node_tail<T_VY>(a, ix, iy, vy3);
+  } else if (ix >= 1 && iy >= 1) {  // writes centre node (ix, iy)
+    const Acc nu[3] = {cur[0], cur[1], cur[5]};
+    node_tail<T_CENTRE_NU>(a, ix - 1, iy - 1, nu);
+    node_tail<T_CENTRE_S>(a, ix - 1, iy - 1, cur + 2);
   } else {
     // a centre node no cell has (first column or row)
     const Nodes &N = a.N;
@@ -694,6 +797,11 @@ __global__ void k_dphis(Grid g, float *phis) {
 
 }  // namespace
 
+cudaError_t m2n_init() {
+  return cudaFuncSetAttribute(k_m2n, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sizeof(Smem));
+}
+
 void launch_m2n(const M2NArgs &a, cudaStream_t st) {
   if (a.S.p.interpolationmod == 1) {
     const unsigned nb = (unsigned)((a.g.nn + 127) / 128);
@@ -704,7 +812,7 @@ void launch_m2n(const M2NArgs &a, cudaStream_t st) {
     return;
   }
   dim3 grid((a.g.xn + a.TX - 1) / a.TX, (a.g.yn + TY - 1) / TY);
-  k_m2n<6><<<grid, NTH, 0, st>>>(a);
+  k_m2n<<<grid, NTH, sizeof(Smem), st>>>(a);
 }
 
 void launch_sticky(const Nodes &N, const uint32_t *key, long nn, cudaStream_t st) {
