@@ -253,27 +253,21 @@ int check_params(const v2c_params *p) {
   return V2C_OK;
 }
 
-// Column strip of the gather: the widest up to 32 columns that still gives
-// 1.5 waves of 7 resident CTAs on each of the 152 SMs (a strip of tx columns
-// restages one halo column).
-int pick_tx(const v2c_ctx *c, int max_tx) {
-  long rows = (c->yn + 31) / 32;
-  int tx = max_tx;
-  while (tx > 4 && rows * ((c->xn + tx - 1) / tx) < 152 * 7 * 3 / 2) tx /= 2;
-  return tx;
-}
-
-// Column strip of the scatter: the widest up to 16 columns that still gives
-// 3 waves of its 4 resident CTAs per SM.  Wide strips save the halo column
-// (C4, 13 waves: 2.98 ms at 16 columns, 3.27 at 4), narrow ones balance the
-// last wave (1001 x 401 lines: 0.385 ms at 8 columns and 2.7 waves, 0.382 at
-// 4 and 5.4) and, where one wave holds the grid, the columns a CTA takes in
-// turn are the kernel's time (51 x 21 lines: 49, 34 and 25 us at 4, 2 and 1).
-int scatter_tx(const v2c_ctx *c) {
-  const long rows = (c->yn + 31) / 32;
-  int tx = 16;
-  while (tx > 1 && rows * ((c->xn + tx - 1) / tx) < 152 * 4 * 3) tx /= 2;
-  return tx;
+// Column strip of the two sweeps: the widest up to 16 columns that gives 2
+// waves of their 4 resident CTAs per SM (wide strips save the halo column,
+// narrower ones balance the last wave), else the widest that fills about one
+// wave, else one column (the columns a CTA takes in turn are the kernel's
+// time then).  Scatter / gather in us at strips of 16, 8, 4, 2, 1:
+//   4001 x 1001 lines  2976 3252 3275 3644 4460 / 2368 2489 2732 3169 4185
+//   1001 x 401 lines    500  385  382  407  491 /  323  277  299  335  435
+//   301 x 101 lines     228  124   69   47   48 /   98   56   40   33   40
+//   51 x 21 lines       170   92   49   34   25 /   85   48   30   21   16
+int sweep_tx(const v2c_ctx *c) {
+  const long rows = (c->yn + 31) / 32, wave = 152 * 4;
+  for (long least : {2 * wave, wave * 9 / 10})
+    for (int tx = 16; tx > 1; tx /= 2)
+      if (rows * ((c->xn + tx - 1) / tx) >= least) return tx;
+  return 1;
 }
 
 }  // namespace
@@ -345,7 +339,7 @@ extern "C" int v2c_create(const v2c_params *p, long max_markers, void *cuda_stre
   AL(ctx->sb.blocksum, ctx->sb.blocksum_cap);
   AL(ctx->d_stage64, cap); AL(ctx->d_stage64b, cap);
 #undef AL
-  if (m2n_init() != cudaSuccess) { v2c_destroy(ctx); return V2C_ERR_CUDA; }
+  if (m2n_init() != cudaSuccess || n2m_init() != cudaSuccess) { v2c_destroy(ctx); return V2C_ERR_CUDA; }
   if (newton_init(ctx->nw, cap) != cudaSuccess) { v2c_destroy(ctx); return V2C_ERR_CUDA; }
   if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) { v2c_destroy(ctx); return V2C_ERR_CUDA; }
   *out = ctx;
@@ -986,7 +980,7 @@ extern "C" int v2c_marker2nodes(v2c_ctx *ctx) {
   a.stat = ctx->d_stat;
   a.gxf = ctx->d_gxf;
   a.gyf = ctx->d_gyf;
-  a.TX = scatter_tx(ctx);
+  a.TX = sweep_tx(ctx);
   a.n = ctx->n;
   CK(cudaMemsetAsync(ctx->d_sticky, 0, sizeof(uint32_t) * ctx->nn, st));
   ctx->dsxx_valid = false;  // the scatter writes sxxe
@@ -1008,7 +1002,7 @@ extern "C" int v2c_marker2nodes(v2c_ctx *ctx) {
   {
     Prof pr(ctx, V2C_PROF_M2N);
     launch_m2n(a, st);
-    ctx->launches += ctx->p.interpolationmod == 1 ? 4 : 1;
+    ctx->launches += 1;
   }
   ctx->props_valid = true;
   {
@@ -1157,8 +1151,7 @@ static int n2m_move(v2c_ctx *ctx, int do_n2m, int do_move) {
   a.gyf = ctx->d_gyf;
   a.quad = ctx->d_quad;
   a.n = ctx->n;
-  a.TX = pick_tx(ctx, 32);
-  a.do_n2m = 1;
+  a.TX = sweep_tx(ctx);
   if (do_n2m && ctx->p.interpolationmod == 1 && ctx->p.antidiffinter == 1) {
     // the full-stencil back-scatter: one payload record per marker
     if (!ctx->d_bs) return fail(ctx, V2C_ERR_STATE);
@@ -1167,7 +1160,7 @@ static int n2m_move(v2c_ctx *ctx, int do_n2m, int do_move) {
   if (do_n2m) {
     Prof pr(ctx, V2C_PROF_N2M);
     launch_n2m(a, st);
-    ctx->launches += a.bs ? 3 : 1;
+    ctx->launches += a.bs ? 2 : 1;
   }
   if (do_move) {
     ctx->props_valid = false;

@@ -176,8 +176,7 @@ struct N2MArgs {
   const float *gyf;  // FP32 line positions (coarse depth test)
   float4 *quad;      // allinteri's bilinear forms per cell quarter [ncell * QUAD_FLOAT4]
   long n;            // markers
-  int TX;
-  int do_n2m;
+  int TX;            // node columns per CTA
   // interpolationmod 1: the tile sweep writes each marker's back-scatter
   // payload (BS_N fields, SoA by sorted position) here and per-node gather
   // kernels sum it; null for interpolationmod 2
@@ -190,7 +189,9 @@ struct N2MArgs {
 enum { BS_U = 0, BS_V, BS_PHIS, BS_SXY, BS_EXY, BS_ES, BS_PR, BS_SXX, BS_EXX, BS_N };
 // float4 coefficient sets per cell: 4 quarters x (VX, VY, ESP)
 constexpr int QUAD_FLOAT4 = 12;
-// nodes2markers: gather, marker update, back-scatter (cell-column tiles)
+// nodes2markers: gather, marker update, back-scatter (cell-column tiles);
+// n2m_init sets the sweep's shared-memory size on the current device
+cudaError_t n2m_init();
 void launch_n2m(const N2MArgs &a, cudaStream_t st);
 // moveandrotatemarkers: one thread per marker, new positions to *_out
 void launch_move(const N2MArgs &a, cudaStream_t st);

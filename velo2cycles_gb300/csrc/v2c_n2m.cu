@@ -1,14 +1,17 @@
 // v2c_n2m.cu -- nodes2markers (interpolation.c:929-1490) and
 // moveandrotatemarkers (moveandrotatemarkers.c:1-178).
 //
-// nodes2markers: same tiling as the marker2nodes sweep (see v2c_m2n.cu).
-// Staging a marker gathers the 19 node fields of interpolate_mechanical from
-// the four staggered stencils in cell-local FP32 coordinates and keeps the
-// quantities the antidiffusion correction scatters back (PHIS, SXY, EXY, ES
-// to basic nodes, PR, SXX, EXX to the centre node, VX*MRO, VY*MRO and MRO to
-// vx/vy nodes); the tile that owns the marker applies the marker update.
-// The back-scatter sums are formed per node by one thread each, in sorted
-// marker order with two-sum compensation, exactly as in marker2nodes.
+// nodes2markers with antidiffusion and interpolationmod 2 (k_n2m): same
+// tiling as the marker2nodes sweep (see v2c_m2n.cu).  A thread gathers a
+// marker's nine node fields from the four staggered stencils of
+// interpolate_mechanical, updates the marker where its tile owns it, and
+// leaves the quantities the antidiffusion correction scatters back (PHIS,
+// SXY, EXY, ES to basic nodes, PR, SXX, EXX to the centre node, VX*MRO,
+// VY*MRO and MRO to vx/vy nodes) in shared memory, where one lane per node
+// row sums them per node, in sorted marker order with two-sum compensation,
+// exactly as in marker2nodes.  The other settings gather without the sweep
+// (k_gather): no back-scatter without antidiffusion, per-node kernels for
+// the full stencils of interpolationmod 1.
 //
 // moveandrotatemarkers: one thread per marker, Euler or RK4 through four
 // allinteri evaluations (interpolation.c:1688-1758) from per-quarter
@@ -22,16 +25,6 @@
 namespace v2c {
 
 namespace {
-
-constexpr int TY = 32;
-constexpr int NTH = 4 * TY;
-constexpr int CHUNK = 384;
-
-enum { Q_U = 0, Q_V, Q_PHIS, Q_SXY, Q_EXY, Q_ES, Q_PR, Q_SXX, Q_EXX, Q_VX, Q_VY, Q_MRO, Q_N };
-
-struct Smem {
-  float q[Q_N][CHUNK];
-};
 
 struct Pos {
   int ix, iy;
@@ -183,17 +176,7 @@ __device__ __forceinline__ void vel_at(const Grid &g, const float4 *Q, Pos p, fl
   ESP = fmaf(dY, fmaf(e.w, dX, e.z), fmaf(e.y, dX, e.x));
 }
 
-// basic-node back-scatter into a named register array
-#define ADD_BS(A, q, w)                                                 \
-  do {                                                                  \
-    A[0].add(sm.q[Q_PHIS][q] * (w)); A[1].add(sm.q[Q_SXY][q] * (w));    \
-    A[2].add(sm.q[Q_EXY][q] * (w)); A[3].add(sm.q[Q_ES][q] * (w));      \
-    A[4].add(w);                                                        \
-  } while (0)
-
-// Marker values without antidiffusion (interpolation.c:985-1011), in a
-// kernel instance of their own (PLAIN) so that the common antidiffusion
-// path keeps its registers: the previous node fields interpolated (change = false: a marker's first
+// Marker values without antidiffusion (interpolation.c:985-1011): the previous node fields interpolated (change = false: a marker's first
 // values), or the change of the node fields since then (change = true),
 // interpolated as one field of node differences -- the same bilinear form,
 // so the same value in exact arithmetic, but the FP32 node differences of
@@ -236,304 +219,537 @@ __device__ __forceinline__ void plain_values(const Grid &g, const Nodes &N, Axis
                 : bil(N.f(V2C_NF_MVY), m3, yn, e, n);
 }
 
-template <bool BS, bool PLAIN>
-__global__ void __launch_bounds__(NTH, 7) k_n2m(N2MArgs a) {
-  __shared__ Smem sm;
+// ------------------------------------------------------------ the sweep
+constexpr int TY = 32;
+constexpr int NTH = 8 * 32;
+// markers staged at once: 33 cells of 23, in the 56 KB that four resident
+// CTAs leave each other
+constexpr int CHUNK = 768;
+constexpr int SLOTS = CHUNK + CHUNK / 16;
+// the marker at position p of a chunk, in slot p + p / 16 (see v2c_m2n.cu)
+__device__ __forceinline__ int slot_of(int p) { return p + (p >> 4); }
+
+// staged quantities, in pairs for packed FP32 sums
+enum { Q_UV = 0, Q_PHSXY, Q_EXYES, Q_PRSXX, Q_EXXMRO, Q_VXVY, Q_N };
+
+// The node columns ci-1 .. ci+2 that the markers of cell column ci read, in
+// a ring of five (the fifth arrives for the next column while this one is
+// gathered), rows j0-2 .. j0+33.
+constexpr int RING = 5, ROWS = TY + 4;
+struct NodeColumn {
+  float4 basic[ROWS];   // PHIS_IT, SXY, EXY, PES
+  float4 centre[ROWS];  // PR, SXX, EXX
+  float2 vel[ROWS];     // VX, VY
+};
+// One axis of a stencil: the weight (position - a) r of its second line, and
+// where its lines are: in y, the first line relative to the marker's cell
+// row; in x, the byte offsets of the two node columns in the ring.
+struct Side {
+  float a, r;
+  int o0, o1;
+};
+enum { S_BASIC = 0, S_CLO, S_CHI, S_LINE, S_HALF, S_HALFLO, S_N };
+struct Smem {
+  float2 q[Q_N][SLOTS];
+  int32_t idx[CHUNK];
+  NodeColumn ring[RING];
+  Side x[2][S_N], y[TY + 1][S_N];  // x: this column's and the next's
+};
+
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void *p) {
+  asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
+}
+
+// The weights of one axis for a marker in cell i of it, by stencil: basic
+// nodes, pressure nodes with the marker in the lower or upper half, lines
+// (vx in x, vy in y), half lines (vy in x, vx in y) with the marker in the
+// upper or lower half -- the four stencils of stencil_basic, stencil_centre,
+// stencil_vx and stencil_vy, whose first line and divisor depend on the cell
+// and the half only.
+__device__ __forceinline__ void axis_side(const float *w, int nc, int n, int i, int which,
+                                          bool x, Side &s) {
+  const Axis ax = make_axis(w, nc, i, 0.f);
+  int m;
+  float A, B;
+  if (which == S_BASIC || which == S_LINE) {
+    m = which == S_BASIC ? min(max(i, 1), n - 3) : i;
+    const int q = m - i;
+    A = ax.G(q);
+    B = ax.G(q + 1) - ax.G(q);
+  } else if (which == S_CLO || which == S_CHI) {
+    m = max(min(i + (which == S_CHI), n - 2), 1);
+    const int q = m - i;
+    A = (ax.G(q - 1) + ax.G(q)) * 0.5f;
+    B = (ax.G(q + 1) - ax.G(q - 1)) * 0.5f;
+  } else {
+    m = min(max(i - (which == S_HALFLO), 0), n - 3);
+    const int q = m - i;
+    A = (ax.G(q) + ax.G(q + 1)) * 0.5f;
+    B = (ax.G(q + 2) - ax.G(q)) * 0.5f;
+  }
+  s.a = A;
+  s.r = __fdividef(1.f, B);
+  s.o0 = x ? m % RING * (int)sizeof(NodeColumn) : m - i;
+  s.o1 = x ? (m + 1) % RING * (int)sizeof(NodeColumn) : 0;
+}
+
+// Start copying node column c (rows r0 .. r0+ROWS-1) to its place in the ring
+__device__ __forceinline__ void load_column(const N2MArgs &a, Smem &sm, int c, int r0, int tid) {
+  if (c < 0 || c >= a.g.xn) return;
+  NodeColumn &R = sm.ring[c % RING];
+  const long m0 = (long)c * a.g.yn + r0;
+  const Nodes &N = a.N;
+#pragma unroll 1
+  for (int t = tid; t < ROWS * 9; t += NTH) {
+    const int f = t / ROWS, r = t - f * ROWS;
+    if (r0 + r < 0 || r0 + r >= a.g.yn) continue;
+    static const int field[9] = {V2C_NF_PHIS_IT, V2C_NF_SXY, V2C_NF_EXY, V2C_NF_PES, V2C_NF_PR,
+                                 V2C_NF_SXX, V2C_NF_EXX, V2C_NF_VX, V2C_NF_VY};
+    float *dst = f < 4 ? &R.basic[r].x + f : f < 7 ? &R.centre[r].x + (f - 4) : &R.vel[r].x + (f - 7);
+    cp_async4(dst, N.f(field[f]) + m0 + r);
+  }
+}
+
+// Ahead of the chunk at sorted positions [b, e): its sort indices, and the
+// L2 lines of what the gather reads of its markers
+__device__ __forceinline__ void start_chunk(const N2MArgs &a, Smem &sm, int b, int e, int tid) {
+#pragma unroll 1
+  for (int s = b + tid; s < e; s += NTH) cp_async4(&sm.idx[s - b], a.perm + s);
+  const int s = b + 32 * (tid & 31);
+  if (s >= e) return;
+  switch (tid >> 5) {
+    case 0: prefetch_l2(a.m.cell_in + s); break;
+    case 1: prefetch_l2(a.m.u_in + s); break;
+    case 2: prefetch_l2(a.m.v_in + s); break;
+    case 3: prefetch_l2(a.m.tk + s); break;
+    case 4: if ((tid & 3) == 0) prefetch_l2(a.m.type + s); break;
+  }
+}
+
+// bilinear interpolation from node values (v2c_rheology.cuh's bil)
+__device__ __forceinline__ float bil_of(const float (&d)[4], float f0, float f1, float f2,
+                                        float f3) {
+  return d[0] * f0 + d[1] * f1 + d[2] * f2 + d[3] * f3;
+}
+__device__ __forceinline__ void weights_of(float e, float n, float (&d)[4]) {
+  d[0] = (1.f - e) * (1.f - n); d[1] = (1.f - e) * n; d[2] = e * (1.f - n); d[3] = e * n;
+}
+
+// Gather of the chunk's marker at position p (array index i) of cell column
+// ci: interpolate_mechanical and the marker update of nodes2markers
+// (interpolation.c:943-984); what the back-scatter sums goes to its slot.
+__device__ __forceinline__ void gather_marker(const N2MArgs &a, Smem &sm, int ci, int jlo, int r0,
+                                              int i0, int j0, int p, int i, int c, float u,
+                                              float v, int t, float tk) {
+  const Grid &g = a.g;
+  const int iy = c - ci * g.ncy;
+  const bool owned = ci >= i0 && iy >= j0;
+  // of the halo column only the right halves reach a node of this tile, of
+  // the halo row only the bottom halves
+  if ((ci < i0 && !(u > 0.5f)) || (iy < j0 && !(v > 0.5f))) return;
+  // interpolate_mechanical clamps the point into the model first
+  float uc = u, vc = v;
+  if (ci == 0 && uc < 0.f) uc = 0.f;
+  if (ci == g.ncx - 1 && uc > 1.f) uc = 1.f;
+  if (iy == 0 && vc < 0.f) vc = 0.f;
+  if (iy == g.ncy - 1 && vc > 1.f) vc = 1.f;
+  const float X = __fmul_rn(uc, __ldg(g.wx + ci)), Y = __fmul_rn(vc, __ldg(g.wy + iy));
+  const Side *sx = sm.x[ci & 1], *sy = sm.y[iy - jlo];
+  const char *ring = reinterpret_cast<const char *>(sm.ring);
+  const int row = iy - r0;
+  float d[4];
+  // the weights of a stencil, and its first node row in its two columns
+  auto corner = [&](int hx, int hy, const NodeColumn *&c0, const NodeColumn *&c1) {
+    const Side A = sx[hx], B = sy[hy];
+    weights_of((X - A.a) * A.r, (Y - B.a) * B.r, d);
+    c0 = reinterpret_cast<const NodeColumn *>(ring + A.o0);
+    c1 = reinterpret_cast<const NodeColumn *>(ring + A.o1);
+    return row + B.o0;
+  };
+  const NodeColumn *c0, *c1;
+  int r = corner(S_BASIC, S_BASIC, c0, c1);
+  float4 f0 = c0->basic[r], f1 = c0->basic[r + 1], f2 = c1->basic[r], f3 = c1->basic[r + 1];
+  const float PHIS = bil_of(d, f0.x, f1.x, f2.x, f3.x), SXY = bil_of(d, f0.y, f1.y, f2.y, f3.y);
+  const float EXY = bil_of(d, f0.z, f1.z, f2.z, f3.z), ES = bil_of(d, f0.w, f1.w, f2.w, f3.w);
+  r = corner(uc > 0.5f ? S_CHI : S_CLO, vc > 0.5f ? S_CHI : S_CLO, c0, c1);
+  f0 = c0->centre[r]; f1 = c0->centre[r + 1]; f2 = c1->centre[r]; f3 = c1->centre[r + 1];
+  const float PR = bil_of(d, f0.x, f1.x, f2.x, f3.x), SXX = bil_of(d, f0.y, f1.y, f2.y, f3.y);
+  const float EXX = bil_of(d, f0.z, f1.z, f2.z, f3.z);
+  r = corner(S_LINE, vc < 0.5f ? S_HALFLO : S_HALF, c0, c1);
+  const float VX = bil_of(d, c0->vel[r].x, c0->vel[r + 1].x, c1->vel[r].x, c1->vel[r + 1].x);
+  r = corner(uc < 0.5f ? S_HALFLO : S_HALF, S_LINE, c0, c1);
+  const float VY = bil_of(d, c0->vel[r].y, c0->vel[r + 1].y, c1->vel[r].y, c1->vel[r + 1].y);
+  const int q = slot_of(p);
+  sm.q[Q_UV][q] = make_float2(uc, vc);
+  sm.q[Q_PHSXY][q] = make_float2(PHIS, SXY);
+  sm.q[Q_EXYES][q] = make_float2(EXY, ES);
+  sm.q[Q_PRSXX][q] = make_float2(PR, SXX);
+  sm.q[Q_EXXMRO][q] = make_float2(EXX, a.R(RK_RO, t));
+  sm.q[Q_VXVY][q] = make_float2(VX, VY);
+  if (!owned || t >= 50) return;
+  // marker update: strictly inside with no temperature yet, or in the grid
+  const bool in_strict = (ci > 0 || u > 0.f) && (ci < g.ncx - 1 || u < 1.f) &&
+                         (iy > 0 || v > 0.f) && (iy < g.ncy - 1 || v < 1.f);
+  const bool in_grid = (ci > 0 || u >= 0.f) && (ci < g.ncx - 1 || u <= 1.f) &&
+                       (iy > 0 || v >= 0.f) && (iy < g.ncy - 1 || v <= 1.f);
+  if (tk <= 0.f ? in_strict : (in_grid && tk > 0.f)) {
+    a.m.phi[i] = PHIS; a.m.exx[i] = EXX; a.m.exy[i] = EXY;
+    a.m.sxx[i] = SXX; a.m.sxy[i] = SXY; a.m.p[i] = PR;
+    a.m.vx[i] = VX; a.m.vy[i] = VY; a.m.e[i] = ES;
+    if (tk <= 0.f && !a.S.p.tempmod) {
+      a.m.tk[i] = a.S.eps2_f;
+      a.m.tk_lo[i] = a.S.eps2_lo;
+    }
+  }
+}
+
+// Back-scatter lists of one lane: two runs of sorted positions, walked as
+// one list (see v2c_m2n.cu)
+struct Runs {
+  int p, n1, n, jump;
+};
+__device__ __forceinline__ Runs two_runs(int cs, int ce, int b1, int e1, int b2, int e2) {
+  b1 = max(b1, cs); e1 = min(e1, ce); b2 = max(b2, cs); e2 = min(e2, ce);
+  Runs r;
+  r.n1 = max(e1 - b1, 0);
+  r.n = r.n1 + max(e2 - b2, 0);
+  r.p = b1 - cs;
+  r.jump = (b2 - cs) - (r.p + r.n1);
+  return r;
+}
+#define FOR_RUNS(R)                                                          \
+  _Pragma("unroll 1") for (int i_ = 0, p = (R).p; i_ < (R).n; ++i_, ++p)     \
+    if (p += (i_ == (R).n1) ? (R).jump : 0; true)
+
+// Warps 0, 1 sum the basic nodes of even and odd node columns, warp 2 the
+// centre nodes, warp 3 vy, warps 4, 5 vx of even and odd node columns; all
+// eight gather.
+// C4 (80 M markers, 20 per cell): 4.77 -> 2.37 ms against four warps of
+// 384-marker chunks gathering through L1; a 1001 x 401-line model of 20 (16)
+// per cell 0.606 -> 0.277 (0.589 -> 0.237) ms, 301 x 101 lines 98 -> 33 us,
+// 51 x 21 lines 52 -> 16 us.  Bound by instruction issue (64 % active, 28
+// warp instructions per marker) and shared-memory reads.  The node values
+// come from shared memory (16 reads per marker instead of 36 through L1), a
+// stencil's line offsets and reciprocals from tables per cell row and
+// column, and the temperature is written only where it changes.  Halo
+// markers that reach no node of the tile are not gathered.
+__global__ void __launch_bounds__(NTH, 4) k_n2m(N2MArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
   const Grid &g = a.g;
   const Nodes &N = a.N;
-  const int tid = threadIdx.x, role = tid / TY, jl = tid % TY;
+  const int tid = threadIdx.x, warp = tid >> 5, jl = tid & 31;
   const int i0 = blockIdx.x * a.TX, j0 = blockIdx.y * TY;
   const int j = j0 + jl;
   const bool jvalid = j < g.yn;
   const int ncy = g.ncy;
   const int ci_end = min(i0 + a.TX, g.xn);
-  const v2c_params &P = a.S.p;
-  // interpolationmod 1 back-scatters through a.bs and the gather kernels
-  const int backscatter = a.do_n2m && !PLAIN && !BS;
-  const long yn = g.yn;
+  const int jlo = max(j0 - 1, 0), jhi = min(j0 + TY - 1, ncy - 1), r0 = jlo - 1;
+  const int c_end = min(ci_end, g.ncx), c0 = max(i0 - 1, 0);
 
-  // role 0: PHIS, SXY, EXY, ES, w (basic)   role 1: PR, SXX, EXX, w (centre)
-  // role 2: VX*MRO, MRO, w (vx)             role 3: VY*MRO, MRO, w (vy)
-  Acc cur[5], car[5];
-#pragma unroll
-  for (int q = 0; q < 5; q++) { cur[q].zero(); car[q].zero(); }
+  // row weights, the first columns' nodes, column weights and chunk
+  for (int t = tid; t < (jhi - jlo + 1) * S_N; t += NTH)
+    axis_side(g.wy, ncy, g.yn, jlo + t / S_N, t % S_N, false, sm.y[t / S_N][t % S_N]);
+  if (c0 < c_end) {
+    for (int c = c0 - 1; c <= c0 + 2; c++) load_column(a, sm, c, r0, tid);
+    if (tid < S_N) axis_side(g.wx, g.ncx, g.xn, c0, tid, true, sm.x[c0 & 1][tid]);
+    const int b = __ldg(a.start + (long)c0 * ncy + jlo);
+    start_chunk(a, sm, b, min(b + CHUNK, __ldg(a.start + (long)c0 * ncy + jhi + 1)), tid);
+  }
 
-  for (int ci = max(i0 - 1, 0); ci < ci_end; ++ci) {
-#pragma unroll
-    for (int q = 0; q < 5; q++) { cur[q] = car[q]; car[q].zero(); }
-    if (role == 1 || role == 3) {
-#pragma unroll
-      for (int q = 0; q < 5; q++) cur[q].zero();
-    }
+  // basic: PHIS, SXY | EXY, ES and w   centre: PR, SXX | EXX, w
+  // vx, vy: v*MRO, MRO and w
+  Acc2 acc[2];
+  Acc wt;
+  acc[0].zero(); acc[1].zero(); wt.zero();
+
+  for (int ci = c0; ci < ci_end; ++ci) {
+    const bool owned = ci >= i0, next = ci + 1 < ci_end;
+    // warps 0, 1, 4, 5: node column ci is this warp's
+    const bool mine = ((ci ^ warp) & 1) == 0;
     if (ci < g.ncx) {
-      const int jlo = max(j0 - 1, 0), jhi = min(j0 + TY - 1, ncy - 1);
       const long cb = (long)ci * ncy;
       const int seg_b = __ldg(a.start + cb + jlo), seg_e = __ldg(a.start + cb + jhi + 1);
-
-      const bool owned_col = ci >= i0;
-      for (int cs = seg_b; cs < seg_e; cs += CHUNK) {
-        const int ce = min(cs + CHUNK, seg_e);
-        if (backscatter) __syncthreads();
-        // the chunk's sort indices of this thread, read together (three
-        // markers per thread: one round of latency rather than three)
-        static_assert(CHUNK == 3 * NTH, "three staging rounds per chunk");
-        int pidx[3];
-#pragma unroll
-        for (int jj = 0; jj < 3; jj++)
-          pidx[jj] = tid + jj * NTH < ce - cs ? __ldg(a.perm + cs + tid + jj * NTH) : 0;
-#pragma unroll 1
-        for (int jj = 0; jj < 3; jj++) {
-          const int k = tid + jj * NTH;
-          if (k >= ce - cs) break;
-          // ---------------------------------------------- stage marker
-          const int idx = jj == 0 ? pidx[0] : (jj == 1 ? pidx[1] : pidx[2]);
-          const int c = a.m.cell_in[idx];
-          const int ix = c / ncy, iy = c - ix * ncy;
-          const float u = a.m.u_in[idx], v = a.m.v_in[idx];
-          const int t = a.m.type[idx];
-          const bool owned = owned_col && iy >= j0 && iy < j0 + TY;
-          if (!owned && !backscatter) continue;
-          // interpolate_mechanical clamps the point into the model first
-          float uc = u, vc = v;
-          if (ix == 0 && uc < 0.f) uc = 0.f;
-          if (ix == g.ncx - 1 && uc > 1.f) uc = 1.f;
-          if (iy == 0 && vc < 0.f) vc = 0.f;
-          if (iy == g.ncy - 1 && vc > 1.f) vc = 1.f;
-          const float wxc = __ldg(g.wx + ix), wyc = __ldg(g.wy + iy);
-          const Axis ax = make_axis(g.wx, g.ncx, ix, uc * wxc);
-          const Axis ay = make_axis(g.wy, g.ncy, iy, vc * wyc);
-          float eb, nb, ec, ncc, e, n;
-          const long mb = stencil_basic(g, ax, ay, eb, nb);
-          const float EXY = bil(N.f(V2C_NF_EXY), mb, yn, eb, nb);
-          const float SXY = bil(N.f(V2C_NF_SXY), mb, yn, eb, nb);
-          const float ES = bil(N.f(V2C_NF_PES), mb, yn, eb, nb);
-          const float PHIS = bil(N.f(V2C_NF_PHIS_IT), mb, yn, eb, nb);
-          const long mc = stencil_centre(g, ax, ay, uc > 0.5f, vc > 0.5f, ec, ncc);
-          const float EXX = bil(N.f(V2C_NF_EXX), mc, yn, ec, ncc);
-          const float SXX = bil(N.f(V2C_NF_SXX), mc, yn, ec, ncc);
-          const float PR = bil(N.f(V2C_NF_PR), mc, yn, ec, ncc);
-          long m3 = stencil_vx(g, ax, ay, vc < 0.5f, g.xn - 2, e, n);
-          const float VX = bil(N.f(V2C_NF_VX), m3, yn, e, n);
-          m3 = stencil_vy(g, ax, ay, uc < 0.5f, g.yn - 2, e, n);
-          const float VY = bil(N.f(V2C_NF_VY), m3, yn, e, n);
-          if (backscatter) {
-            sm.q[Q_U][k] = uc; sm.q[Q_V][k] = vc;
-            sm.q[Q_PHIS][k] = PHIS; sm.q[Q_SXY][k] = SXY; sm.q[Q_EXY][k] = EXY;
-            sm.q[Q_ES][k] = ES; sm.q[Q_PR][k] = PR; sm.q[Q_SXX][k] = SXX;
-            sm.q[Q_EXX][k] = EXX; sm.q[Q_VX][k] = VX; sm.q[Q_VY][k] = VY;
-            sm.q[Q_MRO][k] = a.R(RK_RO, t);
-          }
-          if (!owned) continue;
-          if (BS) {
-            const long s = cs + k, n = a.n;
-            a.bs[BS_U * n + s] = uc; a.bs[BS_V * n + s] = vc;
-            a.bs[BS_PHIS * n + s] = PHIS; a.bs[BS_SXY * n + s] = SXY;
-            a.bs[BS_EXY * n + s] = EXY; a.bs[BS_ES * n + s] = ES;
-            a.bs[BS_PR * n + s] = PR; a.bs[BS_SXX * n + s] = SXX;
-            a.bs[BS_EXX * n + s] = EXX;
-          }
-          // ------------------------------------- marker update (:943-1011)
-          const bool in_strict = (ix > 0 || u > 0.f) && (ix < g.ncx - 1 || u < 1.f) &&
-                                 (iy > 0 || v > 0.f) && (iy < g.ncy - 1 || v < 1.f);
-          const bool in_grid = (ix > 0 || u >= 0.f) && (ix < g.ncx - 1 || u <= 1.f) &&
-                               (iy > 0 || v >= 0.f) && (iy < g.ncy - 1 || v <= 1.f);
-          float tk = a.m.tk[idx];
-          // the marker's own values are read only without antidiffusion,
-          // where it keeps them plus the change of the node fields; with
-          // it, an updated marker takes all nine from the nodes
-          float phi = 0.f, mexx = 0.f, mexy = 0.f, msxx = 0.f, msxy = 0.f, mp = 0.f;
-          float mvx = 0.f, mvy = 0.f, me = 0.f;
-          if (PLAIN) {
-            phi = a.m.phi[idx]; mexx = a.m.exx[idx]; mexy = a.m.exy[idx];
-            msxx = a.m.sxx[idx]; msxy = a.m.sxy[idx]; mp = a.m.p[idx];
-            mvx = a.m.vx[idx]; mvy = a.m.vy[idx]; me = a.m.e[idx];
-          }
-          bool changed = false, tk_set = false;
-          if (a.do_n2m) {
-            if (in_strict && t < 50 && tk <= 0.f) {
-              if (!PLAIN) {
-                msxx = SXX; msxy = SXY; mp = PR; mexx = EXX; mexy = EXY;
-                mvx = VX; mvy = VY; phi = PHIS; me = ES;
-              } else {
-                Plain o;
-                plain_values(g, N, ax, ay, uc, vc, false, o);
-                msxx = o.sxx; msxy = o.sxy; mp = o.p; mexx = o.exx; mexy = o.exy;
-                mvx = o.vx; mvy = o.vy; phi = o.phi; me = o.e;
-              }
-              if (!P.tempmod) {
-                tk = a.S.eps2_f;
-                tk_set = true;
-              }
-              changed = true;
-            }
-            if (in_grid && t < 50 && tk > 0.f) {
-              if (!PLAIN) {
-                phi = PHIS; mexx = EXX; mexy = EXY; msxx = SXX; msxy = SXY;
-                mp = PR; mvx = VX; mvy = VY; me = ES;
-              } else {
-                Plain o;
-                plain_values(g, N, ax, ay, uc, vc, true, o);
-                phi += o.phi; mexx += o.exx; mexy += o.exy;
-                msxx += o.sxx; msxy += o.sxy; mp += o.p;
-                mvx += o.vx; mvy += o.vy; me += o.e;
-              }
-              changed = true;
-            }
-          }
-
-          if (changed) {
-            a.m.phi[idx] = phi; a.m.exx[idx] = mexx; a.m.exy[idx] = mexy;
-            a.m.sxx[idx] = msxx; a.m.sxy[idx] = msxy; a.m.p[idx] = mp;
-            a.m.vx[idx] = mvx; a.m.vy[idx] = mvy; a.m.e[idx] = me;
-            a.m.tk[idx] = tk;
-            if (tk_set) a.m.tk_lo[idx] = a.S.eps2_lo;
-          }
-        }
-        if (!backscatter) continue;
-        __syncthreads();
-        if (!jvalid) continue;
-        // quarter class starts of cell (ci, j-1) (lower) and (ci, j) (upper),
-        // read here rather than held through the staging
-        int4 ql = make_int4(0, 0, 0, 0), qu = make_int4(0, 0, 0, 0);
-        int lo_e = 0, up_e = 0;
-        float s1lo = 0.f, s1up = 0.f;
+      const int nseg_b = ci + 1 < c_end ? __ldg(a.start + cb + ncy + jlo) : 0;
+      const int nseg_e = ci + 1 < c_end ? __ldg(a.start + cb + ncy + jhi + 1) : 0;
+      // quarter class starts of cells (ci, j-1) (lower) and (ci, j) (upper)
+      int4 ql = make_int4(0, 0, 0, 0), qu = make_int4(0, 0, 0, 0);
+      int lo_e = 0, up_e = 0;
+      float s1lo = 0.f, s1up = 0.f;
+      if (warp < 6) {
         const float iwx = 1.f / __ldg(g.wx + ci);
-        if (j - 1 >= 0 && j - 1 <= ncy - 1) {
-          ql = __ldg(a.qstart + cb + j - 1); lo_e = __ldg(a.start + cb + j);
+        if (jvalid && j - 1 >= 0 && j - 1 <= ncy - 1) {
+          ql = __ldg(a.qstart + cb + j - 1);
+          lo_e = __ldg(a.start + cb + j);
           s1lo = iwx / __ldg(g.wy + j - 1);
         }
-        if (j <= ncy - 1) {
-          qu = __ldg(a.qstart + cb + j); up_e = __ldg(a.start + cb + j + 1);
+        if (jvalid && j <= ncy - 1) {
+          qu = __ldg(a.qstart + cb + j);
+          up_e = __ldg(a.start + cb + j + 1);
           s1up = iwx / __ldg(g.wy + j);
         }
-        // ---------------------------------------------- back-scatter
-        // over the quarter class runs of cell (ci, j-1) and (ci, j); the
-        // conditions inside hold for the whole run except at exact halves
-#define CLASS_RUN(b, e) \
-  for (int s = max((b), cs), s_e = min((e), ce), q = s - cs; s < s_e; ++s, q = s - cs)
-        if (role == 0) {
-          CLASS_RUN(ql.z, ql.w) {  // cell (ci, j-1), v > 1/2, u <= 1/2
-            const float u = sm.q[Q_U][q], v = sm.q[Q_V][q];
-            if (u < 0.5f) {
-              const float w = s1lo * (1.f - 2.f * u) * (2.f * v - 1.f);
-              ADD_BS(cur, q, w);
+      }
+      if (seg_b == seg_e) start_chunk(a, sm, nseg_b, min(nseg_b + CHUNK, nseg_e), tid);
+      for (int cs = seg_b; cs < seg_e; cs += CHUNK) {
+        const int ce = min(cs + CHUNK, seg_e);
+        cp_async_wait_all();
+        __syncthreads();  // indices and nodes are there, the previous chunk is summed
+        {
+          // each thread's next marker is read while the current one is gathered
+          int p = tid, i = 0, c = 0, t = 0;
+          float u = 0.f, v = 0.f, tk = 0.f;
+          auto read = [&]() {
+            if (p >= ce - cs) return;
+            i = sm.idx[p];
+            c = a.m.cell_in[i]; u = a.m.u_in[i]; v = a.m.v_in[i];
+            t = a.m.type[i]; tk = a.m.tk[i];
+          };
+          read();
+#pragma unroll 1
+          while (p < ce - cs) {
+            const int p_ = p, i_ = i, c_ = c, t_ = t;
+            const float u_ = u, v_ = v, tk_ = tk;
+            p += NTH;
+            read();
+            gather_marker(a, sm, ci, jlo, r0, i0, j0, p_, i_, c_, u_, v_, t_, tk_);
+          }
+        }
+        __syncthreads();
+        {
+          const int nb = ce == seg_e ? nseg_b : ce;
+          start_chunk(a, sm, nb, min(nb + CHUNK, ce == seg_e ? nseg_e : seg_e), tid);
+        }
+        if (warp < 2) {
+          // left halves (of node column ci), right halves (of ci+1) of cell
+          // (ci, j-1), bottom quarter, and cell (ci, j), top quarter
+          if (mine ? owned : next) {
+            const Runs R = mine ? two_runs(cs, ce, ql.z, ql.w, qu.x, qu.y)
+                                : two_runs(cs, ce, ql.w, lo_e, qu.y, qu.z);
+            const float s1 = mine ? -s1lo : s1lo, s2 = mine ? s1up : -s1up;
+            FOR_RUNS(R) {
+              const int q = slot_of(p);
+              const float2 uv = sm.q[Q_UV][q], f = sm.q[Q_PHSXY][q], h = sm.q[Q_EXYES][q];
+              const float w = (i_ < R.n1 ? s1 : s2) * fmaf(2.f, uv.x, -1.f) * fmaf(2.f, uv.y, -1.f);
+              if (w > 0.f) {
+                acc[0].add(mul_w(f.x, f.y, w));
+                acc[1].add(mul_w(h.x, h.y, w));
+                wt.add(w);
+              }
             }
           }
-          CLASS_RUN(ql.w, lo_e) {  // cell (ci, j-1), v > 1/2, u > 1/2
-            const float u = sm.q[Q_U][q], v = sm.q[Q_V][q];
-            const float w = s1lo * (2.f * u - 1.f) * (2.f * v - 1.f);
-            ADD_BS(car, q, w);
-          }
-          CLASS_RUN(qu.x, qu.y) {  // cell (ci, j), v <= 1/2, u <= 1/2
-            const float u = sm.q[Q_U][q], v = sm.q[Q_V][q];
-            if (u < 0.5f && v < 0.5f) {
-              const float w = s1up * (1.f - 2.f * u) * (1.f - 2.f * v);
-              ADD_BS(cur, q, w);
+        } else if (warp == 2) {
+          // the whole cell (ci, j) to its centre node
+          if (owned) {
+            const Runs R = two_runs(cs, ce, qu.x, up_e, 0, 0);
+#pragma unroll 1
+            for (int k = 0, p = R.p; k < R.n; ++k, ++p) {
+              const int q = slot_of(p);
+              const float2 uv = sm.q[Q_UV][q], f = sm.q[Q_PRSXX][q];
+              const float ex = sm.q[Q_EXXMRO][q].x;
+              const float w = s1up * tent(uv.x) * tent(uv.y);
+              acc[0].add(mul_w(f.x, f.y, w));
+              acc[1].add(pack2(__fmul_rn(ex, w), w));
             }
           }
-          CLASS_RUN(qu.y, qu.z) {  // cell (ci, j), v <= 1/2, u > 1/2
-            const float u = sm.q[Q_U][q], v = sm.q[Q_V][q];
-            if (v < 0.5f) {
-              const float w = s1up * (2.f * u - 1.f) * (1.f - 2.f * v);
-              ADD_BS(car, q, w);
-            }
-          }
-        } else if (role == 1) {
-          CLASS_RUN(qu.x, up_e) {  // the whole cell (ci, j) to its centre node
-            const float u = sm.q[Q_U][q], v = sm.q[Q_V][q];
-            const float w = s1up * tent(u) * tent(v);
-            cur[0].add(sm.q[Q_PR][q] * w); cur[1].add(sm.q[Q_SXX][q] * w);
-            cur[2].add(sm.q[Q_EXX][q] * w); cur[3].add(w);
-          }
-        } else if (role == 2) {
-          // vx node (ci, j) from u < 1/2 (classes 0, 2), (ci+1, j) from u > 1/2
-          CLASS_RUN(qu.x, qu.y) {
-            const float u = sm.q[Q_U][q], v = sm.q[Q_V][q];
-            if (u < 0.5f) {
-              const float mro = sm.q[Q_MRO][q];
-              const float w = s1up * (1.f - u) * (1.f - fabsf(v - 0.5f));
-              cur[0].add(sm.q[Q_VX][q] * mro * w); cur[1].add(mro * w); cur[2].add(w);
-            }
-          }
-          CLASS_RUN(qu.y, qu.z) {
-            const float u = sm.q[Q_U][q], v = sm.q[Q_V][q];
-            const float mro = sm.q[Q_MRO][q];
-            const float w = s1up * u * (1.f - fabsf(v - 0.5f));
-            car[0].add(sm.q[Q_VX][q] * mro * w); car[1].add(mro * w); car[2].add(w);
-          }
-          CLASS_RUN(qu.z, qu.w) {
-            const float u = sm.q[Q_U][q], v = sm.q[Q_V][q];
-            if (u < 0.5f) {
-              const float mro = sm.q[Q_MRO][q];
-              const float w = s1up * (1.f - u) * (1.f - fabsf(v - 0.5f));
-              cur[0].add(sm.q[Q_VX][q] * mro * w); cur[1].add(mro * w); cur[2].add(w);
-            }
-          }
-          CLASS_RUN(qu.w, up_e) {
-            const float u = sm.q[Q_U][q], v = sm.q[Q_V][q];
-            const float mro = sm.q[Q_MRO][q];
-            const float w = s1up * u * (1.f - fabsf(v - 0.5f));
-            car[0].add(sm.q[Q_VX][q] * mro * w); car[1].add(mro * w); car[2].add(w);
-          }
-        } else {
+        } else if (warp == 3) {
           // vy node (ci, j) from v > 1/2 of cell (ci, j-1) (classes 2, 3) and
           // v < 1/2 of cell (ci, j) (classes 0, 1)
-          CLASS_RUN(ql.z, lo_e) {
-            const float u = sm.q[Q_U][q], v = sm.q[Q_V][q];
-            const float mro = sm.q[Q_MRO][q];
-            const float w = s1lo * (1.f - fabsf(u - 0.5f)) * v;
-            cur[0].add(sm.q[Q_VY][q] * mro * w); cur[1].add(mro * w); cur[2].add(w);
+          if (owned) {
+            const Runs R = two_runs(cs, ce, ql.z, lo_e, qu.x, qu.z);
+            FOR_RUNS(R) {
+              const int q = slot_of(p);
+              const float2 uv = sm.q[Q_UV][q];
+              const float vy = sm.q[Q_VXVY][q].y, mro = sm.q[Q_EXXMRO][q].y;
+              const bool lo = i_ < R.n1;
+              if (lo || uv.y < 0.5f) {
+                const float w = (lo ? s1lo : s1up) * (1.f - fabsf(uv.x - 0.5f)) *
+                                (lo ? uv.y : 1.f - uv.y);
+                acc[0].add(mul_w(__fmul_rn(vy, mro), mro, w));
+                wt.add(w);
+              }
+            }
           }
-          CLASS_RUN(qu.x, qu.z) {
-            const float u = sm.q[Q_U][q], v = sm.q[Q_V][q];
-            if (v < 0.5f) {
-              const float mro = sm.q[Q_MRO][q];
-              const float w = s1up * (1.f - fabsf(u - 0.5f)) * (1.f - v);
-              cur[0].add(sm.q[Q_VY][q] * mro * w); cur[1].add(mro * w); cur[2].add(w);
+        } else if (warp == 4 || warp == 5) {
+          // vx node (ci, j) from u < 1/2 (classes 0, 2), (ci+1, j) from
+          // u > 1/2 (classes 1, 3)
+          if (mine ? owned : next) {
+            const Runs R = mine ? two_runs(cs, ce, qu.x, qu.y, qu.z, qu.w)
+                                : two_runs(cs, ce, qu.y, qu.z, qu.w, up_e);
+            FOR_RUNS(R) {
+              const int q = slot_of(p);
+              const float2 uv = sm.q[Q_UV][q];
+              const float vx = sm.q[Q_VXVY][q].x, mro = sm.q[Q_EXXMRO][q].y;
+              if (!mine || uv.x < 0.5f) {
+                const float w = s1up * (mine ? 1.f - uv.x : uv.x) * (1.f - fabsf(uv.y - 0.5f));
+                acc[0].add(mul_w(__fmul_rn(vx, mro), mro, w));
+                wt.add(w);
+              }
             }
           }
         }
-#undef CLASS_RUN
+      }
+      // for the next column: its weights and the node column it adds
+      if (ci + 1 < c_end) {
+        if (warp == 7 && jl < S_N)
+          axis_side(g.wx, g.ncx, g.xn, ci + 1, jl, true, sm.x[(ci + 1) & 1][jl]);
+        load_column(a, sm, ci + 3, r0, tid);
       }
     }
 
     // ----------------------------------------------- sums and normalisation
-    if (!backscatter || ci < i0 || !jvalid) continue;
-    const long m3 = (long)ci * yn + j;
-    if (role == 0) {
-      const float w = cur[4].value();
-      const float ph = cur[0].value(), sy = cur[1].value(), ey = cur[2].value(), es = cur[3].value();
-      N.f(V2C_NF_PHISUM)[m3] = ph; N.f(V2C_NF_SXYSUM)[m3] = sy;
-      N.f(V2C_NF_EXYSUM)[m3] = ey; N.f(V2C_NF_ESUM)[m3] = es; N.f(V2C_NF_WTPHISUM)[m3] = w;
-      if (w != 0.f && ci >= 1 && j >= 1 && ci < g.xn - 1 && j < g.yn - 1) {
-        N.f(V2C_NF_PHIE)[m3] = __fdividef(ph, w); N.f(V2C_NF_SXYEE)[m3] = __fdividef(sy, w);
-        N.f(V2C_NF_EXYEE)[m3] = __fdividef(ey, w); N.f(V2C_NF_PEE)[m3] = __fdividef(es, w);
-      }
-    } else if (role == 1) {
-      if (ci < g.ncx && j < ncy) {
-        const long mc = (long)(ci + 1) * yn + (j + 1);
-        const float w = cur[3].value();
-        const float ps = cur[0].value(), sx = cur[1].value(), ex = cur[2].value();
-        N.f(V2C_NF_PSUM)[mc] = ps; N.f(V2C_NF_SXXSUM)[mc] = sx;
-        N.f(V2C_NF_EXXSUM)[mc] = ex; N.f(V2C_NF_WTSXXSUM)[mc] = w;
-        if (w != 0.f) {
-          N.f(V2C_NF_SPPEE)[mc] = __fdividef(ps, w); N.f(V2C_NF_SXXEE)[mc] = __fdividef(sx, w);
-          N.f(V2C_NF_EXXEE)[mc] = __fdividef(ex, w);
+    if ((warp < 2 || warp >= 4) && !mine) continue;
+    if (owned && jvalid && warp < 6) {
+      const long m3 = (long)ci * g.yn + j;
+      Acc x, y, z, w;
+      acc[0].split(x, y);
+      if (warp < 2) {
+        acc[1].split(z, w);
+        const float ph = x.value(), sy = y.value(), ey = z.value(), es = w.value();
+        const float sw = wt.value();
+        N.f(V2C_NF_PHISUM)[m3] = ph; N.f(V2C_NF_SXYSUM)[m3] = sy;
+        N.f(V2C_NF_EXYSUM)[m3] = ey; N.f(V2C_NF_ESUM)[m3] = es; N.f(V2C_NF_WTPHISUM)[m3] = sw;
+        if (sw != 0.f && ci >= 1 && j >= 1 && ci < g.xn - 1 && j < g.yn - 1) {
+          N.f(V2C_NF_PHIE)[m3] = __fdividef(ph, sw); N.f(V2C_NF_SXYEE)[m3] = __fdividef(sy, sw);
+          N.f(V2C_NF_EXYEE)[m3] = __fdividef(ey, sw); N.f(V2C_NF_PEE)[m3] = __fdividef(es, sw);
         }
+      } else if (warp == 2) {
+        acc[1].split(z, w);
+        if (ci < g.ncx && j < ncy) {
+          const long mc = m3 + g.yn + 1;
+          const float ps = x.value(), sx = y.value(), ex = z.value(), sw = w.value();
+          N.f(V2C_NF_PSUM)[mc] = ps; N.f(V2C_NF_SXXSUM)[mc] = sx;
+          N.f(V2C_NF_EXXSUM)[mc] = ex; N.f(V2C_NF_WTSXXSUM)[mc] = sw;
+          if (sw != 0.f) {
+            N.f(V2C_NF_SPPEE)[mc] = __fdividef(ps, sw); N.f(V2C_NF_SXXEE)[mc] = __fdividef(sx, sw);
+            N.f(V2C_NF_EXXEE)[mc] = __fdividef(ex, sw);
+          }
+        }
+        if (ci == 0 || j == 0) {
+          N.f(V2C_NF_PSUM)[m3] = 0; N.f(V2C_NF_SXXSUM)[m3] = 0;
+          N.f(V2C_NF_EXXSUM)[m3] = 0; N.f(V2C_NF_WTSXXSUM)[m3] = 0;
+        }
+      } else {
+        const bool X = warp != 3;
+        const float vs = x.value(), mr = y.value(), sw = wt.value();
+        N.f(X ? V2C_NF_VXSUM : V2C_NF_VYSUM)[m3] = vs;
+        N.f(X ? V2C_NF_MRX0 : V2C_NF_MRY0)[m3] = mr;
+        N.f(X ? V2C_NF_WTVXSUM : V2C_NF_WTVYSUM)[m3] = sw;
+        if (sw != 0.f) N.f(X ? V2C_NF_MVXE : V2C_NF_MVYE)[m3] = __fdividef(vs, mr);
       }
-      if (ci == 0 || j == 0) {
-        N.f(V2C_NF_PSUM)[m3] = 0; N.f(V2C_NF_SXXSUM)[m3] = 0;
-        N.f(V2C_NF_EXXSUM)[m3] = 0; N.f(V2C_NF_WTSXXSUM)[m3] = 0;
-      }
-    } else if (role == 2) {
-      const float w = cur[2].value(), vs = cur[0].value(), mr = cur[1].value();
-      N.f(V2C_NF_VXSUM)[m3] = vs; N.f(V2C_NF_MRX0)[m3] = mr; N.f(V2C_NF_WTVXSUM)[m3] = w;
-      if (w != 0.f) N.f(V2C_NF_MVXE)[m3] = __fdividef(vs, mr);
-    } else {
-      const float w = cur[2].value(), vs = cur[0].value(), mr = cur[1].value();
-      N.f(V2C_NF_VYSUM)[m3] = vs; N.f(V2C_NF_MRY0)[m3] = mr; N.f(V2C_NF_WTVYSUM)[m3] = w;
-      if (w != 0.f) N.f(V2C_NF_MVYE)[m3] = __fdividef(vs, mr);
     }
+    acc[0].zero(); acc[1].zero(); wt.zero();
+  }
+}
+
+// ------------------------------------------------- gather without a sweep
+// nodes2markers where no tile sums are formed: PLAIN, no antidiffusion (no
+// back-scatter); BS, interpolationmod 1 (each marker's back-scatter payload
+// goes to a.bs for the per-node kernel below).  One thread per marker, in
+// sorted order; bound by the latency of its node reads, so 6 resident CTAs
+// (811 x 309 lines, 4.5 M markers, PLAIN: 215 us, 235 at the registers the
+// compiler takes by itself, 288 at 4 CTAs; BS, 433 x 187 lines: 121 -> 100
+// us against the chunked sweep).
+template <bool BS, bool PLAIN>
+__global__ void __launch_bounds__(256, 6) k_gather(N2MArgs a) {
+  const Grid &g = a.g;
+  const Nodes &N = a.N;
+  const int ncy = g.ncy;
+  const v2c_params &P = a.S.p;
+  const long yn = g.yn;
+  const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (s >= a.n) return;
+  const int idx = __ldg(a.perm + s);
+  const int c = a.m.cell_in[idx];
+  const int ix = c / ncy, iy = c - ix * ncy;
+  const float u = a.m.u_in[idx], v = a.m.v_in[idx];
+  const int t = a.m.type[idx];
+  // interpolate_mechanical clamps the point into the model first
+  float uc = u, vc = v;
+  if (ix == 0 && uc < 0.f) uc = 0.f;
+  if (ix == g.ncx - 1 && uc > 1.f) uc = 1.f;
+  if (iy == 0 && vc < 0.f) vc = 0.f;
+  if (iy == g.ncy - 1 && vc > 1.f) vc = 1.f;
+  const float wxc = __ldg(g.wx + ix), wyc = __ldg(g.wy + iy);
+  const Axis ax = make_axis(g.wx, g.ncx, ix, uc * wxc);
+  const Axis ay = make_axis(g.wy, g.ncy, iy, vc * wyc);
+  float EXY = 0.f, SXY = 0.f, ES = 0.f, PHIS = 0.f, EXX = 0.f, SXX = 0.f, PR = 0.f;
+  float VX = 0.f, VY = 0.f;
+  if (!PLAIN) {
+    float eb, nb, ec, ncc, e, n;
+    const long mb = stencil_basic(g, ax, ay, eb, nb);
+    EXY = bil(N.f(V2C_NF_EXY), mb, yn, eb, nb);
+    SXY = bil(N.f(V2C_NF_SXY), mb, yn, eb, nb);
+    ES = bil(N.f(V2C_NF_PES), mb, yn, eb, nb);
+    PHIS = bil(N.f(V2C_NF_PHIS_IT), mb, yn, eb, nb);
+    const long mc = stencil_centre(g, ax, ay, uc > 0.5f, vc > 0.5f, ec, ncc);
+    EXX = bil(N.f(V2C_NF_EXX), mc, yn, ec, ncc);
+    SXX = bil(N.f(V2C_NF_SXX), mc, yn, ec, ncc);
+    PR = bil(N.f(V2C_NF_PR), mc, yn, ec, ncc);
+    long m3 = stencil_vx(g, ax, ay, vc < 0.5f, g.xn - 2, e, n);
+    VX = bil(N.f(V2C_NF_VX), m3, yn, e, n);
+    m3 = stencil_vy(g, ax, ay, uc < 0.5f, g.yn - 2, e, n);
+    VY = bil(N.f(V2C_NF_VY), m3, yn, e, n);
+  }
+  if (BS) {
+    const long n = a.n;
+    a.bs[BS_U * n + s] = uc; a.bs[BS_V * n + s] = vc;
+    a.bs[BS_PHIS * n + s] = PHIS; a.bs[BS_SXY * n + s] = SXY;
+    a.bs[BS_EXY * n + s] = EXY; a.bs[BS_ES * n + s] = ES;
+    a.bs[BS_PR * n + s] = PR; a.bs[BS_SXX * n + s] = SXX;
+    a.bs[BS_EXX * n + s] = EXX;
+  }
+  // ------------------------------------- marker update (:943-1011)
+  if (t >= 50) return;
+  const bool in_strict = (ix > 0 || u > 0.f) && (ix < g.ncx - 1 || u < 1.f) &&
+                         (iy > 0 || v > 0.f) && (iy < g.ncy - 1 || v < 1.f);
+  const bool in_grid = (ix > 0 || u >= 0.f) && (ix < g.ncx - 1 || u <= 1.f) &&
+                       (iy > 0 || v >= 0.f) && (iy < g.ncy - 1 || v <= 1.f);
+  float tk = a.m.tk[idx];
+  // PLAIN: the marker's own values plus the change of the node fields; with
+  // antidiffusion an updated marker takes all nine from the nodes
+  float phi = PHIS, mexx = EXX, mexy = EXY, msxx = SXX, msxy = SXY, mp = PR, mvx = VX, mvy = VY;
+  float me = ES;
+  if (PLAIN) {
+    phi = a.m.phi[idx]; mexx = a.m.exx[idx]; mexy = a.m.exy[idx];
+    msxx = a.m.sxx[idx]; msxy = a.m.sxy[idx]; mp = a.m.p[idx];
+    mvx = a.m.vx[idx]; mvy = a.m.vy[idx]; me = a.m.e[idx];
+  }
+  bool changed = false;
+  if (in_strict && tk <= 0.f) {
+    if (PLAIN) {
+      Plain o;
+      plain_values(g, N, ax, ay, uc, vc, false, o);
+      msxx = o.sxx; msxy = o.sxy; mp = o.p; mexx = o.exx; mexy = o.exy;
+      mvx = o.vx; mvy = o.vy; phi = o.phi; me = o.e;
+    }
+    if (!P.tempmod) {
+      tk = a.S.eps2_f;
+      a.m.tk[idx] = tk;
+      a.m.tk_lo[idx] = a.S.eps2_lo;
+    }
+    changed = true;
+  }
+  if (in_grid && tk > 0.f) {
+    if (PLAIN) {
+      Plain o;
+      plain_values(g, N, ax, ay, uc, vc, true, o);
+      phi += o.phi; mexx += o.exx; mexy += o.exy;
+      msxx += o.sxx; msxy += o.sxy; mp += o.p;
+      mvx += o.vx; mvy += o.vy; me += o.e;
+    }
+    changed = true;
+  }
+  if (changed) {
+    a.m.phi[idx] = phi; a.m.exx[idx] = mexx; a.m.exy[idx] = mexy;
+    a.m.sxx[idx] = msxx; a.m.sxy[idx] = msxy; a.m.p[idx] = mp;
+    a.m.vx[idx] = mvx; a.m.vy[idx] = mvy; a.m.e[idx] = me;
   }
 }
 
@@ -554,7 +770,7 @@ __device__ __forceinline__ float bs_half(int k, float f) {
 }
 
 template <int ROLE>
-__global__ void __launch_bounds__(128) k_n2m_bs_mode1(N2MArgs a) {
+__device__ __forceinline__ void bs_mode1(const N2MArgs &a) {
   const Grid &g = a.g;
   const Nodes &N = a.N;
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -614,6 +830,12 @@ __global__ void __launch_bounds__(128) k_n2m_bs_mode1(N2MArgs a) {
       N.f(V2C_NF_EXXEE)[t] = __fdividef(ex, w);
     }
   }
+}
+
+// both node kinds in one launch, a row of blocks each
+__global__ void __launch_bounds__(128) k_n2m_bs_mode1(N2MArgs a) {
+  if (blockIdx.y == 0) bs_mode1<1>(a);
+  else bs_mode1<0>(a);
 }
 
 // ----------------------------------------------------------- the move
@@ -783,17 +1005,23 @@ __global__ void __launch_bounds__(256) k_move(N2MArgs a) {
 
 }  // namespace
 
+cudaError_t n2m_init() {
+  return cudaFuncSetAttribute(k_n2m, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sizeof(Smem));
+}
+
 void launch_n2m(const N2MArgs &a, cudaStream_t st) {
-  dim3 grid((a.g.xn + a.TX - 1) / a.TX, (a.g.yn + TY - 1) / TY);
-  if (!a.bs) {
-    // PLAIN: the markers take the node fields without antidiffusion
-    if (a.S.p.antidiffinter == 1) k_n2m<false, false><<<grid, NTH, 0, st>>>(a);
-    else k_n2m<false, true><<<grid, NTH, 0, st>>>(a);
-  } else {
-    k_n2m<true, false><<<grid, NTH, 0, st>>>(a);
+  const unsigned mb = (unsigned)((a.n + 255) / 256);
+  if (a.bs) {
+    if (a.n > 0) k_gather<true, false><<<mb, 256, 0, st>>>(a);
     const unsigned nb = (unsigned)((a.g.nn + 127) / 128);
-    k_n2m_bs_mode1<0><<<nb, 128, 0, st>>>(a);
-    k_n2m_bs_mode1<1><<<nb, 128, 0, st>>>(a);
+    k_n2m_bs_mode1<<<dim3(nb, 2), 128, 0, st>>>(a);
+  } else if (a.S.p.antidiffinter == 1) {
+    dim3 grid((a.g.xn + a.TX - 1) / a.TX, (a.g.yn + TY - 1) / TY);
+    k_n2m<<<grid, NTH, sizeof(Smem), st>>>(a);
+  } else if (a.n > 0) {
+    // the markers take the node fields without antidiffusion
+    k_gather<false, true><<<mb, 256, 0, st>>>(a);
   }
 }
 
