@@ -51,6 +51,7 @@ struct v2c_ctx {
   float *d_tol = nullptr;                    // temperature update: node scratch
   float *d_bs = nullptr;                     // interpolationmod 1 back-scatter payload
   unsigned *d_list_n = nullptr;              // count of listed Newton problems
+  char *d_rsfk = nullptr;                    // constants the Newton problems share
   double *d_ts = nullptr;                    // calc_timestep scratch
   // markers
   Markers m{};
@@ -310,6 +311,7 @@ extern "C" int v2c_create(const v2c_params *p, long max_markers, void *cuda_stre
   AL(ctx->d_tol, ctx->nn);
   if (p->interpolationmod == 1) AL(ctx->d_bs, (size_t)BS_N * (ctx->cap > 0 ? ctx->cap : 1));
   AL(ctx->d_list_n, 1);
+  AL(ctx->d_rsfk, rsf_const_bytes());
   AL(ctx->d_ts, TIMESTEP_SCRATCH);
   AL(ctx->d_stat, ST_N);
   ctx->red_cap = 2 + 2 * ((ctx->nn + 255) / 256);
@@ -369,7 +371,7 @@ extern "C" int v2c_destroy(v2c_ctx *ctx) {
   if (ctx->d_slip) cudaFree(ctx->d_slip);
   if (ctx->d_mslip) cudaFree(ctx->d_mslip);
   void *ptrs[] = {ctx->d_gx, ctx->d_gy, ctx->d_wx, ctx->d_wy, ctx->d_gxf, ctx->d_gyf,
-                  ctx->d_rock, ctx->d_node, ctx->d_node64, ctx->d_sticky, ctx->d_quad, ctx->d_tol, ctx->d_list_n, ctx->d_ts,
+                  ctx->d_rock, ctx->d_node, ctx->d_node64, ctx->d_sticky, ctx->d_quad, ctx->d_tol, ctx->d_list_n, ctx->d_rsfk, ctx->d_ts,
                   ctx->d_stat, ctx->d_red, ctx->d_nstage,
                   ctx->sb.counts, ctx->sb.start, ctx->sb.qstart, ctx->sb.slot, ctx->sb.tmp, ctx->sb.perm,
                   ctx->sb.blocksum, ctx->d_stage64, ctx->d_stage64b, ctx->bc_mem,
@@ -994,10 +996,11 @@ extern "C" int v2c_marker2nodes(v2c_ctx *ctx) {
     // between sorts (capacity: one entry per marker)
     ph.list = ctx->sb.slot;
     ph.list_n = ctx->d_list_n;
+    ph.rk = reinterpret_cast<RsfConst *>(ctx->d_rsfk);
     ph.guess = reinterpret_cast<float *>(ctx->sb.tmp);  // likewise free between sorts
     Prof pr(ctx, ctx->p.newton_guess == V2C_GUESS_OFF ? V2C_PROF_PHYS : V2C_PROF_NEWTON);
     launch_phys(ph, st);
-    ctx->launches += ctx->p.newton_guess == V2C_GUESS_OFF ? 1 : (ph.mlp && ctx->p.newton_guess == V2C_GUESS_LEARNED ? 3 : 2);
+    ctx->launches += ctx->p.newton_guess == V2C_GUESS_OFF ? 1 : (ph.mlp && ctx->p.newton_guess == V2C_GUESS_LEARNED ? 4 : 3);
   }
   {
     Prof pr(ctx, V2C_PROF_M2N);

@@ -24,6 +24,8 @@
 #pragma once
 #include <math.h>
 
+#include "v2c_f32x2.cuh"
+
 namespace v2c {
 
 struct ff {
@@ -55,10 +57,16 @@ __device__ __forceinline__ float two_prod(float a, float b, float &e) {
   return p;
 }
 
+// The two-sums of the high and of the low words are one packed two-sum (6
+// instructions for both instead of 12; a pair's two words are a register
+// pair already).
 __device__ __forceinline__ ff ff_add(ff a, ff b) {
-  float s2, t2;
-  float s1 = two_sum(a.hi, b.hi, s2);
-  const float t1 = two_sum(a.lo, b.lo, t2);
+  const f32x2 x = pack2(a.hi, a.lo), y = pack2(b.hi, b.lo);
+  const f32x2 s = add2(x, y), yy = sub2(s, x);
+  const f32x2 e = add2(sub2(x, sub2(s, yy)), sub2(y, yy));
+  float s1, t1, s2, t2;
+  unpack2(s, s1, t1);
+  unpack2(e, s2, t2);
   s2 = __fadd_rn(s2, t1);
   s1 = fast_two_sum(s1, s2, s2);
   s2 = __fadd_rn(s2, t2);

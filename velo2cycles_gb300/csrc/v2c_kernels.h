@@ -75,6 +75,8 @@ struct M2NArgs {
 cudaError_t m2n_init();
 void launch_m2n(const M2NArgs &a, cudaStream_t st);
 
+struct RsfConst;
+size_t rsf_const_bytes();
 // per-marker physics (+ optional RSF Newton), marker array order
 struct PhysArgs {
   Grid g;
@@ -96,6 +98,7 @@ struct PhysArgs {
   // marker indices (capacity n) and their count (device)
   int32_t *list = nullptr;
   unsigned *list_n = nullptr;
+  RsfConst *rk = nullptr;  // constants the Newton problems share (v2c_rsf.cuh; scratch)
   float *guess = nullptr;  // the network's start per listed problem (capacity n)
 };
 void launch_phys(const PhysArgs &a, cudaStream_t st);

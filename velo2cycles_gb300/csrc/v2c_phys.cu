@@ -46,18 +46,19 @@ __device__ __forceinline__ void warp_max_bits(unsigned long long *p, unsigned lo
 enum { PHYS_OFF = 0, PHYS_SPLIT, PHYS_FP64, PHYS_COLLECT };
 
 // Friction parameters of a marker (calc_frictionpara, calc_RSF.c:224-295)
-// and its new state: FP32 position away from the band, FP64 near it.
+// and its new state: FP32 position away from the band (far), FP64 near it.
 __device__ __forceinline__ float marker_friction(const PhysArgs &a, int ix, int iy, float u,
                                                  float v, float Xc, float Yc, int t, float phi,
-                                                 Fric &fr) {
+                                                 Fric &fr, bool &far) {
   const Grid &g = a.g;
   const v2c_params &P = a.S.p;
   const Scal &S = a.S;
   const float xf = __ldg(a.gxf + ix) + Xc, yf = __ldg(a.gyf + iy) + Yc;
   const float rad = fabsf(yf - (S.fault_y_f + S.fault_slope_f * xf));
-  if (t > 0 && rad > S.fault_hw1_f) {
+  far = t > 0 && rad > S.fault_hw1_f;
+  if (far) {
     fr.a = S.a_hr_f; fr.b = S.b_hr_f; fr.L = S.L_hr_f; fr.V0 = S.V0_hr_f; fr.mu0 = 0.6f;
-    return 50.f;
+    return RSF_FAR_STATE;
   }
   const double x = g.gx[ix] + (double)u * (g.gx[ix + 1] - g.gx[ix]);
   const double y = g.gy[iy] + (double)v * (g.gy[iy + 1] - g.gy[iy]);
@@ -68,17 +69,18 @@ __device__ __forceinline__ float marker_friction(const PhysArgs &a, int ix, int 
 // its viscosity and state
 __device__ __forceinline__ void marker_problem(const PhysArgs &a, long i, const ff &dt_ff,
                                                const ff &W_ff, const ff &sn_ff, RsfIn &in,
-                                               float &uplain) {
+                                               float &uplain, int &t, bool &far) {
   const Grid &g = a.g;
   const v2c_params &P = a.S.p;
   const int c = a.m.cell_in[i];
   const int ix = c / g.ncy, iy = c - ix * g.ncy;
   const float u = a.m.u_in[i], v = a.m.v_in[i];
-  const int t = a.m.type[i];
+  t = a.m.type[i];
   Fric fr{0.f, 0.f, 1.f, 1.f, 0.f};
   const float phi = a.m.phi[i];
   (void)marker_friction(a, ix, iy, u, v, u * __ldg(g.wx + ix), v * __ldg(g.wy + iy), t, phi,
-                        fr);
+                        fr, far);
+  far = far && phi == RSF_FAR_STATE;
   const float sxx = a.m.sxx[i], sxy = a.m.sxy[i], exx = a.m.exx[i], exy = a.m.exy[i];
   in.a = ff_f(fr.a); in.b = ff_f(fr.b); in.L = ff_f(fr.L); in.V0 = ff_f(fr.V0);
   in.mu0 = ff_f(fr.mu0);
@@ -93,8 +95,11 @@ __device__ __forceinline__ void marker_problem(const PhysArgs &a, long i, const 
   uplain = (vold > 0.f) ? __logf(vold) : -30.f;
 }
 
+// Bound by instruction issue (110 warp instructions per marker at dt = 1e8 s,
+// 74-80 % issue active, FMA pipe half busy).  8 CTAs per SM (61 registers):
+// C4 physics + Newton 8.30 ms at 7, 7.98 at 8, 8.11 at 10 (spills).
 template <int MODE>
-__global__ void __launch_bounds__(PT, 5) k_phys(PhysArgs a) {
+__global__ void __launch_bounds__(PT, 8) k_phys(PhysArgs a) {
   const Grid &g = a.g;
   const bool collect = MODE == PHYS_COLLECT;
   const bool newton = MODE == PHYS_SPLIT || MODE == PHYS_FP64;
@@ -110,6 +115,7 @@ __global__ void __launch_bounds__(PT, 5) k_phys(PhysArgs a) {
     bool solve = false;
     float mnu = 0.f, sigin = 0.f, phi = 0.f;
     int t = 0;
+    bool far = false;
     Fric fr{0.f, 0.f, 1.f, 1.f, 0.f};
     if (valid) {
       const int c = a.m.cell_in[i];
@@ -153,7 +159,7 @@ __global__ void __launch_bounds__(PT, 5) k_phys(PhysArgs a) {
         const ff sig2 = ff_add(ff_mul(ff_f(sxx), ff_f(sxx)), ff_mul(ff_f(sxy), ff_f(sxy)));
         mnu = ductile_visc32(a.R, a.S, t, sig2, T, a.m.tk_lo[i], mpb_ff);
         const float phi0 = a.m.phi[i];
-        phi = marker_friction(a, ix, iy, u, v, ax.X, ay.X, t, phi0, fr);
+        phi = marker_friction(a, ix, iy, u, v, ax.X, ay.X, t, phi0, fr, far);
         if (!collect) {
           if (phi != phi0) a.m.phi[i] = phi;
           a.m.mnu[i] = mnu;
@@ -202,7 +208,7 @@ __global__ void __launch_bounds__(PT, 5) k_phys(PhysArgs a) {
       in.edot = ff_f(sqrtf(exx * exx + exy * exy)); in.eta = ff_f(mnu);
       in.G = ff_f(a.R(RK_GG, t));
       float A_floor;
-      if (rsf_floor_certain(rsf32_of(in), A_floor)) {
+      if (rsf_floor_certain(rsf32_of(in, a.rk, far), A_floor)) {
         a.m.slipv[i] = 1e-40f;
         it += 1;
         need = false;
@@ -236,10 +242,11 @@ __global__ void __launch_bounds__(PT, 4) k_guess(PhysArgs a, float *guess) {
     const bool valid = e < cnt;
     RsfIn in;
     float uplain = 0.f, rp = 0.f, up = 0.f;
-    bool need = false;
+    bool need = false, far = false;
+    int t = 0;
     if (valid) {
-      marker_problem(a, a.list[e], dt_ff, W_ff, sn_ff, in, uplain);
-      rp = rsf_start_residual(rsf32_of(in), uplain, up);
+      marker_problem(a, a.list[e], dt_ff, W_ff, sn_ff, in, uplain, t, far);
+      rp = rsf_start_residual(rsf32_of(in, a.rk, far), uplain, up);
       need = !(rp <= RSF_NET_MIN_RES);
     }
     float u0 = uplain;
@@ -251,19 +258,38 @@ __global__ void __launch_bounds__(PT, 4) k_guess(PhysArgs a, float *guess) {
       __syncwarp();
       mlp_warp_forward(S, wl);
       float un;
-      if (need && rsf_start_residual(rsf32_of(in), S.yout[wl][lane][0], un) < rp) u0 = un;
+      if (need && rsf_start_residual(rsf32_of(in, a.rk, far), S.yout[wl][lane][0], un) < rp) u0 = un;
       __syncwarp();
     }
     if (valid) guess[e] = u0;
   }
 }
 
+// The FP64 Newton of marker i from u, for the split solve's rare fallback:
+// the problem is read again, so that the solve need not keep it.
+static __device__ __noinline__ void marker_finish64(const PhysArgs &a, long i, double u,
+                                                    RsfResult &r) {
+  const v2c_params &P = a.S.p;
+  const ff dt_ff{a.S.dt_hi, a.S.dt_lo}, W_ff{a.S.W_hi, a.S.W_lo}, sn_ff{a.S.sn_hi, a.S.sn_lo};
+  RsfIn in;
+  float uplain;
+  int t;
+  bool far;
+  marker_problem(a, i, dt_ff, W_ff, sn_ff, in, uplain, t, far);
+  rsf_finish64(in, u, P.newton_rtol, P.newton_maxit, r);
+}
+
 // The listed Newton problems, 32 per warp, densely: the split or FP64 solve
 // from the plain start or (LEARNED) the network's guess[e], restarting from
 // the plain start when that does not converge.  The list order comes from
 // integer atomics; each problem's result depends only on its own inputs.
+// Bound by instruction issue and fetch (some 2000 float-pair instructions per
+// problem).  The constants shared by all far-field markers (RsfConst) took
+// the refined 1001 x 401-line model's 6.4 M problems from 788 to about 540
+// us; one copy of the solve and 8 CTAs per SM the C4 list's share of the
+// stage from 7.77 to 7.63 ms.
 template <bool FP64, bool LEARNED>
-__global__ void __launch_bounds__(PT, 5) k_newton(PhysArgs a, const float *guess) {
+__global__ void __launch_bounds__(PT, 8) k_newton(PhysArgs a, const float *guess) {
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const long nwarps = (long)gridDim.x * (PT / 32);
   const long cnt = *a.list_n;
@@ -276,17 +302,25 @@ __global__ void __launch_bounds__(PT, 5) k_newton(PhysArgs a, const float *guess
     const long i = a.list[e];
     RsfIn in;
     float uplain;
-    marker_problem(a, i, dt_ff, W_ff, sn_ff, in, uplain);
+    int t;
+    bool far;
+    marker_problem(a, i, dt_ff, W_ff, sn_ff, in, uplain, t, far);
     const float u0 = LEARNED ? guess[e] : uplain;
-    RsfResult r = FP64 ? rsf_solve64(in, (double)u0, P.newton_rtol, P.newton_maxit)
-                       : rsf_solve_split(in, rsf32_of(in), u0, P.newton_rtol, P.newton_maxit);
-    it += r.it32 + r.itff + r.it64;
-    if (!r.ok && LEARNED && u0 != uplain) {
-      RsfResult r2 = FP64 ? rsf_solve64(in, (double)uplain, P.newton_rtol, P.newton_maxit)
-                          : rsf_solve_split(in, rsf32_of(in), uplain, P.newton_rtol, P.newton_maxit);
-      it += r2.it32 + r2.itff + r2.it64;
+    auto solve = [&](float start) {
+      if (FP64) return rsf_solve64(in, (double)start, P.newton_rtol, P.newton_maxit);
+      return rsf_solve_split(in, rsf32_of(in, a.rk, far), start, P.newton_rtol, P.newton_maxit,
+                             [&](RsfFF &q) { rsf_setup_marker(q, in, *a.rk, t, far); },
+                             [&](double u, RsfResult &r) { marker_finish64(a, i, u, r); });
+    };
+    RsfResult r;
+    float start = u0;
+#pragma unroll 1
+    for (;;) {  // one copy of the solve for both starts
+      r = solve(start);
+      it += r.it32 + r.itff + r.it64;
+      if (r.ok || !LEARNED || start == uplain) break;
       fb += 1;
-      r = r2;
+      start = uplain;
     }
     if (!r.ok) nc += 1;
     a.m.slipv[i] = r.Vf;
@@ -301,6 +335,21 @@ __global__ void __launch_bounds__(PT, 5) k_newton(PhysArgs a, const float *guess
   warp_add(a.stat + ST_NEWTON_NONCONV, nc);
 }
 
+// the call's shared Newton constants; empties the problem list
+__global__ void k_rsf_const(Rock R, Scal S, RsfConst *k, unsigned *list_n) {
+  const int t = threadIdx.x;
+  if (t == 0) {
+    RsfIn in;
+    in.a = ff_f(S.a_hr_f); in.b = ff_f(S.b_hr_f); in.L = ff_f(S.L_hr_f); in.V0 = ff_f(S.V0_hr_f);
+    in.mu0 = ff_f(0.6f); in.sn = ff{S.sn_hi, S.sn_lo}; in.dt = ff{S.dt_hi, S.dt_lo};
+    in.W = ff{S.W_hi, S.W_lo}; in.phio = ff_f(RSF_FAR_STATE);
+    in.tau_old = in.edot = ff_f(0.f); in.eta = in.G = ff_f(1.f);
+    rsf_const_far(*k, in);
+    *list_n = 0;
+  }
+  rsf_const_type(*k, t, ff_f(R(RK_GG, t)), ff{S.dt_hi, S.dt_lo}, ff{S.W_hi, S.W_lo});
+}
+
 // resident blocks of a kernel on the whole GPU (grid-stride launches)
 template <class K>
 unsigned resident_grid(K kernel, int threads) {
@@ -313,11 +362,14 @@ unsigned resident_grid(K kernel, int threads) {
 
 }  // namespace
 
+size_t rsf_const_bytes() { return sizeof(RsfConst); }
+
 void launch_phys(const PhysArgs &a, cudaStream_t st) {
   if (a.n <= 0) return;
-  long warps = (a.n + 31) / 32;
-  long blocks = (warps + PT / 32 - 1) / (PT / 32);
-  if (blocks > 152 * 16) blocks = 152 * 16;
+  // one pass of 32 markers per warp: the blocks' times differ with the creep
+  // iterations of their markers, and many short blocks fill the SMs to the
+  // end where 16 long ones per SM left the last wave a third empty
+  const long blocks = (a.n + PT - 1) / PT;
   const v2c_params &p = a.S.p;
   const bool learned = p.newton_guess == V2C_GUESS_LEARNED && a.mlp != nullptr;
   const bool fp64 = p.newton_precision == V2C_NEWTON_FP64;
@@ -330,7 +382,7 @@ void launch_phys(const PhysArgs &a, cudaStream_t st) {
     k_phys<PHYS_OFF><<<nb, PT, 0, st>>>(a);
     return;
   }
-  cudaMemsetAsync(a.list_n, 0, sizeof(unsigned), st);
+  k_rsf_const<<<1, 128, 0, st>>>(a.R, a.S, a.rk, a.list_n);
   if (fp64) k_phys<PHYS_FP64><<<nb, PT, 0, st>>>(a);
   else k_phys<PHYS_SPLIT><<<nb, PT, 0, st>>>(a);
   if (learned) k_guess<<<resident_grid(k_guess, PT), PT, 0, st>>>(a, a.guess);

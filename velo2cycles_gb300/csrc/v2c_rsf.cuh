@@ -186,6 +186,56 @@ __device__ __forceinline__ void rsf_setup_ff(RsfFF &q, const RsfIn &in) {
   q.inv_a = ff_div(ff_f(1.f), in.a);
 }
 
+// What the set-ups of one call's markers share: almost every marker lies
+// outside the frictional band, where the friction parameters are the far
+// field's and the state is 50, and G dt depends on the rock type only.  The
+// terms built from these alone are evaluated once per call (k_rsf_const) by
+// the same device functions, so a marker's set-up has the same bits with one
+// division instead of four and neither the exponential nor the logarithm.
+constexpr float RSF_FAR_STATE = 50.f;
+struct RsfConst {
+  ff inv_a, dtL, V0dtL, V0s, ln2V0, ephio;  // far field, state 50
+  float ephio32, lg2V032;                   // the same for the FP32 phase
+  ff Gdt[128], GdtW2[128];                  // by rock type: G dt, 2 G dt / W
+};
+
+__device__ __forceinline__ void rsf_const_far(RsfConst &k, const RsfIn &in) {
+  RsfFF q;
+  rsf_setup_ff(q, in);
+  k.inv_a = q.inv_a; k.dtL = q.dtL; k.V0dtL = q.V0dtL; k.V0s = q.V0s; k.ln2V0 = q.ln2V0;
+  k.ephio = q.ephio;
+  k.ephio32 = expf(in.phio.hi);
+  k.lg2V032 = logf(2.f * in.V0.hi);
+}
+__device__ __forceinline__ void rsf_const_type(RsfConst &k, int t, ff G, ff dt, ff W) {
+  const ff Gdt = ff_mul(G, dt);
+  k.Gdt[t] = Gdt;
+  k.GdtW2[t] = ff_scale(ff_div(Gdt, W), 2.f);
+}
+
+// rsf_setup_ff of a marker of rock type t (far: far-field friction, state 50)
+__device__ __forceinline__ void rsf_setup_marker(RsfFF &q, const RsfIn &in, const RsfConst &k,
+                                                 int t, bool far) {
+  const ff Gdt = k.Gdt[t];
+  q.Ts = ff_add(in.tau_old, ff_scale(ff_mul(Gdt, in.edot), 2.f));
+  const ff c1 = ff_add_f(ff_div(Gdt, in.eta), 1.f);
+  q.klin = ff_add(ff_mul_f(c1, 4330300.f), k.GdtW2[t]);
+  q.snac1 = ff_mul(ff_mul(in.sn, in.a), c1);
+  q.mu0 = in.mu0;
+  q.b = in.b;
+  if (far) {
+    q.inv_a = k.inv_a; q.dtL = k.dtL; q.V0dtL = k.V0dtL; q.V0s = k.V0s; q.ln2V0 = k.ln2V0;
+    q.ephio = k.ephio;
+  } else {
+    q.ephio = ff_exp(in.phio);
+    q.dtL = ff_div(in.dt, in.L);
+    q.V0dtL = ff_mul(in.V0, q.dtL);
+    q.V0s = ff_scale(in.V0, V2C_TWO64);
+    q.ln2V0 = ff_log(ff_scale(in.V0, 2.f));
+    q.inv_a = ff_div(ff_f(1.f), in.a);
+  }
+}
+
 // F and lhs = F + T* at u (float-float); phi and A at u.  Mirrors
 // rsf_eval64 term by term.
 __device__ __forceinline__ ff rsf_eval_ff(const RsfFF &q, ff u, ff &lhs, ff &phi, ff &A,
@@ -255,7 +305,9 @@ struct Rsf32 {
 };
 // FP32 constants straight from the inputs (no float-float set-up needed
 // for the FP32 phase)
-__device__ __forceinline__ Rsf32 rsf32_of(const RsfIn &in) {
+// (far: the constants k of the far field and state 50, see RsfConst)
+__device__ __forceinline__ Rsf32 rsf32_of(const RsfIn &in, const RsfConst *k = nullptr,
+                                          bool far = false) {
   Rsf32 r;
   r.a = in.a.hi; r.b = in.b.hi; r.L = in.L.hi; r.V0 = in.V0.hi; r.mu0 = in.mu0.hi;
   r.dt = in.dt.hi;
@@ -264,8 +316,13 @@ __device__ __forceinline__ Rsf32 rsf32_of(const RsfIn &in) {
   const float c1 = 1.f + Gdt / in.eta.hi;
   r.klin = 4330300.f * c1 + 2.f * Gdt / in.W.hi;
   r.snac1 = in.sn.hi * in.a.hi * c1;
-  r.ephio = expf(in.phio.hi);
-  r.lg2V0 = logf(2.f * in.V0.hi);
+  if (far) {
+    r.ephio = k->ephio32;
+    r.lg2V0 = k->lg2V032;
+  } else {
+    r.ephio = expf(in.phio.hi);
+    r.lg2V0 = logf(2.f * in.V0.hi);
+  }
   r.uhi = logf(r.Ts / r.klin);
   return r;
 }
@@ -355,9 +412,12 @@ __device__ __forceinline__ float rsf_start_residual(const Rsf32 &q, float u0, fl
 constexpr float RSF_NET_MIN_RES = 1e-2f;
 
 // Split solve from the start u0 (FP32 phase, float-float phase, FP64
-// fallback).  q32 = rsf32_of(in).
+// fallback).  q32 = rsf32_of(in); setup(q) fills the float-float constants,
+// finish(u, r) runs the FP64 Newton from u.
+template <class Setup, class Finish>
 __device__ __forceinline__ RsfResult rsf_solve_split(const RsfIn &in, const Rsf32 &q32, float u0,
-                                                     double rtol, int maxit) {
+                                                     double rtol, int maxit, Setup setup,
+                                                     Finish finish) {
   RsfResult r{};
   r.phi = in.phio.hi;
   const float floor32 = (float)RSF_LOG_FLOOR;
@@ -368,7 +428,7 @@ __device__ __forceinline__ RsfResult rsf_solve_split(const RsfIn &in, const Rsf3
   float dF32;
   const float u32 = rsf_newton32(q32, u0, floor32, q32.uhi, maxit, r.it32, dF32);
   RsfFF q;
-  rsf_setup_ff(q, in);
+  setup(q);
   const ff floor_u = ff_from_double(RSF_LOG_FLOOR);
   ff u = (u32 <= floor32 + 1e-6f) ? floor_u : ff_f(u32);
   // the ratio |F|/(F+T*) needs a few significant digits: F and F+T* come
@@ -399,9 +459,14 @@ __device__ __forceinline__ RsfResult rsf_solve_split(const RsfIn &in, const Rsf3
     if (!(dF32 > 0.f)) break;
     u = ff_add_f(u, -F.hi / dF32);
   }
-  // the FP64 Newton finishes
-  rsf_finish64(in, ff_to_double(u), rtol, maxit, r);
+  finish(ff_to_double(u), r);  // the FP64 Newton finishes
   return r;
+}
+// with the state's own constants
+__device__ __forceinline__ RsfResult rsf_solve_split(const RsfIn &in, const Rsf32 &q32, float u0,
+                                                     double rtol, int maxit) {
+  return rsf_solve_split(in, q32, u0, rtol, maxit, [&](RsfFF &q) { rsf_setup_ff(q, in); },
+                         [&](double u, RsfResult &r) { rsf_finish64(in, u, rtol, maxit, r); });
 }
 
 // The floor as a result (one FP32 residual evaluation)
