@@ -1,6 +1,7 @@
 // v2c_api.cu -- the C ABI (include/v2c.h): context life cycle, transfers,
 // and the step entry points that replace the reference's global-array
 // routines.
+#include <cuda.h>
 #include <math.h>
 #include <cmath>
 #include <stdio.h>
@@ -53,6 +54,7 @@ struct v2c_ctx {
   unsigned *d_list_n = nullptr;              // count of listed Newton problems
   char *d_rsfk = nullptr;                    // constants the Newton problems share
   double *d_ts = nullptr;                    // calc_timestep scratch
+  double *h_res = nullptr;                   // pinned: small results kernels write
   // markers
   Markers m{};
   void *marker_mem[32] = {};
@@ -96,7 +98,6 @@ struct v2c_ctx {
   int bc_n = 0;
   void *bc_mem = nullptr;
   BcRows bc{};
-  float *d_bc_scratch = nullptr;
   // status
   unsigned long long *d_stat = nullptr;
   double *d_red = nullptr;
@@ -313,11 +314,17 @@ extern "C" int v2c_create(const v2c_params *p, long max_markers, void *cuda_stre
   AL(ctx->d_list_n, 1);
   AL(ctx->d_rsfk, rsf_const_bytes());
   AL(ctx->d_ts, TIMESTEP_SCRATCH);
+  cudaMemsetAsync(ctx->d_ts, 0, sizeof(double) * TIMESTEP_SCRATCH, ctx->stream);
   AL(ctx->d_stat, ST_N);
   ctx->red_cap = 2 + 2 * ((ctx->nn + 255) / 256);
   AL(ctx->d_red, ctx->red_cap);
   cudaMemsetAsync(ctx->d_node, 0, sizeof(float) * V2C_NF_N * ctx->nn, ctx->stream);
   cudaMemsetAsync(ctx->d_stat, 0, sizeof(unsigned long long) * ST_N, ctx->stream);
+  if (cudaHostAlloc((void **)&ctx->h_res, sizeof(double) * RESULT_DOUBLES, cudaHostAllocDefault) !=
+      cudaSuccess) {
+    v2c_destroy(ctx);
+    return V2C_ERR_CUDA;
+  }
   // markers
   long cap = max_markers;
   Markers &m = ctx->m;
@@ -334,14 +341,17 @@ extern "C" int v2c_create(const v2c_params *p, long max_markers, void *cuda_stre
 #undef AM
   ctx->n_marker_mem = k;
   // sort
-  AL(ctx->sb.counts, ctx->ncell); AL(ctx->sb.start, ctx->ncell + 1);
+  AL(ctx->sb.counts, ctx->ncell);
+  cudaMemsetAsync(ctx->sb.counts, 0, sizeof(int32_t) * ctx->ncell, ctx->stream);
+  AL(ctx->sb.start, ctx->ncell + 1);
   AL(ctx->sb.qstart, ctx->ncell + 1);
   AL(ctx->sb.slot, cap); AL(ctx->sb.tmp, cap); AL(ctx->sb.perm, cap);
   ctx->sb.blocksum_cap = (ctx->ncell + 4095) / 4096 + 1;
   AL(ctx->sb.blocksum, ctx->sb.blocksum_cap);
   AL(ctx->d_stage64, cap); AL(ctx->d_stage64b, cap);
 #undef AL
-  if (m2n_init() != cudaSuccess || n2m_init() != cudaSuccess) { v2c_destroy(ctx); return V2C_ERR_CUDA; }
+  if (m2n_init() != cudaSuccess || n2m_init() != cudaSuccess ||
+      timestep_init() != cudaSuccess) { v2c_destroy(ctx); return V2C_ERR_CUDA; }
   if (newton_init(ctx->nw, cap) != cudaSuccess) { v2c_destroy(ctx); return V2C_ERR_CUDA; }
   if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) { v2c_destroy(ctx); return V2C_ERR_CUDA; }
   *out = ctx;
@@ -358,6 +368,7 @@ extern "C" int v2c_destroy(v2c_ctx *ctx) {
   if (ctx->ev_conv) cudaEventDestroy(ctx->ev_conv);
   if (ctx->ev_copy) cudaEventDestroy(ctx->ev_copy);
   if (ctx->d_astage) cudaFree(ctx->d_astage);
+  if (ctx->h_res) cudaFreeHost(ctx->h_res);
   for (auto &gr : ctx->graphs) cudaGraphExecDestroy(gr.exec);
   ctx->graphs.clear();
   for (float *v : ctx->d_cyc_v)
@@ -374,8 +385,7 @@ extern "C" int v2c_destroy(v2c_ctx *ctx) {
                   ctx->d_rock, ctx->d_node, ctx->d_node64, ctx->d_sticky, ctx->d_quad, ctx->d_tol, ctx->d_list_n, ctx->d_rsfk, ctx->d_ts,
                   ctx->d_stat, ctx->d_red, ctx->d_nstage,
                   ctx->sb.counts, ctx->sb.start, ctx->sb.qstart, ctx->sb.slot, ctx->sb.tmp, ctx->sb.perm,
-                  ctx->sb.blocksum, ctx->d_stage64, ctx->d_stage64b, ctx->bc_mem,
-                  ctx->d_bc_scratch};
+                  ctx->sb.blocksum, ctx->d_stage64, ctx->d_stage64b, ctx->bc_mem};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   for (int i = 0; i < ctx->n_marker_mem; i++)
@@ -595,7 +605,6 @@ int build_bc(v2c_ctx *ctx) {
   }
   int n = (int)fld.size();
   if (ctx->bc_mem) { cudaFree(ctx->bc_mem); ctx->bc_mem = nullptr; }
-  if (ctx->d_bc_scratch) { cudaFree(ctx->d_bc_scratch); ctx->d_bc_scratch = nullptr; }
   ctx->bc_n = n;
   ctx->bc = BcRows{};
   ctx->bc.n = n;
@@ -605,7 +614,6 @@ int build_bc(v2c_ctx *ctx) {
                  n * M * (sizeof(int) + sizeof(long) + sizeof(float)) + 64;
   char *mem;
   if (cudaMalloc((void **)&mem, bytes) != cudaSuccess) return V2C_ERR_CUDA;
-  if (cudaMalloc((void **)&ctx->d_bc_scratch, sizeof(float) * n) != cudaSuccess) return V2C_ERR_CUDA;
   ctx->bc_mem = mem;
   size_t off = 0;
   auto put = [&](const void *src, size_t sz) {
@@ -800,23 +808,29 @@ extern "C" int v2c_download_cells(v2c_ctx *ctx, int32_t *cell, long n) {
 // ============================================================== node arrays
 // node fields live in FP32 on the device; they are converted on the way in
 // and out (the conversion kernels run on the context stream)
-// keep the FP64 copy of an uploaded velocity or temperature field (staged
-// at dev64)
-static int keep_node64(v2c_ctx *ctx, int field, const double *dev64) {
+// the FP64 copy kept of an uploaded velocity or temperature field (null for
+// others), and keeping it from dev64
+static int node64_of(v2c_ctx *ctx, int field, double *&dst) {
+  dst = nullptr;
   if (field == V2C_NF_TK || field == V2C_NF_TK2) {
     const int k = field == V2C_NF_TK ? 0 : 1;
     if (!ctx->d_tk64) CK(cudaMalloc(&ctx->d_tk64, sizeof(double) * 2 * ctx->nn));
-    CK(cudaMemcpyAsync(ctx->d_tk64 + k * ctx->nn, dev64, sizeof(double) * ctx->nn,
-                       cudaMemcpyDeviceToDevice, ctx->stream));
+    dst = ctx->d_tk64 + k * ctx->nn;
     ctx->tk64_ok[k] = true;
-    return V2C_OK;
+  } else if (field == V2C_NF_VX || field == V2C_NF_VY) {
+    const int k = field == V2C_NF_VX ? 0 : 1;
+    if (!ctx->d_vel64) CK(cudaMalloc(&ctx->d_vel64, sizeof(double) * 2 * ctx->nn));
+    dst = ctx->d_vel64 + k * ctx->nn;
+    ctx->vel64_ok[k] = true;
   }
-  if (field != V2C_NF_VX && field != V2C_NF_VY) return V2C_OK;
-  const int k = field == V2C_NF_VX ? 0 : 1;
-  if (!ctx->d_vel64) CK(cudaMalloc(&ctx->d_vel64, sizeof(double) * 2 * ctx->nn));
-  CK(cudaMemcpyAsync(ctx->d_vel64 + k * ctx->nn, dev64, sizeof(double) * ctx->nn,
-                     cudaMemcpyDeviceToDevice, ctx->stream));
-  ctx->vel64_ok[k] = true;
+  return V2C_OK;
+}
+static int keep_node64(v2c_ctx *ctx, int field, const double *dev64) {
+  double *dst;
+  if (int rc = node64_of(ctx, field, dst)) return rc;
+  if (dst)
+    CK(cudaMemcpyAsync(dst, dev64, sizeof(double) * ctx->nn, cudaMemcpyDeviceToDevice,
+                       ctx->stream));
   return V2C_OK;
 }
 
@@ -849,6 +863,48 @@ static int node_field_list_ok(int count, const int *fields, const void *const *p
   return 1;
 }
 
+// Whether every array (nn doubles) lies in one pinned host allocation that
+// the device reads and writes at the same address: then a kernel moves the
+// fields itself.  Each copy costs about 2 us on its stream and 1 us to issue,
+// so at 301 x 101 nodes eight of them took 28 us and the kernel takes 8; at
+// 4 M nodes both run at the host link's rate (210 GB/s in, 193 out) and the
+// kernel saves the staging area's traffic.
+static bool all_pinned(const void *const *ptrs, int count, long nn) {
+  typedef CUresult (*AttrFn)(void *, CUpointer_attribute, CUdeviceptr);
+  static const AttrFn range_of = [] {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault,
+                                         &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    cudaGetLastError();
+    return reinterpret_cast<AttrFn>(fn);
+  }();
+  if (!range_of) return false;
+  const size_t bytes = sizeof(double) * (size_t)nn;
+  for (int k = 0; k < count; k++) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, ptrs[k]) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (at.type != cudaMemoryTypeHost || at.devicePointer != ptrs[k] || (uintptr_t)ptrs[k] % 8)
+      return false;
+    unsigned long long begin = 0;
+    size_t size = 0;
+    const unsigned long long p = (unsigned long long)ptrs[k];
+    if (range_of(&begin, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) ||
+        range_of(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) || p < begin ||
+        p + bytes > begin + size)
+      return false;
+  }
+  return true;
+}
+// A field this size goes to the host by the copy engine, which takes no SMs
+// from the kernels it runs under; smaller ones together in one kernel.
+constexpr long ENGINE_COPY_NODES = 1 << 17;
+
 static int grow_node_stage(v2c_ctx *ctx, int count) {
   if (count <= ctx->nstage_cap) return V2C_OK;
   CK(cudaStreamSynchronize(ctx->stream));
@@ -866,6 +922,15 @@ extern "C" int v2c_upload_node_fields(v2c_ctx *ctx, int count, const int *fields
   if (!node_field_list_ok(count, fields, (const void *const *)src)) return fail(ctx, V2C_ERR_ARG);
   if (count == 0) return V2C_OK;
   ctx->dsxx_valid = false;
+  if (all_pinned((const void *const *)src, count, ctx->nn)) {
+    double *keep[V2C_NF_N];
+    for (int k = 0; k < count; k++)
+      if (int rc2 = node64_of(ctx, fields[k], keep[k])) return fail(ctx, rc2);
+    launch_host_to_fields(src, fields, keep, count, ctx->nn, ctx->d_node, ctx->stream);
+    ctx->launches += 1;
+    CK(cudaGetLastError());
+    return V2C_OK;
+  }
   int rc = grow_node_stage(ctx, count);
   if (rc) return fail(ctx, rc);
   for (int k = 0; k < count; k++)
@@ -907,7 +972,14 @@ extern "C" int v2c_download_node_fields_async(v2c_ctx *ctx, int count, const int
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev_conv, st));
   CK(cudaStreamWaitEvent(ctx->xfer, ctx->ev_conv, 0));
-  for (int k = 0; k < count; k++)
+  const bool engine = ctx->nn > ENGINE_COPY_NODES ||
+                      !all_pinned((const void *const *)dst, count, ctx->nn);
+  if (!engine) {
+    launch_stage_to_host(ctx->d_astage, dst, count, ctx->nn, ctx->xfer);
+    ctx->launches += 1;
+    CK(cudaGetLastError());
+  }
+  for (int k = 0; engine && k < count; k++)
     CK(cudaMemcpyAsync(dst[k], ctx->d_astage + (long)k * ctx->nn, sizeof(double) * ctx->nn,
                        cudaMemcpyDeviceToHost, ctx->xfer));
   CK(cudaEventRecord(ctx->ev_copy, ctx->xfer));
@@ -929,6 +1001,13 @@ extern "C" int v2c_download_node_fields(v2c_ctx *ctx, int count, const int *fiel
   if (!ctx) return V2C_ERR_ARG;
   if (!node_field_list_ok(count, fields, (const void *const *)dst)) return fail(ctx, V2C_ERR_ARG);
   if (count == 0) return V2C_OK;
+  if (all_pinned((const void *const *)dst, count, ctx->nn)) {
+    launch_fields_to_host(ctx->d_node, fields, dst, count, ctx->nn, ctx->stream);
+    ctx->launches += 1;
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(ctx->stream));
+    return V2C_OK;
+  }
   int rc = grow_node_stage(ctx, count);
   if (rc) return fail(ctx, rc);
   launch_fields_to_f64(ctx->d_node, ctx->nn, fields, count, ctx->d_nstage, ctx->stream);
@@ -962,7 +1041,7 @@ extern "C" int v2c_marker2nodes(v2c_ctx *ctx) {
     Prof pr(ctx, V2C_PROF_SORT);
     launch_sort(ctx->m.cell_in, ctx->m.u_in, ctx->m.v_in, ctx->n, ctx->ncell, ctx->sb,
                 ctx->d_stat, st);
-    ctx->launches += ctx->n > 0 ? 6 : 3;
+    ctx->launches += ctx->n > 0 ? 5 : 3;
     ctx->sorted = true;
   }
   if (ctx->have_bonds) {
@@ -984,7 +1063,6 @@ extern "C" int v2c_marker2nodes(v2c_ctx *ctx) {
   a.gyf = ctx->d_gyf;
   a.TX = sweep_tx(ctx);
   a.n = ctx->n;
-  CK(cudaMemsetAsync(ctx->d_sticky, 0, sizeof(uint32_t) * ctx->nn, st));
   ctx->dsxx_valid = false;  // the scatter writes sxxe
   ctx->tk64_ok[0] = false;  // and the node temperature
   {
@@ -1000,7 +1078,9 @@ extern "C" int v2c_marker2nodes(v2c_ctx *ctx) {
     ph.guess = reinterpret_cast<float *>(ctx->sb.tmp);  // likewise free between sorts
     Prof pr(ctx, ctx->p.newton_guess == V2C_GUESS_OFF ? V2C_PROF_PHYS : V2C_PROF_NEWTON);
     launch_phys(ph, st);
-    ctx->launches += ctx->p.newton_guess == V2C_GUESS_OFF ? 1 : (ph.mlp && ctx->p.newton_guess == V2C_GUESS_LEARNED ? 4 : 3);
+    ctx->launches += ctx->p.newton_guess == V2C_GUESS_OFF                       ? 2
+                     : ph.mlp && ctx->p.newton_guess == V2C_GUESS_LEARNED ? 4
+                                                                                : 3;
   }
   {
     Prof pr(ctx, V2C_PROF_M2N);
@@ -1010,10 +1090,9 @@ extern "C" int v2c_marker2nodes(v2c_ctx *ctx) {
   ctx->props_valid = true;
   {
     Prof pr(ctx, V2C_PROF_M2N_TAIL);
-    launch_sticky(a.N, ctx->d_sticky, ctx->nn, st);
+    launch_m2n_tail(ctx->have_bonds ? ctx->bc : BcRows{}, a.N, ctx->d_sticky, ctx->nn, st);
     ctx->launches += 1;
     if (ctx->p.Dphis > 0) { launch_dphis(a.g, a.N, st); ctx->launches += 1; }
-    if (ctx->have_bonds && ctx->bc.n > 0) { launch_bc(ctx->bc, a.N, ctx->d_bc_scratch, st); ctx->launches += 2; }
   }
   CK(cudaGetLastError());
   return V2C_OK;
@@ -1117,14 +1196,13 @@ extern "C" int v2c_compute_after_solve(v2c_ctx *ctx, double dt, int rk, double *
   {
     Prof pr(ctx, V2C_PROF_AFTER);
     launch_after_solve(make_grid(ctx), make_nodes(ctx), make_scal(ctx->p, ctx->h_rt), dt, rk,
-                       ctx->d_red, ctx->stream);
+                       ctx->d_red, deltas ? ctx->h_res : nullptr, ctx->stream);
   }
-  ctx->launches += 2;
+  ctx->launches += deltas ? 2 : 1;
   CK(cudaGetLastError());
   if (deltas) {
-    double h[2];
-    CK(cudaMemcpyAsync(h, ctx->d_red, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    const double *h = ctx->h_res;
     *deltas = h[1] > 0 ? sqrt(h[0] / h[1]) : 0.0;
   }
   return V2C_OK;
@@ -1138,7 +1216,7 @@ static int n2m_move(v2c_ctx *ctx, int do_n2m, int do_move) {
     Prof pr(ctx, V2C_PROF_SORT);
     launch_sort(ctx->m.cell_in, ctx->m.u_in, ctx->m.v_in, ctx->n, ctx->ncell, ctx->sb,
                 ctx->d_stat, st);
-    ctx->launches += ctx->n > 0 ? 6 : 3;
+    ctx->launches += ctx->n > 0 ? 5 : 3;
     ctx->sorted = true;
   }
   N2MArgs a;
@@ -1194,7 +1272,7 @@ static int n2m_move(v2c_ctx *ctx, int do_n2m, int do_move) {
     Prof pr(ctx, V2C_PROF_SORT);
     launch_sort(ctx->m.cell_in, ctx->m.u_in, ctx->m.v_in, ctx->n, ctx->ncell, ctx->sb,
                 ctx->d_stat, st);
-    ctx->launches += ctx->n > 0 ? 6 : 3;
+    ctx->launches += ctx->n > 0 ? 5 : 3;
   }
   CK(cudaGetLastError());
   return V2C_OK;
@@ -1213,7 +1291,7 @@ extern "C" int v2c_calc_timestep(v2c_ctx *ctx, int oldornew, const v2c_timestep_
   {
     Prof pr(ctx, V2C_PROF_TIMESTEP);
     rc = calc_timestep_device(make_grid(ctx), make_nodes(ctx), make_scal(ctx->p, ctx->h_rt), *ctl,
-                              oldornew, ctx->d_ts, TIMESTEP_SCRATCH, info, ctx->stream);
+                              oldornew, ctx->d_ts, TIMESTEP_SCRATCH, ctx->h_res, info, ctx->stream);
   }
   ctx->launches += 2;
   if (rc) return fail(ctx, rc);
@@ -1239,7 +1317,7 @@ extern "C" int v2c_marker_temperature(v2c_ctx *ctx, double heatdif) {
   if (!ctx->sorted) {
     launch_sort(ctx->m.cell_in, ctx->m.u_in, ctx->m.v_in, ctx->n, ctx->ncell, ctx->sb,
                 ctx->d_stat, st);
-    ctx->launches += ctx->n > 0 ? 6 : 3;
+    ctx->launches += ctx->n > 0 ? 5 : 3;
     ctx->sorted = true;
   }
   TempArgs a;

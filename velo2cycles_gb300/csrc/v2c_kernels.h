@@ -7,7 +7,7 @@
 namespace v2c {
 
 struct SortBufs {
-  int32_t *counts;   // [ncell]
+  int32_t *counts;   // [ncell], zero between sorts
   int32_t *start;    // [ncell+1]
   int4 *qstart;      // [ncell+1]: start of each quarter class of a cell (see launch_sort)
   int32_t *slot;     // [cap]
@@ -102,12 +102,13 @@ struct PhysArgs {
   float *guess = nullptr;  // the network's start per listed problem (capacity n)
 };
 void launch_phys(const PhysArgs &a, cudaStream_t st);
-void launch_sticky(const Nodes &N, const uint32_t *key, long nn, cudaStream_t st);
 void launch_dphis(const Grid &g, const Nodes &N, cudaStream_t st);
 
-// boundary corrections: flattened rows x[row] = c + sum coef*value[ref]
+// boundary corrections: flattened rows x[row] = c + sum coef*value[ref], the
+// references all rows without an equation of their own (no row reads
+// another's result)
 struct BcRows {
-  int n;            // rows
+  int n = 0;        // rows
   const int *field; // node field written
   const long *node; // node written
   const float *c;   // constant
@@ -117,7 +118,10 @@ struct BcRows {
   const float *rcoef;
 };
 #define V2C_BC_MAXREF 8
-void launch_bc(const BcRows &rows, const Nodes &N, float *scratch, cudaStream_t st);
+// the end of marker2nodes: sticky-air flags from their candidates, and the
+// boundary rows
+void launch_m2n_tail(const BcRows &rows, const Nodes &N, const uint32_t *sticky_key, long nn,
+                     cudaStream_t st);
 void launch_node_to_f32(const double *src, float *dst, long n, cudaStream_t st);
 void launch_node_to_f64(const float *src, double *dst, long n, cudaStream_t st);
 // count node fields (ids in fields[], count <= V2C_NF_N) to / from a staging
@@ -125,6 +129,15 @@ void launch_node_to_f64(const float *src, double *dst, long n, cudaStream_t st);
 void launch_fields_to_f64(const float *base, long nn, const int *fields, int count, double *stage,
                           cudaStream_t st);
 void launch_fields_to_f32(const double *stage, long nn, const int *fields, int count, float *base,
+                          cudaStream_t st);
+
+// the same from / to pinned host arrays directly (keep[k]: where to keep an
+// FP64 copy of field k, or null), and a staging area to pinned host arrays
+void launch_host_to_fields(const double *const *src, const int *fields, double *const *keep,
+                           int count, long nn, float *base, cudaStream_t st);
+void launch_fields_to_host(const float *base, const int *fields, double *const *dst, int count,
+                           long nn, cudaStream_t st);
+void launch_stage_to_host(const double *stage, double *const *dst, int count, long nn,
                           cudaStream_t st);
 
 void launch_c2b_old(const Grid &g, const Nodes &N, cudaStream_t st);
@@ -140,8 +153,9 @@ void launch_unpermute_f64(const double *src, const int32_t *id, double *out, lon
 void launch_slip_acc(const Grid &g, const Nodes &N, double dt, double *acc, cudaStream_t st);
 void launch_before_solve(const Grid &g, const Nodes &N, const Scal &S, double dt, int rk,
                          unsigned long long *stat, cudaStream_t st);
+// out: two doubles (sum of squared misfits, count) the host reads, or null
 void launch_after_solve(const Grid &g, const Nodes &N, const Scal &S, double dt, int rk,
-                        double *red, cudaStream_t st);
+                        double *red, double *out, cudaStream_t st);
 
 // Immobile markers (moveandrotatemarkers.c:88-171): what the move kernel
 // records per reference marker number, and the scratch of the compaction
@@ -218,11 +232,14 @@ struct TempArgs {
 void launch_temperature(const TempArgs &a, cudaStream_t st);
 
 // calc_timestep over the device node fields (synchronises the stream);
-// scratch: TIMESTEP_SCRATCH doubles
+// scratch: TIMESTEP_SCRATCH doubles, zero before the first call; result:
+// RESULT_DOUBLES of pinned host memory
+constexpr int RESULT_DOUBLES = 64;
 constexpr long TIMESTEP_SCRATCH = (152 * 4 * 8 + 1) * 32 + 64;
+cudaError_t timestep_init();  // shared-memory size of the fold, once per device
 int calc_timestep_device(const Grid &g, const Nodes &N, const Scal &S, const v2c_timestep_ctl &c,
                          int oldornew, double *scratch, long scratch_doubles,
-                         v2c_timestep_info *info, cudaStream_t st);
+                         double *result, v2c_timestep_info *info, cudaStream_t st);
 
 // upload / download helpers
 void launch_assign(const Grid &g, const double *x, const double *y, long n, Markers m,

@@ -783,14 +783,6 @@ __global__ void __launch_bounds__(128) k_m2n_mode1(M2NArgs a) {
   }
 }
 
-__global__ void k_sticky(float *st, const uint32_t *key, long nn) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i < nn) {
-    uint32_t k = key[i];
-    st[i] = k ? (float)(k & 3u) : 0.f;
-  }
-}
-
 // ghost copy of the state when it diffuses, interpolation.c:827-859
 __global__ void k_dphis(Grid g, float *phis) {
   long m3 = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -823,10 +815,6 @@ void launch_m2n(const M2NArgs &a, cudaStream_t st) {
   }
   dim3 grid((a.g.xn + a.TX - 1) / a.TX, (a.g.yn + TY - 1) / TY);
   k_m2n<<<grid, NTH, sizeof(Smem), st>>>(a);
-}
-
-void launch_sticky(const Nodes &N, const uint32_t *key, long nn, cudaStream_t st) {
-  k_sticky<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(N.f(V2C_NF_STICKY01), key, nn);
 }
 
 void launch_dphis(const Grid &g, const Nodes &N, cudaStream_t st) {

@@ -335,19 +335,20 @@ __global__ void __launch_bounds__(PT, 8) k_newton(PhysArgs a, const float *guess
   warp_add(a.stat + ST_NEWTON_NONCONV, nc);
 }
 
-// the call's shared Newton constants; empties the problem list
-__global__ void k_rsf_const(Rock R, Scal S, RsfConst *k, unsigned *list_n) {
+// What marker2nodes clears before its marker passes, and the shared Newton
+// constants, in one launch: no sticky-air candidates, an empty problem list.
+// The constants' long chains go to different warps of block 0.
+__global__ void __launch_bounds__(256) k_phys_init(PhysArgs a, bool newton) {
+  const long nn = a.g.nn;
+  for (long i = blockIdx.x * 256l + threadIdx.x; i < nn; i += gridDim.x * 256l) a.sticky_key[i] = 0;
+  if (!newton || blockIdx.x != 0) return;
+  const Scal &S = a.S;
   const int t = threadIdx.x;
-  if (t == 0) {
-    RsfIn in;
-    in.a = ff_f(S.a_hr_f); in.b = ff_f(S.b_hr_f); in.L = ff_f(S.L_hr_f); in.V0 = ff_f(S.V0_hr_f);
-    in.mu0 = ff_f(0.6f); in.sn = ff{S.sn_hi, S.sn_lo}; in.dt = ff{S.dt_hi, S.dt_lo};
-    in.W = ff{S.W_hi, S.W_lo}; in.phio = ff_f(RSF_FAR_STATE);
-    in.tau_old = in.edot = ff_f(0.f); in.eta = in.G = ff_f(1.f);
-    rsf_const_far(*k, in);
-    *list_n = 0;
-  }
-  rsf_const_type(*k, t, ff_f(R(RK_GG, t)), ff{S.dt_hi, S.dt_lo}, ff{S.W_hi, S.W_lo});
+  const ff dt{S.dt_hi, S.dt_lo}, W{S.W_hi, S.W_lo};
+  if (t < 128) rsf_const_type(*a.rk, t, ff_f(a.R(RK_GG, t)), dt, W);
+  else if (t % 32 == 0)
+    rsf_const_far(*a.rk, (t - 128) / 32, S.a_hr_f, S.L_hr_f, S.V0_hr_f, dt);
+  if (t == 0) *a.list_n = 0;
 }
 
 // resident blocks of a kernel on the whole GPU (grid-stride launches)
@@ -365,12 +366,17 @@ unsigned resident_grid(K kernel, int threads) {
 size_t rsf_const_bytes() { return sizeof(RsfConst); }
 
 void launch_phys(const PhysArgs &a, cudaStream_t st) {
+  const v2c_params &p = a.S.p;
+  if (!a.xs) {
+    const long nb = (a.g.nn + 255) / 256;
+    k_phys_init<<<(unsigned)(nb < 608 ? nb : 608), 256, 0, st>>>(
+        a, a.n > 0 && p.newton_guess != V2C_GUESS_OFF);
+  }
   if (a.n <= 0) return;
   // one pass of 32 markers per warp: the blocks' times differ with the creep
   // iterations of their markers, and many short blocks fill the SMs to the
   // end where 16 long ones per SM left the last wave a third empty
   const long blocks = (a.n + PT - 1) / PT;
-  const v2c_params &p = a.S.p;
   const bool learned = p.newton_guess == V2C_GUESS_LEARNED && a.mlp != nullptr;
   const bool fp64 = p.newton_precision == V2C_NEWTON_FP64;
   const unsigned nb = (unsigned)blocks;
@@ -382,7 +388,6 @@ void launch_phys(const PhysArgs &a, cudaStream_t st) {
     k_phys<PHYS_OFF><<<nb, PT, 0, st>>>(a);
     return;
   }
-  k_rsf_const<<<1, 128, 0, st>>>(a.R, a.S, a.rk, a.list_n);
   if (fp64) k_phys<PHYS_FP64><<<nb, PT, 0, st>>>(a);
   else k_phys<PHYS_SPLIT><<<nb, PT, 0, st>>>(a);
   if (learned) k_guess<<<resident_grid(k_guess, PT), PT, 0, st>>>(a, a.guess);

@@ -189,7 +189,7 @@ __device__ __forceinline__ void rsf_setup_ff(RsfFF &q, const RsfIn &in) {
 // What the set-ups of one call's markers share: almost every marker lies
 // outside the frictional band, where the friction parameters are the far
 // field's and the state is 50, and G dt depends on the rock type only.  The
-// terms built from these alone are evaluated once per call (k_rsf_const) by
+// terms built from these alone are evaluated once per call (k_phys_init) by
 // the same device functions, so a marker's set-up has the same bits with one
 // division instead of four and neither the exponential nor the logarithm.
 constexpr float RSF_FAR_STATE = 50.f;
@@ -199,13 +199,24 @@ struct RsfConst {
   ff Gdt[128], GdtW2[128];                  // by rock type: G dt, 2 G dt / W
 };
 
-__device__ __forceinline__ void rsf_const_far(RsfConst &k, const RsfIn &in) {
-  RsfFF q;
-  rsf_setup_ff(q, in);
-  k.inv_a = q.inv_a; k.dtL = q.dtL; k.V0dtL = q.V0dtL; k.V0s = q.V0s; k.ln2V0 = q.ln2V0;
-  k.ephio = q.ephio;
-  k.ephio32 = expf(in.phio.hi);
-  k.lg2V032 = logf(2.f * in.V0.hi);
+// the far-field terms, in four independent parts
+__device__ __forceinline__ void rsf_const_far(RsfConst &k, int part, float a, float L, float V0,
+                                              ff dt) {
+  if (part == 0) {
+    k.dtL = ff_div(dt, ff_f(L));
+    k.V0dtL = ff_mul(ff_f(V0), k.dtL);
+  } else if (part == 1) {
+    k.ln2V0 = ff_log(ff_scale(ff_f(V0), 2.f));
+    k.lg2V032 = logf(2.f * V0);
+  } else if (part == 2) {
+    k.inv_a = ff_div(ff_f(1.f), ff_f(a));
+    k.V0s = ff_scale(ff_f(V0), V2C_TWO64);
+  } else {
+    float state = RSF_FAR_STATE;
+    asm volatile("" : "+f"(state));  // the device's exponentials, not a folded constant
+    k.ephio = ff_exp(ff_f(state));
+    k.ephio32 = expf(state);
+  }
 }
 __device__ __forceinline__ void rsf_const_type(RsfConst &k, int t, ff G, ff dt, ff W) {
   const ff Gdt = ff_mul(G, dt);

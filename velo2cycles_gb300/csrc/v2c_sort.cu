@@ -49,62 +49,71 @@ __global__ void k_count(const int32_t *cell, long n, int32_t *counts, int32_t *s
   slot[i] = base + __popc(grp & ((1u << lane) - 1));
 }
 
-// exclusive scan, three passes: per-block scan of 4 elements per thread
+// Exclusive scan in two launches.  First each block scans its SB * SE
+// elements (4 per thread) and leaves their sum; CLEAR also zeroes the input,
+// so that the sort's counters are zero again for its next call.
 constexpr int SB = 1024, SE = 4;
-__global__ void k_scan_block(const int32_t *in, long m, int32_t *out, int32_t *bsum) {
-  __shared__ int32_t sh[SB];
-  long base = (long)blockIdx.x * SB * SE + (long)threadIdx.x * SE;
+
+// inclusive scan of one value per thread over the block
+__device__ __forceinline__ int32_t block_scan(int32_t v, int32_t *warp_sum) {
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t t = __shfl_up_sync(V2C_FULL, v, o);
+    if (lane >= o) v += t;
+  }
+  if (lane == 31) warp_sum[wl] = v;
+  __syncthreads();
+  if (wl == 0) {
+    int32_t w = warp_sum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int32_t t = __shfl_up_sync(V2C_FULL, w, o);
+      if (lane >= o) w += t;
+    }
+    warp_sum[lane] = w;
+  }
+  __syncthreads();
+  return v + (wl > 0 ? warp_sum[wl - 1] : 0);
+}
+
+template <bool CLEAR>
+__global__ void __launch_bounds__(SB) k_scan_block(int32_t *in, long m, int32_t *out,
+                                                   int32_t *bsum) {
+  __shared__ int32_t ws[32];
+  const long base = (long)blockIdx.x * SB * SE + (long)threadIdx.x * SE;
   int32_t v[SE], s = 0;
 #pragma unroll
   for (int k = 0; k < SE; k++) {
     v[k] = (base + k < m) ? in[base + k] : 0;
     s += v[k];
   }
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int off = 1; off < SB; off <<= 1) {
-    int32_t t = (threadIdx.x >= off) ? sh[threadIdx.x - off] : 0;
-    __syncthreads();
-    sh[threadIdx.x] += t;
-    __syncthreads();
-  }
-  int32_t run = sh[threadIdx.x] - s;
+  const int32_t incl = block_scan(s, ws);
+  int32_t run = incl - s;
 #pragma unroll
   for (int k = 0; k < SE; k++) {
-    if (base + k < m) out[base + k] = run;
+    if (base + k < m) {
+      out[base + k] = run;
+      if (CLEAR) in[base + k] = 0;
+    }
     run += v[k];
   }
-  if (threadIdx.x == SB - 1) bsum[blockIdx.x] = sh[SB - 1];
+  if (threadIdx.x == SB - 1) bsum[blockIdx.x] = incl;
 }
 
-__global__ void k_scan_sums(int32_t *bsum, long nb, int32_t *total_out) {
-  // single block, sequential chunks of SB
-  __shared__ int32_t sh[SB];
-  __shared__ int32_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (long c0 = 0; c0 < nb; c0 += SB) {
-    long i = c0 + threadIdx.x;
-    int32_t v = (i < nb) ? bsum[i] : 0;
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int off = 1; off < SB; off <<= 1) {
-      int32_t t = (threadIdx.x >= off) ? sh[threadIdx.x - off] : 0;
-      __syncthreads();
-      sh[threadIdx.x] += t;
-      __syncthreads();
-    }
-    if (i < nb) bsum[i] = carry + sh[threadIdx.x] - v;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += sh[SB - 1];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *total_out = carry;
-}
-
-__global__ void k_scan_add(int32_t *out, long m, const int32_t *bsum) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i < m) out[i] += bsum[i / (SB * SE)];
+// Then each block adds the sum of the blocks before its own (each sums them
+// for itself: at most a thousand or so), and the last leaves the total.
+__global__ void __launch_bounds__(SB) k_scan_add(int32_t *out, long m, const int32_t *bsum,
+                                                 int nb) {
+  __shared__ int32_t ws[32];
+  int32_t s = 0;
+  for (int i = threadIdx.x; i < (int)blockIdx.x; i += SB) s += bsum[i];
+  block_scan(s, ws);
+  const int32_t before = ws[31];
+  const long base = (long)blockIdx.x * SB * SE;
+  if (before)
+    for (long i = base + threadIdx.x; i < min(base + SB * SE, m); i += SB) out[i] += before;
+  if (blockIdx.x == nb - 1 && threadIdx.x == 0) out[m] = before + bsum[nb - 1];
 }
 
 // key of marker i: quarter class in bits 30-31, array index below
@@ -280,21 +289,25 @@ void launch_assign(const Grid &g, const double *x, const double *y, long n, Mark
 
 long scan_blocks(long m) { return (m + SB * SE - 1) / (SB * SE); }
 
+namespace {
+// exclusive scan of in[0, m), m > 0
+template <bool CLEAR>
+void scan(int32_t *in, long m, int32_t *out, int32_t *blocksum, cudaStream_t st) {
+  const int nb = (int)scan_blocks(m);
+  k_scan_block<CLEAR><<<nb, SB, 0, st>>>(in, m, out, blocksum);
+  k_scan_add<<<nb, SB, 0, st>>>(out, m, blocksum, nb);
+}
+}  // namespace
+
 void launch_scan(const int32_t *in, long m, int32_t *out, int32_t *blocksum, cudaStream_t st) {
-  const long nb = scan_blocks(m);
-  if (nb > 0) k_scan_block<<<(unsigned)nb, SB, 0, st>>>(in, m, out, blocksum);
-  k_scan_sums<<<1, SB, 0, st>>>(blocksum, nb, out + m);
-  if (m > 0) k_scan_add<<<nblk(m, 256), 256, 0, st>>>(out, m, blocksum);
+  if (m > 0) scan<false>(const_cast<int32_t *>(in), m, out, blocksum, st);
+  else cudaMemsetAsync(out, 0, sizeof(int32_t), st);
 }
 
 void launch_sort(const int32_t *cell, const float *u, const float *v, long n, long ncell,
                  SortBufs &b, unsigned long long *stat, cudaStream_t st) {
-  cudaMemsetAsync(b.counts, 0, sizeof(int32_t) * ncell, st);
   if (n > 0) k_count<<<nblk(n, 256), 256, 0, st>>>(cell, n, b.counts, b.slot);
-  long nb = (ncell + SB * SE - 1) / (SB * SE);
-  k_scan_block<<<(unsigned)nb, SB, 0, st>>>(b.counts, ncell, b.start, b.blocksum);
-  k_scan_sums<<<1, SB, 0, st>>>(b.blocksum, nb, b.start + ncell);
-  k_scan_add<<<nblk(ncell, 256), 256, 0, st>>>(b.start, ncell, b.blocksum);
+  scan<true>(b.counts, ncell, b.start, b.blocksum, st);
   uint32_t *keys = reinterpret_cast<uint32_t *>(b.tmp);
   if (n > 0) k_slots<<<nblk(n, 256), 256, 0, st>>>(cell, u, v, n, b.start, b.slot, keys);
   k_rank<<<nblk((ncell + RG - 1) / RG * 32, 256), 256, 0, st>>>(b.start, ncell, keys, b.perm,

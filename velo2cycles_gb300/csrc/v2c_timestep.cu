@@ -16,7 +16,8 @@
 // node range and walks it in 32-node slices; segment states combine with
 //   (A then B): reset = A.reset | B.reset, all = min(A.all, B.all),
 //               after = B.reset ? B.after : min(A.after, B.all),
-// which is associative, so the warp ranges fold in order in a tree.  The
+// which is associative, so the warp ranges fold in order in a tree (lanes,
+// warps of a block, blocks: adjacent pairs at every level).  The
 // lambda carry crosses slices but not warp ranges: a NaN-chi node at the
 // start of a range takes 1/5 (MINV(NaN, 1/5) in the reference's order).
 // chi == 0 (where the reference stops) sets an error flag.
@@ -53,26 +54,128 @@ __device__ __forceinline__ int ts_kind(int k) {  // 0 min, 1 max, 2 sum, 3 order
   }
 }
 
-__device__ __forceinline__ void ts_init(double *s) {
-  for (int k = 0; k < TS_N; k++) s[k] = 0.0;
-  s[TS_DTNVP] = s[TS_DTD] = s[TS_PHI_ALL] = s[TS_L_ALL] = s[TS_PHI_AFTER] = s[TS_L_AFTER] = 1e30;
-  s[TS_MINS0] = s[TS_MINV0] = s[TS_MINS1] = s[TS_MINV1] = 1e30;
+// Entry k of "A then B" (B follows A in node order)
+__device__ __forceinline__ double ts_combined(int k, const double *a, const double *b) {
+  const int kind = ts_kind(k);
+  if (kind == 0) return b[k] <= a[k] ? b[k] : a[k];
+  if (kind == 1) return b[k] >= a[k] ? b[k] : a[k];
+  if (kind == 2) return a[k] + b[k];
+  const bool br = b[TS_RESET] != 0.0;
+  if (k == TS_RESET) return (a[TS_RESET] != 0.0 || br) ? 1.0 : 0.0;
+  if (k == TS_PHI_ALL || k == TS_L_ALL) return b[k] <= a[k] ? b[k] : a[k];
+  const double all = b[k == TS_PHI_AFTER ? TS_PHI_ALL : TS_L_ALL];
+  return br ? b[k] : (all <= a[k] ? all : a[k]);
 }
 
-// a := a then b (b follows a in node order)
-__device__ __forceinline__ void ts_combine(double *a, const double *b) {
-  for (int k = 0; k < TS_N; k++) {
-    const int kind = ts_kind(k);
-    if (kind == 0) a[k] = b[k] <= a[k] ? b[k] : a[k];
-    else if (kind == 1) a[k] = b[k] >= a[k] ? b[k] : a[k];
-    else if (kind == 2) a[k] += b[k];
+// Fold n partials in order, pairs (2i, 2i+1) at each level, a warp per pair
+// and a lane per entry; the result is partial 0.  All threads of the block.
+__device__ __forceinline__ void ts_fold(double (*p)[TS_N], long n, int warp, int warps, int lane) {
+  for (long step = 1; step < n; step <<= 1) {
+    for (long i = warp; 2 * i * step + step < n; i += warps) {
+      double *A = p[2 * i * step];
+      const double *B = p[2 * i * step + step];
+      const double v = lane < TS_N ? ts_combined(lane, A, B) : 0.0;
+      __syncwarp();
+      if (lane < TS_N) A[lane] = v;
+    }
+    __syncthreads();
   }
-  const bool br = b[TS_RESET] != 0.0;
-  a[TS_PHI_AFTER] = br ? b[TS_PHI_AFTER] : (b[TS_PHI_ALL] <= a[TS_PHI_AFTER] ? b[TS_PHI_ALL] : a[TS_PHI_AFTER]);
-  a[TS_L_AFTER] = br ? b[TS_L_AFTER] : (b[TS_L_ALL] <= a[TS_L_AFTER] ? b[TS_L_ALL] : a[TS_L_AFTER]);
-  a[TS_PHI_ALL] = b[TS_PHI_ALL] <= a[TS_PHI_ALL] ? b[TS_PHI_ALL] : a[TS_PHI_ALL];
-  a[TS_L_ALL] = b[TS_L_ALL] <= a[TS_L_ALL] ? b[TS_L_ALL] : a[TS_L_ALL];
-  a[TS_RESET] = (a[TS_RESET] != 0.0 || br) ? 1.0 : 0.0;
+}
+
+// One warp's running state.  The minima and maxima are FP32 values (the node
+// arithmetic is FP32), kept and folded as such: FP64 compares run at 1/64 of
+// the rate.  Their FP64 initial value 1e30 is put back at the end.
+enum {
+  F_DTNVP = 0, F_DTD, F_MINS0, F_MINV0, F_MINS1, F_MINV1,              // minima
+  F_MAXVX, F_MAXVEL, F_MAXS0, F_MAXV0, F_MAXS1, F_MAXV1,               // maxima
+  F_N,
+  D_NR0 = 0, D_SUMS0, D_SUM2S0, D_SUMV0, D_SUM2V0, D_NR1, D_SUMS1, D_SUM2S1, D_SUMV1, D_SUM2V1,
+  D_N
+};
+constexpr int F_MINS = F_MAXVX;
+struct TsState {
+  float f[F_N];
+  double d[D_N];
+  float all[2], after[2];  // state limit, slip-length limit
+  bool reset;
+  __device__ __forceinline__ void init() {
+#pragma unroll
+    for (int k = 0; k < F_N; k++) f[k] = k < F_MINS ? INFINITY : 0.f;
+#pragma unroll
+    for (int k = 0; k < D_N; k++) d[k] = 0.0;
+    all[0] = all[1] = after[0] = after[1] = INFINITY;
+    reset = false;
+  }
+};
+__device__ __forceinline__ float ts_min(float a, float b) { return b <= a ? b : a; }
+__device__ __forceinline__ float ts_max(float a, float b) { return b >= a ? b : a; }
+
+// fold the warp's lanes in order (adjacent pairs, lower lane first); the
+// statistics of sticky01 == 1 and == 2 nodes only where a lane has some
+__device__ __forceinline__ void ts_fold_lanes(TsState &s, bool any0, bool any1, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const bool take = (lane & (2 * o - 1)) == 0;
+    auto stat = [&](int fmin, int fmax, int d0) {
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const float mn = __shfl_down_sync(V2C_FULL, s.f[fmin + k], o);
+        const float mx = __shfl_down_sync(V2C_FULL, s.f[fmax + k], o);
+        if (take) { s.f[fmin + k] = ts_min(s.f[fmin + k], mn); s.f[fmax + k] = ts_max(s.f[fmax + k], mx); }
+      }
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+        const double v = __shfl_down_sync(V2C_FULL, s.d[d0 + k], o);
+        if (take) s.d[d0 + k] += v;
+      }
+    };
+    if (any0) stat(F_MINS0, F_MAXS0, D_NR0);
+    if (any1) stat(F_MINS1, F_MAXS1, D_NR1);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const float mn = __shfl_down_sync(V2C_FULL, s.f[F_DTNVP + k], o);
+      const float mx = __shfl_down_sync(V2C_FULL, s.f[F_MAXVX + k], o);
+      if (take) { s.f[F_DTNVP + k] = ts_min(s.f[F_DTNVP + k], mn); s.f[F_MAXVX + k] = ts_max(s.f[F_MAXVX + k], mx); }
+    }
+    const bool br = __shfl_down_sync(V2C_FULL, (int)s.reset, o);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const float ball = __shfl_down_sync(V2C_FULL, s.all[k], o);
+      const float baft = __shfl_down_sync(V2C_FULL, s.after[k], o);
+      if (take) {
+        s.after[k] = br ? baft : ts_min(s.after[k], ball);
+        s.all[k] = ts_min(s.all[k], ball);
+      }
+    }
+    if (take) s.reset = s.reset || br;
+  }
+}
+// a := a then b
+__device__ __forceinline__ void ts_append(TsState &a, const TsState &b) {
+#pragma unroll
+  for (int k = 0; k < F_N; k++) a.f[k] = k < F_MINS ? ts_min(a.f[k], b.f[k]) : ts_max(a.f[k], b.f[k]);
+#pragma unroll
+  for (int k = 0; k < D_N; k++) a.d[k] += b.d[k];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    a.after[k] = b.reset ? b.after[k] : ts_min(a.after[k], b.all[k]);
+    a.all[k] = ts_min(a.all[k], b.all[k]);
+  }
+  a.reset = a.reset || b.reset;
+}
+__device__ __forceinline__ void ts_store(const TsState &s, double *p) {
+  auto lim = [](float v) { return (double)v <= 1e30 ? (double)v : 1e30; };
+  p[TS_DTNVP] = lim(s.f[F_DTNVP]); p[TS_DTD] = lim(s.f[F_DTD]);
+  p[TS_MAXVX] = s.f[F_MAXVX]; p[TS_MAXVEL] = s.f[F_MAXVEL];
+  p[TS_PHI_ALL] = lim(s.all[0]); p[TS_L_ALL] = lim(s.all[1]);
+  p[TS_PHI_AFTER] = lim(s.after[0]); p[TS_L_AFTER] = lim(s.after[1]);
+  p[TS_RESET] = s.reset ? 1.0 : 0.0;
+  p[TS_NR0] = s.d[D_NR0]; p[TS_MAXS0] = s.f[F_MAXS0]; p[TS_MINS0] = lim(s.f[F_MINS0]);
+  p[TS_SUMS0] = s.d[D_SUMS0]; p[TS_SUM2S0] = s.d[D_SUM2S0]; p[TS_MAXV0] = s.f[F_MAXV0];
+  p[TS_MINV0] = lim(s.f[F_MINV0]); p[TS_SUMV0] = s.d[D_SUMV0]; p[TS_SUM2V0] = s.d[D_SUM2V0];
+  p[TS_NR1] = s.d[D_NR1]; p[TS_MAXS1] = s.f[F_MAXS1]; p[TS_MINS1] = lim(s.f[F_MINS1]);
+  p[TS_SUMS1] = s.d[D_SUMS1]; p[TS_SUM2S1] = s.d[D_SUM2S1]; p[TS_MAXV1] = s.f[F_MAXV1];
+  p[TS_MINV1] = lim(s.f[F_MINV1]); p[TS_SUMV1] = s.d[D_SUMV1]; p[TS_SUM2V1] = s.d[D_SUM2V1];
 }
 
 struct TsArgs {
@@ -82,11 +185,13 @@ struct TsArgs {
   v2c_timestep_ctl c;
   int oldornew;
   long per_warp;   // nodes per warp range (a multiple of 32)
-  double *part;    // [warps][TS_N]
+  double *part;    // [blocks][TS_N]
   double *out;     // [TS_OUT_N]
 };
 
-// node pass: one warp per contiguous range
+// node pass: one warp per contiguous range, the block's warps folded at its
+// end (301 x 101 lines: 22 us with FP64 minima and a serial fold per lane,
+// 16 us)
 __global__ void __launch_bounds__(TW * 32) k_ts_nodes(TsArgs a) {
   const Grid &g = a.g;
   const Nodes &N = a.N;
@@ -95,17 +200,18 @@ __global__ void __launch_bounds__(TW * 32) k_ts_nodes(TsArgs a) {
   const long warp = (long)blockIdx.x * TW + (threadIdx.x >> 5);
   const long lo = warp * a.per_warp, hi = min(lo + a.per_warp, g.nn);
   const long yn = g.yn;
-  double s[TS_N];
-  ts_init(s);
+  __shared__ double part[TW][TS_N];
+  TsState s;
+  s.init();
   float lam_carry = __int_as_float(0x7fc00000);  // NaN: none yet
   for (long b0 = lo; b0 < hi; b0 += 32) {
     const long m3 = b0 + lane;
     const long m2 = m3 % yn, m1 = (m3 - m2) / yn;
     const bool interior = m3 < hi && m1 >= 1 && m2 >= 1 && m1 < g.xn - 1 && m2 < yn - 1;
-    double d[TS_N];
-    ts_init(d);
+    TsState d;
+    d.init();
     bool rsf_node = false, chi_ok = false, reset = false, has_phi = false;
-    float lam_raw = 0.f, LoV = 0.f, dtphi = 0.f;
+    float lam_raw = 0.f, LoV = 0.f, dtphi = 0.f, st = 0.f;
     if (interior) {
       const float dx = __ldg(g.wx + m1), dy = __ldg(g.wy + m2);
       const float faultwidth = 2.f * 0.5f * (dx + dy);
@@ -123,14 +229,14 @@ __global__ void __launch_bounds__(TW * 32) k_ts_nodes(TsArgs a) {
       } else {
         NUVP = (nu_m2c > 1.00e+26f) ? N.f(V2C_NF_NU)[m3] : 5.00e+26f;
       }
-      d[TS_DTNVP] = (float)a.c.tcnvp * NUVP / gg;
+      d.f[F_DTNVP] = (float)a.c.tcnvp * NUVP / gg;
       const float VXn = a.oldornew == 1 ? N.f(V2C_NF_VX)[m3] : N.f(V2C_NF_MVX)[m3];
       const float VYn = a.oldornew == 1 ? N.f(V2C_NF_VY)[m3] : N.f(V2C_NF_MVY)[m3];
       if (VXn != 0.f && VYn != 0.f) {
         const float ax = fabsf(VXn), ay = fabsf(VYn);
-        d[TS_MAXVX] = ax >= ay ? ax : ay;
+        d.f[F_MAXVX] = ax >= ay ? ax : ay;
         const float rx = fabsf(VXn / dx), ry = fabsf(VYn / dy);
-        d[TS_DTD] = (float)a.c.tcd * 1.f / (rx >= ry ? rx : ry);
+        d.f[F_DTD] = (float)a.c.tcd * 1.f / (rx >= ry ? rx : ry);
       }
       if (P.RSFmode == 1) {
         rsf_node = true;
@@ -162,22 +268,24 @@ __global__ void __launch_bounds__(TW * 32) k_ts_nodes(TsArgs a) {
         }
       }
       const float sx = N.f(V2C_NF_SXXS)[m3], sy = N.f(V2C_NF_SXY)[m3];
-      const double sg = sqrtf(sx * sx + sy * sy), nv = N.f(V2C_NF_NU)[m3];
-      const float st = N.f(V2C_NF_STICKY01)[m3];
-      if (st == 2.f) {
-        const double l = log10(nv);
-        d[TS_NR1] = 1; d[TS_MAXS1] = d[TS_MINS1] = d[TS_SUMS1] = sg; d[TS_SUM2S1] = sg * sg;
-        d[TS_MAXV1] = d[TS_MINV1] = nv; d[TS_SUMV1] = l; d[TS_SUM2V1] = l * l;
-      }
-      if (st == 1.f) {
-        const double l = log10(nv);
-        d[TS_NR0] = 1; d[TS_MAXS0] = d[TS_MINS0] = d[TS_SUMS0] = sg; d[TS_SUM2S0] = sg * sg;
-        d[TS_MAXV0] = d[TS_MINV0] = nv; d[TS_SUMV0] = l; d[TS_SUM2V0] = l * l;
-        if (m1 == 50 && m2 == 50) { a.out[TS_P1S] = sg; a.out[TS_P1V] = nv; }
-        if (m1 == 500 && m2 == 50) { a.out[TS_P2S] = sg; a.out[TS_P2V] = nv; }
+      const float sgf = sqrtf(sx * sx + sy * sy), nvf = N.f(V2C_NF_NU)[m3];
+      st = N.f(V2C_NF_STICKY01)[m3];
+      if (st == 1.f || st == 2.f) {
+        const double sg = sgf, l = log10((double)nvf);
+        if (st == 2.f) {
+          d.f[F_MINS1] = d.f[F_MAXS1] = sgf; d.f[F_MINV1] = d.f[F_MAXV1] = nvf;
+          d.d[D_NR1] = 1; d.d[D_SUMS1] = sg; d.d[D_SUM2S1] = sg * sg;
+          d.d[D_SUMV1] = l; d.d[D_SUM2V1] = l * l;
+        } else {
+          d.f[F_MINS0] = d.f[F_MAXS0] = sgf; d.f[F_MINV0] = d.f[F_MAXV0] = nvf;
+          d.d[D_NR0] = 1; d.d[D_SUMS0] = sg; d.d[D_SUM2S0] = sg * sg;
+          d.d[D_SUMV0] = l; d.d[D_SUM2V0] = l * l;
+          if (m1 == 50 && m2 == 50) { a.out[TS_P1S] = sg; a.out[TS_P1V] = nvf; }
+          if (m1 == 500 && m2 == 50) { a.out[TS_P2S] = sg; a.out[TS_P2V] = nvf; }
+        }
       }
       const float V = a.oldornew == 0 ? N.f(V2C_NF_RK_SLIPRS_FINAL)[m3] : N.f(V2C_NF_RK_SLIPRS_SOLVED)[m3];
-      if (V > 0.f) d[TS_MAXVEL] = V;
+      if (V > 0.f) d.f[F_MAXVEL] = V;
     }
     // lambda: the node's own, or that of the last earlier node with a
     // defined chi (within the slice, else carried from earlier slices)
@@ -189,50 +297,54 @@ __global__ void __launch_bounds__(TW * 32) k_ts_nodes(TsArgs a) {
     if (okm) lam_carry = __shfl_sync(V2C_FULL, lam_raw, 31 - __clz(okm));
     if (rsf_node) {
       if (reset) {
-        d[TS_RESET] = 1.0;
+        d.reset = true;
       } else if (has_phi) {
         const float lamc = lam <= 0.2f ? lam : 0.2f;  // MINV(lambda, 1/5)
-        const double dl = lamc * LoV;
-        d[TS_PHI_ALL] = d[TS_PHI_AFTER] = dtphi;
-        d[TS_L_ALL] = d[TS_L_AFTER] = dl;
+        d.all[0] = d.after[0] = dtphi;
+        d.all[1] = d.after[1] = lamc * LoV;
       }
     }
-    // fold the slice in lane order (adjacent pairs, lower lane first)
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      double e[TS_N];
-#pragma unroll
-      for (int k = 0; k < TS_N; k++) e[k] = __shfl_down_sync(V2C_FULL, d[k], o);
-      if ((lane & (2 * o - 1)) == 0 && lane + o < 32) ts_combine(d, e);
-    }
-    if (lane == 0) ts_combine(s, d);
+    ts_fold_lanes(d, __any_sync(V2C_FULL, st == 1.f), __any_sync(V2C_FULL, st == 2.f), lane);
+    if (lane == 0) ts_append(s, d);
   }
-  if (lane == 0) {
-    double *p = a.part + warp * TS_N;
-    for (int k = 0; k < TS_N; k++) p[k] = s[k];
-  }
+  const int wl = threadIdx.x >> 5;
+  if (lane == 0) ts_store(s, part[wl]);
+  __syncthreads();
+  ts_fold(part, TW, wl, TW, lane);
+  if (threadIdx.x < TS_N) a.part[(long)blockIdx.x * TS_N + threadIdx.x] = part[0][threadIdx.x];
 }
 
-// fold the warp partials in order: pairs (2i, 2i+1) at each level
-__global__ void k_ts_fold(double *part, long nw, double *out) {
-  for (long step = 1; step < nw; step <<= 1) {
-    for (long i = threadIdx.x; 2 * i * step + step < nw; i += blockDim.x) {
-      double *A = part + (2 * i * step) * TS_N;
-      const double *B = part + (2 * i * step + step) * TS_N;
-      ts_combine(A, B);
-    }
-    __syncthreads();
+// fold the block partials in order, in shared memory (301 x 101 lines: 68 us
+// as a tree in global memory with a thread per pair, 17 us)
+constexpr int TF = 16;  // warps
+// The results go to the host's memory, and the slots that the node pass sets
+// by hand are zero again for the next call.
+__global__ void __launch_bounds__(TF * 32) k_ts_fold(const double *part, int nb, double *out,
+                                                     double *result) {
+  extern __shared__ double p[][TS_N];
+  for (int i = threadIdx.x; i < nb * TS_N; i += TF * 32) p[i / TS_N][i % TS_N] = part[i];
+  __syncthreads();
+  ts_fold(p, nb, threadIdx.x >> 5, TF, threadIdx.x & 31);
+  const int t = threadIdx.x;
+  if (t < TS_OUT_N) {
+    result[t] = t < TS_N ? p[0][t] : out[t];
+    out[t] = 0.0;
   }
-  if (threadIdx.x < TS_N) out[threadIdx.x] = part[threadIdx.x];
 }
+static_assert(TS_OUT_N <= RESULT_DOUBLES, "result buffer");
+constexpr long TS_MAX_WARPS = 152 * 4 * TW;
 
 }  // namespace
 
+cudaError_t timestep_init() {
+  return cudaFuncSetAttribute(k_ts_fold, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(sizeof(double) * TS_N * (TS_MAX_WARPS / TW)));
+}
+
 int calc_timestep_device(const Grid &g, const Nodes &N, const Scal &S, const v2c_timestep_ctl &c,
                          int oldornew, double *scratch, long scratch_doubles,
-                         v2c_timestep_info *info, cudaStream_t st) {
-  const long warps_max = 152 * 4 * TW;
-  long per_warp = (g.nn + warps_max - 1) / warps_max;
+                         double *result, v2c_timestep_info *info, cudaStream_t st) {
+  long per_warp = (g.nn + TS_MAX_WARPS - 1) / TS_MAX_WARPS;
   per_warp = (per_warp + 31) / 32 * 32;
   const long warps = (g.nn + per_warp - 1) / per_warp;
   if ((warps + 1) * TS_N + TS_OUT_N > scratch_doubles) return V2C_ERR_CAPACITY;
@@ -240,15 +352,14 @@ int calc_timestep_device(const Grid &g, const Nodes &N, const Scal &S, const v2c
   a.g = g; a.N = N; a.S = S; a.c = c; a.oldornew = oldornew; a.per_warp = per_warp;
   a.out = scratch;
   a.part = scratch + TS_OUT_N;
-  if (cudaMemsetAsync(a.out, 0, sizeof(double) * TS_OUT_N, st) != cudaSuccess) return V2C_ERR_CUDA;
   const long blocks = (warps + TW - 1) / TW;
   // warps past the node range write empty partials
   k_ts_nodes<<<(unsigned)blocks, TW * 32, 0, st>>>(a);
-  k_ts_fold<<<1, 512, 0, st>>>(a.part, blocks * TW, a.out);
-  double h[TS_OUT_N];
-  if (cudaMemcpyAsync(h, a.out, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
+  k_ts_fold<<<1, TF * 32, sizeof(double) * TS_N * blocks, st>>>(a.part, (int)blocks, a.out,
+                                                                  result);
+  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
     return V2C_ERR_CUDA;
+  const double *h = result;
   if (h[TS_CHI0] != 0.0) return V2C_ERR_TIMESTEP;
   const double dtphi = h[TS_RESET] != 0.0 ? (h[TS_PHI_AFTER] <= c.maxtmstep ? h[TS_PHI_AFTER] : c.maxtmstep)
                                           : h[TS_PHI_ALL];
