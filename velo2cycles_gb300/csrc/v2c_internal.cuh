@@ -81,7 +81,23 @@ struct Grid {
   int xn, yn, ncx, ncy;
   long nn;
   double xsize, ysize;
+  unsigned div_m;  // c / ncy = c div_m >> 31 + div_s for 0 <= c < 2^31
+  int div_s;
+  // cell column and row of cell c = ix ncy + iy, without the division
+  __device__ __forceinline__ void cell_at(int c, int &ix, int &iy) const {
+    ix = (int)(((unsigned long long)(unsigned)c * div_m) >> (31 + div_s));
+    iy = c - ix * ncy;
+  }
 };
+
+// div_s = ceil(log2 d), div_m = floor(2^(31 + div_s) / d) + 1: with
+// e = div_m d - 2^(31 + div_s) in (0, d], the quotient's error
+// c e / (d 2^(31 + div_s)) stays below 1 / d for every c < 2^31.
+inline void set_divider(Grid &g) {
+  g.div_s = 0;
+  while ((1l << g.div_s) < g.ncy) g.div_s++;
+  g.div_m = (unsigned)((1ull << (31 + g.div_s)) / (unsigned)g.ncy + 1);
+}
 
 struct Nodes {
   float *base;

@@ -660,14 +660,14 @@ template <bool BS, bool PLAIN>
 __global__ void __launch_bounds__(256, 6) k_gather(N2MArgs a) {
   const Grid &g = a.g;
   const Nodes &N = a.N;
-  const int ncy = g.ncy;
   const v2c_params &P = a.S.p;
   const long yn = g.yn;
   const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (s >= a.n) return;
   const int idx = __ldg(a.perm + s);
   const int c = a.m.cell_in[idx];
-  const int ix = c / ncy, iy = c - ix * ncy;
+  int ix, iy;
+  g.cell_at(c, ix, iy);
   const float u = a.m.u_in[idx], v = a.m.v_in[idx];
   const int t = a.m.type[idx];
   // interpolate_mechanical clamps the point into the model first
@@ -840,21 +840,31 @@ __global__ void __launch_bounds__(128) k_n2m_bs_mode1(N2MArgs a) {
 
 // ----------------------------------------------------------- the move
 // moveandrotatemarkers (moveandrotatemarkers.c:1-178), one thread per
-// marker in cell order: Euler or RK4 through allinteri, stress rotation,
-// markers from depth, out-of-grid reset.  New positions go to the second
-// position buffer.
-__global__ void __launch_bounds__(256) k_move(N2MArgs a) {
+// marker: Euler or RK4 through allinteri, stress rotation, markers from
+// depth, out-of-grid reset.  New positions go to the second position buffer.
+// In array order, which stays near cell order (the markers of a warp share
+// their cells' forms in L1): the sort's order would make ten marker arrays
+// follow the permutation.  Bound by the latency of the integration's chain
+// of form reads, so six resident CTAs, and the stresses, which are rotated
+// after it, are asked for at the start.  4001 x 1001 lines, 60 M markers,
+// with the quarters' forms: 1725 -> 1525 us (1616 in array order alone, 1566
+// with the stresses asked for).
+__global__ void __launch_bounds__(256, 6) k_move(N2MArgs a) {
   const Grid &g = a.g;
   const v2c_params &P = a.S.p;
   const int ncy = g.ncy;
   const float dt = a.S.dt;
-  for (long s = blockIdx.x * (long)blockDim.x + threadIdx.x; s < a.n;
-       s += (long)gridDim.x * blockDim.x) {
-    const int idx = __ldg(a.perm + s);
+  {
+    const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (idx >= a.n) return;
     const int c = a.m.cell_in[idx];
-    const int ix = c / ncy, iy = c - ix * ncy;
+    int ix, iy;
+    g.cell_at(c, ix, iy);
     const float u = a.m.u_in[idx], v = a.m.v_in[idx];
     const int t = a.m.type[idx];
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(a.m.sxx + idx));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(a.m.sxy + idx));
+    float tk = a.m.tk[idx];
     const bool in_grid = (ix > 0 || u >= 0.f) && (ix < g.ncx - 1 || u <= 1.f) &&
                          (iy > 0 || v >= 0.f) && (iy < g.ncy - 1 || v <= 1.f);
     int nix = ix, niy = iy;
@@ -921,7 +931,7 @@ __global__ void __launch_bounds__(256) k_move(N2MArgs a) {
         // (markk, markv), as it does when it strays more than ystpy from it
         const bool inside = (nix > 0 || nu_ >= 0.f) && (nix < g.ncx - 1 || nu_ <= 1.f) &&
                             (niy > 0 || nv_ >= 0.f) && (niy < g.ncy - 1 || nv_ <= 1.f);
-        const double ax = (double)a.m.tk[idx] + (double)a.m.tk_lo[idx];
+        const double ax = (double)tk + (double)a.m.tk_lo[idx];
         const double ay = (double)a.m.mv[idx] + (double)a.m.mv_lo[idx];
         double x = g.gx[nix] + (double)nu_ * (g.gx[nix + 1] - g.gx[nix]);
         double y = g.gy[niy] + (double)nv_ * (g.gy[niy + 1] - g.gy[niy]);
@@ -964,7 +974,7 @@ __global__ void __launch_bounds__(256) k_move(N2MArgs a) {
       // (the temperature pair's high word decides tk < tdeep; the two can
       // differ only for a temperature within half an FP32 ulp of tdeep, where
       // resetting or not leaves the same temperature to that half ulp)
-      float tk = a.m.tk[idx], tk_lo = 0.f;
+      float tk_lo = 0.f;
       bool reset = false;
       if (vy0 < 0.f && tk < a.S.tdeep_f &&
           __ldg(a.gyf + niy) + nv_ * __ldg(g.wy + niy) > a.S.zdeep_lo_f) {
@@ -1029,9 +1039,7 @@ void launch_move(const N2MArgs &a, cudaStream_t st) {
   const long quarters = (long)a.g.ncx * a.g.ncy * 4;
   k_vel_quads<<<(unsigned)((quarters + 255) / 256), 256, 0, st>>>(a.g, a.N, a.quad);
   if (a.n <= 0) return;
-  long blocks = (a.n + 255) / 256;
-  if (blocks > 152 * 8 * 4) blocks = 152 * 8 * 4;
-  k_move<<<(unsigned)blocks, 256, 0, st>>>(a);
+  k_move<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a);
 }
 
 }  // namespace v2c

@@ -73,7 +73,8 @@ __device__ __forceinline__ void marker_problem(const PhysArgs &a, long i, const 
   const Grid &g = a.g;
   const v2c_params &P = a.S.p;
   const int c = a.m.cell_in[i];
-  const int ix = c / g.ncy, iy = c - ix * g.ncy;
+  int ix, iy;
+  g.cell_at(c, ix, iy);
   const float u = a.m.u_in[i], v = a.m.v_in[i];
   t = a.m.type[i];
   Fric fr{0.f, 0.f, 1.f, 1.f, 0.f};
@@ -119,7 +120,8 @@ __global__ void __launch_bounds__(PT, 8) k_phys(PhysArgs a) {
     Fric fr{0.f, 0.f, 1.f, 1.f, 0.f};
     if (valid) {
       const int c = a.m.cell_in[i];
-      const int ix = c / g.ncy, iy = c - ix * g.ncy;
+      int ix, iy;
+      g.cell_at(c, ix, iy);
       const float u = a.m.u_in[i], v = a.m.v_in[i];
       t = a.m.type[i];
       // sticky-air flag candidates: every marker, last in reference order wins

@@ -56,7 +56,8 @@ __global__ void k_temp_markers(TempArgs a) {
     a.wt[s] = 0.f;
     const int idx = __ldg(a.perm + s);
     const int c = a.m.cell_in[idx];
-    const int ix = c / g.ncy, iy = c - ix * g.ncy;
+    int ix, iy;
+    g.cell_at(c, ix, iy);
     const float u = a.m.u_in[idx], v = a.m.v_in[idx];
     const int t = a.m.type[idx];
     if (t >= 100 || !inside_model(g, ix, iy, u, v)) continue;
@@ -128,7 +129,8 @@ __global__ void k_temp_anti(TempArgs a) {
     if (a.wt[s] == 0.f) continue;  // rock markers inside the model only
     const int idx = __ldg(a.perm + s);
     const int c = a.m.cell_in[idx];
-    const int ix = c / g.ncy, iy = c - ix * g.ncy;
+    int ix, iy;
+    g.cell_at(c, ix, iy);
     const float t = a.tol[(long)ix * g.yn + iy];
     if (t != 0.f) {
       const float u = a.m.u_in[idx], v = a.m.v_in[idx];
