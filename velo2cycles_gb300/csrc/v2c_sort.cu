@@ -21,7 +21,7 @@ __global__ void k_assign(Grid g, const double *x, const double *y, long n, Marke
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   double xi = x[i], yi = y[i];
-  int ix = nsearch64(g.gx, g.xn, xi), iy = nsearch64(g.gy, g.yn, yi);
+  int ix = nsearch_bits(g.gx, g.xn, xi), iy = nsearch_bits(g.gy, g.yn, yi);
   double u = (xi - g.gx[ix]) / (g.gx[ix + 1] - g.gx[ix]);
   double v = (yi - g.gy[iy]) / (g.gy[iy + 1] - g.gy[iy]);
   m.cell_in[i] = ix * g.ncy + iy;

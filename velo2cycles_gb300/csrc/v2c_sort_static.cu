@@ -31,20 +31,21 @@ constexpr long MAX_BLOCKS = (MAX_CELLS + SB * SE - 1) / (SB * SE);
 constexpr long SCRATCH_WORDS = MAX_CELLS + MAX_BLOCKS;  // counters, then block sums
 
 // 4 Mi counters + 1 Ki block sums = 16 MiB + 4 KiB per device.  The counters
-// must be zero before the counting pass and again before the fill pass; every
-// call zeroes them itself on its stream, so nothing has to be zero on entry.
+// must be zero before the counting pass; every call zeroes them itself on its
+// stream, so nothing has to be zero on entry.
 static __device__ __align__(256) int32_t g_scratch[SCRATCH_WORDS];
 
 constexpr int MAX_DEVICES = 64;
 std::mutex g_setup_mu;
 int32_t *g_scratch_ptr[MAX_DEVICES] = {};
 
-__global__ void k_assign_count(const double *gx, int xn, const double *gy, int yn,
-                               const double *x, const double *y, long n, int32_t *cell,
-                               int32_t *count) {
+__global__ void __launch_bounds__(256) k_assign_count(const double *gx, int xn, const double *gy,
+                                                      int yn, const double *x, const double *y,
+                                                      long n, int32_t *cell, int32_t *count) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int ix = nsearch64(gx, xn, x[i]), iy = nsearch64(gy, yn, y[i]);
+  const double xi = x[i], yi = y[i];
+  const int ix = nsearch_bits(gx, xn, xi), iy = nsearch_bits(gy, yn, yi);
   const int c = ix * (yn - 1) + iy;
   cell[i] = c;
   atomicAdd(count + c, 1);
@@ -98,39 +99,46 @@ __global__ void k_scan_add_s(int32_t *out, long m, const int32_t *bsum) {
   if (i < m) out[i] += bsum[i / (SB * SE)];
 }
 
-// every marker takes a slot in its cell's segment (slot order is whatever
-// the atomics give; k_order_cells makes it index order)
-__global__ void k_fill(const int32_t *cell, long n, const int32_t *start, int32_t *cursor,
-                       int32_t *perm) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int c = cell[i];
-  perm[start[c] + atomicAdd(cursor + c, 1)] = (int32_t)i;
+// every marker takes a slot in its cell's segment, counting the cell's
+// counter back down (slot order is whatever the atomics give; k_order_cells
+// makes it index order).  FM markers per thread, so that FM atomics and then
+// FM stores are in flight: 9 M markers 61 -> 56 us.
+constexpr int FM = 4;
+__global__ void __launch_bounds__(256) k_fill(const int32_t *cell, long n, const int32_t *start,
+                                              int32_t *count, int32_t *perm) {
+  const long i0 = blockIdx.x * (256l * FM) + threadIdx.x;
+  int c[FM], at[FM];
+#pragma unroll
+  for (int k = 0; k < FM; k++) c[k] = i0 + 256 * k < n ? cell[i0 + 256 * k] : -1;
+#pragma unroll
+  for (int k = 0; k < FM; k++)
+    if (c[k] >= 0) at[k] = __ldg(start + c[k]) + atomicSub(count + c[k], 1) - 1;
+#pragma unroll
+  for (int k = 0; k < FM; k++)
+    if (c[k] >= 0) perm[at[k]] = (int32_t)(i0 + 256 * k);
 }
 
-// One warp per cell sorts the cell's segment of perm ascending, in place.
-// Up to 32 entries: rank in registers, then write.  Longer segments: a
-// bitonic network in the form whose every compare puts the smaller value at
-// the lower position (first stage of each merge compares a with its mirror
-// in the block), so positions past the segment act as +infinity and are
-// never touched.  Every position is in one pair per stage; __syncwarp()
-// orders the stages' global-memory accesses among the warp's lanes.
-__global__ void k_order_cells(const int32_t *start, long ncell, int32_t *perm) {
-  const long c = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (c >= ncell) return;  // uniform across the warp
-  const int s = start[c], L = start[c + 1] - s;
-  if (L < 2) return;
-  int32_t *p = perm + s;
-  if (L <= 32) {
-    const int32_t v = (lane < L) ? p[lane] : INT_MAX;
-    int rank = 0;
+// ascending over the warp's lanes (W = 32) or each of its halves (W = 16)
+template <int W>
+__device__ __forceinline__ int32_t bitonic(int32_t key, int lane) {
 #pragma unroll
-    for (int k = 0; k < 32; k++) rank += (__shfl_sync(V2C_FULL, v, k) < v);
-    __syncwarp();
-    if (lane < L) p[rank] = v;  // marker indices are distinct
-    return;
-  }
+  for (int k = 2; k <= W; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      const int32_t other = __shfl_xor_sync(V2C_FULL, key, j);
+      const bool keep_min = ((lane & j) == 0) == ((lane & k & (W - 1)) == 0);
+      key = keep_min ? min(key, other) : max(key, other);
+    }
+  return key;
+}
+
+// A segment of L > 32 entries: a bitonic network in the form whose every
+// compare puts the smaller value at the lower position (first stage of each
+// merge compares a with its mirror in the block), so positions past the
+// segment act as +infinity and are never touched.  Every position is in one
+// pair per stage; __syncwarp() orders the stages' global-memory accesses
+// among the warp's lanes.
+__device__ __noinline__ void order_large(int32_t *p, int L, int lane) {
   int P = 64;
   while (P < L) P <<= 1;
   for (int k = 2; k <= P; k <<= 1) {
@@ -154,6 +162,54 @@ __global__ void k_order_cells(const int32_t *start, long ncell, int32_t *perm) {
         }
       }
       __syncwarp();
+    }
+  }
+}
+
+// One warp per OG consecutive cells sorts each cell's segment of perm
+// ascending, in place.  The cells' starts come in one read and all their
+// entries in the next (two rounds of memory latency per warp); the entries
+// wait in shared memory, so that the sorting code is one loop, which takes
+// two cells at a time, half a warp each, where both have at most 16 markers.
+// 600 000 cells of 15 markers: 144 -> 79 us against a warp per cell.
+constexpr int OG = 8;
+__global__ void __launch_bounds__(256) k_order_cells(const int32_t *start, long ncell,
+                                                     int32_t *perm) {
+  __shared__ int32_t keys[8][OG][32];
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long c0 = (blockIdx.x * 8l + wl) * OG;
+  if (c0 >= ncell) return;  // uniform across the warp
+  const int ng = (int)min((long)OG, ncell - c0);
+  // (lanes past the last cell repeat its end: empty cells)
+  const int sv = start[c0 + min(lane, ng)];
+  int32_t val[OG];
+#pragma unroll
+  for (int g = 0; g < OG; g++) {
+    const int s = __shfl_sync(V2C_FULL, sv, g), L = __shfl_sync(V2C_FULL, sv, g + 1) - s;
+    val[g] = (lane < L && L <= 32) ? perm[s + lane] : INT_MAX;
+  }
+#pragma unroll
+  for (int g = 0; g < OG; g++) keys[wl][g][lane] = val[g];
+  __syncwarp();
+#pragma unroll 1
+  for (int g = 0; g < ng; g += 2) {
+    const int s0 = __shfl_sync(V2C_FULL, sv, g), s1 = __shfl_sync(V2C_FULL, sv, g + 1);
+    const int L0 = s1 - s0, L1 = __shfl_sync(V2C_FULL, sv, g + 2) - s1;
+    if (L0 <= 16 && L1 <= 16) {
+      const int half = lane >> 4, l = lane & 15;
+      const int32_t key = bitonic<16>(keys[wl][g + half][l], lane);
+      if (l < (half ? L1 : L0)) perm[(half ? s1 : s0) + l] = key;
+      continue;
+    }
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+      const int s = h ? s1 : s0, L = h ? L1 : L0;
+      if (L > 32) {
+        order_large(perm + s, L, lane);
+      } else {
+        const int32_t key = bitonic<32>(keys[wl][g + h][lane], lane);
+        if (lane < L) perm[s + lane] = key;
+      }
     }
   }
 }
@@ -235,10 +291,9 @@ extern "C" int v2c_sort_cells_static(const double *gx_dev, long xnumx, const dou
   k_scan_add_s<<<nblk(ncell, 256), 256, 0, st>>>(start_dev, ncell, bsum);
   if (!launched()) return V2C_ERR_CUDA;
   if (n > 0) {
-    if (cudaMemsetAsync(count, 0, sizeof(int32_t) * ncell, st) != cudaSuccess) return V2C_ERR_CUDA;
-    k_fill<<<nblk(n, 256), 256, 0, st>>>(cell_dev, n, start_dev, count, perm_dev);
+    k_fill<<<nblk(n, 256 * FM), 256, 0, st>>>(cell_dev, n, start_dev, count, perm_dev);
     if (!launched()) return V2C_ERR_CUDA;
-    k_order_cells<<<nblk(ncell * 32, 256), 256, 0, st>>>(start_dev, ncell, perm_dev);
+    k_order_cells<<<nblk(ncell, 8 * OG), 256, 0, st>>>(start_dev, ncell, perm_dev);
     if (!launched()) return V2C_ERR_CUDA;
   }
   return V2C_OK;
