@@ -27,6 +27,38 @@ using namespace v2c;
     }                                                              \
   } while (0)
 
+namespace {
+// A device block grown as needed and handed out in 256-byte-aligned pieces.
+struct DevArena {
+  char *p = nullptr;
+  size_t cap = 0, used = 0;
+  cudaError_t reserve(size_t bytes) {
+    used = 0;
+    if (bytes <= cap) return cudaSuccess;
+    release();
+    const cudaError_t e = cudaMalloc((void **)&p, bytes);
+    if (e == cudaSuccess) cap = bytes;
+    else p = nullptr;
+    return e;
+  }
+  template <class T>
+  static size_t bytes_of(long n) {
+    return (sizeof(T) * (size_t)(n > 0 ? n : 1) + 255) / 256 * 256;
+  }
+  template <class T>
+  T *take(long n) {
+    T *q = reinterpret_cast<T *>(p + used);
+    used += bytes_of<T>(n);
+    return q;
+  }
+  void release() {
+    if (p) cudaFree(p);
+    p = nullptr;
+    cap = used = 0;
+  }
+};
+}  // namespace
+
 struct v2c_ctx {
   v2c_params p;
   cudaStream_t stream = nullptr;
@@ -68,6 +100,8 @@ struct v2c_ctx {
   cudaStream_t xfer = nullptr;
   cudaEvent_t ev_conv = nullptr, ev_copy = nullptr;
   double *d_astage = nullptr;
+  DevArena stokes_ws, stokes_out, stokes_bonds;  // Stokes assembly: rows, result, boundary table
+  bool stokes_bonds_ok = false;                  // the table is the last v2c_set_bonds's
   int astage_fields = 0;
   bool dl_pending = false;
   // sort
@@ -370,6 +404,9 @@ extern "C" int v2c_destroy(v2c_ctx *ctx) {
   if (ctx->ev_copy) cudaEventDestroy(ctx->ev_copy);
   if (ctx->d_astage) cudaFree(ctx->d_astage);
   if (ctx->h_res) cudaFreeHost(ctx->h_res);
+  ctx->stokes_ws.release();
+  ctx->stokes_out.release();
+  ctx->stokes_bonds.release();
   for (auto &gr : ctx->graphs) cudaGraphExecDestroy(gr.exec);
   ctx->graphs.clear();
   for (float *v : ctx->d_cyc_v)
@@ -499,6 +536,7 @@ extern "C" int v2c_set_bonds(v2c_ctx *ctx, const long *bondm, const long *bondn,
     if (bondm[i] < 0 || bondm[i] >= bondnum) return fail(ctx, V2C_ERR_ARG);
   ctx->have_bonds = true;
   ctx->bc_built_compressible = -1;
+  ctx->stokes_bonds_ok = false;
   return V2C_OK;
 }
 
@@ -1351,56 +1389,44 @@ extern "C" int v2c_marker_temperature(v2c_ctx *ctx, double heatdif) {
 }
 
 // ====================================================== Stokes assembly
-namespace {
-// device memory of one call, freed on every return path
-struct DevBuf {
-  void *p = nullptr;
-  ~DevBuf() {
-    if (p) cudaFree(p);
-  }
-  template <class T>
-  cudaError_t alloc(long n) {
-    return cudaMalloc(&p, sizeof(T) * (size_t)(n > 0 ? n : 1));
-  }
-  template <class T>
-  T *get() const {
-    return static_cast<T *>(p);
-  }
-};
-}  // namespace
+// What the assembly keeps between calls: beyond this it is freed at the end of
+// each (an allocation then costs little beside the rows).
+constexpr size_t STOKES_KEEP_BYTES = size_t(256) << 20;
 
-extern "C" int v2c_stokes_assemble(v2c_ctx *ctx, const v2c_stokes_ctl *ctl, long cap, int *ia,
-                                   int *ja, double *a, double *b, long *nnz) {
-  if (!ctx || !ctl || !nnz || cap < 0 || (ja == nullptr) != (a == nullptr)) return V2C_ERR_ARG;
-  if (!ctx->have_grid || !ctx->have_bonds) return fail(ctx, V2C_ERR_STATE);
-  const long rows = 3 * ctx->nn;
-  if (rows + 1 > 0x7fffffffL) return fail(ctx, V2C_ERR_CAPACITY);
-  cudaStream_t st = ctx->stream;
-  const long nb = ctx->bondnum;
-  DevBuf bm, bn, bv, cnt, rhs, bsum, err, dja, da, ecol, evalb;
-  CK(bm.alloc<long>(ctx->nn * 4));
-  CK(bn.alloc<long>(nb * 3));
-  CK(bv.alloc<double>(nb * 4));
-  CK(cnt.alloc<int32_t>(rows + 1));
-  CK(rhs.alloc<double>(rows));
-  CK(bsum.alloc<int32_t>(scan_blocks(rows)));
-  CK(err.alloc<int>(1));
-  CK(cudaMemcpyAsync(bm.p, ctx->h_bondm.data(), sizeof(long) * ctx->nn * 4,
-                     cudaMemcpyHostToDevice, st));
-  if (nb > 0) {
-    CK(cudaMemcpyAsync(bn.p, ctx->h_bondn.data(), sizeof(long) * nb * 3, cudaMemcpyHostToDevice,
-                       st));
-    CK(cudaMemcpyAsync(bv.p, ctx->h_bondv.data(), sizeof(double) * nb * 4,
-                       cudaMemcpyHostToDevice, st));
+// The boundary table on the device, uploaded once after v2c_set_bonds.
+static int stokes_bonds(v2c_ctx *ctx, StokesArgs &s) {
+  const long nn = ctx->nn, nb = ctx->bondnum;
+  DevArena &w = ctx->stokes_bonds;
+  CK(w.reserve(DevArena::bytes_of<long>(nn * 4) + DevArena::bytes_of<long>(nb * 3) +
+               DevArena::bytes_of<double>(nb * 4)));
+  long *bm = w.take<long>(nn * 4), *bn = w.take<long>(nb * 3);
+  double *bv = w.take<double>(nb * 4);
+  if (!ctx->stokes_bonds_ok) {
+    CK(cudaMemcpyAsync(bm, ctx->h_bondm.data(), sizeof(long) * nn * 4, cudaMemcpyHostToDevice,
+                       ctx->stream));
+    if (nb > 0) {
+      CK(cudaMemcpyAsync(bn, ctx->h_bondn.data(), sizeof(long) * nb * 3, cudaMemcpyHostToDevice,
+                         ctx->stream));
+      CK(cudaMemcpyAsync(bv, ctx->h_bondv.data(), sizeof(double) * nb * 4,
+                         cudaMemcpyHostToDevice, ctx->stream));
+    }
+    ctx->stokes_bonds_ok = true;
   }
-  CK(cudaMemsetAsync(err.p, 0, sizeof(int), st));
+  s.bondm = bm;
+  s.bondn = bn;
+  s.bondv = bv;
+  s.bondnum = nb;
+  return V2C_OK;
+}
+
+static int stokes_assemble(v2c_ctx *ctx, const v2c_stokes_ctl *ctl, long cap, int *ia, int *ja,
+                           double *a, double *b, long *nnz) {
+  const long rows = 3 * ctx->nn;
+  cudaStream_t st = ctx->stream;
   StokesArgs s;
   s.g = make_grid(ctx);
   s.N = make_nodes(ctx);
-  s.bondm = bm.get<long>();
-  s.bondn = bn.get<long>();
-  s.bondv = bv.get<double>();
-  s.bondnum = nb;
+  if (int rc = stokes_bonds(ctx, s)) return rc;
   s.mukoef = ctl->mukoef;
   s.dt = ctl->dt;
   s.gxkoef = ctl->gxkoef;
@@ -1412,55 +1438,53 @@ extern "C" int v2c_stokes_assemble(v2c_ctx *ctx, const v2c_stokes_ctl *ctl, long
   s.nubeg = ctx->p.nubeg;
   s.inertyn = ctx->p.inertyn;
   s.compressible = ctx->p.compressiblemode;
-  s.cnt = cnt.get<int32_t>();
-  s.b = rhs.get<double>();
+  // when the caller has room for the coefficients the count pass keeps the
+  // rows, so the FP64 work is done once
+  const long kept = ja ? rows * STOKES_ROW_MAX : 0;
+  DevArena &w = ctx->stokes_ws;
+  CK(w.reserve(DevArena::bytes_of<int32_t>(rows + 2) + DevArena::bytes_of<double>(rows) +
+               DevArena::bytes_of<int32_t>(scan_blocks(rows)) +
+               DevArena::bytes_of<int32_t>(kept) + DevArena::bytes_of<double>(kept)));
+  s.cnt = w.take<int32_t>(rows + 2);  // row starts, their total, then the error word
+  s.b = w.take<double>(rows);
+  int32_t *bsum = w.take<int32_t>(scan_blocks(rows));
+  s.ell_col = kept ? w.take<int32_t>(kept) : nullptr;
+  s.ell_val = kept ? w.take<double>(kept) : nullptr;
   s.ja = nullptr;
   s.a = nullptr;
-  s.ell_col = nullptr;
-  s.ell_val = nullptr;
-  if (ja) {
-    // the caller has room for the coefficients: the count pass keeps the
-    // rows, so the FP64 work is done once
-    CK(ecol.alloc<int32_t>(rows * STOKES_ROW_MAX));
-    CK(evalb.alloc<double>(rows * STOKES_ROW_MAX));
-    s.ell_col = ecol.get<int32_t>();
-    s.ell_val = evalb.get<double>();
-  }
-  s.err = err.get<int>();
-  int h_err = 0;
-  int32_t total = 0;
+  s.err = s.cnt + rows + 1;
+  CK(cudaMemsetAsync(s.err, 0, sizeof(int), st));
   {
     Prof pr(ctx, V2C_PROF_STOKES);
     launch_stokes_count(s, st);
-    launch_scan(s.cnt, rows, s.cnt, bsum.get<int32_t>(), st);
-    ctx->launches += 4;
+    launch_scan(s.cnt, rows, s.cnt, bsum, st);
+    ctx->launches += 3;
   }
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(&h_err, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(&total, s.cnt + rows, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  int32_t *res = reinterpret_cast<int32_t *>(ctx->h_res);
+  CK(cudaMemcpyAsync(res, s.cnt + rows, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  if (h_err) return fail(ctx, V2C_ERR_UNSUPPORTED);
+  const int32_t total = res[0];
+  if (res[1]) return fail(ctx, V2C_ERR_UNSUPPORTED);
   if (total < 0) return fail(ctx, V2C_ERR_CAPACITY);  // more than 2^31 - 1 coefficients
   *nnz = total;
-  if (ia) {
-    CK(cudaMemcpyAsync(ia, s.cnt, sizeof(int32_t) * (rows + 1), cudaMemcpyDeviceToHost, st));
+  if (ja && cap >= total) {
+    CK(ctx->stokes_out.reserve(DevArena::bytes_of<int32_t>(total) +
+                               DevArena::bytes_of<double>(total)));
+    s.ja = ctx->stokes_out.take<int32_t>(total);
+    s.a = ctx->stokes_out.take<double>(total);
+    Prof pr(ctx, V2C_PROF_STOKES);
+    launch_stokes_fill(s, st);
+    ctx->launches += 1;
+    CK(cudaGetLastError());
   }
+  if (ia) CK(cudaMemcpyAsync(ia, s.cnt, sizeof(int32_t) * (rows + 1), cudaMemcpyDeviceToHost, st));
   if (b) CK(cudaMemcpyAsync(b, s.b, sizeof(double) * rows, cudaMemcpyDeviceToHost, st));
   if (ja) {
     if (cap < total) {
       CK(cudaStreamSynchronize(st));
       return fail(ctx, V2C_ERR_CAPACITY);
     }
-    CK(dja.alloc<int32_t>(total));
-    CK(da.alloc<double>(total));
-    s.ja = dja.get<int32_t>();
-    s.a = da.get<double>();
-    {
-      Prof pr(ctx, V2C_PROF_STOKES);
-      launch_stokes_fill(s, st);
-      ctx->launches += 1;
-    }
-    CK(cudaGetLastError());
     CK(cudaMemcpyAsync(ja, s.ja, sizeof(int32_t) * total, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(a, s.a, sizeof(double) * total, cudaMemcpyDeviceToHost, st));
   }
@@ -1469,6 +1493,19 @@ extern "C" int v2c_stokes_assemble(v2c_ctx *ctx, const v2c_stokes_ctl *ctl, long
   if (ia)
     for (long r = 0; r <= rows; r++) ia[r] += 1;
   return V2C_OK;
+}
+
+extern "C" int v2c_stokes_assemble(v2c_ctx *ctx, const v2c_stokes_ctl *ctl, long cap, int *ia,
+                                   int *ja, double *a, double *b, long *nnz) {
+  if (!ctx || !ctl || !nnz || cap < 0 || (ja == nullptr) != (a == nullptr)) return V2C_ERR_ARG;
+  if (!ctx->have_grid || !ctx->have_bonds) return fail(ctx, V2C_ERR_STATE);
+  if (3 * ctx->nn + 1 > 0x7fffffffL) return fail(ctx, V2C_ERR_CAPACITY);
+  const int rc = stokes_assemble(ctx, ctl, cap, ia, ja, a, b, nnz);
+  if (ctx->stokes_ws.cap + ctx->stokes_out.cap > STOKES_KEEP_BYTES) {
+    ctx->stokes_ws.release();
+    ctx->stokes_out.release();
+  }
+  return rc;
 }
 
 // ======================================================= seismic cycle
