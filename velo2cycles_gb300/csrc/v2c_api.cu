@@ -676,6 +676,46 @@ int build_bc(v2c_ctx *ctx) {
 
 }  // namespace
 
+// ======================================================== pinned host arrays
+// Whether every array (n doubles) lies in one pinned host allocation that
+// the device reads and writes at the same address: then a kernel moves the
+// fields itself.  Each copy costs about 2 us on its stream and 1 us to issue,
+// so at 301 x 101 nodes eight of them took 28 us and the kernel takes 8; at
+// 4 M nodes both run at the host link's rate (210 GB/s in, 193 out) and the
+// kernel saves the staging area's traffic.
+static bool all_pinned(const void *const *ptrs, int count, long n) {
+  typedef CUresult (*AttrFn)(void *, CUpointer_attribute, CUdeviceptr);
+  static const AttrFn range_of = [] {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault,
+                                         &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    cudaGetLastError();
+    return reinterpret_cast<AttrFn>(fn);
+  }();
+  if (!range_of) return false;
+  const size_t bytes = sizeof(double) * (size_t)n;
+  for (int k = 0; k < count; k++) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, ptrs[k]) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (at.type != cudaMemoryTypeHost || at.devicePointer != ptrs[k] || (uintptr_t)ptrs[k] % 8)
+      return false;
+    unsigned long long begin = 0;
+    size_t size = 0;
+    const unsigned long long p = (unsigned long long)ptrs[k];
+    if (range_of(&begin, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) ||
+        range_of(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) || p < begin ||
+        p + bytes > begin + size)
+      return false;
+  }
+  return true;
+}
+
 // ============================================================ marker arrays
 // the compaction scratch of immobile markers, one allocation for the
 // context's capacity (ImmBufs in v2c_kernels.h)
@@ -782,7 +822,27 @@ extern "C" int v2c_download_markers(v2c_ctx *ctx, double *const *fields, signed 
   cudaStream_t st = ctx->stream;
   Markers &m = ctx->m;
   Grid g = make_grid(ctx);
-  if (fields[V2C_MF_X] || fields[V2C_MF_Y]) {
+  struct F { int id; const float *src; const float *lo; } ff[] = {
+      {V2C_MF_K, m.tk, m.tk_lo}, {V2C_MF_V, m.mv, m.mv_lo}, {V2C_MF_E, m.e, nullptr},
+      {V2C_MF_P, m.p, nullptr},
+      {V2C_MF_XX, m.sxx, nullptr}, {V2C_MF_XY, m.sxy, nullptr}, {V2C_MF_EXX, m.exx, nullptr},
+      {V2C_MF_EXY, m.exy, nullptr}, {V2C_MF_VX, m.vx, nullptr}, {V2C_MF_VY, m.vy, nullptr},
+      {V2C_MF_PHI, m.phi, nullptr}, {V2C_MF_C, m.coh, nullptr}, {V2C_MF_SLIPV, m.slipv, nullptr}};
+  // pinned arrays are written by one kernel (456 000 markers, 13 fields: the
+  // copies and a wait after each and conversions took 440 us of the call, the kernel 300)
+  MarkerFields mf;
+  if (fields[V2C_MF_X]) mf.add(MARKER_X, nullptr, nullptr, fields[V2C_MF_X]);
+  if (fields[V2C_MF_Y]) mf.add(MARKER_Y, nullptr, nullptr, fields[V2C_MF_Y]);
+  for (auto &f : ff)
+    if (fields[f.id]) mf.add(f.lo ? MARKER_PAIR : MARKER_F32, f.src, f.lo, fields[f.id]);
+  const bool direct = all_pinned((const void *const *)mf.dst, mf.n, n);
+  if (direct) {
+    // the sort's slot buffer holds nothing between sorts
+    launch_markers_to_host(g, m, n, mf, ctx->sb.slot, st);
+    ctx->launches += n > 0 && mf.n > 0 ? 2 : 0;
+    CK(cudaGetLastError());
+  }
+  if (!direct && (fields[V2C_MF_X] || fields[V2C_MF_Y])) {
     launch_positions(g, m, n, ctx->d_stage64, ctx->d_stage64b, st);
     if (fields[V2C_MF_X])
       CK(cudaMemcpyAsync(fields[V2C_MF_X], ctx->d_stage64, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
@@ -790,14 +850,8 @@ extern "C" int v2c_download_markers(v2c_ctx *ctx, double *const *fields, signed 
       CK(cudaMemcpyAsync(fields[V2C_MF_Y], ctx->d_stage64b, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
   }
-  struct F { int id; const float *src; const float *lo; } ff[] = {
-      {V2C_MF_K, m.tk, m.tk_lo}, {V2C_MF_V, m.mv, m.mv_lo}, {V2C_MF_E, m.e, nullptr},
-      {V2C_MF_P, m.p, nullptr},
-      {V2C_MF_XX, m.sxx, nullptr}, {V2C_MF_XY, m.sxy, nullptr}, {V2C_MF_EXX, m.exx, nullptr},
-      {V2C_MF_EXY, m.exy, nullptr}, {V2C_MF_VX, m.vx, nullptr}, {V2C_MF_VY, m.vy, nullptr},
-      {V2C_MF_PHI, m.phi, nullptr}, {V2C_MF_C, m.coh, nullptr}, {V2C_MF_SLIPV, m.slipv, nullptr}};
   for (auto &f : ff) {
-    if (!fields[f.id]) continue;
+    if (direct || !fields[f.id]) continue;
     if (f.lo) launch_unpermute_pair(f.src, f.lo, m.id, ctx->d_stage64, n, st);
     else launch_unpermute_f32(f.src, m.id, ctx->d_stage64, n, st);
     CK(cudaMemcpyAsync(fields[f.id], ctx->d_stage64, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
@@ -902,44 +956,6 @@ static int node_field_list_ok(int count, const int *fields, const void *const *p
   return 1;
 }
 
-// Whether every array (nn doubles) lies in one pinned host allocation that
-// the device reads and writes at the same address: then a kernel moves the
-// fields itself.  Each copy costs about 2 us on its stream and 1 us to issue,
-// so at 301 x 101 nodes eight of them took 28 us and the kernel takes 8; at
-// 4 M nodes both run at the host link's rate (210 GB/s in, 193 out) and the
-// kernel saves the staging area's traffic.
-static bool all_pinned(const void *const *ptrs, int count, long nn) {
-  typedef CUresult (*AttrFn)(void *, CUpointer_attribute, CUdeviceptr);
-  static const AttrFn range_of = [] {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault,
-                                         &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      fn = nullptr;
-    cudaGetLastError();
-    return reinterpret_cast<AttrFn>(fn);
-  }();
-  if (!range_of) return false;
-  const size_t bytes = sizeof(double) * (size_t)nn;
-  for (int k = 0; k < count; k++) {
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, ptrs[k]) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    if (at.type != cudaMemoryTypeHost || at.devicePointer != ptrs[k] || (uintptr_t)ptrs[k] % 8)
-      return false;
-    unsigned long long begin = 0;
-    size_t size = 0;
-    const unsigned long long p = (unsigned long long)ptrs[k];
-    if (range_of(&begin, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) ||
-        range_of(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) || p < begin ||
-        p + bytes > begin + size)
-      return false;
-  }
-  return true;
-}
 // A field this size goes to the host by the copy engine, which takes no SMs
 // from the kernels it runs under; smaller ones together in one kernel.
 constexpr long ENGINE_COPY_NODES = 1 << 17;

@@ -259,6 +259,23 @@ void launch_unpermute_i32(const int32_t *src, const int32_t *id, int32_t *out, l
 void launch_unpermute_u8(const uint8_t *src, const int32_t *id, uint8_t *out, long n, cudaStream_t st);
 void launch_unpermute_i8(const int8_t *src, const int32_t *id, int8_t *out, long n, cudaStream_t st);
 // FP64 positions in reference numbering
+// marker fields straight to host arrays that the device writes: an entry per
+// array
+constexpr int MARKER_FIELDS_MAX = 16;
+enum { MARKER_F32, MARKER_PAIR, MARKER_X, MARKER_Y };
+struct MarkerFields {
+  const float *src[MARKER_FIELDS_MAX], *lo[MARKER_FIELDS_MAX];
+  double *dst[MARKER_FIELDS_MAX];
+  int kind[MARKER_FIELDS_MAX];
+  int n = 0;
+  void add(int k, const float *s, const float *l, double *d) {
+    kind[n] = k; src[n] = s; lo[n] = l; dst[n] = d;
+    n++;
+  }
+};
+// inv: scratch of n entries
+void launch_markers_to_host(const Grid &g, const Markers &m, long n, const MarkerFields &f,
+                            int32_t *inv, cudaStream_t st);
 void launch_positions(const Grid &g, const Markers &m, long n, double *x, double *y,
                       cudaStream_t st);
 

@@ -301,6 +301,35 @@ __global__ void k_positions(Grid g, Markers m, long n, double *x, double *y) {
   y[k] = g.gy[iy] + (double)m.v_in[i] * (g.gy[iy + 1] - g.gy[iy]);
 }
 
+// where each marker of the host's numbering lies (-1: nowhere)
+__global__ void k_marker_inverse(const int32_t *id, long n, int32_t *inv) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i < n) inv[id[i]] = (int32_t)i;
+}
+// One row of blocks per field, in the host's order: the device's reads are
+// gathered (from L2), the host's arrays written in full lines over the link.
+__global__ void __launch_bounds__(256) k_markers_to_host(Grid g, Markers m, long n,
+                                                         const __grid_constant__ MarkerFields F,
+                                                         const int32_t *inv) {
+  const int f = blockIdx.y, kind = F.kind[f];
+  const float *src = F.src[f], *lo = F.lo[f];
+  double *dst = F.dst[f];
+  for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
+    const int i = inv[k];
+    if (i < 0) continue;
+    if (kind == MARKER_F32) {
+      dst[k] = (double)src[i];
+    } else if (kind == MARKER_PAIR) {
+      dst[k] = (double)src[i] + (double)lo[i];
+    } else {
+      int ix, iy;
+      g.cell_at(m.cell_in[i], ix, iy);
+      dst[k] = kind == MARKER_X ? g.gx[ix] + (double)m.u_in[i] * (g.gx[ix + 1] - g.gx[ix])
+                                : g.gy[iy] + (double)m.v_in[i] * (g.gy[iy + 1] - g.gy[iy]);
+    }
+  }
+}
+
 inline unsigned nblk(long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
@@ -378,6 +407,17 @@ void launch_unpermute_i8(const int8_t *src, const int32_t *id, int8_t *out, long
 void launch_positions(const Grid &g, const Markers &m, long n, double *x, double *y,
                       cudaStream_t st) {
   if (n > 0) k_positions<<<nblk(n, 256), 256, 0, st>>>(g, m, n, x, y);
+}
+
+void launch_markers_to_host(const Grid &g, const Markers &m, long n, const MarkerFields &f,
+                            int32_t *inv, cudaStream_t st) {
+  if (n <= 0 || f.n <= 0) return;
+  cudaMemsetAsync(inv, 0xff, sizeof(int32_t) * n, st);
+  k_marker_inverse<<<nblk(n, 256), 256, 0, st>>>(m.id, n, inv);
+  // enough blocks to keep the host link busy, no more
+  const unsigned want = nblk(n, 256), most = 1216 / (unsigned)f.n + 1;
+  k_markers_to_host<<<dim3(want < most ? want : most, (unsigned)f.n), 256, 0, st>>>(g, m, n, f,
+                                                                                   inv);
 }
 
 }  // namespace v2c
