@@ -38,7 +38,42 @@ __device__ __forceinline__ ff ff_from_double(double d) {
   const float h = __double2float_rn(d);
   return ff{h, __double2float_rn(d - (double)h)};
 }
-__device__ __forceinline__ double ff_to_double(ff a) { return (double)a.hi + (double)a.lo; }
+// The same from the bit pattern: FP64 instructions issue at 1/64 of the FP32
+// rate, and four of them per value (two conversions, a difference, a
+// conversion) were the larger part of the FP64 pipe's work in the Newton on
+// state arrays.  hi is the leading 24 bits rounded to even, the remainder an
+// integer of at most 29 bits, exact, rounded once to lo.  Outside 2^-74..2^127
+// (where hi or lo would not be normal) the plain form.
+static __device__ __noinline__ ff ff_from_double_call(double d) { return ff_from_double(d); }
+__device__ __forceinline__ ff ff_from_double_bits(double d) {
+  const unsigned h = (unsigned)__double2hiint(d), l = (unsigned)__double2loint(d);
+  const int e = (int)((h >> 20) & 0x7ff) - 1023;
+  if ((unsigned)(e + 74) >= 201u && (h << 1 | l) != 0) return ff_from_double_call(d);
+  const unsigned q = (h & 0xfffff) << 3 | l >> 29;   // leading 23 fraction bits
+  const int r = (int)(l & 0x1fffffff);               // the 29 below them
+  const int up = r > 0x10000000 || (r == 0x10000000 && (q & 1));
+  const unsigned sign = h & 0x80000000u;
+  const int rem = r - (up << 29);
+  ff x;
+  x.hi = __uint_as_float(sign | (((unsigned)(e + 127) << 23 | q) + (unsigned)up));
+  x.lo = __fmul_rn(__int2float_rn(sign ? -rem : rem), __int_as_float((e + 75) << 23));
+  if ((h << 1 | l) == 0) x = ff{__uint_as_float(sign), 0.f};
+  return x;
+}
+// (double)f, with BITS from the bit pattern, for the same reason (the plain
+// form for what is neither zero nor normal)
+template <bool BITS = false>
+__device__ __forceinline__ double widen(float f) {
+  const unsigned b = __float_as_uint(f), e = b & 0x7f800000u;
+  if (!BITS || (e == 0 && (b << 1) != 0) || e == 0x7f800000u) return (double)f;
+  const unsigned h = (b & 0x80000000u) | (e == 0 ? 0u : ((b & 0x7fffffffu) >> 3) + 0x38000000u);
+  return __hiloint2double((int)h, (int)(b << 29));
+}
+
+template <bool BITS = false>
+__device__ __forceinline__ double ff_to_double(ff a) {
+  return widen<BITS>(a.hi) + widen<BITS>(a.lo);
+}
 
 __device__ __forceinline__ float two_sum(float a, float b, float &e) {
   const float s = __fadd_rn(a, b);

@@ -65,87 +65,255 @@ __device__ __forceinline__ double st_at(const double *S, long n, int k, long i) 
   return S[(long)k * n + i];
 }
 
-__device__ __forceinline__ void state_of(const double *S, long n, long i, double W, RsfIn &in,
+// BITS: whole pairs without FP64 arithmetic; else the conversion, of which the
+// FP32 uses keep only the high word
+template <bool BITS = false>
+__device__ __forceinline__ void state_of(const double *S, long n, long i, ff W, RsfIn &in,
                                          double &vold) {
+  auto pair = [&](int k) {
+    const double d = st_at(S, n, k, i);
+    return BITS ? ff_from_double_bits(d) : ff_from_double(d);
+  };
   vold = st_at(S, n, V2C_RS_VOLD, i);
-  in.a = ff_from_double(st_at(S, n, V2C_RS_A, i));
-  in.b = ff_from_double(st_at(S, n, V2C_RS_B, i));
-  in.L = ff_from_double(st_at(S, n, V2C_RS_L, i));
-  in.V0 = ff_from_double(st_at(S, n, V2C_RS_V0, i));
-  in.mu0 = ff_from_double(st_at(S, n, V2C_RS_MU0, i));
-  in.sn = ff_from_double(st_at(S, n, V2C_RS_SN, i));
-  in.dt = ff_from_double(st_at(S, n, V2C_RS_DT, i));
-  in.phio = ff_from_double(st_at(S, n, V2C_RS_PHIOLD, i));
-  in.tau_old = ff_from_double(st_at(S, n, V2C_RS_TAUOLD, i));
-  in.edot = ff_from_double(st_at(S, n, V2C_RS_EDOT, i));
-  in.eta = ff_from_double(st_at(S, n, V2C_RS_ETA, i));
-  in.G = ff_from_double(st_at(S, n, V2C_RS_G, i));
-  in.W = ff_from_double(W);
+  in.a = pair(V2C_RS_A);
+  in.b = pair(V2C_RS_B);
+  in.L = pair(V2C_RS_L);
+  in.V0 = pair(V2C_RS_V0);
+  in.mu0 = pair(V2C_RS_MU0);
+  in.sn = pair(V2C_RS_SN);
+  in.dt = pair(V2C_RS_DT);
+  in.phio = pair(V2C_RS_PHIOLD);
+  in.tau_old = pair(V2C_RS_TAUOLD);
+  in.edot = pair(V2C_RS_EDOT);
+  in.eta = pair(V2C_RS_ETA);
+  in.G = pair(V2C_RS_G);
+  in.W = W;
 }
 
 // ---------------------------------------------------------- solve states
-// one instantiation per (arithmetic, start) pair; the learned start comes
-// from the network's outputs guess[i] (k_infer), so this kernel keeps the
-// plain start's occupancy
-template <bool FP64, bool LEARNED>
-__global__ void __launch_bounds__(NT, 4) k_solve_states(const double *S, long n, double W,
-                                                        const float *guess, double rtol, int maxit,
-                                                        double *out, int32_t *iters,
-                                                        unsigned long long *stat) {
-  const bool learned = LEARNED;
-  const bool fp64 = FP64;
+// A solved state's results.
+template <bool BITS = false>
+__device__ __forceinline__ void put_state(const RsfIn &in, const RsfResult &r,
+                                          unsigned long long it, long n, long i, double *out,
+                                          int32_t *iters) {
+  out[(long)V2C_RO_V * n + i] = r.V;
+  out[(long)V2C_RO_PHI * n + i] = widen<BITS>(r.phi);
+  // tau_y = sn a A + 4.3303e6 V at the solution (calc_RSF.c:128), FP64
+  out[(long)V2C_RO_TAU * n + i] =
+      __fma_rn(ff_to_double<BITS>(in.sn) * ff_to_double<BITS>(in.a), r.A, RSF_ETA_RAD * r.V);
+  out[(long)V2C_RO_RES * n + i] = r.res;
+  if (iters) iters[i] = r.ok ? (int32_t)it : -(int32_t)it;
+}
+__device__ __forceinline__ float plain_start(double vold) {
+  return (vold > 0) ? logf((float)vold) : -30.f;
+}
+
+// the statistics of a warp's states
+__device__ __forceinline__ void add_stats(unsigned long long *stat, unsigned long long it,
+                                          unsigned long long fb, unsigned long long nc,
+                                          unsigned long long resbits) {
+  warp_max_bits(stat + ST_NEWTON_MAXRES_BITS, resbits);
+  warp_add(stat + ST_NEWTON_ITERS, it);
+  warp_add(stat + ST_NEWTON_FALLBACK, fb);
+  warp_add(stat + ST_NEWTON_NONCONV, nc);
+}
+
+// The FP64 form: one instantiation per start; the learned start comes from
+// the network's outputs guess[i].
+template <bool LEARNED>
+__global__ void __launch_bounds__(NT, 4) k_solve_states64(const double *S, long n, ff W,
+                                                          const float *guess, double rtol,
+                                                          int maxit, double *out, int32_t *iters,
+                                                          unsigned long long *stat) {
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const long nwarps = (long)gridDim.x * (NT / 32);
   for (long base = ((long)blockIdx.x * (NT / 32) + wl) * 32; base < n; base += nwarps * 32) {
     const long i = base + lane;
-    const bool valid = i < n;
-    RsfIn in;
-    double vold = 1e-9;
-    if (valid) state_of(S, n, i, W, in, vold);
-    const float u_plain = (vold > 0) ? logf((float)vold) : -30.f;
-    // split form: states whose load is certainly below the floor's yield
-    // are done with one FP32 evaluation
-    bool at_floor = false;
-    float A_floor = 0.f;
-    if (valid && !fp64) at_floor = rsf_floor_certain(rsf32_of(in), A_floor);
-    const float u0 = (learned && valid) ? guess[i] : u_plain;
     unsigned long long it = 0, fb = 0, nc = 0, resbits = 0;
-    if (valid) {
-      // the FP64 form starts from the FP64 log of the previous slip rate
-      const double u_plain64 = (fp64 && vold > 0) ? log(vold) : (double)u_plain;
-      RsfResult r = at_floor ? rsf_floor_result(in, A_floor)
-                  : fp64     ? rsf_solve64(in, learned ? (double)u0 : u_plain64, rtol, maxit)
-                             : rsf_solve_split(in, rsf32_of(in), u0, rtol, maxit);
-      it = r.it32 + r.itff + r.it64;
-      if (!r.ok && learned && u0 != u_plain) {
-        RsfResult r2 = fp64 ? rsf_solve64(in, u_plain64, rtol, maxit)
-                            : rsf_solve_split(in, rsf32_of(in), u_plain, rtol, maxit);
-        it += r2.it32 + r2.itff + r2.it64;
+    if (i < n) {
+      RsfIn in;
+      double vold;
+      state_of(S, n, i, W, in, vold);
+      // starts from the FP64 log of the previous slip rate
+      const float u_plain = plain_start(vold);
+      const double u_plain64 = vold > 0 ? log(vold) : (double)u_plain;
+      const float u0 = LEARNED ? guess[i] : u_plain;
+      RsfResult r = rsf_solve64(in, LEARNED ? (double)u0 : u_plain64, rtol, maxit);
+      it = r.it64;
+      if (!r.ok && LEARNED && u0 != u_plain) {
+        r = rsf_solve64(in, u_plain64, rtol, maxit);
+        it += r.it64;
         fb = 1;
-        r = r2;
       }
       if (!r.ok) nc = 1;
-      out[(long)V2C_RO_V * n + i] = r.V;
-      out[(long)V2C_RO_PHI * n + i] = r.phi;
-      // tau_y = sn a A + 4.3303e6 V at the solution (calc_RSF.c:128), FP64
-      out[(long)V2C_RO_TAU * n + i] =
-          ff_to_double(in.sn) * ff_to_double(in.a) * r.A + RSF_ETA_RAD * r.V;
-      out[(long)V2C_RO_RES * n + i] = r.res;
-      if (iters) iters[i] = r.ok ? (int32_t)it : -(int32_t)it;
+      put_state(in, r, it, n, i, out, iters);
       if (r.res > 0) resbits = (unsigned long long)__double_as_longlong(r.res);
     }
-    warp_max_bits(stat + ST_NEWTON_MAXRES_BITS, resbits);
-    warp_add(stat + ST_NEWTON_ITERS, it);
-    warp_add(stat + ST_NEWTON_FALLBACK, fb);
-    warp_add(stat + ST_NEWTON_NONCONV, nc);
+    add_stats(stat, it, fb, nc, resbits);
   }
+}
+
+// The split form, a kernel per phase: FP32, float-float, and FP64 for the
+// states that need it.  In one kernel the states of a block were in different
+// phases and at different iterations of 50 KB of code, so that instruction
+// fetch was the bound (7 of 13 stall cycles per instruction), and a warp ran
+// the FP64 Newton for one lane.  4 M states of the benchmark's
+// distributions, plain start: 2510 -> 1085 us (FP32 252, float-float 731, FP64
+// 100; with the FP64 Newton inside the float-float kernel 1340 for the two).
+//
+// A phase leaves its result in the state's own outputs, which the next one
+// reads and then writes.
+enum { PH_POLISH = 0, PH_FLOOR = 1, PH_DEGENERATE = 2 };
+struct Phase32 {  // in the places of the slip rate and the state variable
+  float u, dF;    // FP32 iterate (PH_FLOOR: the friction term) and derivative
+  int it, what;   // iterations; what the next phase does
+};
+__device__ __forceinline__ void put_phase32(double *out, long n, long i, const Phase32 &p) {
+  reinterpret_cast<float2 *>(out)[(long)V2C_RO_V * n + i] = make_float2(p.u, p.dF);
+  reinterpret_cast<int2 *>(out)[(long)V2C_RO_PHI * n + i] = make_int2(p.it, p.what);
+}
+__device__ __forceinline__ Phase32 get_phase32(const double *out, long n, long i) {
+  const float2 a = reinterpret_cast<const float2 *>(out)[(long)V2C_RO_V * n + i];
+  const int2 b = reinterpret_cast<const int2 *>(out)[(long)V2C_RO_PHI * n + i];
+  return Phase32{a.x, a.y, b.x, b.y};
+}
+__device__ __forceinline__ bool resume(const Phase32 &p, RsfResult &r, float &u, float &dF) {
+  r.it32 = p.it;
+  u = p.u;
+  dF = p.dF;
+  return true;
+}
+// states left to the FP64 phase, by a mark in the residual's place (NaNs that
+// no arithmetic returns): from the iterate in the slip rate's place, with the
+// iterations so far and the state variable in the state variable's; or from a
+// load degenerate in FP32, Phase32 left as it was; or (LEARNED) a whole solve
+// from the plain start
+constexpr unsigned long long MARK_NEWTON = 0x7ff4563243324301ull;
+constexpr unsigned long long MARK_DEGENERATE = 0x7ff4563243324302ull;
+
+template <bool LEARNED>
+__global__ void __launch_bounds__(NT) k_states_fp32(const double *S, long n, ff W,
+                                                    const float *guess, int maxit, double *out) {
+  const long i = blockIdx.x * (long)NT + threadIdx.x;
+  if (i >= n) return;
+  RsfIn in;
+  double vold;
+  state_of(S, n, i, W, in, vold);
+  const Rsf32 q = rsf32_of(in);
+  Phase32 p{0.f, 0.f, 1, PH_FLOOR};
+  // states whose load is certainly below the floor's yield are done with
+  // one FP32 evaluation
+  if (!rsf_floor_certain(q, p.u)) {
+    p.what = rsf_degenerate32(q) ? PH_DEGENERATE : PH_POLISH;
+    p.u = rsf_newton32(q, LEARNED ? guess[i] : plain_start(vold), (float)RSF_LOG_FLOOR, q.uhi,
+                       maxit, p.it, p.dF);
+  }
+  put_phase32(out, n, i, p);
+}
+
+__global__ void __launch_bounds__(NT, 8) k_states_polish(const double *S, long n, ff W, float rtolf,
+                                                         double *out, int32_t *iters,
+                                                         unsigned long long *stat) {
+  const long i = blockIdx.x * (long)NT + threadIdx.x;
+  unsigned long long it = 0, resbits = 0;
+  if (i < n) {
+    const Phase32 p = get_phase32(out, n, i);
+    double *mark = out + (long)V2C_RO_RES * n + i;
+    if (p.what == PH_DEGENERATE) {
+      *mark = __longlong_as_double(MARK_DEGENERATE);
+    } else {
+      RsfIn in;
+      double vold;
+      state_of<true>(S, n, i, W, in, vold);
+      RsfResult r{};
+      bool left = false;
+      if (p.what == PH_FLOOR) {
+        r = rsf_floor_result(in, p.u);
+      } else {
+        r = rsf_solve_phases<true>(
+            in, [&](RsfResult &rr, float &u, float &dF) { return resume(p, rr, u, dF); }, rtolf,
+            [&](RsfFF &q) { rsf_setup_ff(q, in); },
+            [&](double u, RsfResult &rr) {
+              left = true;
+              out[(long)V2C_RO_V * n + i] = u;
+              reinterpret_cast<int2 *>(out)[(long)V2C_RO_PHI * n + i] =
+                  make_int2(rr.it32 + rr.itff, __float_as_int(rr.phi));
+              *mark = __longlong_as_double(MARK_NEWTON);
+            });
+      }
+      if (!left) {
+        it = r.it32 + r.itff;
+        put_state<true>(in, r, it, n, i, out, iters);
+        if (r.res > 0) resbits = (unsigned long long)__double_as_longlong(r.res);
+      }
+    }
+  }
+  add_stats(stat, it, 0, 0, resbits);
+}
+
+// The states left to the FP64 phase, gathered by each block from FIN states.
+constexpr int FIN = 4096;
+template <bool LEARNED>
+__global__ void __launch_bounds__(NT) k_states_finish(const double *S, long n, ff W,
+                                                      const float *guess, double rtol, int maxit,
+                                                      double *out, int32_t *iters,
+                                                      unsigned long long *stat) {
+  __shared__ int list[FIN], count;
+  if (threadIdx.x == 0) count = 0;
+  __syncthreads();
+  const long base = blockIdx.x * (long)FIN;
+  for (int k = threadIdx.x; k < FIN && base + k < n; k += NT) {
+    const unsigned long long m =
+        (unsigned long long)__double_as_longlong(out[(long)V2C_RO_RES * n + base + k]);
+    if (m == MARK_NEWTON || m == MARK_DEGENERATE) list[atomicAdd(&count, 1)] = k;
+  }
+  __syncthreads();
+  unsigned long long it_sum = 0, fb = 0, nc = 0, resbits = 0;
+  for (int k = threadIdx.x; k < count; k += NT) {
+    const long i = base + list[k];
+    RsfIn in;
+    double vold;
+    state_of(S, n, i, W, in, vold);
+    RsfResult r{};
+    r.phi = in.phio.hi;
+    if ((unsigned long long)__double_as_longlong(out[(long)V2C_RO_RES * n + i]) == MARK_NEWTON) {
+      const int2 b = reinterpret_cast<const int2 *>(out)[(long)V2C_RO_PHI * n + i];
+      r.it32 = b.x;
+      r.phi = __int_as_float(b.y);
+      rsf_finish64(in, out[(long)V2C_RO_V * n + i], rtol, maxit, r);
+    } else if (rsf_degenerate_in(in)) {
+      r.V = 1e-40;
+      r.ok = true;
+    } else {
+      const Phase32 p = get_phase32(out, n, i);
+      r = rsf_solve_phases<false>(
+          in, [&](RsfResult &rr, float &u, float &dF) { return resume(p, rr, u, dF); },
+          (float)rtol, [&](RsfFF &q) { rsf_setup_ff(q, in); },
+          [&](double u, RsfResult &rr) { rsf_finish64(in, u, rtol, maxit, rr); });
+    }
+    unsigned long long it = r.it32 + r.itff + r.it64;
+    const float u_plain = plain_start(vold);
+    if (LEARNED && !r.ok && guess[i] != u_plain) {
+      r = rsf_solve_split(in, rsf32_of(in), u_plain, rtol, maxit);
+      it += r.it32 + r.itff + r.it64;
+      fb++;
+    }
+    if (!r.ok) nc++;
+    it_sum += it;
+    put_state(in, r, it, n, i, out, iters);
+    if (r.res > 0) {
+      const unsigned long long b = (unsigned long long)__double_as_longlong(r.res);
+      if (b > resbits) resbits = b;
+    }
+  }
+  add_stats(stat, it_sum, fb, nc, resbits);
 }
 
 // The learned start of every state (the k_guess rule of the MIC step):
 // the plain start where its FP32 residual ratio is below RSF_NET_MIN_RES,
 // else the better of it and the network's proposal, the network evaluated
 // by a warp only when one of its states needs it.
-__global__ void __launch_bounds__(NT) k_learned_start(const double *S, long n, double W,
+__global__ void __launch_bounds__(NT) k_learned_start(const double *S, long n, ff W,
                                                       const float *mlp, float *u0_out) {
   __shared__ MlpSmem M;
   mlp_load_smem(M, mlp);
@@ -185,7 +353,7 @@ __global__ void __launch_bounds__(NT) k_learned_start(const double *S, long n, d
 }
 
 // network outputs (log V, phi) for every state
-__global__ void __launch_bounds__(NT) k_infer(const double *S, long n, double W, const float *mlp,
+__global__ void __launch_bounds__(NT) k_infer(const double *S, long n, ff W, const float *mlp,
                                               float *out) {
   __shared__ MlpSmem M;
   mlp_load_smem(M, mlp);
@@ -215,7 +383,7 @@ __global__ void __launch_bounds__(NT) k_infer(const double *S, long n, double W,
 
 // ------------------------------------------------------- training inputs
 // X[n][8] features, Y[n][2] = (log V, phi) targets, both FP32
-__global__ void k_features(const double *S, const double *T, long n, double W, float *X, float *Y) {
+__global__ void k_features(const double *S, const double *T, long n, ff W, float *X, float *Y) {
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   RsfIn in;
@@ -519,6 +687,12 @@ __global__ void k_sum_loss(const float *lp, int np, float *out) {
   }
 }
 
+// a double as a float pair, on the host
+ff pair_of(double d) {
+  const float h = (float)d;
+  return ff{h, (float)(d - (double)h)};
+}
+
 uint64_t splitmix(uint64_t &x) {
   uint64_t z = (x += 0x9e3779b97f4a7c15ull);
   z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
@@ -542,6 +716,7 @@ extern "C" int v2c_rsf_newton(v2c_ctx *ctx, const double *states_dev, long n, in
   if (guess == V2C_GUESS_LEARNED && !v2c_ctx_newton(ctx)->have_mlp) return V2C_ERR_STATE;
   if (n == 0) return V2C_OK;
   const v2c_params *p = v2c_ctx_params(ctx);
+  const ff W = pair_of(p->faultwidth);
   cudaStream_t st = v2c_ctx_stream(ctx);
   long warps = (n + 31) / 32;
   long blocks = (warps + 3) / 4;
@@ -559,14 +734,26 @@ extern "C" int v2c_rsf_newton(v2c_ctx *ctx, const double *states_dev, long n, in
       CKR(cudaMalloc((void **)&ns->d_guess, sizeof(float) * 2 * n));
       ns->guess_cap = n;
     }
-    k_learned_start<<<(unsigned)blocks, NT, 0, st>>>(states_dev, n, p->faultwidth, ns->d_mlp,
+    k_learned_start<<<(unsigned)blocks, NT, 0, st>>>(states_dev, n, W, ns->d_mlp,
                                                      ns->d_guess);
     v2c_ctx_count_launches(ctx, 1);
   }
-  auto kern = fp64 ? (learned ? k_solve_states<true, true> : k_solve_states<true, false>)
-                   : (learned ? k_solve_states<false, true> : k_solve_states<false, false>);
-  kern<<<(unsigned)blocks, NT, 0, st>>>(states_dev, n, p->faultwidth, ns->d_guess, p->newton_rtol,
-                                        p->newton_maxit, out_dev, iters_dev, v2c_ctx_stat(ctx));
+  if (fp64) {
+    (learned ? k_solve_states64<true> : k_solve_states64<false>)<<<(unsigned)blocks, NT, 0, st>>>(
+        states_dev, n, W, ns->d_guess, p->newton_rtol, p->newton_maxit, out_dev,
+        iters_dev, v2c_ctx_stat(ctx));
+  } else {
+    const unsigned nb = (unsigned)((n + NT - 1) / NT);
+    (learned ? k_states_fp32<true> : k_states_fp32<false>)<<<nb, NT, 0, st>>>(
+        states_dev, n, W, ns->d_guess, p->newton_maxit, out_dev);
+    k_states_polish<<<nb, NT, 0, st>>>(states_dev, n, W, (float)p->newton_rtol, out_dev, iters_dev,
+                                       v2c_ctx_stat(ctx));
+    const unsigned nf = (unsigned)((n + FIN - 1) / FIN);
+    (learned ? k_states_finish<true> : k_states_finish<false>)<<<nf, NT, 0, st>>>(
+        states_dev, n, W, ns->d_guess, p->newton_rtol, p->newton_maxit, out_dev, iters_dev,
+        v2c_ctx_stat(ctx));
+    v2c_ctx_count_launches(ctx, 2);
+  }
   v2c_ctx_prof_end(ctx, V2C_PROF_NEWTON, ev);
   v2c_ctx_count_launches(ctx, 1);
   CKR(cudaGetLastError());
@@ -620,7 +807,7 @@ int prepare(v2c_ctx *ctx, const double *S, const double *T, long n, int batch, T
   CKR(cudaMalloc((void **)&b.stats, sizeof(double) * 20));
   CKR(cudaMemsetAsync(b.m1, 0, sizeof(float) * NG, st));
   CKR(cudaMemsetAsync(b.m2, 0, sizeof(float) * NG, st));
-  k_features<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S, T, n, p->faultwidth, b.X, b.Y);
+  k_features<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S, T, n, pair_of(p->faultwidth), b.X, b.Y);
   v2c_ctx_count_launches(ctx, 1);
   if (set_norm) {
     k_colstats<<<8, 256, 0, st>>>(b.X, n, 8, b.stats, b.stats + 8);
@@ -743,7 +930,7 @@ extern "C" int v2c_mlp_infer(v2c_ctx *ctx, const double *states_dev, long n, flo
   if (n == 0) return V2C_OK;
   long blocks = ((n + 31) / 32 + 3) / 4;
   if (blocks > 152 * 16) blocks = 152 * 16;
-  k_infer<<<(unsigned)blocks, NT, 0, v2c_ctx_stream(ctx)>>>(states_dev, n, v2c_ctx_params(ctx)->faultwidth,
+  k_infer<<<(unsigned)blocks, NT, 0, v2c_ctx_stream(ctx)>>>(states_dev, n, pair_of(v2c_ctx_params(ctx)->faultwidth),
                                                            v2c_ctx_newton(ctx)->d_mlp, out_dev);
   v2c_ctx_count_launches(ctx, 1);
   CKR(cudaGetLastError());

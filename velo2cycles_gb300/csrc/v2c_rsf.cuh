@@ -170,20 +170,24 @@ struct RsfFF {
 #define V2C_TWO64 1.8446744073709552e19f
 #define V2C_TWOM64 5.4210108624275222e-20f
 
+// Out of line for the set-up of a state, which divides four times (3 KB of
+// code each inline).
+static __device__ __noinline__ ff ff_div_call(ff a, ff b) { return ff_div(a, b); }
+
 __device__ __forceinline__ void rsf_setup_ff(RsfFF &q, const RsfIn &in) {
   const ff Gdt = ff_mul(in.G, in.dt);
   q.Ts = ff_add(in.tau_old, ff_scale(ff_mul(Gdt, in.edot), 2.f));
-  const ff c1 = ff_add_f(ff_div(Gdt, in.eta), 1.f);
-  q.klin = ff_add(ff_mul_f(c1, 4330300.f), ff_scale(ff_div(Gdt, in.W), 2.f));
+  const ff c1 = ff_add_f(ff_div_call(Gdt, in.eta), 1.f);
+  q.klin = ff_add(ff_mul_f(c1, 4330300.f), ff_scale(ff_div_call(Gdt, in.W), 2.f));
   q.snac1 = ff_mul(ff_mul(in.sn, in.a), c1);
   q.ephio = ff_exp(in.phio);
-  q.dtL = ff_div(in.dt, in.L);
+  q.dtL = ff_div_call(in.dt, in.L);
   q.V0dtL = ff_mul(in.V0, q.dtL);
   q.V0s = ff_scale(in.V0, V2C_TWO64);
   q.ln2V0 = ff_log(ff_scale(in.V0, 2.f));
   q.mu0 = in.mu0;
   q.b = in.b;
-  q.inv_a = ff_div(ff_f(1.f), in.a);
+  q.inv_a = ff_div_call(ff_f(1.f), in.a);
 }
 
 // What the set-ups of one call's markers share: almost every marker lies
@@ -422,22 +426,23 @@ __device__ __forceinline__ float rsf_start_residual(const Rsf32 &q, float u0, fl
 // two.
 constexpr float RSF_NET_MIN_RES = 1e-2f;
 
-// Split solve from the start u0 (FP32 phase, float-float phase, FP64
-// fallback).  q32 = rsf32_of(in); setup(q) fills the float-float constants,
-// finish(u, r) runs the FP64 Newton from u.
-template <class Setup, class Finish>
-__device__ __forceinline__ RsfResult rsf_solve_split(const RsfIn &in, const Rsf32 &q32, float u0,
-                                                     double rtol, int maxit, Setup setup,
-                                                     Finish finish) {
+// whether the FP32 form of a load is degenerate (FP64 decides)
+__device__ __forceinline__ bool rsf_degenerate32(const Rsf32 &q) {
+  return !(q.Ts > 0.f) || !(q.uhi > (float)RSF_LOG_FLOOR);
+}
+
+// Split solve.  phase32(r, u32, dF32) gives the FP32 phase's iterate and
+// derivative there, or returns false with a degenerate load's result in r;
+// setup(q) fills the float-float constants, finish(u, r) runs the FP64 Newton
+// from u.  BITS: the FP64 results widened without FP64 conversions.
+template <bool BITS, class Phase32, class Setup, class Finish>
+__device__ __forceinline__ RsfResult rsf_solve_phases(const RsfIn &in, Phase32 phase32, float rtol,
+                                                      Setup setup, Finish finish) {
   RsfResult r{};
   r.phi = in.phio.hi;
   const float floor32 = (float)RSF_LOG_FLOOR;
-  if (!(q32.Ts > 0.f) || !(q32.uhi > floor32)) {
-    // degenerate in FP32: decided in FP64 as the FP64 form does
-    if (rsf_degenerate_in(in)) { r.V = 1e-40; r.Vf = 1e-40f; r.ok = true; return r; }
-  }
-  float dF32;
-  const float u32 = rsf_newton32(q32, u0, floor32, q32.uhi, maxit, r.it32, dF32);
+  float u32, dF32;
+  if (!phase32(r, u32, dF32)) return r;
   RsfFF q;
   setup(q);
   const ff floor_u = ff_from_double(RSF_LOG_FLOOR);
@@ -447,7 +452,7 @@ __device__ __forceinline__ RsfResult rsf_solve_split(const RsfIn &in, const Rsf3
   // at 3/4 of the tolerance: the float-float ratio and the FP64 one at the
   // same slip rate differ by up to ~1.3e-11 (measured on 20 000 states of
   // the C3 distributions), and the returned root must meet rtol in FP64.
-  const float rtolf = 0.75f * (float)rtol;
+  const float rtolf = 0.75f * rtol;
   for (int k = 0; k < 4; k++) {
     ff lhs, phi, A, Vs;
     const ff F = rsf_eval_ff(q, u, lhs, phi, A, Vs);
@@ -455,10 +460,10 @@ __device__ __forceinline__ RsfResult rsf_solve_split(const RsfIn &in, const Rsf3
     const float rel = fabsf(F.hi) / lhs.hi;
     r.phi = phi.hi;
     if (rel <= rtolf) {
-      r.A = ff_to_double(A);
-      r.V = ff_to_double(Vs) * 5.4210108624275222e-20;
+      r.A = ff_to_double<BITS>(A);
+      r.V = ff_to_double<BITS>(Vs) * 5.4210108624275222e-20;
       r.Vf = Vs.hi * V2C_TWOM64;
-      r.res = rel;
+      r.res = widen<BITS>(rel);
       r.ok = true;
       return r;
     }
@@ -472,6 +477,27 @@ __device__ __forceinline__ RsfResult rsf_solve_split(const RsfIn &in, const Rsf3
   }
   finish(ff_to_double(u), r);  // the FP64 Newton finishes
   return r;
+}
+
+// from the start u0; q32 = rsf32_of(in)
+template <class Setup, class Finish>
+__device__ __forceinline__ RsfResult rsf_solve_split(const RsfIn &in, const Rsf32 &q32, float u0,
+                                                     double rtol, int maxit, Setup setup,
+                                                     Finish finish) {
+  return rsf_solve_phases<false>(
+      in,
+      [&](RsfResult &r, float &u32, float &dF32) {
+        if (rsf_degenerate32(q32)) {
+          // degenerate in FP32: decided in FP64 as the FP64 form does
+          if (rsf_degenerate_in(in)) {
+            r.V = 1e-40; r.Vf = 1e-40f; r.ok = true;
+            return false;
+          }
+        }
+        u32 = rsf_newton32(q32, u0, (float)RSF_LOG_FLOOR, q32.uhi, maxit, r.it32, dF32);
+        return true;
+      },
+      (float)rtol, setup, finish);
 }
 // with the state's own constants
 __device__ __forceinline__ RsfResult rsf_solve_split(const RsfIn &in, const Rsf32 &q32, float u0,
