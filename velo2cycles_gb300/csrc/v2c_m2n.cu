@@ -442,6 +442,7 @@ __device__ __forceinline__ void sum_basic(const M2NArgs &a, const Smem &sm, cons
 // (3.15 -> 2.98 ms).  Copying through registers instead of asynchronously
 // was slower (0.47 against 0.44 ms on the smaller model).
 __global__ void __launch_bounds__(NTH, 4) k_m2n(M2NArgs a) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
   const Grid &g = a.g;
@@ -775,6 +776,7 @@ __device__ __forceinline__ void mode1_node(const M2NArgs &a) {
 // groups fill each other's gaps (433 x 187 lines, 0.84 M markers: 378 us
 // against 488 in four launches).
 __global__ void __launch_bounds__(128) k_m2n_mode1(M2NArgs a) {
+  after_previous();
   switch (blockIdx.y) {
     case 0: mode1_node<2>(a); break;  // most cells per node: first
     case 1: mode1_node<3>(a); break;
@@ -785,6 +787,7 @@ __global__ void __launch_bounds__(128) k_m2n_mode1(M2NArgs a) {
 
 // ghost copy of the state when it diffuses, interpolation.c:827-859
 __global__ void k_dphis(Grid g, float *phis) {
+  after_previous();
   long m3 = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (m3 >= g.nn) return;
   const int yn = g.yn, xn = g.xn;
@@ -810,15 +813,15 @@ cudaError_t m2n_init() {
 void launch_m2n(const M2NArgs &a, cudaStream_t st) {
   if (a.S.p.interpolationmod == 1) {
     const unsigned nb = (unsigned)((a.g.nn + 127) / 128);
-    k_m2n_mode1<<<dim3(nb, 4), 128, 0, st>>>(a);
+    launch_after(k_m2n_mode1, dim3(nb, 4), 128, 0, st, a);
     return;
   }
   dim3 grid((a.g.xn + a.TX - 1) / a.TX, (a.g.yn + TY - 1) / TY);
-  k_m2n<<<grid, NTH, sizeof(Smem), st>>>(a);
+  launch_after(k_m2n, grid, NTH, sizeof(Smem), st, a);
 }
 
 void launch_dphis(const Grid &g, const Nodes &N, cudaStream_t st) {
-  k_dphis<<<(unsigned)((g.nn + 255) / 256), 256, 0, st>>>(g, N.f(V2C_NF_PHIS));
+  launch_after(k_dphis, (unsigned)((g.nn + 255) / 256), 256, 0, st, g, N.f(V2C_NF_PHIS));
 }
 
 }  // namespace v2c

@@ -110,6 +110,7 @@ __device__ __forceinline__ float4 blend(float4 p, float4 s, float xrat) {
 // one thread per cell quarter t = 4 cell + 2 qy + qx; stencils as in
 // stencil_basic / stencil_centre / stencil_vx / stencil_vy
 __global__ void k_vel_quads(Grid g, Nodes N, float4 *Q) {
+  after_previous();
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (t >= (long)g.ncx * g.ncy * 4) return;
   const long c = t >> 2;
@@ -441,6 +442,7 @@ __device__ __forceinline__ Runs two_runs(int cs, int ce, int b1, int e1, int b2,
 // column, and the temperature is written only where it changes.  Halo
 // markers that reach no node of the tile are not gathered.
 __global__ void __launch_bounds__(NTH, 4) k_n2m(N2MArgs a) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
   const Grid &g = a.g;
@@ -658,6 +660,7 @@ __global__ void __launch_bounds__(NTH, 4) k_n2m(N2MArgs a) {
 // us against the chunked sweep).
 template <bool BS, bool PLAIN>
 __global__ void __launch_bounds__(256, 6) k_gather(N2MArgs a) {
+  after_previous();
   const Grid &g = a.g;
   const Nodes &N = a.N;
   const v2c_params &P = a.S.p;
@@ -834,6 +837,7 @@ __device__ __forceinline__ void bs_mode1(const N2MArgs &a) {
 
 // both node kinds in one launch, a row of blocks each
 __global__ void __launch_bounds__(128) k_n2m_bs_mode1(N2MArgs a) {
+  after_previous();
   if (blockIdx.y == 0) bs_mode1<1>(a);
   else bs_mode1<0>(a);
 }
@@ -850,6 +854,7 @@ __global__ void __launch_bounds__(128) k_n2m_bs_mode1(N2MArgs a) {
 // with the quarters' forms: 1725 -> 1525 us (1616 in array order alone, 1566
 // with the stresses asked for).
 __global__ void __launch_bounds__(256, 6) k_move(N2MArgs a) {
+  after_previous();
   const Grid &g = a.g;
   const v2c_params &P = a.S.p;
   const int ncy = g.ncy;
@@ -1023,23 +1028,23 @@ cudaError_t n2m_init() {
 void launch_n2m(const N2MArgs &a, cudaStream_t st) {
   const unsigned mb = (unsigned)((a.n + 255) / 256);
   if (a.bs) {
-    if (a.n > 0) k_gather<true, false><<<mb, 256, 0, st>>>(a);
+    if (a.n > 0) launch_after(k_gather<true, false>, mb, 256, 0, st, a);
     const unsigned nb = (unsigned)((a.g.nn + 127) / 128);
-    k_n2m_bs_mode1<<<dim3(nb, 2), 128, 0, st>>>(a);
+    launch_after(k_n2m_bs_mode1, dim3(nb, 2), 128, 0, st, a);
   } else if (a.S.p.antidiffinter == 1) {
     dim3 grid((a.g.xn + a.TX - 1) / a.TX, (a.g.yn + TY - 1) / TY);
-    k_n2m<<<grid, NTH, sizeof(Smem), st>>>(a);
+    launch_after(k_n2m, grid, NTH, sizeof(Smem), st, a);
   } else if (a.n > 0) {
     // the markers take the node fields without antidiffusion
-    k_gather<false, true><<<mb, 256, 0, st>>>(a);
+    launch_after(k_gather<false, true>, mb, 256, 0, st, a);
   }
 }
 
 void launch_move(const N2MArgs &a, cudaStream_t st) {
   const long quarters = (long)a.g.ncx * a.g.ncy * 4;
-  k_vel_quads<<<(unsigned)((quarters + 255) / 256), 256, 0, st>>>(a.g, a.N, a.quad);
+  launch_after(k_vel_quads, (unsigned)((quarters + 255) / 256), 256, 0, st, a.g, a.N, a.quad);
   if (a.n <= 0) return;
-  k_move<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a);
+  launch_after(k_move, (unsigned)((a.n + 255) / 256), 256, 0, st, a);
 }
 
 }  // namespace v2c

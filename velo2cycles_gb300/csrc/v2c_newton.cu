@@ -194,6 +194,7 @@ constexpr unsigned long long MARK_DEGENERATE = 0x7ff4563243324302ull;
 template <bool LEARNED>
 __global__ void __launch_bounds__(NT) k_states_fp32(const double *S, long n, ff W,
                                                     const float *guess, int maxit, double *out) {
+  after_previous();
   const long i = blockIdx.x * (long)NT + threadIdx.x;
   if (i >= n) return;
   RsfIn in;
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(NT) k_states_fp32(const double *S, long n, ff 
 __global__ void __launch_bounds__(NT, 8) k_states_polish(const double *S, long n, ff W, float rtolf,
                                                          double *out, int32_t *iters,
                                                          unsigned long long *stat) {
+  after_previous();
   const long i = blockIdx.x * (long)NT + threadIdx.x;
   unsigned long long it = 0, resbits = 0;
   if (i < n) {
@@ -258,6 +260,7 @@ __global__ void __launch_bounds__(NT) k_states_finish(const double *S, long n, f
                                                       const float *guess, double rtol, int maxit,
                                                       double *out, int32_t *iters,
                                                       unsigned long long *stat) {
+  after_previous();
   __shared__ int list[FIN], count;
   if (threadIdx.x == 0) count = 0;
   __syncthreads();
@@ -315,6 +318,7 @@ __global__ void __launch_bounds__(NT) k_states_finish(const double *S, long n, f
 // by a warp only when one of its states needs it.
 __global__ void __launch_bounds__(NT) k_learned_start(const double *S, long n, ff W,
                                                       const float *mlp, float *u0_out) {
+  after_previous();
   __shared__ MlpSmem M;
   mlp_load_smem(M, mlp);
   __syncthreads();
@@ -734,8 +738,8 @@ extern "C" int v2c_rsf_newton(v2c_ctx *ctx, const double *states_dev, long n, in
       CKR(cudaMalloc((void **)&ns->d_guess, sizeof(float) * 2 * n));
       ns->guess_cap = n;
     }
-    k_learned_start<<<(unsigned)blocks, NT, 0, st>>>(states_dev, n, W, ns->d_mlp,
-                                                     ns->d_guess);
+    launch_after(k_learned_start, (unsigned)blocks, NT, 0, st, states_dev, n, W, ns->d_mlp,
+                 ns->d_guess);
     v2c_ctx_count_launches(ctx, 1);
   }
   if (fp64) {
@@ -744,14 +748,18 @@ extern "C" int v2c_rsf_newton(v2c_ctx *ctx, const double *states_dev, long n, in
         iters_dev, v2c_ctx_stat(ctx));
   } else {
     const unsigned nb = (unsigned)((n + NT - 1) / NT);
-    (learned ? k_states_fp32<true> : k_states_fp32<false>)<<<nb, NT, 0, st>>>(
-        states_dev, n, W, ns->d_guess, p->newton_maxit, out_dev);
-    k_states_polish<<<nb, NT, 0, st>>>(states_dev, n, W, (float)p->newton_rtol, out_dev, iters_dev,
-                                       v2c_ctx_stat(ctx));
+    if (learned) launch_after(k_states_fp32<true>, nb, NT, 0, st, states_dev, n, W, ns->d_guess,
+                              p->newton_maxit, out_dev);
+    else launch_after(k_states_fp32<false>, nb, NT, 0, st, states_dev, n, W, ns->d_guess,
+                      p->newton_maxit, out_dev);
+    launch_after(k_states_polish, nb, NT, 0, st, states_dev, n, W, (float)p->newton_rtol, out_dev,
+                 iters_dev, v2c_ctx_stat(ctx));
     const unsigned nf = (unsigned)((n + FIN - 1) / FIN);
-    (learned ? k_states_finish<true> : k_states_finish<false>)<<<nf, NT, 0, st>>>(
-        states_dev, n, W, ns->d_guess, p->newton_rtol, p->newton_maxit, out_dev, iters_dev,
-        v2c_ctx_stat(ctx));
+    if (learned) launch_after(k_states_finish<true>, nf, NT, 0, st, states_dev, n, W, ns->d_guess,
+                              p->newton_rtol, p->newton_maxit, out_dev, iters_dev,
+                              v2c_ctx_stat(ctx));
+    else launch_after(k_states_finish<false>, nf, NT, 0, st, states_dev, n, W, ns->d_guess,
+                      p->newton_rtol, p->newton_maxit, out_dev, iters_dev, v2c_ctx_stat(ctx));
     v2c_ctx_count_launches(ctx, 2);
   }
   v2c_ctx_prof_end(ctx, V2C_PROF_NEWTON, ev);

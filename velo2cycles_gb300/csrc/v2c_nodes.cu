@@ -108,6 +108,7 @@ __device__ __forceinline__ ff new_state_ff(float ph, float V, ff dt, float L, fl
 // sxx - sxxe is taken from DSXX, which recompute_stress_strainrate wrote
 // for the current sxx and sxxe (the FP32 difference cancels at small dt)
 __global__ void k_c2b(Grid g, Nodes N, float dt, float dt_lo, int use_dsxx) {
+  after_previous();
   long m3 = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (m3 >= g.nn) return;
   const long yn = g.yn;
@@ -159,6 +160,7 @@ __device__ __forceinline__ int centre_stencil(const double *gl, const float *w, 
 // interpolate_basic2center (interpolation.c:1639-1685): nd at every node
 // with m1, m2 >= 1 as the harmonic mean of nu over the basic stencil
 __global__ void k_b2c(Grid g, Nodes N, unsigned long long *stat) {
+  after_previous();
   long m3 = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (m3 >= g.nn) return;
   const long yn = g.yn;
@@ -202,6 +204,7 @@ __device__ __forceinline__ ff nueff_ff(float nvp, float ggeff, ff dt, float nube
 // the FP64 line spacings, each output rounded once.
 __global__ void k_recompute(Grid g, Nodes N, float dt, float dt_lo, float nubeg,
                             const double *vx64, const double *vy64) {
+  after_previous();
   long m3 = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (m3 >= g.nn) return;
   const long yn = g.yn;
@@ -252,6 +255,7 @@ __global__ void k_recompute(Grid g, Nodes N, float dt, float dt_lo, float nubeg,
 // copyarrays (momentum_continuity_iterate.c:265-281): the solved slip and
 // state rates become the final ones
 __global__ void k_copyarrays(Grid g, Nodes N) {
+  after_previous();
   long m3 = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (m3 >= g.nn) return;
   const long yn = g.yn;
@@ -265,12 +269,14 @@ __global__ void k_copyarrays(Grid g, Nodes N) {
 
 // accumulated slip of every marker (the per-marker Newton's slip rate)
 __global__ void k_marker_slip_acc(const float *slipv, long n, double dt, double *acc) {
+  after_previous();
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i < n) acc[i] += dt * (double)slipv[i];
 }
 
 // accumulated slip of every interior basic node: acc += dt * slip rate
 __global__ void k_slip_acc(Grid g, const float *v, double dt, double *acc) {
+  after_previous();
   long m3 = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (m3 >= g.nn) return;
   const long yn = g.yn;
@@ -279,6 +285,7 @@ __global__ void k_slip_acc(Grid g, const float *v, double dt, double *acc) {
 }
 
 __global__ void k_c2b_old(Grid g, Nodes N) {
+  after_previous();
   long m3 = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (m3 >= g.nn) return;
   const long yn = g.yn;
@@ -293,6 +300,7 @@ __global__ void k_c2b_old(Grid g, Nodes N) {
 
 __global__ void k_before(Grid g, Nodes N, Scal S, float dt, float dt_lo, int rk,
                          unsigned long long *stat) {
+  after_previous();
   long m3 = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (m3 >= g.nn) return;
   const v2c_params &p = S.p;
@@ -379,6 +387,7 @@ __global__ void k_before(Grid g, Nodes N, Scal S, float dt, float dt_lo, int rk,
 // per-block partial sums of (syield - sigin)^2 and counts
 constexpr int AB = 256;
 __global__ void k_after(Grid g, Nodes N, Scal S, float dt, float *part) {
+  after_previous();
   __shared__ float sd[AB];
   __shared__ float sc[AB];
   long m3 = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -463,6 +472,7 @@ __global__ void k_after(Grid g, Nodes N, Scal S, float dt, float *part) {
 // fold the block partials in block order (single block, fixed order); the
 // few thousand partials are summed in FP64
 __global__ void k_after_fold(const float *part, long nb, double *out) {
+  after_previous();
   __shared__ double sd[AB], sc[AB];
   double d = 0, c = 0;
   for (long i = threadIdx.x; i < nb; i += AB) {
@@ -489,6 +499,7 @@ __global__ void k_after_fold(const float *part, long nb, double *out) {
 // need no order among themselves; the sticky-air flags are a field of their
 // own.  One launch where three took 8 us of a 51 x 21-line step's 270.
 __global__ void k_m2n_tail(BcRows r, Nodes N, const uint32_t *key, long nn) {
+  after_previous();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i < nn) {
     const uint32_t k = key[i];
@@ -519,6 +530,7 @@ struct FieldList {
   int f[V2C_NF_N];
 };
 __global__ void k_fields_to_f64(const float *base, long nn, FieldList L, double *stage) {
+  after_previous();
   const float *src = base + (long)L.f[blockIdx.y] * nn;
   double *dst = stage + (long)blockIdx.y * nn;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nn; i += (long)gridDim.x * blockDim.x)
@@ -550,6 +562,7 @@ struct HostCopies {
 };
 // __grid_constant__: the block's row is indexed in the parameter itself
 __global__ void k_host_to_fields(const __grid_constant__ HostFields H, long nn, float *base) {
+  after_previous();
   const double *src = H.src[blockIdx.y];
   float *dst = base + (long)H.f[blockIdx.y] * nn;
   double *keep = H.keep[blockIdx.y];
@@ -560,12 +573,14 @@ __global__ void k_host_to_fields(const __grid_constant__ HostFields H, long nn, 
   }
 }
 __global__ void k_fields_to_host(const float *base, long nn, const __grid_constant__ HostCopies H) {
+  after_previous();
   const float *src = base + (long)H.f[blockIdx.y] * nn;
   double *dst = H.dst[blockIdx.y];
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nn; i += (long)gridDim.x * blockDim.x)
     dst[i] = (double)src[i];
 }
 __global__ void k_stage_to_host(const double *stage, long nn, const __grid_constant__ HostCopies H) {
+  after_previous();
   const double *src = stage + (long)H.f[blockIdx.y] * nn;
   double *dst = H.dst[blockIdx.y];
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nn; i += (long)gridDim.x * blockDim.x)
@@ -580,34 +595,34 @@ dim3 host_grid(long nn, int count) {
 }  // namespace
 
 void launch_c2b_old(const Grid &g, const Nodes &N, cudaStream_t st) {
-  k_c2b_old<<<nblk(g.nn, 256), 256, 0, st>>>(g, N);
+  launch_after(k_c2b_old, nblk(g.nn, 256), 256, 0, st, g, N);
 }
 
 void launch_c2b(const Grid &g, const Nodes &N, double dt, int use_dsxx, cudaStream_t st) {
   const float hi = (float)dt, lo = (float)(dt - (double)hi);
-  k_c2b<<<nblk(g.nn, 256), 256, 0, st>>>(g, N, hi, lo, use_dsxx);
+  launch_after(k_c2b, nblk(g.nn, 256), 256, 0, st, g, N, hi, lo, use_dsxx);
 }
 void launch_recompute(const Grid &g, const Nodes &N, const Scal &S, double dt, const double *vx64,
                       const double *vy64, cudaStream_t st) {
   const float hi = (float)dt, lo = (float)(dt - (double)hi);
-  k_recompute<<<nblk(g.nn, 256), 256, 0, st>>>(g, N, hi, lo, S.nubeg_f, vx64, vy64);
+  launch_after(k_recompute, nblk(g.nn, 256), 256, 0, st, g, N, hi, lo, S.nubeg_f, vx64, vy64);
 }
 void launch_copyarrays(const Grid &g, const Nodes &N, cudaStream_t st) {
-  k_copyarrays<<<nblk(g.nn, 256), 256, 0, st>>>(g, N);
+  launch_after(k_copyarrays, nblk(g.nn, 256), 256, 0, st, g, N);
 }
 void launch_marker_slip_acc(const float *slipv, long n, double dt, double *acc, cudaStream_t st) {
-  if (n > 0) k_marker_slip_acc<<<nblk(n, 256), 256, 0, st>>>(slipv, n, dt, acc);
+  if (n > 0) launch_after(k_marker_slip_acc, nblk(n, 256), 256, 0, st, slipv, n, dt, acc);
 }
 void launch_slip_acc(const Grid &g, const Nodes &N, double dt, double *acc, cudaStream_t st) {
-  k_slip_acc<<<nblk(g.nn, 256), 256, 0, st>>>(g, N.f(V2C_NF_RK_SLIPRS_FINAL), dt, acc);
+  launch_after(k_slip_acc, nblk(g.nn, 256), 256, 0, st, g, N.f(V2C_NF_RK_SLIPRS_FINAL), dt, acc);
 }
 void launch_b2c(const Grid &g, const Nodes &N, unsigned long long *stat, cudaStream_t st) {
-  k_b2c<<<nblk(g.nn, 256), 256, 0, st>>>(g, N, stat);
+  launch_after(k_b2c, nblk(g.nn, 256), 256, 0, st, g, N, stat);
 }
 void launch_before_solve(const Grid &g, const Nodes &N, const Scal &S, double dt, int rk,
                          unsigned long long *stat, cudaStream_t st) {
   const float hi = (float)dt, lo = (float)(dt - (double)hi);
-  k_before<<<nblk(g.nn, 256), 256, 0, st>>>(g, N, S, hi, lo, rk, stat);
+  launch_after(k_before, nblk(g.nn, 256), 256, 0, st, g, N, S, hi, lo, rk, stat);
 }
 
 void launch_after_solve(const Grid &g, const Nodes &N, const Scal &S, double dt, int rk,
@@ -615,14 +630,14 @@ void launch_after_solve(const Grid &g, const Nodes &N, const Scal &S, double dt,
   (void)rk;
   long nb = (g.nn + AB - 1) / AB;
   float *part = (float *)red;
-  k_after<<<(unsigned)nb, AB, 0, st>>>(g, N, S, (float)dt, part);
-  if (out) k_after_fold<<<1, AB, 0, st>>>(part, nb, out);
+  launch_after(k_after, (unsigned)nb, AB, 0, st, g, N, S, (float)dt, part);
+  if (out) launch_after(k_after_fold, 1, AB, 0, st, part, nb, out);
 }
 
 void launch_m2n_tail(const BcRows &rows, const Nodes &N, const uint32_t *sticky_key, long nn,
                      cudaStream_t st) {
   const long n = nn > rows.n ? nn : rows.n;
-  k_m2n_tail<<<nblk(n, 256), 256, 0, st>>>(rows, N, sticky_key, nn);
+  launch_after(k_m2n_tail, nblk(n, 256), 256, 0, st, rows, N, sticky_key, nn);
 }
 
 void launch_node_to_f32(const double *src, float *dst, long n, cudaStream_t st) {
@@ -635,8 +650,8 @@ void launch_fields_to_f64(const float *base, long nn, const int *fields, int cou
                           cudaStream_t st) {
   if (nn <= 0 || count <= 0) return;
   const unsigned bx = nblk(nn, 256) < 152 * 8 ? nblk(nn, 256) : 152 * 8;
-  k_fields_to_f64<<<dim3(bx, (unsigned)count), 256, 0, st>>>(base, nn, field_list(fields, count),
-                                                             stage);
+  launch_after(k_fields_to_f64, dim3(bx, (unsigned)count), 256, 0, st, base, nn, field_list(fields,
+               count), stage);
 }
 void launch_host_to_fields(const double *const *src, const int *fields, double *const *keep,
                            int count, long nn, float *base, cudaStream_t st) {
@@ -647,7 +662,7 @@ void launch_host_to_fields(const double *const *src, const int *fields, double *
     H.f[k] = fields[k];
     H.keep[k] = keep[k];
   }
-  k_host_to_fields<<<host_grid(nn, count), 256, 0, st>>>(H, nn, base);
+  launch_after(k_host_to_fields, host_grid(nn, count), 256, 0, st, H, nn, base);
 }
 void launch_fields_to_host(const float *base, const int *fields, double *const *dst, int count,
                            long nn, cudaStream_t st) {
@@ -657,7 +672,7 @@ void launch_fields_to_host(const float *base, const int *fields, double *const *
     H.dst[k] = dst[k];
     H.f[k] = fields[k];
   }
-  k_fields_to_host<<<host_grid(nn, count), 256, 0, st>>>(base, nn, H);
+  launch_after(k_fields_to_host, host_grid(nn, count), 256, 0, st, base, nn, H);
 }
 void launch_stage_to_host(const double *stage, double *const *dst, int count, long nn,
                           cudaStream_t st) {
@@ -667,7 +682,7 @@ void launch_stage_to_host(const double *stage, double *const *dst, int count, lo
     H.dst[k] = dst[k];
     H.f[k] = k;
   }
-  k_stage_to_host<<<host_grid(nn, count), 256, 0, st>>>(stage, nn, H);
+  launch_after(k_stage_to_host, host_grid(nn, count), 256, 0, st, stage, nn, H);
 }
 void launch_fields_to_f32(const double *stage, long nn, const int *fields, int count, float *base,
                           cudaStream_t st) {

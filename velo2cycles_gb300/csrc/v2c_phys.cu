@@ -101,6 +101,7 @@ __device__ __forceinline__ void marker_problem(const PhysArgs &a, long i, const 
 // C4 physics + Newton 8.30 ms at 7, 7.98 at 8, 8.11 at 10 (spills).
 template <int MODE>
 __global__ void __launch_bounds__(PT, 8) k_phys(PhysArgs a) {
+  after_previous();
   const Grid &g = a.g;
   const bool collect = MODE == PHYS_COLLECT;
   const bool newton = MODE == PHYS_SPLIT || MODE == PHYS_FP64;
@@ -232,6 +233,7 @@ __global__ void __launch_bounds__(PT, 8) k_phys(PhysArgs a) {
 // problems needs it), written to guess[e]; a kernel of its own so the
 // Newton kernel keeps the occupancy of the plain start.
 __global__ void __launch_bounds__(PT, 4) k_guess(PhysArgs a, float *guess) {
+  after_previous();
   __shared__ MlpSmem S;
   mlp_load_smem(S, a.mlp);
   __syncthreads();
@@ -292,6 +294,7 @@ static __device__ __noinline__ void marker_finish64(const PhysArgs &a, long i, d
 // stage from 7.77 to 7.63 ms.
 template <bool FP64, bool LEARNED>
 __global__ void __launch_bounds__(PT, 8) k_newton(PhysArgs a, const float *guess) {
+  after_previous();
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const long nwarps = (long)gridDim.x * (PT / 32);
   const long cnt = *a.list_n;
@@ -341,6 +344,7 @@ __global__ void __launch_bounds__(PT, 8) k_newton(PhysArgs a, const float *guess
 // constants, in one launch: no sticky-air candidates, an empty problem list.
 // The constants' long chains go to different warps of block 0.
 __global__ void __launch_bounds__(256) k_phys_init(PhysArgs a, bool newton) {
+  after_previous();
   const long nn = a.g.nn;
   for (long i = blockIdx.x * 256l + threadIdx.x; i < nn; i += gridDim.x * 256l) a.sticky_key[i] = 0;
   if (!newton || blockIdx.x != 0) return;
@@ -371,8 +375,8 @@ void launch_phys(const PhysArgs &a, cudaStream_t st) {
   const v2c_params &p = a.S.p;
   if (!a.xs) {
     const long nb = (a.g.nn + 255) / 256;
-    k_phys_init<<<(unsigned)(nb < 608 ? nb : 608), 256, 0, st>>>(
-        a, a.n > 0 && p.newton_guess != V2C_GUESS_OFF);
+    launch_after(k_phys_init, (unsigned)(nb < 608 ? nb : 608), 256, 0, st, a,
+                 a.n > 0 && p.newton_guess != V2C_GUESS_OFF);
   }
   if (a.n <= 0) return;
   // one pass of 32 markers per warp: the blocks' times differ with the creep
@@ -383,24 +387,28 @@ void launch_phys(const PhysArgs &a, cudaStream_t st) {
   const bool fp64 = p.newton_precision == V2C_NEWTON_FP64;
   const unsigned nb = (unsigned)blocks;
   if (a.xs) {
-    k_phys<PHYS_COLLECT><<<nb, PT, 0, st>>>(a);
+    launch_after(k_phys<PHYS_COLLECT>, nb, PT, 0, st, a);
     return;
   }
   if (p.newton_guess == V2C_GUESS_OFF) {
-    k_phys<PHYS_OFF><<<nb, PT, 0, st>>>(a);
+    launch_after(k_phys<PHYS_OFF>, nb, PT, 0, st, a);
     return;
   }
-  if (fp64) k_phys<PHYS_FP64><<<nb, PT, 0, st>>>(a);
-  else k_phys<PHYS_SPLIT><<<nb, PT, 0, st>>>(a);
-  if (learned) k_guess<<<resident_grid(k_guess, PT), PT, 0, st>>>(a, a.guess);
+  if (fp64) launch_after(k_phys<PHYS_FP64>, nb, PT, 0, st, a);
+  else launch_after(k_phys<PHYS_SPLIT>, nb, PT, 0, st, a);
+  if (learned) launch_after(k_guess, resident_grid(k_guess, PT), PT, 0, st, a, a.guess);
   if (fp64 && learned)
-    k_newton<true, true><<<resident_grid(k_newton<true, true>, PT), PT, 0, st>>>(a, a.guess);
+    launch_after(k_newton<true, true>, resident_grid(k_newton<true, true>, PT), PT, 0, st, a,
+                 a.guess);
   else if (fp64)
-    k_newton<true, false><<<resident_grid(k_newton<true, false>, PT), PT, 0, st>>>(a, a.guess);
+    launch_after(k_newton<true, false>, resident_grid(k_newton<true, false>, PT), PT, 0, st, a,
+                 a.guess);
   else if (learned)
-    k_newton<false, true><<<resident_grid(k_newton<false, true>, PT), PT, 0, st>>>(a, a.guess);
+    launch_after(k_newton<false, true>, resident_grid(k_newton<false, true>, PT), PT, 0, st, a,
+                 a.guess);
   else
-    k_newton<false, false><<<resident_grid(k_newton<false, false>, PT), PT, 0, st>>>(a, a.guess);
+    launch_after(k_newton<false, false>, resident_grid(k_newton<false, false>, PT), PT, 0, st, a,
+                 a.guess);
 }
 
 }  // namespace v2c

@@ -40,6 +40,7 @@ __global__ void k_assign(Grid g, const double *x, const double *y, long n, Marke
 constexpr int MK = 4;
 __global__ void __launch_bounds__(256) k_count(const int32_t *cell, long n, int32_t *counts,
                                                int32_t *slot) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const long i0 = (blockIdx.x * 8l + (threadIdx.x >> 5)) * (32 * MK) + lane;
   int c[MK], base[MK];
@@ -90,6 +91,7 @@ __device__ __forceinline__ int32_t block_scan(int32_t v, int32_t *warp_sum) {
 template <bool CLEAR>
 __global__ void __launch_bounds__(SB) k_scan_block(int32_t *in, long m, int32_t *out,
                                                    int32_t *bsum) {
+  after_previous();
   __shared__ int32_t ws[32];
   const long base = (long)blockIdx.x * SB * SE + (long)threadIdx.x * SE;
   int32_t v[SE], s = 0;
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(SB) k_scan_block(int32_t *in, long m, int32_t 
 // for itself: at most a thousand or so), and the last leaves the total.
 __global__ void __launch_bounds__(SB) k_scan_add(int32_t *out, long m, const int32_t *bsum,
                                                  int nb) {
+  after_previous();
   __shared__ int32_t ws[32];
   int32_t s = 0;
   for (int i = threadIdx.x; i < (int)blockIdx.x; i += SB) s += bsum[i];
@@ -130,6 +133,7 @@ __global__ void __launch_bounds__(SB) k_scan_add(int32_t *out, long m, const int
 __global__ void __launch_bounds__(256) k_slots(const int32_t *cell, const float *u, const float *v,
                                                long n, const int32_t *start, const int32_t *slot,
                                                uint32_t *tmp) {
+  after_previous();
   const long i0 = blockIdx.x * (256l * MK) + threadIdx.x;
   int c[MK], at[MK];
   uint32_t q[MK];
@@ -214,6 +218,7 @@ constexpr int RG = 8;
 __global__ void __launch_bounds__(256) k_rank(const int32_t *start, long ncell,
                                               const uint32_t *tmp, int32_t *perm, int4 *qstart,
                                               unsigned long long *stat) {
+  after_previous();
   __shared__ int bmax;
   __shared__ uint32_t keys[8][RG][32];
   if (threadIdx.x == 0) bmax = 0;
@@ -303,6 +308,7 @@ __global__ void k_positions(Grid g, Markers m, long n, double *x, double *y) {
 
 // where each marker of the host's numbering lies (-1: nowhere)
 __global__ void k_marker_inverse(const int32_t *id, long n, int32_t *inv) {
+  after_previous();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i < n) inv[id[i]] = (int32_t)i;
 }
@@ -311,6 +317,7 @@ __global__ void k_marker_inverse(const int32_t *id, long n, int32_t *inv) {
 __global__ void __launch_bounds__(256) k_markers_to_host(Grid g, Markers m, long n,
                                                          const __grid_constant__ MarkerFields F,
                                                          const int32_t *inv) {
+  after_previous();
   const int f = blockIdx.y, kind = F.kind[f];
   const float *src = F.src[f], *lo = F.lo[f];
   double *dst = F.dst[f];
@@ -347,8 +354,8 @@ namespace {
 template <bool CLEAR>
 void scan(int32_t *in, long m, int32_t *out, int32_t *blocksum, cudaStream_t st) {
   const int nb = (int)scan_blocks(m);
-  k_scan_block<CLEAR><<<nb, SB, 0, st>>>(in, m, out, blocksum);
-  k_scan_add<<<nb, SB, 0, st>>>(out, m, blocksum, nb);
+  launch_after(k_scan_block<CLEAR>, nb, SB, 0, st, in, m, out, blocksum);
+  launch_after(k_scan_add, nb, SB, 0, st, out, m, blocksum, nb);
 }
 }  // namespace
 
@@ -359,12 +366,13 @@ void launch_scan(const int32_t *in, long m, int32_t *out, int32_t *blocksum, cud
 
 void launch_sort(const int32_t *cell, const float *u, const float *v, long n, long ncell,
                  SortBufs &b, unsigned long long *stat, cudaStream_t st) {
-  if (n > 0) k_count<<<nblk(n, 256 * MK), 256, 0, st>>>(cell, n, b.counts, b.slot);
+  if (n > 0) launch_after(k_count, nblk(n, 256 * MK), 256, 0, st, cell, n, b.counts, b.slot);
   scan<true>(b.counts, ncell, b.start, b.blocksum, st);
   uint32_t *keys = reinterpret_cast<uint32_t *>(b.tmp);
-  if (n > 0) k_slots<<<nblk(n, 256 * MK), 256, 0, st>>>(cell, u, v, n, b.start, b.slot, keys);
-  k_rank<<<nblk((ncell + RG - 1) / RG * 32, 256), 256, 0, st>>>(b.start, ncell, keys, b.perm,
-                                                                 b.qstart, stat);
+  if (n > 0) launch_after(k_slots, nblk(n, 256 * MK), 256, 0, st, cell, u, v, n, b.start, b.slot,
+                          keys);
+  launch_after(k_rank, nblk((ncell + RG - 1) / RG * 32, 256), 256, 0, st, b.start, ncell, keys,
+               b.perm, b.qstart, stat);
 }
 
 void launch_f64_to_f32(const double *src, float *dst, long n, cudaStream_t st) {
@@ -413,11 +421,11 @@ void launch_markers_to_host(const Grid &g, const Markers &m, long n, const Marke
                             int32_t *inv, cudaStream_t st) {
   if (n <= 0 || f.n <= 0) return;
   cudaMemsetAsync(inv, 0xff, sizeof(int32_t) * n, st);
-  k_marker_inverse<<<nblk(n, 256), 256, 0, st>>>(m.id, n, inv);
+  launch_after(k_marker_inverse, nblk(n, 256), 256, 0, st, m.id, n, inv);
   // enough blocks to keep the host link busy, no more
   const unsigned want = nblk(n, 256), most = 1216 / (unsigned)f.n + 1;
-  k_markers_to_host<<<dim3(want < most ? want : most, (unsigned)f.n), 256, 0, st>>>(g, m, n, f,
-                                                                                   inv);
+  launch_after(k_markers_to_host, dim3(want < most ? want : most, (unsigned)f.n), 256, 0, st, g, m,
+               n, f, inv);
 }
 
 }  // namespace v2c

@@ -42,6 +42,7 @@ int32_t *g_scratch_ptr[MAX_DEVICES] = {};
 __global__ void __launch_bounds__(256) k_assign_count(const double *gx, int xn, const double *gy,
                                                       int yn, const double *x, const double *y,
                                                       long n, int32_t *cell, int32_t *count) {
+  after_previous();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double xi = x[i], yi = y[i];
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(256) k_assign_count(const double *gx, int xn, 
 }
 
 __global__ void k_scan_block_s(const int32_t *in, long m, int32_t *out, int32_t *bsum) {
+  after_previous();
   __shared__ int32_t sh[SB];
   const long base = (long)blockIdx.x * SB * SE + (long)threadIdx.x * SE;
   int32_t v[SE], s = 0;
@@ -80,6 +82,7 @@ __global__ void k_scan_block_s(const int32_t *in, long m, int32_t *out, int32_t 
 // exclusive scan of at most SB block sums in one block; the total goes to
 // *total (start[ncell])
 __global__ void k_scan_sums_s(int32_t *bsum, int nb, int32_t *total) {
+  after_previous();
   __shared__ int32_t sh[SB];
   const int32_t v = (threadIdx.x < nb) ? bsum[threadIdx.x] : 0;
   sh[threadIdx.x] = v;
@@ -95,6 +98,7 @@ __global__ void k_scan_sums_s(int32_t *bsum, int nb, int32_t *total) {
 }
 
 __global__ void k_scan_add_s(int32_t *out, long m, const int32_t *bsum) {
+  after_previous();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i < m) out[i] += bsum[i / (SB * SE)];
 }
@@ -106,6 +110,7 @@ __global__ void k_scan_add_s(int32_t *out, long m, const int32_t *bsum) {
 constexpr int FM = 4;
 __global__ void __launch_bounds__(256) k_fill(const int32_t *cell, long n, const int32_t *start,
                                               int32_t *count, int32_t *perm) {
+  after_previous();
   const long i0 = blockIdx.x * (256l * FM) + threadIdx.x;
   int c[FM], at[FM];
 #pragma unroll
@@ -175,6 +180,7 @@ __device__ __noinline__ void order_large(int32_t *p, int L, int lane) {
 constexpr int OG = 8;
 __global__ void __launch_bounds__(256) k_order_cells(const int32_t *start, long ncell,
                                                      int32_t *perm) {
+  after_previous();
   __shared__ int32_t keys[8][OG][32];
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long c0 = (blockIdx.x * 8l + wl) * OG;
@@ -279,21 +285,21 @@ extern "C" int v2c_sort_cells_static(const double *gx_dev, long xnumx, const dou
 
   if (cudaMemsetAsync(count, 0, sizeof(int32_t) * ncell, st) != cudaSuccess) return V2C_ERR_CUDA;
   if (n > 0) {
-    k_assign_count<<<nblk(n, 256), 256, 0, st>>>(gx_dev, (int)xnumx, gy_dev, (int)ynumy, x_dev,
-                                                 y_dev, n, cell_dev, count);
+    launch_after(k_assign_count, nblk(n, 256), 256, 0, st, gx_dev, (int)xnumx, gy_dev, (int)ynumy,
+                 x_dev, y_dev, n, cell_dev, count);
     if (!launched()) return V2C_ERR_CUDA;
   }
   const long nb = (ncell + SB * SE - 1) / (SB * SE);
-  k_scan_block_s<<<(unsigned)nb, SB, 0, st>>>(count, ncell, start_dev, bsum);
+  launch_after(k_scan_block_s, (unsigned)nb, SB, 0, st, count, ncell, start_dev, bsum);
   if (!launched()) return V2C_ERR_CUDA;
-  k_scan_sums_s<<<1, SB, 0, st>>>(bsum, (int)nb, start_dev + ncell);
+  launch_after(k_scan_sums_s, 1, SB, 0, st, bsum, (int)nb, start_dev + ncell);
   if (!launched()) return V2C_ERR_CUDA;
-  k_scan_add_s<<<nblk(ncell, 256), 256, 0, st>>>(start_dev, ncell, bsum);
+  launch_after(k_scan_add_s, nblk(ncell, 256), 256, 0, st, start_dev, ncell, bsum);
   if (!launched()) return V2C_ERR_CUDA;
   if (n > 0) {
-    k_fill<<<nblk(n, 256 * FM), 256, 0, st>>>(cell_dev, n, start_dev, count, perm_dev);
+    launch_after(k_fill, nblk(n, 256 * FM), 256, 0, st, cell_dev, n, start_dev, count, perm_dev);
     if (!launched()) return V2C_ERR_CUDA;
-    k_order_cells<<<nblk(ncell, 8 * OG), 256, 0, st>>>(start_dev, ncell, perm_dev);
+    launch_after(k_order_cells, nblk(ncell, 8 * OG), 256, 0, st, start_dev, ncell, perm_dev);
     if (!launched()) return V2C_ERR_CUDA;
   }
   return V2C_OK;

@@ -365,6 +365,7 @@ __device__ __forceinline__ void build_row(const Ctx &C, Out &O, long m1, long m2
 }
 
 __global__ void __launch_bounds__(128) k_stokes_count(StokesArgs a) {
+  after_previous();
   const long nn = a.g.nn, m3 = blockIdx.x * 128l + threadIdx.x;
   if (m3 >= nn) return;
   const Ctx C{a, a.g.yn, a.g.xn, nn};
@@ -380,6 +381,7 @@ __global__ void __launch_bounds__(128) k_stokes_count(StokesArgs a) {
 
 // the rows the count pass kept, moved to their CSR positions
 __global__ void __launch_bounds__(256) k_stokes_move(StokesArgs a) {
+  after_previous();
   const long nn = a.g.nn, m3 = blockIdx.x * 256l + threadIdx.x;
   if (m3 >= nn) return;
   const int kind = blockIdx.y;
@@ -397,11 +399,11 @@ inline unsigned nblk(long n, int t) { return (unsigned)((n + t - 1) / t); }
 }  // namespace
 
 void launch_stokes_count(const StokesArgs &a, cudaStream_t st) {
-  if (a.g.nn > 0) k_stokes_count<<<dim3(nblk(a.g.nn, 128), 3), 128, 0, st>>>(a);
+  if (a.g.nn > 0) launch_after(k_stokes_count, dim3(nblk(a.g.nn, 128), 3), 128, 0, st, a);
 }
 
 void launch_stokes_fill(const StokesArgs &a, cudaStream_t st) {
-  if (a.g.nn > 0) k_stokes_move<<<dim3(nblk(a.g.nn, 256), 3), 256, 0, st>>>(a);
+  if (a.g.nn > 0) launch_after(k_stokes_move, dim3(nblk(a.g.nn, 256), 3), 256, 0, st, a);
 }
 
 }  // namespace v2c

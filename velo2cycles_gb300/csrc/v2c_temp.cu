@@ -46,6 +46,7 @@ __device__ __forceinline__ bool inside_model(const Grid &g, int ix, int iy, floa
 }
 
 __global__ void k_temp_markers(TempArgs a) {
+  after_previous();
   const Grid &g = a.g;
   const long yn = g.yn;
   const float *tk = a.N.f(V2C_NF_TK), *tk2 = a.N.f(V2C_NF_TK2);
@@ -104,6 +105,7 @@ __global__ void k_temp_markers(TempArgs a) {
 
 // per cell: the normalised diffusion change at its upper-left node
 __global__ void k_temp_cells(TempArgs a) {
+  after_previous();
   const long c = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (c >= a.ncell) return;
   const int b = __ldg(a.start + c), e = __ldg(a.start + c + 1);
@@ -123,6 +125,7 @@ __global__ void k_temp_cells(TempArgs a) {
 }
 
 __global__ void k_temp_anti(TempArgs a) {
+  after_previous();
   const Grid &g = a.g;
   for (long s = blockIdx.x * (long)blockDim.x + threadIdx.x; s < a.n;
        s += (long)gridDim.x * blockDim.x) {
@@ -149,10 +152,10 @@ void launch_temperature(const TempArgs &a, cudaStream_t st) {
   cudaMemsetAsync(a.tol, 0, sizeof(float) * a.g.nn, st);
   if (a.n <= 0) return;
   const unsigned gb = nblk(a.n, 256) < 152 * 16 ? nblk(a.n, 256) : 152 * 16;
-  k_temp_markers<<<gb, 256, 0, st>>>(a);
+  launch_after(k_temp_markers, gb, 256, 0, st, a);
   if (a.heatdif == 0.f) return;
-  k_temp_cells<<<nblk(a.ncell, 256), 256, 0, st>>>(a);
-  k_temp_anti<<<gb, 256, 0, st>>>(a);
+  launch_after(k_temp_cells, nblk(a.ncell, 256), 256, 0, st, a);
+  launch_after(k_temp_anti, gb, 256, 0, st, a);
 }
 
 }  // namespace v2c

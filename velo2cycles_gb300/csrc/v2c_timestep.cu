@@ -193,6 +193,7 @@ struct TsArgs {
 // end (301 x 101 lines: 22 us with FP64 minima and a serial fold per lane,
 // 16 us)
 __global__ void __launch_bounds__(TW * 32) k_ts_nodes(TsArgs a) {
+  after_previous();
   const Grid &g = a.g;
   const Nodes &N = a.N;
   const v2c_params &P = a.S.p;
@@ -321,6 +322,7 @@ constexpr int TF = 16;  // warps
 // by hand are zero again for the next call.
 __global__ void __launch_bounds__(TF * 32) k_ts_fold(const double *part, int nb, double *out,
                                                      double *result) {
+  after_previous();
   extern __shared__ double p[][TS_N];
   for (int i = threadIdx.x; i < nb * TS_N; i += TF * 32) p[i / TS_N][i % TS_N] = part[i];
   __syncthreads();
@@ -354,9 +356,9 @@ int calc_timestep_device(const Grid &g, const Nodes &N, const Scal &S, const v2c
   a.part = scratch + TS_OUT_N;
   const long blocks = (warps + TW - 1) / TW;
   // warps past the node range write empty partials
-  k_ts_nodes<<<(unsigned)blocks, TW * 32, 0, st>>>(a);
-  k_ts_fold<<<1, TF * 32, sizeof(double) * TS_N * blocks, st>>>(a.part, (int)blocks, a.out,
-                                                                  result);
+  launch_after(k_ts_nodes, (unsigned)blocks, TW * 32, 0, st, a);
+  launch_after(k_ts_fold, 1, TF * 32, sizeof(double) * TS_N * blocks, st, a.part, (int)blocks,
+               a.out, result);
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
     return V2C_ERR_CUDA;
   const double *h = result;
