@@ -2,7 +2,7 @@
 half-warps and its bit-pattern bisection can go wrong (GPU): cells of 0 to
 300 markers in random array order, cell counts that are no multiple of a
 group, markers on the lines, outside the model, at zeros of both signs and on
-lines below zero.  Against numpy's search and stable sort; integer results,
+lines below zero, lines closer than their upper words tell apart.  Against numpy's search and stable sort; integer results,
 equal."""
 import numpy as np
 import pytest
@@ -18,6 +18,8 @@ SHAPES = [
     (12, 8, [0, 1, 16, 17, 31, 32, 33], 0.0),
     (9, 14, [3, 64, 65, 300], -2.0),
     (40, 31, [0, 2, 16, 20], 0.0),
+    (4, 5, [0, 1022, 1023, 1024, 2500], 0.0),  # slots past the ten bits
+    (6200, 3, [0, 1, 2], 0.0),     # more lines than shared memory takes
 ]
 
 
@@ -27,6 +29,8 @@ def test_cells_and_order(built_lib, xn, yn, fill, x0):
     rng = np.random.default_rng(xn * 100 + yn)
     gx = x0 + np.concatenate([[0.0], np.cumsum(rng.uniform(0.1, 2.0, xn - 1))])
     gy = x0 + np.concatenate([[0.0], np.cumsum(rng.uniform(0.1, 2.0, yn - 1))])
+    if xn == 40:
+        gx = 1000.0 + np.arange(xn) * 2.0 ** -25
     count = rng.choice(fill, size=(xn - 1) * (yn - 1))
     c = np.repeat(np.arange(count.size), count)
     c = rng.permutation(c)

@@ -39,17 +39,75 @@ constexpr int MAX_DEVICES = 64;
 std::mutex g_setup_mu;
 int32_t *g_scratch_ptr[MAX_DEVICES] = {};
 
+// Line search among the upper words of the lines in shared memory, for an x
+// without a sign bit: the largest line whose upper word does not exceed x's.
+__device__ __forceinline__ int search_upper(const int32_t *upper, const double *g, int n,
+                                            double x) {
+  const long long xb = __double_as_longlong(x);
+  const int32_t xh = (int32_t)(xb >> 32);
+  int lo = 0;
+  for (int len = n - 1; len > 1;) {  // the line sought is one of lo .. lo + len - 1
+    const int half = len >> 1;
+    if (upper[lo + half] <= xh) lo += half;
+    len -= half;
+  }
+  if (upper[lo] != xh || __ldg(reinterpret_cast<const long long *>(g) + lo) <= xb) return lo;
+  // that line shares x's upper word and lies above it: the one before, unless
+  // it shares the word too (lines closer than 2^-20 of the coordinate)
+  if (lo == 0 || upper[lo - 1] != xh) return lo > 0 ? lo - 1 : 0;
+  return nsearch_bits(g, n, x);
+}
+
+// Cells and the markers' slots in them (whatever the atomics give).  The slot
+// rides in the upper ten bits of the cell (fewer than 2^22 cells) to k_fill,
+// which then needs no atomics; SLOT_LATE stands for that and all above.
+// AM markers per thread; LINES: the grid's upper words fit in shared memory.
+// 9 M markers on 1501 x 401 lines: 341 us with FP64 comparisons, 97 with
+// 64-bit integer ones, 79 so, slots included, and k_fill, which
+// waited for its atomics, 57 -> 36.
+static_assert(MAX_CELLS <= 1l << 22, "cells and slots share a word");
+constexpr int SLOT_SHIFT = 22, SLOT_LATE = 1023;
+constexpr int AM = 4;
+constexpr int MAX_LINES = 6144;
+template <bool LINES>
 __global__ void __launch_bounds__(256) k_assign_count(const double *gx, int xn, const double *gy,
                                                       int yn, const double *x, const double *y,
                                                       long n, int32_t *cell, int32_t *count) {
   after_previous();
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double xi = x[i], yi = y[i];
-  const int ix = nsearch_bits(gx, xn, xi), iy = nsearch_bits(gy, yn, yi);
-  const int c = ix * (yn - 1) + iy;
-  cell[i] = c;
-  atomicAdd(count + c, 1);
+  extern __shared__ int32_t upper[];
+  if (LINES) {
+    for (int k = threadIdx.x; k < xn + yn; k += 256)
+      upper[k] = __double2hiint(k < xn ? gx[k] : gy[k - xn]);
+    __syncthreads();
+  }
+  const long i0 = blockIdx.x * (256l * AM) + threadIdx.x;
+  double xi[AM], yi[AM];
+#pragma unroll
+  for (int k = 0; k < AM; k++) {
+    const bool in = i0 + 256 * k < n;
+    xi[k] = in ? x[i0 + 256 * k] : 0.0;
+    yi[k] = in ? y[i0 + 256 * k] : 0.0;
+  }
+  int c[AM];
+#pragma unroll
+  for (int k = 0; k < AM; k++) {
+    int ix, iy;
+    if (LINES && (__double2hiint(xi[k]) | __double2hiint(yi[k])) >= 0) {
+      ix = search_upper(upper, gx, xn, xi[k]);
+      iy = search_upper(upper + xn, gy, yn, yi[k]);
+    } else {
+      ix = nsearch_bits(gx, xn, xi[k]);
+      iy = nsearch_bits(gy, yn, yi[k]);
+    }
+    c[k] = ix * (yn - 1) + iy;
+  }
+#pragma unroll
+  for (int k = 0; k < AM; k++)
+    if (i0 + 256 * k < n) {
+      const int slot = atomicAdd(count + c[k], 1);
+      cell[i0 + 256 * k] =
+          (int32_t)((uint32_t)c[k] | (uint32_t)min(slot, SLOT_LATE) << SLOT_SHIFT);
+    }
 }
 
 __global__ void k_scan_block_s(const int32_t *in, long m, int32_t *out, int32_t *bsum) {
@@ -103,24 +161,30 @@ __global__ void k_scan_add_s(int32_t *out, long m, const int32_t *bsum) {
   if (i < m) out[i] += bsum[i / (SB * SE)];
 }
 
-// every marker takes a slot in its cell's segment, counting the cell's
-// counter back down (slot order is whatever the atomics give; k_order_cells
-// makes it index order).  FM markers per thread, so that FM atomics and then
-// FM stores are in flight: 9 M markers 61 -> 56 us.
+// Every marker goes to its slot of its cell's segment (k_order_cells makes
+// slot order index order), the late ones to what they count the counter down
+// to, and the cells are left without the slots.
 constexpr int FM = 4;
-__global__ void __launch_bounds__(256) k_fill(const int32_t *cell, long n, const int32_t *start,
+__global__ void __launch_bounds__(256) k_fill(int32_t *cell, long n, const int32_t *start,
                                               int32_t *count, int32_t *perm) {
   after_previous();
   const long i0 = blockIdx.x * (256l * FM) + threadIdx.x;
-  int c[FM], at[FM];
+  uint32_t w[FM];
+  int at[FM];
 #pragma unroll
-  for (int k = 0; k < FM; k++) c[k] = i0 + 256 * k < n ? cell[i0 + 256 * k] : -1;
+  for (int k = 0; k < FM; k++) w[k] = i0 + 256 * k < n ? (uint32_t)cell[i0 + 256 * k] : 0u;
+#pragma unroll
+  for (int k = 0; k < FM; k++) {
+    const int c = (int)(w[k] & ((1u << SLOT_SHIFT) - 1)), slot = (int)(w[k] >> SLOT_SHIFT);
+    at[k] = __ldg(start + c) + slot;
+    if (i0 + 256 * k < n) {
+      if (slot == SLOT_LATE) at[k] += atomicSub(count + c, 1) - 1 - SLOT_LATE;
+      cell[i0 + 256 * k] = c;
+    }
+  }
 #pragma unroll
   for (int k = 0; k < FM; k++)
-    if (c[k] >= 0) at[k] = __ldg(start + c[k]) + atomicSub(count + c[k], 1) - 1;
-#pragma unroll
-  for (int k = 0; k < FM; k++)
-    if (c[k] >= 0) perm[at[k]] = (int32_t)(i0 + 256 * k);
+    if (i0 + 256 * k < n) perm[at[k]] = (int32_t)(i0 + 256 * k);
 }
 
 // ascending over the warp's lanes (W = 32) or each of its halves (W = 16)
@@ -173,51 +237,68 @@ __device__ __noinline__ void order_large(int32_t *p, int L, int lane) {
 
 // One warp per OG consecutive cells sorts each cell's segment of perm
 // ascending, in place.  The cells' starts come in one read and all their
-// entries in the next (two rounds of memory latency per warp); the entries
-// wait in shared memory, so that the sorting code is one loop, which takes
-// two cells at a time, half a warp each, where both have at most 16 markers.
-// 600 000 cells of 15 markers: 144 -> 79 us against a warp per cell.
+// entries, one run of perm, in the next (two rounds of memory latency per
+// warp, full lines); the entries wait in shared memory, so that the sorting
+// code is one loop, which takes two cells at a time, half a warp each, where
+// both have at most 16 markers, and go back the way they came.  600 000 cells
+// of 15 markers: 144 us with a warp per cell, 79 with a read and a write per
+// cell, 72 so.
 constexpr int OG = 8;
 __global__ void __launch_bounds__(256) k_order_cells(const int32_t *start, long ncell,
                                                      int32_t *perm) {
   after_previous();
-  __shared__ int32_t keys[8][OG][32];
+  __shared__ int32_t keys[8][OG * 32];
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long c0 = (blockIdx.x * 8l + wl) * OG;
   if (c0 >= ncell) return;  // uniform across the warp
   const int ng = (int)min((long)OG, ncell - c0);
   // (lanes past the last cell repeat its end: empty cells)
   const int sv = start[c0 + min(lane, ng)];
+  const int s0 = __shfl_sync(V2C_FULL, sv, 0), total = __shfl_sync(V2C_FULL, sv, OG) - s0;
+  const int len = __shfl_down_sync(V2C_FULL, sv, 1) - sv;
+  if (__any_sync(V2C_FULL, lane < OG && len > 32)) {
+#pragma unroll 1
+    for (int g = 0; g < ng; g++) {
+      const int s = __shfl_sync(V2C_FULL, sv, g), L = __shfl_sync(V2C_FULL, sv, g + 1) - s;
+      if (L > 32) {
+        order_large(perm + s, L, lane);
+      } else if (L > 1) {
+        const int32_t key = bitonic<32>(lane < L ? perm[s + lane] : INT_MAX, lane);
+        if (lane < L) perm[s + lane] = key;
+      }
+    }
+    return;
+  }
+  int32_t *buf = keys[wl];
   int32_t val[OG];
 #pragma unroll
-  for (int g = 0; g < OG; g++) {
-    const int s = __shfl_sync(V2C_FULL, sv, g), L = __shfl_sync(V2C_FULL, sv, g + 1) - s;
-    val[g] = (lane < L && L <= 32) ? perm[s + lane] : INT_MAX;
-  }
+  for (int k = 0; k < OG; k++) val[k] = k * 32 + lane < total ? perm[s0 + k * 32 + lane] : 0;
 #pragma unroll
-  for (int g = 0; g < OG; g++) keys[wl][g][lane] = val[g];
+  for (int k = 0; k < OG; k++) buf[k * 32 + lane] = val[k];
   __syncwarp();
 #pragma unroll 1
   for (int g = 0; g < ng; g += 2) {
-    const int s0 = __shfl_sync(V2C_FULL, sv, g), s1 = __shfl_sync(V2C_FULL, sv, g + 1);
-    const int L0 = s1 - s0, L1 = __shfl_sync(V2C_FULL, sv, g + 2) - s1;
+    const int o0 = __shfl_sync(V2C_FULL, sv, g) - s0, o1 = __shfl_sync(V2C_FULL, sv, g + 1) - s0;
+    const int L0 = o1 - o0, L1 = __shfl_sync(V2C_FULL, sv, g + 2) - s0 - o1;
     if (L0 <= 16 && L1 <= 16) {
-      const int half = lane >> 4, l = lane & 15;
-      const int32_t key = bitonic<16>(keys[wl][g + half][l], lane);
-      if (l < (half ? L1 : L0)) perm[(half ? s1 : s0) + l] = key;
+      const int half = lane >> 4, l = lane & 15, at = (half ? o1 : o0) + l;
+      const bool in = l < (half ? L1 : L0);
+      const int32_t key = bitonic<16>(in ? buf[at] : INT_MAX, lane);
+      if (in) buf[at] = key;
       continue;
     }
 #pragma unroll 1
     for (int h = 0; h < 2; h++) {
-      const int s = h ? s1 : s0, L = h ? L1 : L0;
-      if (L > 32) {
-        order_large(perm + s, L, lane);
-      } else {
-        const int32_t key = bitonic<32>(keys[wl][g + h][lane], lane);
-        if (lane < L) perm[s + lane] = key;
-      }
+      const int at = (h ? o1 : o0) + lane;
+      const bool in = lane < (h ? L1 : L0);
+      const int32_t key = bitonic<32>(in ? buf[at] : INT_MAX, lane);
+      if (in) buf[at] = key;
     }
   }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < OG; k++)
+    if (k * 32 + lane < total) perm[s0 + k * 32 + lane] = buf[k * 32 + lane];
 }
 
 inline unsigned nblk(long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -285,8 +366,10 @@ extern "C" int v2c_sort_cells_static(const double *gx_dev, long xnumx, const dou
 
   if (cudaMemsetAsync(count, 0, sizeof(int32_t) * ncell, st) != cudaSuccess) return V2C_ERR_CUDA;
   if (n > 0) {
-    launch_after(k_assign_count, nblk(n, 256), 256, 0, st, gx_dev, (int)xnumx, gy_dev, (int)ynumy,
-                 x_dev, y_dev, n, cell_dev, count);
+    const bool lines = xnumx + ynumy <= MAX_LINES;
+    launch_after(lines ? k_assign_count<true> : k_assign_count<false>, nblk(n, 256 * AM), 256,
+                 lines ? sizeof(int32_t) * (xnumx + ynumy) : 0, st, gx_dev, (int)xnumx, gy_dev,
+                 (int)ynumy, x_dev, y_dev, n, cell_dev, count);
     if (!launched()) return V2C_ERR_CUDA;
   }
   const long nb = (ncell + SB * SE - 1) / (SB * SE);
