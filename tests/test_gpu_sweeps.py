@@ -73,3 +73,26 @@ def test_scatter_and_gather_edges(built_lib, oracle_built, xn, yn, fill, kw):
     bad = over(marker_errors(m.download_markers(N2M_MARK), ref.marks, N2M_MARK, floors))
     assert not bad, bad
     m.close()
+
+
+@pytest.mark.parametrize("mode", [1, 2])
+def test_markers_at_the_model_edges(built_lib, oracle_built, mode):
+    """Markers on, inside and outside the model's edges by distances on both
+    sides of what an FP32 position resolves: only those strictly inside
+    count (FP64 decides where FP32 cannot)."""
+    case = synth.make_case("c1", seed=4, window=(0, 0, 12, 9), interpolationmod=mode)
+    x, y = case.marks[abi.MF_X], case.marks[abi.MF_Y]
+    xs, ys = case.gx[-1], case.gy[-1]
+    d = np.array([0.0, 1e-9, 1e-4, 1e-2, 0.3, 3.0, 30.0])
+    d = np.concatenate([d, -d[1:]])
+    rng = np.random.default_rng(1)
+    at = rng.permutation(case.n)[:8 * d.size].reshape(8, d.size)
+    for k, (p, edge, sign) in enumerate([(x, 0.0, 1), (x, xs, -1), (y, 0.0, 1), (y, ys, -1)] * 2):
+        p[at[k]] = edge + sign * d
+    m = mic.from_case(case)
+    ref = oracle_for(case)
+    m.marker2nodes()
+    ref.marker2nodes()
+    bad = over(node_errors(m.download_nodes(M2N_OUT), ref.nodes, M2N_OUT))
+    assert not bad, bad
+    m.close()

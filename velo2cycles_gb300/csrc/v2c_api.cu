@@ -223,6 +223,7 @@ Grid make_grid(const v2c_ctx *c) {
   g.gx = c->d_gx; g.gy = c->d_gy; g.wx = c->d_wx; g.wy = c->d_wy;
   g.xn = c->xn; g.yn = c->yn; g.ncx = c->ncx; g.ncy = c->ncy; g.nn = c->nn;
   g.xsize = c->p.xsize; g.ysize = c->p.ysize;
+  g.xsf = (float)g.xsize; g.ysf = (float)g.ysize;
   set_divider(g);
   return g;
 }

@@ -121,11 +121,11 @@ __device__ __forceinline__ void stage_fields(const M2NArgs &a, Smem &sm, int n, 
       if (!ex && !ey) continue;
       float2 *uv = &sm.p[S_UV][slot_of(p)];
       bool act = true;
-      if (ex) {
+      if (ex && !surely_inside(__ldg(a.gxf + ci), __ldg(g.wx + ci), uv->x, g.xsf)) {
         double x = g.gx[ci] + (double)uv->x * (g.gx[ci + 1] - g.gx[ci]);
         act = act && x > 0 && x < g.xsize;
       }
-      if (ey) {
+      if (ey && !surely_inside(__ldg(a.gyf + iy), __ldg(g.wy + iy), uv->y, g.ysf)) {
         double y = g.gy[iy] + (double)uv->y * (g.gy[iy + 1] - g.gy[iy]);
         act = act && y > 0 && y < g.ysize;
       }
@@ -641,13 +641,16 @@ struct Mk {
   float u, v;
 };
 
-__device__ __forceinline__ bool marker_active(const Grid &g, int cx, int cy, float u, float v) {
+__device__ __forceinline__ bool marker_active(const M2NArgs &a, int cx, int cy, float u, float v) {
+  const Grid &g = a.g;
   bool act = true;
-  if (cx == 0 || cx == g.ncx - 1) {
+  if ((cx == 0 || cx == g.ncx - 1) &&
+      !surely_inside(__ldg(a.gxf + cx), __ldg(g.wx + cx), u, g.xsf)) {
     double x = g.gx[cx] + (double)u * (g.gx[cx + 1] - g.gx[cx]);
     act = act && x > 0 && x < g.xsize;
   }
-  if (cy == 0 || cy == g.ncy - 1) {
+  if ((cy == 0 || cy == g.ncy - 1) &&
+      !surely_inside(__ldg(a.gyf + cy), __ldg(g.wy + cy), v, g.ysf)) {
     double y = g.gy[cy] + (double)v * (g.gy[cy + 1] - g.gy[cy]);
     act = act && y > 0 && y < g.ysize;
   }
@@ -691,57 +694,79 @@ __device__ __forceinline__ void mode1_node(const M2NArgs &a) {
       const long c = (long)cx * ncy + cy;
       // quarter classes (2 (v > 1/2) + (u > 1/2)) that can have weight:
       // a half-cell factor k = 0 needs the lower half, k = 2 the upper
-      constexpr int UX[3] = {0x5, 0xf, 0xa}, VY[3] = {0x3, 0xf, 0xc};
+      auto ux = [](int k) { return 0xaf5 >> (4 * k) & 0xf; };
+      auto vy = [](int k) { return 0xcf3 >> (4 * k) & 0xf; };
       int mask = 0xf;
-      if (ROLE == 2) mask = UX[ax] & VY[by];
-      if (ROLE == 3) mask = (ax >= 0 ? VY[by + 1] : 0) | (by >= 0 ? UX[ax + 1] : 0);
+      if (ROLE == 2) mask = ux(ax) & vy(by);
+      if (ROLE == 3) mask = (ax >= 0 ? vy(by + 1) : 0) | (by >= 0 ? ux(ax + 1) : 0);
       const int4 qs = __ldg(a.qstart + c);
-      const int qb[5] = {qs.x, qs.y, qs.z, qs.w, __ldg(a.start + c + 1)};
+      const int qe = __ldg(a.start + c + 1);
+      auto qb = [&](int q) { return q == 0 ? qs.x : q == 1 ? qs.y : q == 2 ? qs.z : q == 3 ? qs.w : qe; };
+      // runs of classes with weight (one for the basic nodes, at most two)
+#pragma unroll 1
       for (int q = 0; q < 4; q++) {
         if (!((mask >> q) & 1)) continue;
-      for (int s = qb[q]; s < qb[q + 1]; s++) {
-        const int idx = __ldg(a.perm + s);
+        const int b = qb(q);
+        while (q < 3 && ((mask >> (q + 1)) & 1)) q++;
+        const int e = qb(q + 1);
+        if (b >= e) continue;
+        // the index of the marker after next is read while this one is summed,
+        // and every field of a marker at once, also of those without weight:
+        // one round of memory latency per marker instead of three
+        int idx1 = __ldg(a.perm + b);
+#pragma unroll 1
+      for (int s = b; s < e; s++) {
+        const int idx = idx1;
+        if (s + 1 < e) idx1 = __ldg(a.perm + s + 1);
         const float u = a.m.u_in[idx], v = a.m.v_in[idx];
-        if (!marker_active(g, cx, cy, u, v)) continue;
         const int tt = a.m.type[idx];
-        if (ROLE == 0 || ROLE == 1) {
+        if (ROLE == 0) {
+          const float mnu = a.m.mnu[idx], me = a.m.e[idx], sxy = a.m.sxy[idx];
+          const float exy = a.m.exy[idx], coh = a.m.coh[idx], phi = a.m.phi[idx];
+          const float ig = a.R(RK_INV_GG, tt);
+          if (!marker_active(a, cx, cy, u, v)) continue;
           const float w = s1 * (ax ? u : 1.f - u) * (by ? v : 1.f - v);
-          if (ROLE == 0) {
-            const float mnu = a.m.mnu[idx];
-            cur[0].add(mnu * w); cur[1].add(mnu * a.R(RK_INV_GG, tt) * w);
-            cur[2].add(a.m.e[idx] * w); cur[3].add(a.m.sxy[idx] * w);
-            cur[4].add(a.m.exy[idx] * w); cur[5].add(a.m.coh[idx] * w);
-            cur[6].add(a.m.phi[idx] * w); cur[7].add(w);
-          } else {
-            const float T = a.m.tk[idx], bb = a.R(RK_BB, tt);
-            const float ro = a.S.p.densimod ? a.m.mro[idx] : a.R(RK_RO, tt);
-            cur[0].add(ro * w);
-            cur[1].add(__fdividef(bb, 1.f - bb * (T - 298.15f)) * w);
-            cur[2].add(a.R(RK_HT, tt) * w); cur[3].add(a.R(RK_CP, tt) * w);
-            cur[4].add(a.m.mkt[idx] * w); cur[5].add(T * w); cur[6].add(w);
-          }
+          cur[0].add(mnu * w); cur[1].add(mnu * ig * w);
+          cur[2].add(me * w); cur[3].add(sxy * w);
+          cur[4].add(exy * w); cur[5].add(coh * w);
+          cur[6].add(phi * w); cur[7].add(w);
+        } else if (ROLE == 1) {
+          const float T = a.m.tk[idx], kt = a.m.mkt[idx];
+          const float mro = a.S.p.densimod ? a.m.mro[idx] : 0.f;
+          const float bb = a.R(RK_BB, tt);
+          const float ro = a.S.p.densimod ? mro : a.R(RK_RO, tt);
+          if (!marker_active(a, cx, cy, u, v)) continue;
+          const float w = s1 * (ax ? u : 1.f - u) * (by ? v : 1.f - v);
+          cur[0].add(ro * w);
+          cur[1].add(__fdividef(bb, 1.f - bb * (T - 298.15f)) * w);
+          cur[2].add(a.R(RK_HT, tt) * w); cur[3].add(a.R(RK_CP, tt) * w);
+          cur[4].add(kt * w); cur[5].add(T * w); cur[6].add(w);
         } else if (ROLE == 2) {
+          const float mnu = a.m.mnu[idx], sxx = a.m.sxx[idx], exx = a.m.exx[idx];
+          const float mp = a.m.p[idx], ig = a.R(RK_INV_GG, tt);
+          if (!marker_active(a, cx, cy, u, v)) continue;
           const float w = s1 * half_factor(ax, u) * half_factor(by, v);
           if (w != 0.f) {
-            const float mnu = a.m.mnu[idx];
-            cur[0].add(mnu * w); cur[1].add(mnu * a.R(RK_INV_GG, tt) * w);
-            cur[2].add(a.m.sxx[idx] * w); cur[3].add(a.m.exx[idx] * w);
-            cur[4].add(a.m.p[idx] * w); cur[5].add(w);
+            cur[0].add(mnu * w); cur[1].add(mnu * ig * w);
+            cur[2].add(sxx * w); cur[3].add(exx * w);
+            cur[4].add(mp * w); cur[5].add(w);
           }
         } else {
+          const float vx = a.m.vx[idx], vy = a.m.vy[idx];
           const float ro = a.S.p.densimod ? a.m.mro[idx] : a.R(RK_RO, tt);
+          if (!marker_active(a, cx, cy, u, v)) continue;
           // vx node: x bilinear (ax in {0, 1}), y staggered (by + 1 in {0, 1, 2})
           if (ax >= 0) {
             const float w = s1 * (ax ? u : 1.f - u) * half_factor(by + 1, v);
             if (w != 0.f) {
-              cur[0].add(a.m.vx[idx] * ro * w); cur[1].add(ro * w); cur[2].add(w);
+              cur[0].add(vx * ro * w); cur[1].add(ro * w); cur[2].add(w);
             }
           }
           // vy node: x staggered (ax + 1), y bilinear (by in {0, 1})
           if (by >= 0) {
             const float w = s1 * half_factor(ax + 1, u) * (by ? v : 1.f - v);
             if (w != 0.f) {
-              vy3[0].add(a.m.vy[idx] * ro * w); vy3[1].add(ro * w); vy3[2].add(w);
+              vy3[0].add(vy * ro * w); vy3[1].add(ro * w); vy3[2].add(w);
             }
           }
         }
@@ -773,8 +798,10 @@ __device__ __forceinline__ void mode1_node(const M2NArgs &a) {
 
 // The four node groups in one launch, a row of blocks each: a thread walks
 // its node's markers one after the other, so the kernel is latency, and the
-// groups fill each other's gaps (433 x 187 lines, 0.84 M markers: 378 us
-// against 488 in four launches).
+// groups fill each other's gaps.  433 x 187 lines, 0.84 M markers: 488 us in
+// four launches, 378 in one, 346 with each marker's fields read at once and
+// the next one's index ahead, 118 with the edge cells' tests in FP32 where
+// they are sure (surely_inside).
 __global__ void __launch_bounds__(128) k_m2n_mode1(M2NArgs a) {
   after_previous();
   switch (blockIdx.y) {

@@ -136,11 +136,13 @@ __global__ void __launch_bounds__(PT, 8) k_phys(PhysArgs a) {
           atomicMax(a.sticky_key + q, ((uint32_t)a.m.id[i] << 2) | (uint32_t)t);
       }
       bool act = true;
-      if (ix == 0 || ix == g.ncx - 1) {
+      if ((ix == 0 || ix == g.ncx - 1) &&
+          !surely_inside(__ldg(a.gxf + ix), __ldg(g.wx + ix), u, g.xsf)) {
         double x = g.gx[ix] + (double)u * (g.gx[ix + 1] - g.gx[ix]);
         act = act && x > 0 && x < g.xsize;
       }
-      if (iy == 0 || iy == g.ncy - 1) {
+      if ((iy == 0 || iy == g.ncy - 1) &&
+          !surely_inside(__ldg(a.gyf + iy), __ldg(g.wy + iy), v, g.ysf)) {
         double y = g.gy[iy] + (double)v * (g.gy[iy + 1] - g.gy[iy]);
         act = act && y > 0 && y < g.ysize;
       }
