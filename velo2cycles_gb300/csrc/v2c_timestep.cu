@@ -23,6 +23,7 @@
 // chi == 0 (where the reference stops) sets an error flag.
 #include <math.h>
 
+#include "v2c_ff.cuh"
 #include "v2c_kernels.h"
 
 namespace v2c {
@@ -54,17 +55,30 @@ __device__ __forceinline__ int ts_kind(int k) {  // 0 min, 1 max, 2 sum, 3 order
   }
 }
 
-// Entry k of "A then B" (B follows A in node order)
+// b <= a by the bit patterns, as integers (no entry is a NaN: the states
+// start from numbers, and a NaN replaces none)
+__device__ __forceinline__ bool ts_le(double b, double a) {
+  auto key = [](double v) {
+    const long long t = __double_as_longlong(v);
+    return t ^ (t >> 63 & 0x7fffffffffffffffll);
+  };
+  return key(b) <= key(a);
+}
+// Entry k of "A then B" (B follows A in node order).  Only the sums are FP64
+// arithmetic: a fold is one block, and its SM issues two FP64 operations a
+// cycle, so FP64 comparisons of the other entries took most of its time.
 __device__ __forceinline__ double ts_combined(int k, const double *a, const double *b) {
   const int kind = ts_kind(k);
-  if (kind == 0) return b[k] <= a[k] ? b[k] : a[k];
-  if (kind == 1) return b[k] >= a[k] ? b[k] : a[k];
-  if (kind == 2) return a[k] + b[k];
-  const bool br = b[TS_RESET] != 0.0;
-  if (k == TS_RESET) return (a[TS_RESET] != 0.0 || br) ? 1.0 : 0.0;
-  if (k == TS_PHI_ALL || k == TS_L_ALL) return b[k] <= a[k] ? b[k] : a[k];
-  const double all = b[k == TS_PHI_AFTER ? TS_PHI_ALL : TS_L_ALL];
-  return br ? b[k] : (all <= a[k] ? all : a[k]);
+  const double x = a[k], y = b[k];
+  if (kind == 2) return x + y;
+  const bool br = __double_as_longlong(b[TS_RESET]) != 0;
+  if (k == TS_RESET) return br ? y : x;  // (0 or 1)
+  double z = y;
+  if (k == TS_PHI_AFTER || k == TS_L_AFTER) {
+    if (br) return y;
+    z = b[k == TS_PHI_AFTER ? TS_PHI_ALL : TS_L_ALL];
+  }
+  return (kind == 1 ? ts_le(x, z) : ts_le(z, x)) ? z : x;
 }
 
 // Fold n partials in order, pairs (2i, 2i+1) at each level, a warp per pair
@@ -150,12 +164,14 @@ __device__ __forceinline__ void ts_fold_lanes(TsState &s, bool any0, bool any1, 
     if (take) s.reset = s.reset || br;
   }
 }
-// a := a then b
-__device__ __forceinline__ void ts_append(TsState &a, const TsState &b) {
+// a := a then b (sums: b has statistics)
+__device__ __forceinline__ void ts_append(TsState &a, const TsState &b, bool sums) {
 #pragma unroll
   for (int k = 0; k < F_N; k++) a.f[k] = k < F_MINS ? ts_min(a.f[k], b.f[k]) : ts_max(a.f[k], b.f[k]);
+  if (sums) {
 #pragma unroll
-  for (int k = 0; k < D_N; k++) a.d[k] += b.d[k];
+    for (int k = 0; k < D_N; k++) a.d[k] += b.d[k];
+  }
 #pragma unroll
   for (int k = 0; k < 2; k++) {
     a.after[k] = b.reset ? b.after[k] : ts_min(a.after[k], b.all[k]);
@@ -164,17 +180,18 @@ __device__ __forceinline__ void ts_append(TsState &a, const TsState &b) {
   a.reset = a.reset || b.reset;
 }
 __device__ __forceinline__ void ts_store(const TsState &s, double *p) {
-  auto lim = [](float v) { return (double)v <= 1e30 ? (double)v : 1e30; };
+  // (1e30f is the first float above 1e30)
+  auto lim = [](float v) { return v < 1e30f ? widen<true>(v) : 1e30; };
   p[TS_DTNVP] = lim(s.f[F_DTNVP]); p[TS_DTD] = lim(s.f[F_DTD]);
-  p[TS_MAXVX] = s.f[F_MAXVX]; p[TS_MAXVEL] = s.f[F_MAXVEL];
+  p[TS_MAXVX] = widen<true>(s.f[F_MAXVX]); p[TS_MAXVEL] = widen<true>(s.f[F_MAXVEL]);
   p[TS_PHI_ALL] = lim(s.all[0]); p[TS_L_ALL] = lim(s.all[1]);
   p[TS_PHI_AFTER] = lim(s.after[0]); p[TS_L_AFTER] = lim(s.after[1]);
   p[TS_RESET] = s.reset ? 1.0 : 0.0;
-  p[TS_NR0] = s.d[D_NR0]; p[TS_MAXS0] = s.f[F_MAXS0]; p[TS_MINS0] = lim(s.f[F_MINS0]);
-  p[TS_SUMS0] = s.d[D_SUMS0]; p[TS_SUM2S0] = s.d[D_SUM2S0]; p[TS_MAXV0] = s.f[F_MAXV0];
+  p[TS_NR0] = s.d[D_NR0]; p[TS_MAXS0] = widen<true>(s.f[F_MAXS0]); p[TS_MINS0] = lim(s.f[F_MINS0]);
+  p[TS_SUMS0] = s.d[D_SUMS0]; p[TS_SUM2S0] = s.d[D_SUM2S0]; p[TS_MAXV0] = widen<true>(s.f[F_MAXV0]);
   p[TS_MINV0] = lim(s.f[F_MINV0]); p[TS_SUMV0] = s.d[D_SUMV0]; p[TS_SUM2V0] = s.d[D_SUM2V0];
-  p[TS_NR1] = s.d[D_NR1]; p[TS_MAXS1] = s.f[F_MAXS1]; p[TS_MINS1] = lim(s.f[F_MINS1]);
-  p[TS_SUMS1] = s.d[D_SUMS1]; p[TS_SUM2S1] = s.d[D_SUM2S1]; p[TS_MAXV1] = s.f[F_MAXV1];
+  p[TS_NR1] = s.d[D_NR1]; p[TS_MAXS1] = widen<true>(s.f[F_MAXS1]); p[TS_MINS1] = lim(s.f[F_MINS1]);
+  p[TS_SUMS1] = s.d[D_SUMS1]; p[TS_SUM2S1] = s.d[D_SUM2S1]; p[TS_MAXV1] = widen<true>(s.f[F_MAXV1]);
   p[TS_MINV1] = lim(s.f[F_MINV1]); p[TS_SUMV1] = s.d[D_SUMV1]; p[TS_SUM2V1] = s.d[D_SUM2V1];
 }
 
@@ -191,7 +208,7 @@ struct TsArgs {
 
 // node pass: one warp per contiguous range, the block's warps folded at its
 // end (301 x 101 lines: 22 us with FP64 minima and a serial fold per lane,
-// 16 us)
+// 16 with FP32 ones, 14 with the limits and empty sums out of the FP64 pipe)
 __global__ void __launch_bounds__(TW * 32) k_ts_nodes(TsArgs a) {
   after_previous();
   const Grid &g = a.g;
@@ -305,8 +322,9 @@ __global__ void __launch_bounds__(TW * 32) k_ts_nodes(TsArgs a) {
         d.all[1] = d.after[1] = lamc * LoV;
       }
     }
-    ts_fold_lanes(d, __any_sync(V2C_FULL, st == 1.f), __any_sync(V2C_FULL, st == 2.f), lane);
-    if (lane == 0) ts_append(s, d);
+    const bool any0 = __any_sync(V2C_FULL, st == 1.f), any1 = __any_sync(V2C_FULL, st == 2.f);
+    ts_fold_lanes(d, any0, any1, lane);
+    if (lane == 0) ts_append(s, d, any0 || any1);
   }
   const int wl = threadIdx.x >> 5;
   if (lane == 0) ts_store(s, part[wl]);
@@ -316,7 +334,8 @@ __global__ void __launch_bounds__(TW * 32) k_ts_nodes(TsArgs a) {
 }
 
 // fold the block partials in order, in shared memory (301 x 101 lines: 68 us
-// as a tree in global memory with a thread per pair, 17 us)
+// as a tree in global memory with a thread per pair, 17 in shared memory, 10
+// with integer comparisons)
 constexpr int TF = 16;  // warps
 // The results go to the host's memory, and the slots that the node pass sets
 // by hand are zero again for the next call.
