@@ -28,6 +28,19 @@
 
 namespace v2c {
 
+// The approximate reciprocal of a normal b, the one __fdividef multiplies by
+// (its product joins a following addition in one rounding, so callers that
+// add write fmaf), without its handling of a subnormal b: 1 instruction
+// instead of 4.
+__device__ __forceinline__ float rcp_normal(float b) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  return r;
+}
+__device__ __forceinline__ float fdiv_normal(float a, float b) {
+  return __fmul_rn(a, rcp_normal(b));
+}
+
 struct ff {
   float hi, lo;
 };
@@ -157,7 +170,7 @@ __device__ __forceinline__ ff ff_div(ff a, ff b) {
 // error, so the pair is good to ~2^-44 -- for quotients rounded to FP32 at
 // the end, or used to that accuracy.  b.hi a normal, finite nonzero float.
 __device__ __forceinline__ ff ff_div_fast(ff a, ff b) {
-  const float rb = __fdividef(1.f, b.hi);
+  const float rb = fdiv_normal(1.f, b.hi);
   const float q1 = __fmul_rn(a.hi, rb);
   const ff r = ff_sub(a, ff_mul_f(b, q1));
   const float q2 = __fmul_rn(r.hi, rb);
@@ -237,12 +250,11 @@ __device__ const float2 k_ff_exp2_64[64] = {
 // |n| < 2^15), |r| <= ln2/128; expm1(r) by its Taylor series (r^2/2 and
 // r^3/6 in float-float, the r^4 and r^5 terms in float; the first omitted
 // term is below 4e-17), then e^a = 2^k 2^(j/64) (1 + expm1(r)).
-// Out of line (as ff_log): the per-marker viscosity calls them several
-// times, and inlined copies of their ~50 instructions each made the marker
-// physics kernel wait on instruction fetch.
-static __device__ __noinline__ ff ff_exp(ff a) {
-  if (a.hi < -87.0f) return ff_f(0.f);
-  if (a.hi > 88.0f) return ff_f(INFINITY);
+// ff_exp and ff_log are out of line: the per-marker viscosity calls them
+// several times, and inlined copies of their ~100 instructions each made the
+// marker physics kernel wait on instruction fetch.  ff_log has the core of
+// its own (a nested call cost the physics of 60 M markers 140 us of 5850).
+__device__ __forceinline__ ff ff_exp_core(ff a) {
   const float nf = rintf(__fmul_rn(a.hi, 0x1.715476p+6f));  // 64/ln 2
   const int n = (int)nf;
   const float c1 = 0x1.63p-7f, c2 = -0x1.bd0106p-19f, c3 = 0x1.cf79acp-46f;
@@ -257,21 +269,29 @@ static __device__ __noinline__ ff ff_exp(ff a) {
   const float tail = rh * rh * rh * rh * (1.f / 24.f + rh * (1.f / 120.f));
   ff p = ff_add(r, ff_scale(s2, 0.5f));
   p = ff_add(p, ff_mul(s3, ff{1.666666716e-01f, -4.967053879e-09f}));
-  p = ff_add_f(p, tail);
+  float pl;  // |tail| <= |p|
+  const float ph = fast_two_sum(p.hi, tail, pl);
+  p.hi = fast_two_sum(ph, __fadd_rn(pl, p.lo), p.lo);
   const float2 t = __ldg(&k_ff_exp2_64[n & 63]);
   const ff T{t.x, t.y};
   return ff_scale(ff_add(T, ff_mul(T, p)), pow2i(n >> 6));
+}
+static __device__ __noinline__ ff ff_exp(ff a) {
+  if (a.hi < -87.0f) return ff_f(0.f);
+  if (a.hi > 88.0f) return ff_f(INFINITY);
+  return ff_exp_core(a);
 }
 
 // a = m 2^e with m in [0.5, 1); log a = log m + e ln 2, so that e^-log m
 // stays in (1, 2] whatever the size of a (a.hi a positive normal float)
 static __device__ __noinline__ ff ff_log(ff a) {
-  int e;
-  (void)frexpf(a.hi, &e);
+  const unsigned bits = __float_as_uint(a.hi);
+  int e = (int)(bits >> 23) - 126;
+  if (bits - 0x00800000u >= 0x7f000000u) (void)frexpf(a.hi, &e);  // not a positive normal
   const int e1 = e >> 1, e2 = e - e1;
   const ff m = ff_scale(ff_scale(a, pow2i(-e1)), pow2i(-e2));
   const float y = logf(m.hi);
-  const ff z = ff_exp(ff_f(-y));
+  const ff z = ff_exp_core(ff_f(-y));  // (0 <= -y <= ln 2)
   const ff t = ff_add_f(ff_mul(m, z), -1.f);
   return ff_add(ff_add_f(t, y), ff_mul_f(ff_ln2(), (float)e));
 }

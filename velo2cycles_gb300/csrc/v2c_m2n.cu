@@ -419,7 +419,7 @@ __device__ __forceinline__ void sum_basic(const M2NArgs &a, const Smem &sm, cons
       } else {
         const float bb = a.R(RK_BB, t);
         // dencalcomp adiabatic term
-        const float et = __fdividef(bb, 1.f - bb * (kt.y - 298.15f));
+        const float et = fdiv_normal(bb, 1.f - bb * (kt.y - 298.15f));
         acc[0].add(mul_w(marker_ro(a, sm, p, q), et, w));
         acc[1].add(mul_w(a.R(RK_HT, t), a.R(RK_CP, t), w));
         acc[2].add(mul_w(kt.x, kt.y, w));
@@ -738,7 +738,7 @@ __device__ __forceinline__ void mode1_node(const M2NArgs &a) {
           if (!marker_active(a, cx, cy, u, v)) continue;
           const float w = s1 * (ax ? u : 1.f - u) * (by ? v : 1.f - v);
           cur[0].add(ro * w);
-          cur[1].add(__fdividef(bb, 1.f - bb * (T - 298.15f)) * w);
+          cur[1].add(fdiv_normal(bb, 1.f - bb * (T - 298.15f)) * w);
           cur[2].add(a.R(RK_HT, tt) * w); cur[3].add(a.R(RK_CP, tt) * w);
           cur[4].add(kt * w); cur[5].add(T * w); cur[6].add(w);
         } else if (ROLE == 2) {

@@ -67,7 +67,8 @@ struct Lin {
   float e0, s;
 };
 __device__ __forceinline__ Lin lin_w(float X0, float A, float B) {
-  return Lin{__fdividef(X0 - A, B), __fdividef(1.f, B)};
+  const float r = rcp_normal(B);
+  return Lin{__fmul_rn(X0 - A, r), r};
 }
 
 // bilinear interpolation of f over nodes m3, m3+1, m3+yn, m3+yn+1 as

@@ -96,9 +96,14 @@ __device__ __forceinline__ void marker_problem(const PhysArgs &a, long i, const 
   uplain = (vold > 0.f) ? __logf(vold) : -30.f;
 }
 
-// Bound by instruction issue (110 warp instructions per marker at dt = 1e8 s,
-// 74-80 % issue active, FMA pipe half busy).  8 CTAs per SM (61 registers):
-// C4 physics + Newton 8.30 ms at 7, 7.98 at 8, 8.11 at 10 (spills).
+// Bound by instruction issue (3100 warp instructions for 32 markers at dt =
+// 1e8 s, 2300 at coseismic steps; 76-87 % issue active, FMA pipe half busy).
+// 8 CTAs per SM (61 registers): C4 physics + Newton 8.30 ms at 7, 7.98 at 8,
+// 8.11 at 10 (spills).  What the instructions are: the creep replay a third,
+// eight float-pair exponentials and logarithms a third.  Reciprocals without
+// subnormal handling (rcp_normal), the approximate floor test and the
+// logarithm's own exponential core took 60 M markers at 4001 x 1001 lines
+// from 6.31 to 5.67 ms, the refined 1001 x 401 model from 2060 to 1900 us.
 template <int MODE>
 __global__ void __launch_bounds__(PT, 8) k_phys(PhysArgs a) {
   after_previous();
@@ -206,14 +211,10 @@ __global__ void __launch_bounds__(PT, 8) k_phys(PhysArgs a) {
     bool need = solve;
     if (solve && MODE == PHYS_SPLIT) {
       const float exx = a.m.exx[i], exy = a.m.exy[i];
-      RsfIn in;
-      in.a = ff_f(fr.a); in.b = ff_f(fr.b); in.L = ff_f(fr.L); in.V0 = ff_f(fr.V0);
-      in.mu0 = ff_f(fr.mu0); in.sn = (P.pmode == 0) ? sn_ff : ff_f(a.m.p[i]);
-      in.dt = dt_ff; in.W = W_ff; in.phio = ff_f(phi); in.tau_old = ff_f(sigin);
-      in.edot = ff_f(sqrtf(exx * exx + exy * exy)); in.eta = ff_f(mnu);
-      in.G = ff_f(a.R(RK_GG, t));
-      float A_floor;
-      if (rsf_floor_certain(rsf32_of(in, a.rk, far), A_floor)) {
+      float edot;
+      asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(edot) : "f"(exx * exx + exy * exy));
+      if (rsf_floor_marker(*a.rk, t, far, fr.a, fr.b, fr.L, fr.V0, fr.mu0,
+                           (P.pmode == 0) ? sn_ff.hi : a.m.p[i], dt_ff.hi, phi, sigin, edot, mnu)) {
         a.m.slipv[i] = 1e-40f;
         it += 1;
         need = false;

@@ -110,7 +110,7 @@ __device__ __forceinline__ float ductile_visc32(const Rock &R, const Scal &S, in
       const float B = fmaf(ds, g1p, g);
       const float f1c = exp2f(em * __log2f(q * B));  // (q B)^em
       const float fp = 1.f - em * __fdividef(f1c, B) * g1p;
-      float dn = ds - __fdividef(ds - f1c, fp);
+      float dn = fmaf(-(ds - f1c), rcp_normal(fp), ds);
       if (!(dn > 0.f)) dn = 0.5f * ds;
       const bool conv = fabsf(dn - ds) <= 1e-6f * ds;
       ds = dn;
@@ -146,8 +146,7 @@ __device__ __forceinline__ float ductile_visc32(const Rock &R, const Scal &S, in
     for (int counter = 1; counter <= 50; counter++) {
       const float e_old = e;
       const float d_old = ds + e_old;
-      const float m = __fdividef(d_old, d_old + 1.f);   // mnu0 / eta_diff
-      const float gm = g + m;
+      const float gm = fmaf(d_old, rcp_normal(d_old + 1.f), g);  // g + mnu0 / eta_diff
       // B(d)/B* - 1: below -1 the reference's iteration has gone to a
       // negative prefactor, whose power is NaN there and is NaN here (log1pf)
       const float x = e_old * kx;
@@ -159,7 +158,7 @@ __device__ __forceinline__ float ductile_visc32(const Rock &R, const Scal &S, in
         cfB = fmaf(kc, h, kc);
       } else {
         g1 = expm1f(em * log1pf(x));
-        cfB = __fdividef(kc * (1.f + g1), 1.f + x);
+        cfB = fdiv_normal(kc * (1.f + g1), 1.f + x);
       }
       const float f2 = (e_old - c0f1s * g1) + r0;       // f2(d* + e)
       // pow(eta_diff, 2/(eta_diff+eta_disl_old)) / eta_diff, the reference's
@@ -167,7 +166,7 @@ __device__ __forceinline__ float ductile_visc32(const Rock &R, const Scal &S, in
       const float p2 = (invS > 1e-30f && !(p2max < gm * 0x1p-25f))
                            ? __expf(__fdividef(p2fac, 1.f + d_old)) * invS : 0.f;
       const float df = 1.f - em * cfB * (gm + p2);
-      e = e_old - __fdividef(f2, df);
+      e = fmaf(-f2, rcp_normal(df), e_old);
       // relative change of mnu0 from the previous step: (d - d_prev) /
       // (d_prev (1 + d)), tested without the division (the denominator > 0)
       const float D = d_prev * (1.f + d_old), dd = e_old - e_prev;
@@ -247,7 +246,7 @@ static __device__ __noinline__ float friction_marker(const v2c_params &p, int ph
 // the upper-left stencil node and the weights (e, n).
 
 // basic (shear) nodes, interpolation.c:1067-1080: m10 clamped to [1, xn-3]
-// Stencil weights use the fast reciprocal division (__fdividef, 2 ulp): the
+// Stencil weights use the fast reciprocal division (fdiv_normal, 2 ulp): the
 // denominators are cell widths, far inside its range.
 __device__ __forceinline__ long stencil_basic(const Grid &g, const Axis &ax, const Axis &ay,
                                               float &e, float &n) {
@@ -257,8 +256,8 @@ __device__ __forceinline__ long stencil_basic(const Grid &g, const Axis &ax, con
   if (m20 < 1) m20 = 1;
   if (m20 > g.yn - 3) m20 = g.yn - 3;
   int kx = m10 - ax.i, ky = m20 - ay.i;
-  e = __fdividef(ax.X - ax.G(kx), ax.G(kx + 1) - ax.G(kx));
-  n = __fdividef(ay.X - ay.G(ky), ay.G(ky + 1) - ay.G(ky));
+  e = fdiv_normal(ax.X - ax.G(kx), ax.G(kx + 1) - ax.G(kx));
+  n = fdiv_normal(ay.X - ay.G(ky), ay.G(ky + 1) - ay.G(ky));
   return (long)m10 * g.yn + m20;
 }
 
@@ -272,8 +271,8 @@ __device__ __forceinline__ long stencil_centre(const Grid &g, const Axis &ax, co
   if (m10 < 1) m10 = 1;
   if (m20 < 1) m20 = 1;
   int kx = m10 - ax.i, ky = m20 - ay.i;
-  e = __fdividef(ax.X - (ax.G(kx - 1) + ax.G(kx)) * 0.5f, (ax.G(kx + 1) - ax.G(kx - 1)) * 0.5f);
-  n = __fdividef(ay.X - (ay.G(ky - 1) + ay.G(ky)) * 0.5f, (ay.G(ky + 1) - ay.G(ky - 1)) * 0.5f);
+  e = fdiv_normal(ax.X - (ax.G(kx - 1) + ax.G(kx)) * 0.5f, (ax.G(kx + 1) - ax.G(kx - 1)) * 0.5f);
+  n = fdiv_normal(ay.X - (ay.G(ky - 1) + ay.G(ky)) * 0.5f, (ay.G(ky + 1) - ay.G(ky - 1)) * 0.5f);
   return (long)m10 * g.yn + m20;
 }
 
@@ -287,8 +286,8 @@ __device__ __forceinline__ long stencil_vx(const Grid &g, const Axis &ax, const 
   if (m20 < 0) m20 = 0;
   if (m20 > g.yn - 3) m20 = g.yn - 3;
   int kx = m10 - ax.i, ky = m20 - ay.i;
-  e = __fdividef(ax.X - ax.G(kx), ax.G(kx + 1) - ax.G(kx));
-  n = __fdividef(ay.X - (ay.G(ky) + ay.G(ky + 1)) * 0.5f, (ay.G(ky + 2) - ay.G(ky)) * 0.5f);
+  e = fdiv_normal(ax.X - ax.G(kx), ax.G(kx + 1) - ax.G(kx));
+  n = fdiv_normal(ay.X - (ay.G(ky) + ay.G(ky + 1)) * 0.5f, (ay.G(ky + 2) - ay.G(ky)) * 0.5f);
   return (long)m10 * g.yn + m20;
 }
 
@@ -301,8 +300,8 @@ __device__ __forceinline__ long stencil_vy(const Grid &g, const Axis &ax, const 
   if (m20 < 0) m20 = 0;
   if (m20 > yclamp_hi) m20 = yclamp_hi;
   int kx = m10 - ax.i, ky = m20 - ay.i;
-  e = __fdividef(ax.X - (ax.G(kx) + ax.G(kx + 1)) * 0.5f, (ax.G(kx + 2) - ax.G(kx)) * 0.5f);
-  n = __fdividef(ay.X - ay.G(ky), ay.G(ky + 1) - ay.G(ky));
+  e = fdiv_normal(ax.X - (ax.G(kx) + ax.G(kx + 1)) * 0.5f, (ax.G(kx + 2) - ax.G(kx)) * 0.5f);
+  n = fdiv_normal(ay.X - ay.G(ky), ay.G(ky + 1) - ay.G(ky));
   return (long)m10 * g.yn + m20;
 }
 
