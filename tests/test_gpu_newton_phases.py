@@ -65,6 +65,20 @@ def test_phases(ctx, n, guess):
         assert B.rsf_residual(S[:, live], out[abi.RO_V][live]).max() <= 1e-10
 
 
+def test_more_states_left_than_the_list_holds(ctx):
+    """270 000 degenerate loads among ordinary states: the FP64 phase's list
+    (2^18) runs over, and nothing changes."""
+    n = 270_003
+    S = newton.rsf_states(n, seed=5)
+    some = np.arange(n) % 90 == 1
+    S[abi.RS_TAUOLD, ~some] = 0.0
+    S[abi.RS_EDOT, ~some] = 0.0
+    out, it = newton.solve(ctx, S, abi.GUESS_PLAIN)
+    assert (out[abi.RO_V, ~some] == 1e-40).all() and (it[~some] == 0).all()
+    want, wit = newton.solve(ctx, S[:, some], abi.GUESS_PLAIN)
+    assert np.array_equal(out[:, some], want) and np.array_equal(it[some], wit)
+
+
 def test_conversions_by_bit_pattern(tmp_path):
     rng = np.random.default_rng(2)
     x = [np.exp(rng.uniform(-100, 88, 100000)) * rng.choice([-1, 1], 100000)]

@@ -28,13 +28,17 @@ cudaError_t newton_init(NewtonState &s, long cap) {
   s.cap = cap;
   cudaError_t e = cudaMalloc((void **)&s.d_mlp, sizeof(float) * V2C_MLP_NPARAM);
   if (e != cudaSuccess) return e;
+  e = cudaMalloc((void **)&s.d_left, sizeof(int32_t) * (1 + NEWTON_LEFT));
+  if (e != cudaSuccess) return e;
   return cudaMemset(s.d_mlp, 0, sizeof(float) * V2C_MLP_NPARAM);
 }
 
 void newton_free(NewtonState &s) {
   if (s.d_mlp) cudaFree(s.d_mlp);
   if (s.d_guess) cudaFree(s.d_guess);
+  if (s.d_left) cudaFree(s.d_left);
   s.d_mlp = nullptr;
+  s.d_left = nullptr;
   s.d_guess = nullptr;
   s.guess_cap = 0;
 }
@@ -158,8 +162,8 @@ __global__ void __launch_bounds__(NT, 4) k_solve_states64(const double *S, long 
 // phases and at different iterations of 50 KB of code, so that instruction
 // fetch was the bound (7 of 13 stall cycles per instruction), and a warp ran
 // the FP64 Newton for one lane.  4 M states of the benchmark's
-// distributions, plain start: 2510 -> 1085 us (FP32 252, float-float 731, FP64
-// 100; with the FP64 Newton inside the float-float kernel 1340 for the two).
+// distributions, plain start: 2510 -> 1035 us (FP32 252, float-float 731, FP64
+// 50; with the FP64 Newton inside the float-float kernel 1340 for the two).
 //
 // A phase leaves its result in the state's own outputs, which the next one
 // reads and then writes.
@@ -183,18 +187,29 @@ __device__ __forceinline__ bool resume(const Phase32 &p, RsfResult &r, float &u,
   dF = p.dF;
   return true;
 }
-// states left to the FP64 phase, by a mark in the residual's place (NaNs that
-// no arithmetic returns): from the iterate in the slip rate's place, with the
+// States left to the FP64 phase, listed (left[0] counts them) and marked in
+// the residual's place by NaNs that no arithmetic returns (MARK_LATE added
+// past the list's end): from the iterate in the slip rate's place, with the
 // iterations so far and the state variable in the state variable's; or from a
 // load degenerate in FP32, Phase32 left as it was; or (LEARNED) a whole solve
 // from the plain start
 constexpr unsigned long long MARK_NEWTON = 0x7ff4563243324301ull;
 constexpr unsigned long long MARK_DEGENERATE = 0x7ff4563243324302ull;
+constexpr unsigned long long MARK_LATE = 0x10;
+__device__ __forceinline__ void leave(double *out, long n, long i, unsigned long long mark,
+                                      int32_t *left) {
+  const int k = atomicAdd(left, 1);
+  if (k < NEWTON_LEFT) left[1 + k] = (int32_t)i;
+  else mark += MARK_LATE;
+  out[(long)V2C_RO_RES * n + i] = __longlong_as_double((long long)mark);
+}
 
 template <bool LEARNED>
 __global__ void __launch_bounds__(NT) k_states_fp32(const double *S, long n, ff W,
-                                                    const float *guess, int maxit, double *out) {
+                                                    const float *guess, int maxit, double *out,
+                                                    int32_t *left) {
   after_previous();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *left = 0;
   const long i = blockIdx.x * (long)NT + threadIdx.x;
   if (i >= n) return;
   RsfIn in;
@@ -213,22 +228,21 @@ __global__ void __launch_bounds__(NT) k_states_fp32(const double *S, long n, ff 
 }
 
 __global__ void __launch_bounds__(NT, 8) k_states_polish(const double *S, long n, ff W, float rtolf,
-                                                         double *out, int32_t *iters,
+                                                         double *out, int32_t *iters, int32_t *left,
                                                          unsigned long long *stat) {
   after_previous();
   const long i = blockIdx.x * (long)NT + threadIdx.x;
   unsigned long long it = 0, resbits = 0;
   if (i < n) {
     const Phase32 p = get_phase32(out, n, i);
-    double *mark = out + (long)V2C_RO_RES * n + i;
     if (p.what == PH_DEGENERATE) {
-      *mark = __longlong_as_double(MARK_DEGENERATE);
+      leave(out, n, i, MARK_DEGENERATE, left);
     } else {
       RsfIn in;
       double vold;
       state_of<true>(S, n, i, W, in, vold);
       RsfResult r{};
-      bool left = false;
+      bool done = true;
       if (p.what == PH_FLOOR) {
         r = rsf_floor_result(in, p.u);
       } else {
@@ -236,14 +250,14 @@ __global__ void __launch_bounds__(NT, 8) k_states_polish(const double *S, long n
             in, [&](RsfResult &rr, float &u, float &dF) { return resume(p, rr, u, dF); }, rtolf,
             [&](RsfFF &q) { rsf_setup_ff(q, in); },
             [&](double u, RsfResult &rr) {
-              left = true;
+              done = false;
               out[(long)V2C_RO_V * n + i] = u;
               reinterpret_cast<int2 *>(out)[(long)V2C_RO_PHI * n + i] =
                   make_int2(rr.it32 + rr.itff, __float_as_int(rr.phi));
-              *mark = __longlong_as_double(MARK_NEWTON);
+              leave(out, n, i, MARK_NEWTON, left);
             });
       }
-      if (!left) {
+      if (done) {
         it = r.it32 + r.itff;
         put_state<true>(in, r, it, n, i, out, iters);
         if (r.res > 0) resbits = (unsigned long long)__double_as_longlong(r.res);
@@ -253,33 +267,36 @@ __global__ void __launch_bounds__(NT, 8) k_states_polish(const double *S, long n
   add_stats(stat, it, 0, 0, resbits);
 }
 
-// The states left to the FP64 phase, gathered by each block from FIN states.
-constexpr int FIN = 4096;
+constexpr unsigned FINISH_BLOCKS = 152 * 8;
+// The states left to the FP64 phase, 32 per block of one warp: the FP64 pipe
+// of an SM issues an instruction every 16 cycles however many lanes are on, so
+// full warps, spread over the SMs, are what counts (4 M states, 1 % of them
+// left: 50 us against 100 where each block gathered its own of 4096 states;
+// 300 007: 77 against 87, the chain of one state's iterations).
 template <bool LEARNED>
-__global__ void __launch_bounds__(NT) k_states_finish(const double *S, long n, ff W,
+__global__ void __launch_bounds__(32) k_states_finish(const double *S, long n, ff W,
                                                       const float *guess, double rtol, int maxit,
                                                       double *out, int32_t *iters,
+                                                      const int32_t *left,
                                                       unsigned long long *stat) {
   after_previous();
-  __shared__ int list[FIN], count;
-  if (threadIdx.x == 0) count = 0;
-  __syncthreads();
-  const long base = blockIdx.x * (long)FIN;
-  for (int k = threadIdx.x; k < FIN && base + k < n; k += NT) {
-    const unsigned long long m =
-        (unsigned long long)__double_as_longlong(out[(long)V2C_RO_RES * n + base + k]);
-    if (m == MARK_NEWTON || m == MARK_DEGENERATE) list[atomicAdd(&count, 1)] = k;
-  }
-  __syncthreads();
+  const long count = *left, listed = count < NEWTON_LEFT ? count : NEWTON_LEFT;
+  const long total = listed + (count > listed ? n : 0);  // then those past the list's end
   unsigned long long it_sum = 0, fb = 0, nc = 0, resbits = 0;
-  for (int k = threadIdx.x; k < count; k += NT) {
-    const long i = base + list[k];
+  for (long k = blockIdx.x * 32l + threadIdx.x; k < total; k += gridDim.x * 32l) {
+    const long i = k < listed ? left[1 + k] : k - listed;
+    unsigned long long mark =
+        (unsigned long long)__double_as_longlong(out[(long)V2C_RO_RES * n + i]);
+    if (k >= listed) {
+      mark -= MARK_LATE;
+      if (mark != MARK_NEWTON && mark != MARK_DEGENERATE) continue;
+    }
     RsfIn in;
     double vold;
     state_of(S, n, i, W, in, vold);
     RsfResult r{};
     r.phi = in.phio.hi;
-    if ((unsigned long long)__double_as_longlong(out[(long)V2C_RO_RES * n + i]) == MARK_NEWTON) {
+    if (mark == MARK_NEWTON) {
       const int2 b = reinterpret_cast<const int2 *>(out)[(long)V2C_RO_PHI * n + i];
       r.it32 = b.x;
       r.phi = __int_as_float(b.y);
@@ -749,17 +766,17 @@ extern "C" int v2c_rsf_newton(v2c_ctx *ctx, const double *states_dev, long n, in
   } else {
     const unsigned nb = (unsigned)((n + NT - 1) / NT);
     if (learned) launch_after(k_states_fp32<true>, nb, NT, 0, st, states_dev, n, W, ns->d_guess,
-                              p->newton_maxit, out_dev);
+                              p->newton_maxit, out_dev, ns->d_left);
     else launch_after(k_states_fp32<false>, nb, NT, 0, st, states_dev, n, W, ns->d_guess,
-                      p->newton_maxit, out_dev);
+                      p->newton_maxit, out_dev, ns->d_left);
     launch_after(k_states_polish, nb, NT, 0, st, states_dev, n, W, (float)p->newton_rtol, out_dev,
-                 iters_dev, v2c_ctx_stat(ctx));
-    const unsigned nf = (unsigned)((n + FIN - 1) / FIN);
-    if (learned) launch_after(k_states_finish<true>, nf, NT, 0, st, states_dev, n, W, ns->d_guess,
-                              p->newton_rtol, p->newton_maxit, out_dev, iters_dev,
-                              v2c_ctx_stat(ctx));
-    else launch_after(k_states_finish<false>, nf, NT, 0, st, states_dev, n, W, ns->d_guess,
-                      p->newton_rtol, p->newton_maxit, out_dev, iters_dev, v2c_ctx_stat(ctx));
+                 iters_dev, ns->d_left, v2c_ctx_stat(ctx));
+    if (learned) launch_after(k_states_finish<true>, FINISH_BLOCKS, 32, 0, st, states_dev, n, W,
+                              ns->d_guess, p->newton_rtol, p->newton_maxit, out_dev, iters_dev,
+                              ns->d_left, v2c_ctx_stat(ctx));
+    else launch_after(k_states_finish<false>, FINISH_BLOCKS, 32, 0, st, states_dev, n, W,
+                      ns->d_guess, p->newton_rtol, p->newton_maxit, out_dev, iters_dev,
+                      ns->d_left, v2c_ctx_stat(ctx));
     v2c_ctx_count_launches(ctx, 2);
   }
   v2c_ctx_prof_end(ctx, V2C_PROF_NEWTON, ev);

@@ -12,7 +12,11 @@ struct NewtonState {
   long cap = 0;
   float *d_guess = nullptr;  // network outputs [2][guess_cap] for v2c_rsf_newton
   long guess_cap = 0;
+  // states left to the FP64 phase: their count, then the first NEWTON_LEFT of
+  // them
+  int32_t *d_left = nullptr;
 };
+constexpr int NEWTON_LEFT = 1 << 18;
 
 cudaError_t newton_init(NewtonState &s, long cap);
 void newton_free(NewtonState &s);
