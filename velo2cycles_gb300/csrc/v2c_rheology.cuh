@@ -127,6 +127,7 @@ __device__ __forceinline__ float ductile_visc32(const Rock &R, const Scal &S, in
     // the extra derivative term p2 (below) is at most invS e^max(p2fac,0)
     // (d >= 0); under half an ulp of gm it cannot change gm + p2 in FP32
     const float p2max = invS * __expf(fmaxf(p2fac, 0.f));
+    const float p2_from = invS > 1e-30f ? p2max * 0x1p25f : -INFINITY;
     // |log10(m_k / m_k-1)| < 1e-6  <=>  10^-1e-6 - 1 < m_k / m_k-1 - 1 < 10^1e-6 - 1
     const float TLO = -2.30258242e-6f, THI = 2.30258771e-6f;
     const ff e0 = ff_add_f(d0_ff, -ds);
@@ -163,7 +164,7 @@ __device__ __forceinline__ float ductile_visc32(const Rock &R, const Scal &S, in
       const float f2 = (e_old - c0f1s * g1) + r0;       // f2(d* + e)
       // pow(eta_diff, 2/(eta_diff+eta_disl_old)) / eta_diff, the reference's
       // extra term of the derivative (density_ductilevisc_calc.c:190-191)
-      const float p2 = (invS > 1e-30f && !(p2max < gm * 0x1p-25f))
+      const float p2 = !(p2_from < gm)
                            ? __expf(__fdividef(p2fac, 1.f + d_old)) * invS : 0.f;
       const float df = 1.f - em * cfB * (gm + p2);
       e = fmaf(-f2, rcp_normal(df), e_old);
