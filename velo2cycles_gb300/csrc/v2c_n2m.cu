@@ -860,163 +860,161 @@ __global__ void __launch_bounds__(256, 6) k_move(N2MArgs a) {
   const v2c_params &P = a.S.p;
   const int ncy = g.ncy;
   const float dt = a.S.dt;
-  {
-    const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (idx >= a.n) return;
-    const int c = a.m.cell_in[idx];
-    int ix, iy;
-    g.cell_at(c, ix, iy);
-    const float u = a.m.u_in[idx], v = a.m.v_in[idx];
-    const int t = a.m.type[idx];
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(a.m.sxx + idx));
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(a.m.sxy + idx));
-    float tk = a.m.tk[idx];
-    const bool in_grid = (ix > 0 || u >= 0.f) && (ix < g.ncx - 1 || u <= 1.f) &&
-                         (iy > 0 || v >= 0.f) && (iy < g.ncy - 1 || v <= 1.f);
-    int nix = ix, niy = iy;
-    float nu_ = u, nv_ = v;
-    if (!a.R(RK_IM, t) && (in_grid || P.outgrid != 1)) {
-      const float wxc = __ldg(g.wx + ix), wyc = __ldg(g.wy + iy);
-      const Pos p0{ix, iy, u * wxc, v * wyc};
-      float vx0, vy0, sp0, vx1, vy1, sp1;
-      vel_at(g, a.quad, p0, vx1, vy1, sp1);
-      if (P.markmod == 1) {
-        vx0 = vx1; vy0 = vy1; sp0 = sp1;
-      } else {
-        float vx2, vy2, sp2, vx3, vy3, sp3, vx4, vy4, sp4;
-        Pos p = p0;
-        p.X += vx1 * dt / 2.f; p.Y += vy1 * dt / 2.f;
-        settle(g, p, a.stat);
-        vel_at(g, a.quad, p, vx2, vy2, sp2);
-        p = p0;
-        p.X += vx2 * dt / 2.f; p.Y += vy2 * dt / 2.f;
-        settle(g, p, a.stat);
-        vel_at(g, a.quad, p, vx3, vy3, sp3);
-        p = p0;
-        p.X += vx3 * dt; p.Y += vy3 * dt;
-        settle(g, p, a.stat);
-        vel_at(g, a.quad, p, vx4, vy4, sp4);
-        vx0 = (vx1 + 2.f * vx2 + 2.f * vx3 + vx4) / 6.f;
-        vy0 = (vy1 + 2.f * vy2 + 2.f * vy3 + vy4) / 6.f;
-        sp0 = (P.markmod == 2) ? (sp1 + 2.f * sp2 + 2.f * sp3 + sp4) / 6.f : sp1;
+  const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (idx >= a.n) return;
+  const int c = a.m.cell_in[idx];
+  int ix, iy;
+  g.cell_at(c, ix, iy);
+  const float u = a.m.u_in[idx], v = a.m.v_in[idx];
+  const int t = a.m.type[idx];
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(a.m.sxx + idx));
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(a.m.sxy + idx));
+  float tk = a.m.tk[idx];
+  const bool in_grid = (ix > 0 || u >= 0.f) && (ix < g.ncx - 1 || u <= 1.f) &&
+                       (iy > 0 || v >= 0.f) && (iy < g.ncy - 1 || v <= 1.f);
+  int nix = ix, niy = iy;
+  float nu_ = u, nv_ = v;
+  if (!a.R(RK_IM, t) && (in_grid || P.outgrid != 1)) {
+    const float wxc = __ldg(g.wx + ix), wyc = __ldg(g.wy + iy);
+    const Pos p0{ix, iy, u * wxc, v * wyc};
+    float vx0, vy0, sp0, vx1, vy1, sp1;
+    vel_at(g, a.quad, p0, vx1, vy1, sp1);
+    if (P.markmod == 1) {
+      vx0 = vx1; vy0 = vy1; sp0 = sp1;
+    } else {
+      float vx2, vy2, sp2, vx3, vy3, sp3, vx4, vy4, sp4;
+      Pos p = p0;
+      p.X += vx1 * dt / 2.f; p.Y += vy1 * dt / 2.f;
+      settle(g, p, a.stat);
+      vel_at(g, a.quad, p, vx2, vy2, sp2);
+      p = p0;
+      p.X += vx2 * dt / 2.f; p.Y += vy2 * dt / 2.f;
+      settle(g, p, a.stat);
+      vel_at(g, a.quad, p, vx3, vy3, sp3);
+      p = p0;
+      p.X += vx3 * dt; p.Y += vy3 * dt;
+      settle(g, p, a.stat);
+      vel_at(g, a.quad, p, vx4, vy4, sp4);
+      vx0 = (vx1 + 2.f * vx2 + 2.f * vx3 + vx4) / 6.f;
+      vy0 = (vy1 + 2.f * vy2 + 2.f * vy3 + vy4) / 6.f;
+      sp0 = (P.markmod == 2) ? (sp1 + 2.f * sp2 + 2.f * sp3 + sp4) / 6.f : sp1;
+    }
+    if (P.outgrid == 2) {
+      if ((ix == 0 && u < 0.f) || (ix == g.ncx - 1 && u > 1.f)) vy0 = 0.f;
+      if ((iy == 0 && v < 0.f) || (iy == g.ncy - 1 && v > 1.f)) vx0 = 0.f;
+    }
+    // new position: in offset space while the marker stays in its cell
+    // (one FP32 rounding of u), else walked in metres
+    nu_ = u + dt * vx0 / wxc;
+    nv_ = v + dt * vy0 / wyc;
+    const bool interior_x = ix > 0 && ix < g.ncx - 1, interior_y = iy > 0 && iy < g.ncy - 1;
+    if (!(nu_ >= 0.f && nu_ < 1.f && (interior_x || (u >= 0.f && u <= 1.f)))) {
+      Pos p{ix, 0, nu_ * wxc, 0.f};
+      settle(g, p, a.stat);
+      nix = p.ix;
+      const float nwx = __ldg(g.wx + nix);
+      nu_ = p.X / nwx;
+      if (p.X < nwx && nu_ >= 1.f) nu_ = nextafterf(1.f, 0.f);
+      if (p.X < 0.5f * nwx && nu_ >= 0.5f) nu_ = nextafterf(0.5f, 0.f);
+      if (p.X > 0.5f * nwx && nu_ <= 0.5f) nu_ = nextafterf(0.5f, 1.f);
+      if (p.X > nwx && nu_ <= 1.f) nu_ = nextafterf(1.f, 2.f);
+    }
+    if (!(nv_ >= 0.f && nv_ < 1.f && (interior_y || (v >= 0.f && v <= 1.f)))) {
+      Pos p{0, iy, 0.f, nv_ * wyc};
+      settle(g, p, a.stat);
+      niy = p.iy;
+      const float nwy = __ldg(g.wy + niy);
+      nv_ = p.Y / nwy;
+      if (p.Y < nwy && nv_ >= 1.f) nv_ = nextafterf(1.f, 0.f);
+      if (p.Y < 0.5f * nwy && nv_ >= 0.5f) nv_ = nextafterf(0.5f, 0.f);
+      if (p.Y > 0.5f * nwy && nv_ <= 0.5f) nv_ = nextafterf(0.5f, 1.f);
+      if (p.Y > nwy && nv_ <= 1.f) nv_ = nextafterf(1.f, 2.f);
+    }
+    if (t >= 100) {
+      // immobile marker (moveandrotatemarkers.c:88-135): inside the model
+      // it spawns a mobile marker there and goes back to its anchor
+      // (markk, markv), as it does when it strays more than ystpy from it
+      const bool inside = (nix > 0 || nu_ >= 0.f) && (nix < g.ncx - 1 || nu_ <= 1.f) &&
+                          (niy > 0 || nv_ >= 0.f) && (niy < g.ncy - 1 || nv_ <= 1.f);
+      const double ax = (double)tk + (double)a.m.tk_lo[idx];
+      const double ay = (double)a.m.mv[idx] + (double)a.m.mv_lo[idx];
+      double x = g.gx[nix] + (double)nu_ * (g.gx[nix + 1] - g.gx[nix]);
+      double y = g.gy[niy] + (double)nv_ * (g.gy[niy + 1] - g.gy[niy]);
+      if (inside && a.has_imm) {
+        const int id = a.m.id[idx];
+        a.imm.spawn[id] = 1;
+        a.imm.sp_cell[id] = nix * ncy + niy;
+        a.imm.sp_u[id] = nu_;
+        a.imm.sp_v[id] = nv_;
+        x = ax;
+        y = ay;
       }
-      if (P.outgrid == 2) {
-        if ((ix == 0 && u < 0.f) || (ix == g.ncx - 1 && u > 1.f)) vy0 = 0.f;
-        if ((iy == 0 && v < 0.f) || (iy == g.ncy - 1 && v > 1.f)) vx0 = 0.f;
+      const double dx = x - ax, dy = y - ay;
+      if (x == ax && y == ay || sqrt(dx * dx + dy * dy) > P.ystpy) {
+        nix = nsearch64(g.gx, g.xn, ax);
+        niy = nsearch64(g.gy, g.yn, ay);
+        nu_ = offset32((ax - g.gx[nix]) / (g.gx[nix + 1] - g.gx[nix]));
+        nv_ = offset32((ay - g.gy[niy]) / (g.gy[niy + 1] - g.gy[niy]));
       }
-      // new position: in offset space while the marker stays in its cell
-      // (one FP32 rounding of u), else walked in metres
-      nu_ = u + dt * vx0 / wxc;
-      nv_ = v + dt * vy0 / wyc;
-      const bool interior_x = ix > 0 && ix < g.ncx - 1, interior_y = iy > 0 && iy < g.ncy - 1;
-      if (!(nu_ >= 0.f && nu_ < 1.f && (interior_x || (u >= 0.f && u <= 1.f)))) {
-        Pos p{ix, 0, nu_ * wxc, 0.f};
-        settle(g, p, a.stat);
-        nix = p.ix;
-        const float nwx = __ldg(g.wx + nix);
-        nu_ = p.X / nwx;
-        if (p.X < nwx && nu_ >= 1.f) nu_ = nextafterf(1.f, 0.f);
-        if (p.X < 0.5f * nwx && nu_ >= 0.5f) nu_ = nextafterf(0.5f, 0.f);
-        if (p.X > 0.5f * nwx && nu_ <= 0.5f) nu_ = nextafterf(0.5f, 1.f);
-        if (p.X > nwx && nu_ <= 1.f) nu_ = nextafterf(1.f, 2.f);
-      }
-      if (!(nv_ >= 0.f && nv_ < 1.f && (interior_y || (v >= 0.f && v <= 1.f)))) {
-        Pos p{0, iy, 0.f, nv_ * wyc};
-        settle(g, p, a.stat);
-        niy = p.iy;
-        const float nwy = __ldg(g.wy + niy);
-        nv_ = p.Y / nwy;
-        if (p.Y < nwy && nv_ >= 1.f) nv_ = nextafterf(1.f, 0.f);
-        if (p.Y < 0.5f * nwy && nv_ >= 0.5f) nv_ = nextafterf(0.5f, 0.f);
-        if (p.Y > 0.5f * nwy && nv_ <= 0.5f) nv_ = nextafterf(0.5f, 1.f);
-        if (p.Y > nwy && nv_ <= 1.f) nv_ = nextafterf(1.f, 2.f);
-      }
-      if (t >= 100) {
-        // immobile marker (moveandrotatemarkers.c:88-135): inside the model
-        // it spawns a mobile marker there and goes back to its anchor
-        // (markk, markv), as it does when it strays more than ystpy from it
-        const bool inside = (nix > 0 || nu_ >= 0.f) && (nix < g.ncx - 1 || nu_ <= 1.f) &&
-                            (niy > 0 || nv_ >= 0.f) && (niy < g.ncy - 1 || nv_ <= 1.f);
-        const double ax = (double)tk + (double)a.m.tk_lo[idx];
-        const double ay = (double)a.m.mv[idx] + (double)a.m.mv_lo[idx];
-        double x = g.gx[nix] + (double)nu_ * (g.gx[nix + 1] - g.gx[nix]);
-        double y = g.gy[niy] + (double)nv_ * (g.gy[niy + 1] - g.gy[niy]);
-        if (inside && a.has_imm) {
-          const int id = a.m.id[idx];
-          a.imm.spawn[id] = 1;
-          a.imm.sp_cell[id] = nix * ncy + niy;
-          a.imm.sp_u[id] = nu_;
-          a.imm.sp_v[id] = nv_;
-          x = ax;
-          y = ay;
-        }
-        const double dx = x - ax, dy = y - ay;
-        if (x == ax && y == ay || sqrt(dx * dx + dy * dy) > P.ystpy) {
-          nix = nsearch64(g.gx, g.xn, ax);
-          niy = nsearch64(g.gy, g.yn, ay);
-          nu_ = offset32((ax - g.gx[nix]) / (g.gx[nix + 1] - g.gx[nix]));
-          nv_ = offset32((ay - g.gy[niy]) / (g.gy[niy + 1] - g.gy[niy]));
-        }
-      } else {
-      // stress rotation, moveandrotatemarkers.c:58-76
-      float msxx = a.m.sxx[idx], msxy = a.m.sxy[idx];
-      sp0 *= dt;
-      if (P.stoksmod == 1) {
-        float sn, cs;
-        sincosf(sp0, &sn, &cs);
-        const float s2 = 2.f * sn * cs, c2 = cs * cs - sn * sn;  // sin, cos of 2 sp0
-        const float r1 = msxx * cs * cs - msxx * sn * sn + msxy * s2;
-        const float r3 = 0.5f * (-msxx - msxx) * s2 + msxy * c2;
-        msxx = r1; msxy = r3;
-      } else if (P.stoksmod == 2) {
-        const float r1 = msxx + msxy * 2.f * sp0;
-        const float r3 = msxy + 0.5f * (-msxx - msxx) * 2.f * sp0;
-        msxx = r1; msxy = r3;
-      }
-      a.m.sxx[idx] = msxx;
-      a.m.sxy[idx] = msxy;
-      // markers coming from depth, out-of-grid reset (:79-87); the FP64
-      // position only when the FP32 one is within 1 m of zdeep
-      // (the temperature pair's high word decides tk < tdeep; the two can
-      // differ only for a temperature within half an FP32 ulp of tdeep, where
-      // resetting or not leaves the same temperature to that half ulp)
-      float tk_lo = 0.f;
-      bool reset = false;
-      if (vy0 < 0.f && tk < a.S.tdeep_f &&
-          __ldg(a.gyf + niy) + nv_ * __ldg(g.wy + niy) > a.S.zdeep_lo_f) {
-        const double ynew = g.gy[niy] + (double)nv_ * (g.gy[niy + 1] - g.gy[niy]);
-        if (ynew > P.zdeep) {
-          tk = a.S.tdeep_f;
-          tk_lo = a.S.tdeep_lo;
-          reset = true;
-        }
-      }
-      const bool out = (nix == 0 && nu_ < 0.f) || (nix == g.ncx - 1 && nu_ > 1.f) ||
-                       (niy == 0 && nv_ < 0.f) || (niy == g.ncy - 1 && nv_ > 1.f);
-      if (out) {
-        tk = 0.f;
-        tk_lo = 0.f;
+    } else {
+    // stress rotation, moveandrotatemarkers.c:58-76
+    float msxx = a.m.sxx[idx], msxy = a.m.sxy[idx];
+    sp0 *= dt;
+    if (P.stoksmod == 1) {
+      float sn, cs;
+      sincosf(sp0, &sn, &cs);
+      const float s2 = 2.f * sn * cs, c2 = cs * cs - sn * sn;  // sin, cos of 2 sp0
+      const float r1 = msxx * cs * cs - msxx * sn * sn + msxy * s2;
+      const float r3 = 0.5f * (-msxx - msxx) * s2 + msxy * c2;
+      msxx = r1; msxy = r3;
+    } else if (P.stoksmod == 2) {
+      const float r1 = msxx + msxy * 2.f * sp0;
+      const float r3 = msxy + 0.5f * (-msxx - msxx) * 2.f * sp0;
+      msxx = r1; msxy = r3;
+    }
+    a.m.sxx[idx] = msxx;
+    a.m.sxy[idx] = msxy;
+    // markers coming from depth, out-of-grid reset (:79-87); the FP64
+    // position only when the FP32 one is within 1 m of zdeep
+    // (the temperature pair's high word decides tk < tdeep; the two can
+    // differ only for a temperature within half an FP32 ulp of tdeep, where
+    // resetting or not leaves the same temperature to that half ulp)
+    float tk_lo = 0.f;
+    bool reset = false;
+    if (vy0 < 0.f && tk < a.S.tdeep_f &&
+        __ldg(a.gyf + niy) + nv_ * __ldg(g.wy + niy) > a.S.zdeep_lo_f) {
+      const double ynew = g.gy[niy] + (double)nv_ * (g.gy[niy + 1] - g.gy[niy]);
+      if (ynew > P.zdeep) {
+        tk = a.S.tdeep_f;
+        tk_lo = a.S.tdeep_lo;
         reset = true;
-        a.m.e[idx] = 0.f;
-        a.m.flags[idx] |= MFLAG_RESET;
-        atomicAdd(a.stat + ST_OUT_OF_GRID, 1ull);
-      }
-      if (reset) {
-        a.m.tk[idx] = tk;
-        a.m.tk_lo[idx] = tk_lo;
-      }
       }
     }
-    // mobile markers outside the model after the move: the slots that
-    // markers spawned by immobile ones refill (moveandrotatemarkers.c:141-171)
-    if (a.has_imm && t < 100 &&
-        !((nix > 0 || nu_ >= 0.f) && (nix < g.ncx - 1 || nu_ <= 1.f) &&
-          (niy > 0 || nv_ >= 0.f) && (niy < g.ncy - 1 || nv_ <= 1.f)))
-      a.imm.out[a.m.id[idx]] = 1;
-    a.m.cell_out[idx] = nix * ncy + niy;
-    a.m.u_out[idx] = nu_;
-    a.m.v_out[idx] = nv_;
+    const bool out = (nix == 0 && nu_ < 0.f) || (nix == g.ncx - 1 && nu_ > 1.f) ||
+                     (niy == 0 && nv_ < 0.f) || (niy == g.ncy - 1 && nv_ > 1.f);
+    if (out) {
+      tk = 0.f;
+      tk_lo = 0.f;
+      reset = true;
+      a.m.e[idx] = 0.f;
+      a.m.flags[idx] |= MFLAG_RESET;
+      atomicAdd(a.stat + ST_OUT_OF_GRID, 1ull);
+    }
+    if (reset) {
+      a.m.tk[idx] = tk;
+      a.m.tk_lo[idx] = tk_lo;
+    }
+    }
   }
+  // mobile markers outside the model after the move: the slots that
+  // markers spawned by immobile ones refill (moveandrotatemarkers.c:141-171)
+  if (a.has_imm && t < 100 &&
+      !((nix > 0 || nu_ >= 0.f) && (nix < g.ncx - 1 || nu_ <= 1.f) &&
+        (niy > 0 || nv_ >= 0.f) && (niy < g.ncy - 1 || nv_ <= 1.f)))
+    a.imm.out[a.m.id[idx]] = 1;
+  a.m.cell_out[idx] = nix * ncy + niy;
+  a.m.u_out[idx] = nu_;
+  a.m.v_out[idx] = nv_;
 }
 
 }  // namespace
