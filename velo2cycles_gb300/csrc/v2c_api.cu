@@ -1297,7 +1297,7 @@ static int n2m_move(v2c_ctx *ctx, int do_n2m, int do_move) {
   if (do_n2m) {
     Prof pr(ctx, V2C_PROF_N2M);
     launch_n2m(a, st);
-    ctx->launches += a.bs ? 2 : 1;
+    ctx->launches += a.bs || ctx->p.antidiffinter != 1 ? 2 : 1;
   }
   if (do_move) {
     ctx->props_valid = false;

@@ -178,47 +178,82 @@ __device__ __forceinline__ void vel_at(const Grid &g, const float4 *Q, Pos p, fl
   ESP = fmaf(dY, fmaf(e.w, dX, e.z), fmaf(e.y, dX, e.x));
 }
 
-// Marker values without antidiffusion (interpolation.c:985-1011): the previous node fields interpolated (change = false: a marker's first
-// values), or the change of the node fields since then (change = true),
-// interpolated as one field of node differences -- the same bilinear form,
-// so the same value in exact arithmetic, but the FP32 node differences of
-// two states that agree in their leading digits are exact where the
-// separate interpolations would each round at the size of the field.
+// Marker values without antidiffusion (interpolation.c:985-1011): the previous
+// node fields interpolated for a marker's first values, afterwards the change
+// of the node fields since then, interpolated as one field of node differences
+// -- the same bilinear form, so the same value in exact arithmetic, but the
+// FP32 node differences of two states that agree in their leading digits are
+// exact where the separate interpolations would each round at the size of the
+// field.
 struct Plain {
   float phi, exx, exy, sxx, sxy, p, vx, vy, e;
 };
+// a marker that has just come in: the previous node values themselves
 __device__ __forceinline__ void plain_values(const Grid &g, const Nodes &N, Axis ax, Axis ay,
-                                                 float uc, float vc, bool change, Plain &o) {
+                                             float uc, float vc, Plain &o) {
   const long yn = g.yn;
   float e, n;
   long m3 = stencil_basic(g, ax, ay, e, n);
-  if (change) {
-    o.exy = bil_diff(N.f(V2C_NF_EXY), N.f(V2C_NF_EXYE), m3, yn, e, n);
-    o.sxy = bil_diff(N.f(V2C_NF_SXY), N.f(V2C_NF_SXYE), m3, yn, e, n);
-    o.e = bil_diff(N.f(V2C_NF_PES), N.f(V2C_NF_PE), m3, yn, e, n);
-    o.phi = bil_diff(N.f(V2C_NF_PHIS_IT), N.f(V2C_NF_PHIS), m3, yn, e, n);
-  } else {
-    o.exy = bil(N.f(V2C_NF_EXYE), m3, yn, e, n);
-    o.sxy = bil(N.f(V2C_NF_SXYE), m3, yn, e, n);
-    o.e = bil(N.f(V2C_NF_PE), m3, yn, e, n);
-    o.phi = bil(N.f(V2C_NF_PHIS), m3, yn, e, n);
-  }
+  o.exy = bil(N.f(V2C_NF_EXYE), m3, yn, e, n);
+  o.sxy = bil(N.f(V2C_NF_SXYE), m3, yn, e, n);
+  o.e = bil(N.f(V2C_NF_PE), m3, yn, e, n);
+  o.phi = bil(N.f(V2C_NF_PHIS), m3, yn, e, n);
   m3 = stencil_centre(g, ax, ay, uc > 0.5f, vc > 0.5f, e, n);
-  if (change) {
-    o.exx = bil_diff(N.f(V2C_NF_EXX), N.f(V2C_NF_EXXE), m3, yn, e, n);
-    o.sxx = bil_diff(N.f(V2C_NF_SXX), N.f(V2C_NF_SXXE), m3, yn, e, n);
-    o.p = bil_diff(N.f(V2C_NF_PR), N.f(V2C_NF_SPPE), m3, yn, e, n);
-  } else {
-    o.exx = bil(N.f(V2C_NF_EXXE), m3, yn, e, n);
-    o.sxx = bil(N.f(V2C_NF_SXXE), m3, yn, e, n);
-    o.p = bil(N.f(V2C_NF_SPPE), m3, yn, e, n);
-  }
+  o.exx = bil(N.f(V2C_NF_EXXE), m3, yn, e, n);
+  o.sxx = bil(N.f(V2C_NF_SXXE), m3, yn, e, n);
+  o.p = bil(N.f(V2C_NF_SPPE), m3, yn, e, n);
   m3 = stencil_vx(g, ax, ay, vc < 0.5f, g.xn - 2, e, n);
-  o.vx = change ? bil_diff(N.f(V2C_NF_VX), N.f(V2C_NF_MVX), m3, yn, e, n)
-                : bil(N.f(V2C_NF_MVX), m3, yn, e, n);
+  o.vx = bil(N.f(V2C_NF_MVX), m3, yn, e, n);
   m3 = stencil_vy(g, ax, ay, uc < 0.5f, g.yn - 2, e, n);
-  o.vy = change ? bil_diff(N.f(V2C_NF_VY), N.f(V2C_NF_MVY), m3, yn, e, n)
-                : bil(N.f(V2C_NF_MVY), m3, yn, e, n);
+  o.vy = bil(N.f(V2C_NF_MVY), m3, yn, e, n);
+}
+
+// The nine differences of a node side by side: a marker's change is then 16
+// reads instead of 72.  811 x 309 lines, 4.5 M markers: 215 -> 151 us, this
+// pass over the nodes included; 301 x 101: 26 and 26, 51 x 21: 11.2 and 11.6.
+struct PlainNode {
+  float4 basic;   // EXY, SXY, PES, PHIS_IT, each minus its previous value
+  float4 centre;  // EXX, SXX, PR
+  float2 vel;     // VX, VY
+  float2 pad;
+};
+static_assert(sizeof(PlainNode) * 16 <= sizeof(float4) * QUAD_FLOAT4 * 9,
+              "the differences of the smallest grid's nodes fit its cells' forms");
+__global__ void __launch_bounds__(256) k_plain_nodes(Nodes N, long nn, PlainNode *D) {
+  after_previous();
+  const long m = blockIdx.x * 256l + threadIdx.x;
+  if (m >= nn) return;
+  auto d = [&](int f, int g) { return N.f(f)[m] - N.f(g)[m]; };
+  D[m].basic = make_float4(d(V2C_NF_EXY, V2C_NF_EXYE), d(V2C_NF_SXY, V2C_NF_SXYE),
+                           d(V2C_NF_PES, V2C_NF_PE), d(V2C_NF_PHIS_IT, V2C_NF_PHIS));
+  D[m].centre = make_float4(d(V2C_NF_EXX, V2C_NF_EXXE), d(V2C_NF_SXX, V2C_NF_SXXE),
+                            d(V2C_NF_PR, V2C_NF_SPPE), 0.f);
+  D[m].vel = make_float2(d(V2C_NF_VX, V2C_NF_MVX), d(V2C_NF_VY, V2C_NF_MVY));
+}
+__device__ __forceinline__ void plain_change(const Grid &g, const PlainNode *D, Axis ax, Axis ay,
+                                             float uc, float vc, Plain &o) {
+  const long yn = g.yn;
+  float e, n;
+  auto mix = [&](float a, float b, float c, float d) {
+    const float d0 = (1.f - e) * (1.f - n), d1 = (1.f - e) * n, d2 = e * (1.f - n), d3 = e * n;
+    return d0 * a + d1 * b + d2 * c + d3 * d;
+  };
+  auto mix4 = [&](const float4 &a, const float4 &b, const float4 &c, const float4 &d) {
+    return make_float4(mix(a.x, b.x, c.x, d.x), mix(a.y, b.y, c.y, d.y), mix(a.z, b.z, c.z, d.z),
+                       mix(a.w, b.w, c.w, d.w));
+  };
+  const PlainNode *p = D + stencil_basic(g, ax, ay, e, n);
+  const float4 B = mix4(__ldg(&p[0].basic), __ldg(&p[1].basic), __ldg(&p[yn].basic),
+                        __ldg(&p[yn + 1].basic));
+  o.exy = B.x; o.sxy = B.y; o.e = B.z; o.phi = B.w;
+  p = D + stencil_centre(g, ax, ay, uc > 0.5f, vc > 0.5f, e, n);
+  const float4 C = mix4(__ldg(&p[0].centre), __ldg(&p[1].centre), __ldg(&p[yn].centre),
+                        __ldg(&p[yn + 1].centre));
+  o.exx = C.x; o.sxx = C.y; o.p = C.z;
+  p = D + stencil_vx(g, ax, ay, vc < 0.5f, g.xn - 2, e, n);
+  o.vx = mix(__ldg(&p[0].vel.x), __ldg(&p[1].vel.x), __ldg(&p[yn].vel.x), __ldg(&p[yn + 1].vel.x));
+  p = D + stencil_vy(g, ax, ay, uc < 0.5f, g.yn - 2, e, n);
+  o.vy = mix(__ldg(&p[0].vel.y), __ldg(&p[1].vel.y), __ldg(&p[yn].vel.y), __ldg(&p[yn + 1].vel.y));
 }
 
 // ------------------------------------------------------------ the sweep
@@ -656,8 +691,8 @@ __global__ void __launch_bounds__(NTH, 4) k_n2m(N2MArgs a) {
 // back-scatter); BS, interpolationmod 1 (each marker's back-scatter payload
 // goes to a.bs for the per-node kernel below).  One thread per marker, in
 // sorted order; bound by the latency of its node reads, so 6 resident CTAs
-// (811 x 309 lines, 4.5 M markers, PLAIN: 215 us, 235 at the registers the
-// compiler takes by itself, 288 at 4 CTAs; BS, 433 x 187 lines: 121 -> 100
+// (811 x 309 lines, 4.5 M markers, PLAIN before plain_change: 215 us, 235 at
+// the registers the compiler takes by itself, 288 at 4 CTAs; BS, 433 x 187 lines: 121 -> 100
 // us against the chunked sweep).
 template <bool BS, bool PLAIN>
 __global__ void __launch_bounds__(256, 6) k_gather(N2MArgs a) {
@@ -729,7 +764,7 @@ __global__ void __launch_bounds__(256, 6) k_gather(N2MArgs a) {
   if (in_strict && tk <= 0.f) {
     if (PLAIN) {
       Plain o;
-      plain_values(g, N, ax, ay, uc, vc, false, o);
+      plain_values(g, N, ax, ay, uc, vc, o);
       msxx = o.sxx; msxy = o.sxy; mp = o.p; mexx = o.exx; mexy = o.exy;
       mvx = o.vx; mvy = o.vy; phi = o.phi; me = o.e;
     }
@@ -743,7 +778,7 @@ __global__ void __launch_bounds__(256, 6) k_gather(N2MArgs a) {
   if (in_grid && tk > 0.f) {
     if (PLAIN) {
       Plain o;
-      plain_values(g, N, ax, ay, uc, vc, true, o);
+      plain_change(g, reinterpret_cast<const PlainNode *>(a.quad), ax, ay, uc, vc, o);
       phi += o.phi; mexx += o.exx; mexy += o.exy;
       msxx += o.sxx; msxy += o.sxy; mp += o.p;
       mvx += o.vx; mvy += o.vy; me += o.e;
@@ -1035,6 +1070,9 @@ void launch_n2m(const N2MArgs &a, cudaStream_t st) {
     launch_after(k_n2m, grid, NTH, sizeof(Smem), st, a);
   } else if (a.n > 0) {
     // the markers take the node fields without antidiffusion
+    // (the node differences borrow the room of the move's velocity forms)
+    launch_after(k_plain_nodes, (unsigned)((a.g.nn + 255) / 256), 256, 0, st, a.N, a.g.nn,
+                 reinterpret_cast<PlainNode *>(a.quad));
     launch_after(k_gather<false, true>, mb, 256, 0, st, a);
   }
 }

@@ -325,16 +325,4 @@ __device__ __forceinline__ ff bil_ff(const float *f, long m3, long yn, float e, 
   return r;
 }
 
-// bil(f) - bil(g) as one interpolation of the node differences (the same
-// bilinear form, so the same value in exact arithmetic): f and g are
-// consecutive states of one field that agree in their leading digits, and
-// their FP32 node differences are exact where they are within a factor 2
-__device__ __forceinline__ float bil_diff(const float *f, const float *g, long m3, long yn,
-                                          float e, float n) {
-  float d0 = (1.f - e) * (1.f - n), d1 = (1.f - e) * n, d2 = e * (1.f - n), d3 = e * n;
-  return d0 * (__ldg(f + m3) - __ldg(g + m3)) + d1 * (__ldg(f + m3 + 1) - __ldg(g + m3 + 1)) +
-         d2 * (__ldg(f + m3 + yn) - __ldg(g + m3 + yn)) +
-         d3 * (__ldg(f + m3 + yn + 1) - __ldg(g + m3 + yn + 1));
-}
-
 }  // namespace v2c
