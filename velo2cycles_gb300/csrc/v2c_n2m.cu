@@ -825,19 +825,39 @@ __device__ __forceinline__ void bs_mode1(const N2MArgs &a) {
     if (cx < 0 || cx >= g.ncx || cy < 0 || cy >= ncy) return;
     const float s1 = (1.f / __ldg(g.wx + cx)) / __ldg(g.wy + cy);
     const long c = (long)cx * ncy + cy;
-    const int sb = __ldg(a.start + c), se = __ldg(a.start + c + 1);
-    for (int s = sb; s < se; s++) {
-      const float u = bs[BS_U * n + s], v = bs[BS_V * n + s];
-      if (ROLE == 0) {
+    if (ROLE == 0) {
+      const int sb = __ldg(a.start + c), se = __ldg(a.start + c + 1);
+#pragma unroll 2
+      for (int s = sb; s < se; s++) {
+        const float u = bs[BS_U * n + s], v = bs[BS_V * n + s];
         const float w = s1 * (ax ? u : 1.f - u) * (by ? v : 1.f - v);
         sum[0].add(bs[BS_PHIS * n + s] * w); sum[1].add(bs[BS_SXY * n + s] * w);
         sum[2].add(bs[BS_EXY * n + s] * w); sum[3].add(bs[BS_ES * n + s] * w);
         sum[4].add(w);
-      } else {
+      }
+      return;
+    }
+    // only the quarter classes (2 (v > 1/2) + (u > 1/2)) that have weight: a
+    // half-cell factor k = 0 needs the lower half, k = 2 the upper; all fields
+    // of a marker at once (433 x 187 lines, both groups: 57 -> 48 us)
+    const int4 qs = __ldg(a.qstart + c);
+    const int qe = __ldg(a.start + c + 1);
+    const int mask = (0xaf5 >> (4 * ax)) & (0xcf3 >> (4 * by)) & 0xf;
+    auto qb = [&](int q) { return q == 0 ? qs.x : q == 1 ? qs.y : q == 2 ? qs.z : q == 3 ? qs.w : qe; };
+#pragma unroll 1
+    for (int q = 0; q < 4; q++) {
+      if (!((mask >> q) & 1)) continue;
+      const int sb = qb(q);
+      while (q < 3 && ((mask >> (q + 1)) & 1)) q++;
+      const int se = qb(q + 1);
+#pragma unroll 2
+      for (int s = sb; s < se; s++) {
+        const float u = bs[BS_U * n + s], v = bs[BS_V * n + s];
+        const float pr = bs[BS_PR * n + s], sxx = bs[BS_SXX * n + s], exx = bs[BS_EXX * n + s];
         const float w = s1 * bs_half(ax, u) * bs_half(by, v);
         if (w != 0.f) {
-          sum[0].add(bs[BS_PR * n + s] * w); sum[1].add(bs[BS_SXX * n + s] * w);
-          sum[2].add(bs[BS_EXX * n + s] * w); sum[3].add(w);
+          sum[0].add(pr * w); sum[1].add(sxx * w);
+          sum[2].add(exx * w); sum[3].add(w);
         }
       }
     }
