@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(PT, 8) k_phys(PhysArgs a) {
     bool need = solve;
     if (solve && MODE == PHYS_SPLIT) {
       const float exx = a.m.exx[i], exy = a.m.exy[i];
-      float edot;
-      asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(edot) : "f"(exx * exx + exy * exy));
+      float edot;  // (with subnormal squares: strain rates below 1e-19 load a marker too)
+      asm("sqrt.approx.f32 %0, %1;" : "=f"(edot) : "f"(exx * exx + exy * exy));
       if (rsf_floor_marker(*a.rk, t, far, fr.a, fr.b, fr.L, fr.V0, fr.mu0,
                            (P.pmode == 0) ? sn_ff.hi : a.m.p[i], dt_ff.hi, phi, sigin, edot, mnu)) {
         a.m.slipv[i] = 1e-40f;

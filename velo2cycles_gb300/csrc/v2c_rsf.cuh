@@ -407,11 +407,13 @@ __device__ __forceinline__ bool rsf_floor_certain(const Rsf32 &q, float &A_floor
 }
 
 // The same question asked of every marker of a model (far: the constants k of
-// the far field and state 50; t: the rock type), with approximate quotients:
-// their few ulps are as far below the margin, and a "no" only sends the marker
-// to the solve, which finds the floor too.  Without the six IEEE quotients and
-// the logarithm the test is 190 instead of 300 instructions of the 3400 a warp
-// of markers takes at dt = 1e8 s.
+// the far field and state 50; t: the rock type), with approximate quotients.
+// A "yes" is final, so Ts and lhs have to be good to the margin: the quotients
+// (of normal divisors) and edot, the load's strain rate, come within a few
+// ulps, as far below it, the logarithm and the exponential within 1e-4.  A "no"
+// only sends the marker to the solve, which finds the floor too.  Without the
+// six IEEE quotients and the logarithm the test is 190 instead of 300
+// instructions of the 3400 a warp of markers takes at dt = 1e8 s.
 __device__ __forceinline__ bool rsf_floor_marker(const RsfConst &k, int t, bool far, float a,
                                                  float b, float L, float V0, float mu0, float sn,
                                                  float dt, float phio, float tau_old, float edot,
