@@ -487,8 +487,11 @@ int v2c_get_profile(v2c_ctx *ctx, int group, double *ms, long *launches);
  *   eta_vp   = eta tau_y /(2 eta V/W + tau_y)     (calc_RSF.c:142),
  *   Z        = G dt /(G dt + eta_vp).
  * States are device pointers of V2C_RS_N float64 columns of length n
- * (column-major, see V2C_RS_*).  Outputs: V, phi(V), tau_y(V), and the
- * Newton iteration count.  guess = V2C_GUESS_PLAIN starts from V_old,
+ * (column-major, see V2C_RS_*).  Outputs: V, phi(V), tau_y(V), the residual
+ * (V2C_RO_N columns of length n), and the Newton iteration count (or NULL).
+ * out_dev may be columns of the states (states_dev + k n for a whole k): each
+ * state is then read before its outputs replace it, by a slower kernel; iters
+ * must overlap neither.  guess = V2C_GUESS_PLAIN starts from V_old,
  * V2C_GUESS_LEARNED from the network loaded with v2c_mlp_load and falls back
  * to the plain guess when the learned start does not converge. */
 enum {

@@ -122,13 +122,15 @@ __device__ __forceinline__ void add_stats(unsigned long long *stat, unsigned lon
   warp_add(stat + ST_NEWTON_NONCONV, nc);
 }
 
-// The FP64 form: one instantiation per start; the learned start comes from
-// the network's outputs guess[i].
-template <bool LEARNED>
-__global__ void __launch_bounds__(NT, 4) k_solve_states64(const double *S, long n, ff W,
-                                                          const float *guess, double rtol,
-                                                          int maxit, double *out, int32_t *iters,
-                                                          unsigned long long *stat) {
+// A state at a time, read before its results are written: the FP64 form, and
+// the split form (FP64 false) where the outputs lie in rows of the states.  One
+// instantiation per start; the learned start comes from the network's outputs
+// guess[i].
+template <bool FP64, bool LEARNED>
+__global__ void __launch_bounds__(NT, 4) k_solve_states(const double *S, long n, ff W,
+                                                        const float *guess, double rtol, int maxit,
+                                                        double *out, int32_t *iters,
+                                                        unsigned long long *stat) {
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const long nwarps = (long)gridDim.x * (NT / 32);
   for (long base = ((long)blockIdx.x * (NT / 32) + wl) * 32; base < n; base += nwarps * 32) {
@@ -138,15 +140,22 @@ __global__ void __launch_bounds__(NT, 4) k_solve_states64(const double *S, long 
       RsfIn in;
       double vold;
       state_of(S, n, i, W, in, vold);
-      // starts from the FP64 log of the previous slip rate
       const float u_plain = plain_start(vold);
-      const double u_plain64 = vold > 0 ? log(vold) : (double)u_plain;
+      // (the FP64 form's plain start: the FP64 log of the previous slip rate)
+      const double u_plain64 = FP64 && vold > 0 ? log(vold) : (double)u_plain;
       const float u0 = LEARNED ? guess[i] : u_plain;
-      RsfResult r = rsf_solve64(in, LEARNED ? (double)u0 : u_plain64, rtol, maxit);
-      it = r.it64;
+      auto solve = [&](float u, double u64) {
+        if constexpr (FP64) return rsf_solve64(in, u64, rtol, maxit);
+        const Rsf32 q = rsf32_of(in);
+        float A_floor;
+        if (rsf_floor_certain(q, A_floor)) return rsf_floor_result(in, A_floor);
+        return rsf_solve_split(in, q, u, rtol, maxit);
+      };
+      RsfResult r = solve(u0, LEARNED ? (double)u0 : u_plain64);
+      it = r.it32 + r.itff + r.it64;
       if (!r.ok && LEARNED && u0 != u_plain) {
-        r = rsf_solve64(in, u_plain64, rtol, maxit);
-        it += r.it64;
+        r = solve(u_plain, u_plain64);
+        it += r.it32 + r.itff + r.it64;
         fb = 1;
       }
       if (!r.ok) nc = 1;
@@ -759,10 +768,16 @@ extern "C" int v2c_rsf_newton(v2c_ctx *ctx, const double *states_dev, long n, in
                  ns->d_guess);
     v2c_ctx_count_launches(ctx, 1);
   }
-  if (fp64) {
-    (learned ? k_solve_states64<true> : k_solve_states64<false>)<<<(unsigned)blocks, NT, 0, st>>>(
-        states_dev, n, W, ns->d_guess, p->newton_rtol, p->newton_maxit, out_dev,
-        iters_dev, v2c_ctx_stat(ctx));
+  // the phases of the split form keep their intermediate results in the output
+  // rows and read the states again, so outputs among the states take the kernel
+  // that reads a state whole (as the FP64 form always does)
+  const uintptr_t s0 = (uintptr_t)states_dev, o0 = (uintptr_t)out_dev;
+  const bool overlap = s0 < o0 + sizeof(double) * V2C_RO_N * n && o0 < s0 + sizeof(double) * V2C_RS_N * n;
+  if (fp64 || overlap) {
+    auto kern = fp64 ? (learned ? k_solve_states<true, true> : k_solve_states<true, false>)
+                     : (learned ? k_solve_states<false, true> : k_solve_states<false, false>);
+    kern<<<(unsigned)blocks, NT, 0, st>>>(states_dev, n, W, ns->d_guess, p->newton_rtol,
+                                          p->newton_maxit, out_dev, iters_dev, v2c_ctx_stat(ctx));
   } else {
     const unsigned nb = (unsigned)((n + NT - 1) / NT);
     if (learned) launch_after(k_states_fp32<true>, nb, NT, 0, st, states_dev, n, W, ns->d_guess,
