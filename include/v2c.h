@@ -219,7 +219,8 @@ int v2c_set_rock_table(v2c_ctx *ctx, const double *rt);
  * (headevps.c:205-209): bondm[nodenum*4], bondn[bondnum][3],
  * bondv[bondnum][4].  Used by the boundary corrections that end
  * marker2nodes (momentum_continuity_addmatrix_checkerror.c:1002-1184,
- * temperature_iterate.c:828-891). */
+ * temperature_iterate.c:828-891).  A table whose bondm refers outside it is
+ * refused (V2C_ERR_ARG) and leaves the one in force. */
 int v2c_set_bonds(v2c_ctx *ctx, const long *bondm, const long *bondn,
                   const double *bondv, long bondnum);
 

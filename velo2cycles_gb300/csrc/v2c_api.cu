@@ -529,12 +529,13 @@ extern "C" int v2c_set_rock_table(v2c_ctx *ctx, const double *rt) {
 extern "C" int v2c_set_bonds(v2c_ctx *ctx, const long *bondm, const long *bondn,
                              const double *bondv, long bondnum) {
   if (!ctx || !bondm || bondnum < 0 || (bondnum > 0 && (!bondn || !bondv))) return V2C_ERR_ARG;
+  // a refused table leaves the one in force
+  for (long i = 0; i < ctx->nn * 4; i++)
+    if (bondm[i] < 0 || bondm[i] >= bondnum) return fail(ctx, V2C_ERR_ARG);
   ctx->h_bondm.assign(bondm, bondm + ctx->nn * 4);
   ctx->h_bondn.assign(bondn, bondn + bondnum * 3);
   ctx->h_bondv.assign(bondv, bondv + bondnum * 4);
   ctx->bondnum = bondnum;
-  for (long i = 0; i < ctx->nn * 4; i++)
-    if (bondm[i] < 0 || bondm[i] >= bondnum) return fail(ctx, V2C_ERR_ARG);
   ctx->have_bonds = true;
   ctx->bc_built_compressible = -1;
   ctx->stokes_bonds_ok = false;
@@ -1414,8 +1415,10 @@ constexpr size_t STOKES_KEEP_BYTES = size_t(256) << 20;
 static int stokes_bonds(v2c_ctx *ctx, StokesArgs &s) {
   const long nn = ctx->nn, nb = ctx->bondnum;
   DevArena &w = ctx->stokes_bonds;
-  CK(w.reserve(DevArena::bytes_of<long>(nn * 4) + DevArena::bytes_of<long>(nb * 3) +
-               DevArena::bytes_of<double>(nb * 4)));
+  const size_t bytes = DevArena::bytes_of<long>(nn * 4) + DevArena::bytes_of<long>(nb * 3) +
+                       DevArena::bytes_of<double>(nb * 4);
+  if (bytes > w.cap) ctx->stokes_bonds_ok = false;  // a new block holds nothing yet
+  CK(w.reserve(bytes));
   long *bm = w.take<long>(nn * 4), *bn = w.take<long>(nb * 3);
   double *bv = w.take<double>(nb * 4);
   if (!ctx->stokes_bonds_ok) {
