@@ -437,9 +437,10 @@ int v2c_cycle_set_velocity(v2c_ctx *ctx, int regime, const double *vx, const dou
  * counting sort; then timesum += dt.  Asynchronous.
  * use_graph: the step is captured once into a CUDA graph per key (regime,
  * dt, the position buffer holding the current positions, every parameter
- * but timesum, and timesum's classes: zero, positive, equal to dt, above
- * 4e7 s, which are all the kernels see of it) and replayed afterwards; at
- * most 8 graphs are kept (the oldest dropped).  The first step of a key
+ * but timesum, timesum's classes: zero, positive, equal to dt, above 4e7 s,
+ * which are all the kernels see of it, the number of markers, and whether a
+ * network is loaded) and replayed afterwards; at most 8 graphs are kept (the
+ * oldest dropped), none past a new boundary or rock table.  The first step of a key
  * runs the capture (no profiling events there); a capture needs no
  * allocation, so it may run at any point after the context is set up. */
 int v2c_cycle_step(v2c_ctx *ctx, int regime, double dt, int use_graph);

@@ -159,10 +159,18 @@ struct v2c_ctx {
     const void *pos;      // position buffer holding the current positions
     v2c_params p;         // all parameters, timesum zeroed
     int flags;            // the timesum classes the kernels see
+    long n;               // markers
+    bool mlp;             // a network is loaded
     cudaGraphExec_t exec;
     long launches;        // kernels in one replay
   };
   std::vector<CycleGraph> graphs;
+  // what the captured launches hold beyond a graph's key has changed (the rows
+  // of the boundary table, a constant of the rock table): capture again
+  void drop_graphs() {
+    for (auto &gr : graphs) cudaGraphExecDestroy(gr.exec);
+    graphs.clear();
+  }
 };
 
 namespace {
@@ -408,8 +416,7 @@ extern "C" int v2c_destroy(v2c_ctx *ctx) {
   ctx->stokes_ws.release();
   ctx->stokes_out.release();
   ctx->stokes_bonds.release();
-  for (auto &gr : ctx->graphs) cudaGraphExecDestroy(gr.exec);
-  ctx->graphs.clear();
+  ctx->drop_graphs();
   for (float *v : ctx->d_cyc_v)
     if (v) cudaFree(v);
   for (double *v : ctx->d_cyc_v64)
@@ -477,6 +484,7 @@ extern "C" int v2c_set_grid(v2c_ctx *ctx, const double *gx, const double *gy) {
 
 extern "C" int v2c_set_rock_table(v2c_ctx *ctx, const double *rt) {
   if (!ctx || !rt) return V2C_ERR_ARG;
+  ctx->drop_graphs();
   ctx->h_rt.assign(rt, rt + V2C_RT_N * V2C_MAXTMR);
   std::vector<float> f((size_t)RK_N * V2C_MAXTMR, 0.f);
   auto R = [&](int r, int t) { return rt[r * V2C_MAXTMR + t]; };
@@ -645,6 +653,7 @@ int build_bc(v2c_ctx *ctx) {
     }
   }
   int n = (int)fld.size();
+  ctx->drop_graphs();
   if (ctx->bc_mem) { cudaFree(ctx->bc_mem); ctx->bc_mem = nullptr; }
   ctx->bc_n = n;
   ctx->bc = BcRows{};
@@ -1616,9 +1625,10 @@ extern "C" int v2c_cycle_step(v2c_ctx *ctx, int regime, double dt, int use_graph
   pk.timesum = 0;
   const int flags = cycle_flags(ctx);
   const void *pos = ctx->m.cell_in;
+  const bool mlp = ctx->nw.have_mlp != 0;
   for (auto &gr : ctx->graphs) {
     if (gr.regime == regime && gr.dt == dt && gr.pos == pos && gr.flags == flags &&
-        !memcmp(&gr.p, &pk, sizeof(pk))) {
+        gr.n == ctx->n && gr.mlp == mlp && !memcmp(&gr.p, &pk, sizeof(pk))) {
       CK(cudaGraphLaunch(gr.exec, st));
       // the host side of the step the graph replays
       swap_positions(ctx);
@@ -1653,7 +1663,7 @@ extern "C" int v2c_cycle_step(v2c_ctx *ctx, int regime, double dt, int use_graph
     cudaGraphExecDestroy(ctx->graphs.front().exec);
     ctx->graphs.erase(ctx->graphs.begin());
   }
-  ctx->graphs.push_back({regime, dt, pos, pk, flags, exec, ctx->launches - l0});
+  ctx->graphs.push_back({regime, dt, pos, pk, flags, ctx->n, mlp, exec, ctx->launches - l0});
   CK(cudaGraphLaunch(exec, st));
   ctx->p.timesum += dt;
   return V2C_OK;
