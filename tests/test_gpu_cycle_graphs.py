@@ -72,3 +72,27 @@ def test_what_a_graph_holds_changes(built_lib, params):
     for eager, graph in zip(*runs):
         for a, b in zip(eager, graph):
             assert np.array_equal(a, b, equal_nan=True)
+
+
+def test_calls_after_a_replayed_step(built_lib):
+    """What the host knows of the node fields after a step is the same when
+    the step was replayed: marker2nodes has written the temperature, so the
+    one uploaded in FP64 is no longer it, and the stress changes are kept."""
+    case = synth.make_case("tiny", seed=5)
+    fields = cycle.pulse_fields(case, cycle.Schedule())
+    tk2 = case.nodes[abi.NF_TK] + 3.0
+    got = []
+    for graph in (False, True):
+        m = mic.from_case(case)
+        m.cycle_set_velocity(0, *fields[0])
+        for _ in range(3):
+            m.cycle_step(0, 1e8, use_graph=graph)
+        m.upload_nodes({abi.NF_TK: case.nodes[abi.NF_TK] + 50.0, abi.NF_TK2: tk2})
+        m.cycle_step(0, 1e8, use_graph=graph)
+        m.interpolate_center2basic(1e8)
+        m.marker_temperature()
+        mk = m.download_markers([abi.MF_K])[abi.MF_K]
+        got.append([mk] + list(m.download_nodes([abi.NF_EXXPL, abi.NF_EXXEL, abi.NF_TK]).values()))
+        m.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b, equal_nan=True)

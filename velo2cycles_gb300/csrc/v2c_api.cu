@@ -1633,6 +1633,9 @@ extern "C" int v2c_cycle_step(v2c_ctx *ctx, int regime, double dt, int use_graph
       // the host side of the step the graph replays
       swap_positions(ctx);
       ctx->sorted = true;
+      ctx->vel64_ok[0] = ctx->vel64_ok[1] = true;
+      ctx->tk64_ok[0] = false;
+      ctx->dsxx_valid = true;
       ctx->launches += gr.launches;
       ctx->p.timesum += dt;
       return V2C_OK;
