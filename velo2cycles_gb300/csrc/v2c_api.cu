@@ -1416,11 +1416,13 @@ extern "C" int v2c_marker_temperature(v2c_ctx *ctx, double heatdif) {
 }
 
 // ====================================================== Stokes assembly
-// What the assembly keeps between calls: beyond this it is freed at the end of
-// each (an allocation then costs little beside the rows).
+// What the assembly keeps between calls, the boundary table included: beyond
+// this the rows and the result are freed at the end of each (an allocation then
+// costs little beside the rows), and a table larger than this alone (8 M nodes).
 constexpr size_t STOKES_KEEP_BYTES = size_t(256) << 20;
 
-// The boundary table on the device, uploaded once after v2c_set_bonds.
+// The boundary table on the device, uploaded once after v2c_set_bonds (and
+// again where it is not kept).
 static int stokes_bonds(v2c_ctx *ctx, StokesArgs &s) {
   const long nn = ctx->nn, nb = ctx->bondnum;
   DevArena &w = ctx->stokes_bonds;
@@ -1530,9 +1532,13 @@ extern "C" int v2c_stokes_assemble(v2c_ctx *ctx, const v2c_stokes_ctl *ctl, long
   if (!ctx->have_grid || !ctx->have_bonds) return fail(ctx, V2C_ERR_STATE);
   if (3 * ctx->nn + 1 > 0x7fffffffL) return fail(ctx, V2C_ERR_CAPACITY);
   const int rc = stokes_assemble(ctx, ctl, cap, ia, ja, a, b, nnz);
-  if (ctx->stokes_ws.cap + ctx->stokes_out.cap > STOKES_KEEP_BYTES) {
+  if (ctx->stokes_ws.cap + ctx->stokes_out.cap + ctx->stokes_bonds.cap > STOKES_KEEP_BYTES) {
     ctx->stokes_ws.release();
     ctx->stokes_out.release();
+  }
+  if (ctx->stokes_bonds.cap > STOKES_KEEP_BYTES) {
+    ctx->stokes_bonds.release();
+    ctx->stokes_bonds_ok = false;
   }
   return rc;
 }
