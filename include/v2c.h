@@ -227,7 +227,9 @@ int v2c_set_bonds(v2c_ctx *ctx, const long *bondm, const long *bondn,
 /* =========================================================== marker arrays
  * fields[V2C_MF_N] are host pointers (any may be NULL = not transferred;
  * X, Y and markt are required on upload).  Markers keep the reference
- * numbering at the boundary; the device holds them sorted by cell. */
+ * numbering at the boundary; the device holds them sorted by cell.  A
+ * download into pinned arrays only is written by one kernel, any other by a
+ * copy and a wait per field. */
 int v2c_upload_markers(v2c_ctx *ctx, const double *const *fields,
                        const signed char *markt, long n);
 int v2c_download_markers(v2c_ctx *ctx, double *const *fields,
@@ -249,8 +251,8 @@ int v2c_download_marker_properties(v2c_ctx *ctx, double *mnu, double *mkt, long 
 /* ============================================================= node arrays
  * One node field (V2C_NF_*) of nodenum doubles, converted to / from the
  * device's FP32.  The download returns when dst is filled.  The upload is
- * asynchronous on the context stream: from pinned host memory the copy runs
- * later, so src must stay unchanged until a call that synchronises the
+ * asynchronous on the context stream: from pinned host memory src is read
+ * later, so it must stay unchanged until a call that synchronises the
  * stream (any download, v2c_synchronize).  The velocities VX and VY are also
  * kept in FP64 on the device (allocated at their first upload, 2 x nodenum
  * doubles): recompute_stress_strainrate forms strain rates from their
@@ -258,26 +260,29 @@ int v2c_download_marker_properties(v2c_ctx *ctx, double *mnu, double *mkt, long 
 int v2c_upload_node_field(v2c_ctx *ctx, int field, const double *src);
 int v2c_download_node_field(v2c_ctx *ctx, int field, double *dst);
 /* count fields at once (fields[k] a V2C_NF_* id, src[k] / dst[k] nodenum
- * doubles each, count <= V2C_NF_N): one conversion kernel over all of them
- * and one copy per field back to back, one synchronisation at the end of
- * the download; the upload is asynchronous as above.  The first call with
- * more fields than any earlier one allocates a device staging area of
- * count x nodenum doubles (synchronising the stream).  No counterpart in
- * the reference, whose node arrays are host memory. */
+ * doubles each, count <= V2C_NF_N), one synchronisation at the end of the
+ * download; the upload is asynchronous as above.  Where every array is
+ * pinned host memory that the device addresses as the host does, one kernel
+ * reads or writes them all; other arrays (ordinary host memory, as the
+ * binding over the reference's globals passes it) take one copy per field
+ * back to back and one conversion kernel, with a device staging area of
+ * count x nodenum doubles that the first call with more fields than any
+ * earlier one allocates (synchronising the stream).  No counterpart in the
+ * reference, whose node arrays are host memory. */
 int v2c_upload_node_fields(v2c_ctx *ctx, int count, const int *fields,
                            const double *const *src);
 int v2c_download_node_fields(v2c_ctx *ctx, int count, const int *fields, double *const *dst);
 /* The download above without waiting for it: the fields are converted on
  * the context stream after the work enqueued so far (a snapshot: later
- * calls may change them) and copied to dst on a transfer stream of the
- * context, so that the copies run under the kernels the caller enqueues
- * next.  dst (count arrays of nodenum doubles) must be pinned host memory
- * for the copies to overlap, and must not be read before
- * v2c_wait_downloads (or v2c_synchronize) returns.  A second asynchronous
- * download reuses the staging area (count x nodenum doubles, allocated at
- * the first call or when count grows, synchronising both streams) after
- * the first one's copies.  No counterpart in the reference, whose node
- * arrays are host memory. */
+ * calls may change them) and brought to dst on a transfer stream of the
+ * context (small pinned arrays by one kernel, others by copies), under the
+ * kernels the caller enqueues next.  dst (count arrays of nodenum doubles)
+ * must be pinned host memory for that to overlap, and must not be read
+ * before v2c_wait_downloads (or v2c_synchronize) returns.  A second
+ * asynchronous download reuses the staging area (count x nodenum doubles,
+ * allocated at the first call or when count grows, synchronising both
+ * streams) after the first one has left it.  No counterpart in the
+ * reference, whose node arrays are host memory. */
 int v2c_download_node_fields_async(v2c_ctx *ctx, int count, const int *fields,
                                    double *const *dst);
 int v2c_wait_downloads(v2c_ctx *ctx);

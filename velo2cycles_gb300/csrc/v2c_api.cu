@@ -967,8 +967,12 @@ static int node_field_list_ok(int count, const int *fields, const void *const *p
   return 1;
 }
 
-// A field this size goes to the host by the copy engine, which takes no SMs
-// from the kernels it runs under; smaller ones together in one kernel.
+// Fields up to this size leave together in one kernel, which saves the copies'
+// issue: passes in us by engine / by kernel 211 / 200 at 51 x 21 lines, 383 /
+// 373 at 301 x 101, 637 / 631 at 433 x 187 (81 k nodes).  Above, the link's time
+// hides it (811 x 309 lines, 250 k nodes, 1461 / 1458; 401 k nodes 2588 / 2577;
+// 4 M 20.8 / 20.1 ms where runs differ by 5 %), and the engine takes no SMs
+// from the kernels it runs under.
 constexpr long ENGINE_COPY_NODES = 1 << 17;
 
 static int grow_node_stage(v2c_ctx *ctx, int count) {
@@ -1128,7 +1132,6 @@ extern "C" int v2c_marker2nodes(v2c_ctx *ctx) {
   a.gxf = ctx->d_gxf;
   a.gyf = ctx->d_gyf;
   a.TX = sweep_tx(ctx);
-  a.n = ctx->n;
   ctx->dsxx_valid = false;  // the scatter writes sxxe
   ctx->tk64_ok[0] = false;  // and the node temperature
   {

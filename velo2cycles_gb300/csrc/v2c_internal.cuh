@@ -82,11 +82,14 @@ enum { MFLAG_RESET = 1, MFLAG_DNEG = 2 };
 // blocks of the one before leave, and wait in after_previous(), the first
 // statement of every kernel launched that way, until the whole of it, and
 // with it everything before, has ended and its writes are visible.  Pass
-// times 250 -> 199 us at 51 x 21 lines, 421 -> 372 at 301 x 101, 2652 -> 2620
-// at the refined 1001 x 401, 20.29 -> 20.26 ms at 4001 x 1001.  (Letting the
-// next kernel be set up from the start of this one, by launch_dependents, was
-// worse everywhere: 210, 379, 2650 us, 20.60 ms; the waiting blocks take the
-// room of working ones.)
+// times in us, plain launches and these in turn on one build otherwise alike:
+//   51 x 21 lines 239 / 200, 301 x 101 417 / 373, 13-node 433 x 187 679 / 631,
+//   refined 1001 x 401 2542 / 2507, 4001 x 1001 19847 / 19656 (runs of one
+//   side differ by 0.3, 0.2, 0.1, 0.0 and 0.9 %).
+// (Letting the next kernel be set up from the start of this one, by
+// launch_dependents, was worse at every size: 210 against 199, 379 against
+// 372, 2650 against 2620 and 20600 against 20260 us on the first two and last
+// two models; the waiting blocks take the room of working ones.)
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -68,8 +68,7 @@ struct M2NArgs {
   uint32_t *sticky_key;
   unsigned long long *stat;
   const float *gxf, *gyf;  // FP32 line positions (coarse band test)
-  int TX;      // node columns per CTA
-  long n = 0;  // markers
+  int TX;  // node columns per CTA
 };
 // the sweep's shared-memory size, set on the current device (once per context)
 cudaError_t m2n_init();
@@ -194,9 +193,9 @@ struct N2MArgs {
   float4 *quad;      // allinteri's bilinear forms per cell quarter [ncell * QUAD_FLOAT4]
   long n;            // markers
   int TX;            // node columns per CTA
-  // interpolationmod 1: the tile sweep writes each marker's back-scatter
-  // payload (BS_N fields, SoA by sorted position) here and per-node gather
-  // kernels sum it; null for interpolationmod 2
+  // interpolationmod 1: the gather writes each marker's back-scatter payload
+  // (BS_N fields, SoA by sorted position) here and a kernel with a thread per
+  // node sums it; null for interpolationmod 2
   float *bs = nullptr;
   // the move records spawns and out-of-model markers here when the markers
   // include immobile ones (has_imm; device pointers, passed by value)
@@ -258,7 +257,6 @@ void launch_unpermute_f32(const float *src, const int32_t *id, double *out, long
 void launch_unpermute_i32(const int32_t *src, const int32_t *id, int32_t *out, long n, cudaStream_t st);
 void launch_unpermute_u8(const uint8_t *src, const int32_t *id, uint8_t *out, long n, cudaStream_t st);
 void launch_unpermute_i8(const int8_t *src, const int32_t *id, int8_t *out, long n, cudaStream_t st);
-// FP64 positions in reference numbering
 // marker fields straight to host arrays that the device writes: an entry per
 // array
 constexpr int MARKER_FIELDS_MAX = 16;
@@ -276,6 +274,7 @@ struct MarkerFields {
 // inv: scratch of n entries
 void launch_markers_to_host(const Grid &g, const Markers &m, long n, const MarkerFields &f,
                             int32_t *inv, cudaStream_t st);
+// FP64 positions in reference numbering
 void launch_positions(const Grid &g, const Markers &m, long n, double *x, double *y,
                       cudaStream_t st);
 

@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(NTH, 4) k_m2n(M2NArgs a) {
               const float2 uv = sm.p[S_UV][q];
               const float w = C.s1up * tent(uv.x) * tent(uv.y);
               if (w >= 0.f) {
-                        if (warp == 4) {
+                if (warp == 4) {
                   const float nu = sm.p[S_NUE][q].x;
                   acc[0].add(mul_w(nu, __fmul_rn(nu, a.R(RK_INV_GG, sm.type[p])), w));
                   wt.add(w);
@@ -715,62 +715,62 @@ __device__ __forceinline__ void mode1_node(const M2NArgs &a) {
         // one round of memory latency per marker instead of three
         int idx1 = __ldg(a.perm + b);
 #pragma unroll 1
-      for (int s = b; s < e; s++) {
-        const int idx = idx1;
-        if (s + 1 < e) idx1 = __ldg(a.perm + s + 1);
-        const float u = a.m.u_in[idx], v = a.m.v_in[idx];
-        const int tt = a.m.type[idx];
-        if (ROLE == 0) {
-          const float mnu = a.m.mnu[idx], me = a.m.e[idx], sxy = a.m.sxy[idx];
-          const float exy = a.m.exy[idx], coh = a.m.coh[idx], phi = a.m.phi[idx];
-          const float ig = a.R(RK_INV_GG, tt);
-          if (!marker_active(a, cx, cy, u, v)) continue;
-          const float w = s1 * (ax ? u : 1.f - u) * (by ? v : 1.f - v);
-          cur[0].add(mnu * w); cur[1].add(mnu * ig * w);
-          cur[2].add(me * w); cur[3].add(sxy * w);
-          cur[4].add(exy * w); cur[5].add(coh * w);
-          cur[6].add(phi * w); cur[7].add(w);
-        } else if (ROLE == 1) {
-          const float T = a.m.tk[idx], kt = a.m.mkt[idx];
-          const float mro = a.S.p.densimod ? a.m.mro[idx] : 0.f;
-          const float bb = a.R(RK_BB, tt);
-          const float ro = a.S.p.densimod ? mro : a.R(RK_RO, tt);
-          if (!marker_active(a, cx, cy, u, v)) continue;
-          const float w = s1 * (ax ? u : 1.f - u) * (by ? v : 1.f - v);
-          cur[0].add(ro * w);
-          cur[1].add(fdiv_normal(bb, 1.f - bb * (T - 298.15f)) * w);
-          cur[2].add(a.R(RK_HT, tt) * w); cur[3].add(a.R(RK_CP, tt) * w);
-          cur[4].add(kt * w); cur[5].add(T * w); cur[6].add(w);
-        } else if (ROLE == 2) {
-          const float mnu = a.m.mnu[idx], sxx = a.m.sxx[idx], exx = a.m.exx[idx];
-          const float mp = a.m.p[idx], ig = a.R(RK_INV_GG, tt);
-          if (!marker_active(a, cx, cy, u, v)) continue;
-          const float w = s1 * half_factor(ax, u) * half_factor(by, v);
-          if (w != 0.f) {
+        for (int s = b; s < e; s++) {
+          const int idx = idx1;
+          if (s + 1 < e) idx1 = __ldg(a.perm + s + 1);
+          const float u = a.m.u_in[idx], v = a.m.v_in[idx];
+          const int tt = a.m.type[idx];
+          if (ROLE == 0) {
+            const float mnu = a.m.mnu[idx], me = a.m.e[idx], sxy = a.m.sxy[idx];
+            const float exy = a.m.exy[idx], coh = a.m.coh[idx], phi = a.m.phi[idx];
+            const float ig = a.R(RK_INV_GG, tt);
+            if (!marker_active(a, cx, cy, u, v)) continue;
+            const float w = s1 * (ax ? u : 1.f - u) * (by ? v : 1.f - v);
             cur[0].add(mnu * w); cur[1].add(mnu * ig * w);
-            cur[2].add(sxx * w); cur[3].add(exx * w);
-            cur[4].add(mp * w); cur[5].add(w);
-          }
-        } else {
-          const float vx = a.m.vx[idx], vy = a.m.vy[idx];
-          const float ro = a.S.p.densimod ? a.m.mro[idx] : a.R(RK_RO, tt);
-          if (!marker_active(a, cx, cy, u, v)) continue;
-          // vx node: x bilinear (ax in {0, 1}), y staggered (by + 1 in {0, 1, 2})
-          if (ax >= 0) {
-            const float w = s1 * (ax ? u : 1.f - u) * half_factor(by + 1, v);
+            cur[2].add(me * w); cur[3].add(sxy * w);
+            cur[4].add(exy * w); cur[5].add(coh * w);
+            cur[6].add(phi * w); cur[7].add(w);
+          } else if (ROLE == 1) {
+            const float T = a.m.tk[idx], kt = a.m.mkt[idx];
+            const float mro = a.S.p.densimod ? a.m.mro[idx] : 0.f;
+            const float bb = a.R(RK_BB, tt);
+            const float ro = a.S.p.densimod ? mro : a.R(RK_RO, tt);
+            if (!marker_active(a, cx, cy, u, v)) continue;
+            const float w = s1 * (ax ? u : 1.f - u) * (by ? v : 1.f - v);
+            cur[0].add(ro * w);
+            cur[1].add(fdiv_normal(bb, 1.f - bb * (T - 298.15f)) * w);
+            cur[2].add(a.R(RK_HT, tt) * w); cur[3].add(a.R(RK_CP, tt) * w);
+            cur[4].add(kt * w); cur[5].add(T * w); cur[6].add(w);
+          } else if (ROLE == 2) {
+            const float mnu = a.m.mnu[idx], sxx = a.m.sxx[idx], exx = a.m.exx[idx];
+            const float mp = a.m.p[idx], ig = a.R(RK_INV_GG, tt);
+            if (!marker_active(a, cx, cy, u, v)) continue;
+            const float w = s1 * half_factor(ax, u) * half_factor(by, v);
             if (w != 0.f) {
-              cur[0].add(vx * ro * w); cur[1].add(ro * w); cur[2].add(w);
+              cur[0].add(mnu * w); cur[1].add(mnu * ig * w);
+              cur[2].add(sxx * w); cur[3].add(exx * w);
+              cur[4].add(mp * w); cur[5].add(w);
             }
-          }
-          // vy node: x staggered (ax + 1), y bilinear (by in {0, 1})
-          if (by >= 0) {
-            const float w = s1 * half_factor(ax + 1, u) * (by ? v : 1.f - v);
-            if (w != 0.f) {
-              vy3[0].add(vy * ro * w); vy3[1].add(ro * w); vy3[2].add(w);
+          } else {
+            const float vx = a.m.vx[idx], vy = a.m.vy[idx];
+            const float ro = a.S.p.densimod ? a.m.mro[idx] : a.R(RK_RO, tt);
+            if (!marker_active(a, cx, cy, u, v)) continue;
+            // vx node: x bilinear (ax in {0, 1}), y staggered (by + 1 in {0, 1, 2})
+            if (ax >= 0) {
+              const float w = s1 * (ax ? u : 1.f - u) * half_factor(by + 1, v);
+              if (w != 0.f) {
+                cur[0].add(vx * ro * w); cur[1].add(ro * w); cur[2].add(w);
+              }
+            }
+            // vy node: x staggered (ax + 1), y bilinear (by in {0, 1})
+            if (by >= 0) {
+              const float w = s1 * half_factor(ax + 1, u) * (by ? v : 1.f - v);
+              if (w != 0.f) {
+                vy3[0].add(vy * ro * w); vy3[1].add(ro * w); vy3[2].add(w);
+              }
             }
           }
         }
-      }
       }
     }
   }

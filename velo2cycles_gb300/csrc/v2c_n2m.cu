@@ -795,10 +795,9 @@ __global__ void __launch_bounds__(256, 6) k_gather(N2MArgs a) {
 // ------------------------------------------------ interpolationmod 1
 // The back-scatter of interpolate_mechanical (interpolation.c:1104-1158 and
 // 1249-1358) with the full stencils, as a gather: one thread per node sums,
-// cell by cell in sorted order, the payload the tile sweep left per marker
-// — bilinear weights on basic nodes, the staggered centre stencil on
-// pressure nodes (no vx/vy back-scatter in this mode) — and normalises as
-// the tail of nodes2markers does (interpolation.c:1014-1046).  The centre
+// cell by cell in sorted order, the payload k_gather left per marker —
+// bilinear weights on basic nodes, the staggered centre stencil on pressure
+// nodes (no vx/vy back-scatter in this mode) — and normalises as the tail of nodes2markers does (interpolation.c:1014-1046).  The centre
 // stencil's contributions past the last node row land, as in the
 // reference, in the next column's first row (a ghost node whose sums are
 // kept but never normalised).
